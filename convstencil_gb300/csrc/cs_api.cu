@@ -177,6 +177,48 @@ int classify(const Weights &w, int dims, int r)
     return cs::PAT_DENSE;
 }
 
+// Kernel of `steps` steps of a (2r+1)^dims kernel (dims 1 or 2) at the centre
+// of a (2R+1)^dims array: the self-convolution, every sum carried in two
+// doubles (products by fma, sums by TwoSum) and rounded once at the end, what
+// rounding leaves of one weight carried to the next so that their sum keeps
+// its value (see f64_slice_weights). False when the weights' size could
+// take a power of them out of range (such plans keep single steps).
+bool selfconv(const double *w, int dims, int r, int steps, int R, double *out)
+{
+    const int k = 2 * r + 1, K = 2 * R + 1, n = ipow(k, dims), N = ipow(K, dims);
+    double sum = 0.0;
+    for (int i = 0; i < n; ++i) sum += std::fabs(w[i]);
+    if (!(sum > 0x1p-64 && sum < 0x1p64) || steps * r > R) return false;
+    std::vector<double> h(N, 0.0), l(N, 0.0), h2(N), l2(N);
+    const int c = dims == 2 ? R * K + R : R;
+    h[c] = 1.0;
+    for (int s = 0; s < steps; ++s) {
+        std::fill(h2.begin(), h2.end(), 0.0);
+        std::fill(l2.begin(), l2.end(), 0.0);
+        for (int i = 0; i < N; ++i) {
+            if (h[i] == 0.0 && l[i] == 0.0) continue;
+            for (int t = 0; t < n; ++t) {
+                if (w[t] == 0.0) continue;
+                const int j = i + (dims == 2 ? (t / k - r) * K + t % k - r : t - r);
+                const double p = h[i] * w[t], pe = std::fma(h[i], w[t], -p) + l[i] * w[t];
+                const double a = h2[j] + p, b = a - h2[j];
+                l2[j] += (h2[j] - (a - b)) + (p - b) + pe;
+                h2[j] = a;
+            }
+        }
+        h.swap(h2);
+        l.swap(l2);
+    }
+    double carry = 0.0;
+    for (int i = 0; i < N; ++i) {
+        out[i] = 0.0;
+        if (h[i] == 0.0 && l[i] == 0.0) continue;
+        out[i] = h[i] + (l[i] + carry);
+        carry += (h[i] - out[i]) + l[i];
+    }
+    return true;
+}
+
 long long round_up(long long v, long long a) { return (v + a - 1) / a * a; }
 
 void native_layout(int dims, int r, const long long *ext, cs_layout &L)
@@ -218,6 +260,8 @@ std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int, int>, int> g_tune;      // -> algorithm
 std::map<std::tuple<int, int, int, int, int>, int> g_tune_tb;   // -> steps per launch (split FMA)
 std::map<std::tuple<int, int, int, int, int>, int> g_tune_rows; // -> FP64 FMA 2D tile rows
+// -> time of one sweep of the chosen algorithm and of one launch of several steps (FP64)
+std::map<std::tuple<int, int, int, int, int>, std::pair<float, float>> g_tune_steps;
 
 }  // namespace
 
@@ -228,6 +272,9 @@ struct cs_plan {
     int dims, radius, pattern, steps_per_sweep;
     Weights w;
     Weights w7;  // 2D plans: w at the centre of a 7x7 (the 2D tcgen05 kernels' tap window)
+    // FP64 2D radius-1 plans: the 7x7 kernels of 1, 2 and 3 steps (launch_fp64_steps_tc)
+    Weights w_steps[3];
+    int max_steps = 1;  // steps per launch those allow
     cs_layout layout;
     GridView view;
     int algo = CS_ALGO_AUTO;
@@ -397,6 +444,26 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
                                   in, out, st);
 }
 
+// Steps per launch of the tcgen05 digit kernel on this plan and these
+// buffers: 3 for FP64 2D radius-1 plans (three steps of a 3x3 kernel are one
+// 7x7 kernel, the kernel's tap window) from 64 tiles up. Smaller grids leave
+// most SMs without a tile, and a launch of ~12 us loses to single steps on
+// the FP64 FMA kernel (512^2, 64 tiles, is where three of those take as long).
+int fp64_steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base)
+{
+    if (p->max_steps < 2 || !fp64_tc_ok(p) || !fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base))
+        return 1;
+    const long long tiles = ((p->view.ext[0] + 63) / 64) * ((p->view.ext[1] + 63) / 64);
+    return tiles >= 64 ? p->max_steps : 1;
+}
+
+// `steps` (1 .. fp64_steps_per_launch) steps in one launch.
+cudaError_t launch_steps(const cs_plan *p, int steps, const void *in_base, void *out_base, cudaStream_t st)
+{
+    return cs::launch_fp64_steps_tc(p->view, p->w_steps[steps - 1], p->w, steps, p->layout.origin,
+                                    p->layout.elements, (const double *)in_base, (double *)out_base, p->wait, st);
+}
+
 cudaError_t launch_sweep(const cs_plan *p, int algo, const void *in_base, void *out_base, cudaStream_t st)
 {
     return launch_sweep_rows(p, algo, in_base, out_base, 0, p->view.ext[0], st);
@@ -555,6 +622,57 @@ cs_status choose_time_block(cs_plan *p, int algo, const void *a, void *b, cudaSt
     return CS_OK;
 }
 
+// Whether a run of `sweeps` sweeps takes several steps per launch, and then
+// how many (*steps) and the kernel (*algo). Always when FP64_TC is pinned;
+// with AUTO where the time of ceil(sweeps / steps) such launches, measured
+// once per class of plan beside single sweeps of the chosen algorithm
+// (six steps each way, a -> b), is the shorter one. A caller that is capturing
+// its stream gets what is already known.
+cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long long sweeps, int *algo, int *steps)
+{
+    *steps = 1;
+    const int t = fp64_steps_per_launch(p, a, b);
+    if (t < 2 || (p->algo != CS_ALGO_AUTO && p->algo != CS_ALGO_FP64_TC)) return CS_OK;
+    if (p->algo == CS_ALGO_FP64_TC) {
+        *steps = t;
+        return CS_OK;
+    }
+    const auto key = std::make_tuple(p->dims, p->radius, p->pattern, (int)p->prec, size_class(p));
+    std::pair<float, float> ms(0.f, 0.f);
+    {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        auto it = g_tune_steps.find(key);
+        if (it != g_tune_steps.end()) ms = it->second;
+    }
+    if (ms.second == 0.f) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CS_CUDA(cudaStreamIsCapturing(st, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return CS_OK;
+        cudaEvent_t e[3];
+        for (auto &x : e) CS_CUDA(cudaEventCreate(&x));
+        for (int rep = 0; rep < 2; ++rep) {  // rep 0 warms up
+            CS_CUDA(cudaEventRecord(e[0], st));
+            for (int i = 0; i < 6; ++i) CS_CUDA(launch_sweep(p, *algo, a, b, st));
+            CS_CUDA(cudaEventRecord(e[1], st));
+            for (int i = 0; i < 6 / t; ++i) CS_CUDA(launch_steps(p, t, a, b, st));
+            CS_CUDA(cudaEventRecord(e[2], st));
+            CS_CUDA(cudaEventSynchronize(e[2]));
+        }
+        CS_CUDA(cudaEventElapsedTime(&ms.first, e[0], e[1]));
+        CS_CUDA(cudaEventElapsedTime(&ms.second, e[1], e[2]));
+        for (auto &x : e) cudaEventDestroy(x);
+        ms.first /= 6;
+        ms.second /= 6 / t;
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        g_tune_steps[key] = ms;
+    }
+    if (sweeps > 1 && ms.second * (float)((sweeps + t - 1) / t) < ms.first * (float)sweeps) {
+        *steps = t;
+        *algo = CS_ALGO_FP64_TC;
+    }
+    return CS_OK;
+}
+
 // Tile rows of the FP64 FMA 2D kernel (16 or 32 rows per CTA tile): with
 // tile_rows 0 the first run times both once on a -> b (bitwise the same
 // sweep) and remembers the faster for plans of the same class.
@@ -660,6 +778,10 @@ cs_status run_from(cs_plan *p, void *a, void *b, long long first_sweep, long lon
         if (s != CS_OK) return s;
         s = choose_time_block(p, algo, a, b, st, &tb);
         if (s != CS_OK) return s;
+        if (p->prec == CS_PREC_FP64) {
+            s = choose_steps(p, a, b, st, sweeps, &algo, &tb);
+            if (s != CS_OK) return s;
+        }
         int rows = 0;
         s = choose_tile_rows(p, algo, a, b, st, &rows);
         if (s != CS_OK) return s;
@@ -672,6 +794,7 @@ cs_status run_from(cs_plan *p, void *a, void *b, long long first_sweep, long lon
     const long long off = p->layout.origin;
     // One launch of t sweeps from buf[c] to buf[c ^ 1] on stream `on`.
     auto one_launch = [&](int t, int c, cudaStream_t on) -> cudaError_t {
+        if (p->prec == CS_PREC_FP64 && tb >= 2) return launch_steps(p, t, buf[c], buf[c ^ 1], on);
         if (t >= 2)
             return cs::launch_split_sweep_tb(p->view, p->radius, p->pattern, t, p->w,
                                              (const float2 *)buf[c] + off, (float2 *)buf[c ^ 1] + off, on);
@@ -844,6 +967,14 @@ CS_API cs_status cs_plan_create(cs_plan **out, cs_shape shape, cs_semantics sem,
             for (int j = 0; j < k; ++j) p->w7.v[(i + o) * 7 + j + o] = p->w.v[i * k + j];
     } else if (p->dims == 1 && p->radius <= 3) {  // the taps in row 3 of the 7x7
         for (int j = 0; j <= 2 * p->radius; ++j) p->w7.v[3 * 7 + 3 - p->radius + j] = p->w.v[j];
+    }
+    if (prec == CS_PREC_FP64 && p->dims == 2 && p->radius == 1) {
+        bool ok = true;
+        for (int t = 1; t <= 3; ++t) {
+            memset(p->w_steps[t - 1].v, 0, sizeof p->w_steps[t - 1].v);
+            ok = ok && selfconv(p->w.v, 2, 1, t, 3, p->w_steps[t - 1].v);
+        }
+        if (ok) p->max_steps = 3;
     }
     if (layout) {
         const cs_layout &L = *layout;

@@ -81,6 +81,11 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
                                  const double *in_base, double *out_base, const TcWait &wait,
                                  cudaStream_t stream);
+// `steps` (1..3) steps of a 2D radius-1 FP64 grid in one launch: wT is the
+// 7x7 kernel of that many steps (selfconv7), w3x3 the weights of one.
+cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
+                                 long long origin, long long elements, const double *in_base, double *out_base,
+                                 const TcWait &wait, cudaStream_t stream);
 // Batches of 2D radius-3 grids on the tcgen05 kernels (split or FP64): one
 // device record per grid (tc_batch_record_bytes each, 128-byte aligned)
 // holding its tensor map over `in_base`, output, sizes, first tile and

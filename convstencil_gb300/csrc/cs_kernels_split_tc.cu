@@ -220,17 +220,120 @@ __device__ __forceinline__ int grid_of(const TcGrid<F> *grids, int ngrids, int t
     return lo;
 }
 
+// What one launch computes.
+constexpr int kModeGrid = 0;    // one sweep of a 2D grid
+constexpr int kModeRows1d = 1;  // one sweep of a 1D grid, as rows of 64 outputs
+constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
+
+// kModeSteps: T steps of a 3x3 stencil are one sweep of its T-fold
+// self-convolution (7x7 at T = 3) wherever the window of every intermediate
+// step stays inside the grid, that is for outputs at least T - 1 points from
+// the boundary. Those come from the digit pipeline (`sw` holds the convolved
+// weights); the frame of T - 1 points along the boundary is computed step by
+// step with FP64 FMA by the epilogue warps before their first accumulator is
+// ready, from the same input, with the halo each single sweep would read. A
+// launch costs what one step on the 7x7 pipeline costs (its limit is the
+// digits, not the taps): box2d1r 2047 x 1531, 60 steps, GB300: 1818 us at a
+// step per launch, 744 at three; star2d1r 1024^2, 100 steps: 1295 us on the
+// FP64 FMA kernel (the FP64 pipe takes 10 us of each step's 13), 742 so.
+struct StepArgs {
+    const double *in;  // interior point (0, 0) of the source
+    int steps;         // T: 1, 2 or 3
+    unsigned taps;     // bit t: weight t is not zero
+    double w[9];       // weights of one step
+};
+
+// One strip of the frame, by one warp: T steps for the T - 1 points next to
+// an edge, at positions l0 .. l0 + 31 - 2T along it. `edge` is the offset of
+// the edge's first point, `sa` the step away from the edge, `sl` the step
+// along it (`len` points, outputs before `end`); w and taps are the 3x3 weights turned the same
+// way. Lane l holds position l0 - T + l; neighbours along the edge come by
+// shuffles, and every level's outermost lanes fall out of use. A halo cell
+// keeps the value of the buffer that the sweep of its level would read.
+template <int T>
+__device__ __forceinline__ void frame_strip(const double *__restrict__ in, double *__restrict__ out, long long edge,
+                                            long long sa, long long sl, int len, int l0, int end,
+                                            const double (&w)[9], unsigned taps)
+{
+    const int lane = threadIdx.x & 31, p = l0 - T + lane;
+    const bool inside = p >= 0 && p < len, halo = p == -1 || p == len;
+    const long long at = edge + (long long)p * sl;
+    double u0[2 * T], u[2 * T], odd[2 * T - 1];  // row k of the strip is u[k + 1]; odd: halo cells of odd levels
+#pragma unroll
+    for (int j = 0; j < 2 * T; ++j) u[j] = u0[j] = inside || halo ? in[at + (j - 1) * sa] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 2 * T - 1; ++j) odd[j] = halo || (inside && j == 0) ? out[at + (j - 1) * sa] : 0.0;
+#pragma unroll
+    for (int level = 1; level <= T; ++level) {
+        constexpr unsigned all = 0xffffffffu;
+        const int rows = 2 * T - 1 - level;  // rows 0 .. rows - 1 of this level
+        double v[2 * T];
+#pragma unroll
+        for (int k = 0; k < 2 * T - 2; ++k) v[k] = 0.0;
+#pragma unroll
+        for (int j = 0; j < 2 * T; ++j) {
+            if (j > rows + 1) continue;
+            const double x[3] = {__shfl_up_sync(all, u[j], 1), u[j], __shfl_down_sync(all, u[j], 1)};
+#pragma unroll
+            for (int t = 0; t < 9; ++t) {
+                const int k = j - t / 3;  // row k takes u[k + da] through weight row da
+                if (k >= 0 && k < rows && (taps >> t & 1u)) v[k] = fma(w[t], x[t % 3], v[k]);
+            }
+        }
+#pragma unroll
+        for (int k = -1; k < 2 * T - 2; ++k)
+            if (k < rows) {
+                const bool cell = halo || k < 0;  // a halo cell of the next level's input
+                u[k + 1] = cell ? ((level & 1) ? odd[k + 1] : u0[k + 1]) : inside ? v[k < 0 ? 0 : k] : 0.0;
+            }
+    }
+    if (p < end && lane >= T && lane < 32 - T) {
+#pragma unroll
+        for (int k = 0; k < T - 1; ++k) out[at + k * sa] = u[k + 1];
+    }
+}
+
+// The frame of an m x n grid, strip by strip, shared by `nwarps` warps.
+template <int T>
+__device__ __forceinline__ void frame_steps(const StepArgs &s, double *__restrict__ out, int m, int n, long long ld,
+                                            int warp, int nwarps)
+{
+    constexpr int F = T - 1, S = 32 - 2 * T;  // frame width, outputs per strip
+    const int nx = (n + S - 1) / S, ny = (m - 2 * F + S - 1) / S;
+    for (int i = warp; i < 2 * (nx + ny); i += nwarps) {
+        const bool horiz = i < 2 * nx;  // top and bottom rows, whole length
+        const int q = horiz ? i : i - 2 * nx, cnt = horiz ? nx : ny;
+        const bool far = q >= cnt;
+        const int l0 = (far ? q - cnt : q) * S + (horiz ? 0 : F);
+        double w[9];
+        unsigned taps = 0;
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+            const int da = far ? 2 - t / 3 : t / 3, dl = t % 3;
+            const int src = horiz ? 3 * da + dl : 3 * dl + da;
+            w[t] = s.w[src];
+            taps |= (s.taps >> src & 1u) << t;
+        }
+        if (horiz)
+            frame_strip<T>(s.in, out, far ? (long long)(m - 1) * ld : 0, far ? -ld : ld, 1, n, l0, n, w, taps);
+        else  // the corners belong to the rows: columns end F short of them
+            frame_strip<T>(s.in, out, far ? n - 1 : 0, far ? -1 : 1, ld, m, l0, m - F, w, taps);
+    }
+}
+
 // One grid (BATCH = false: kernel parameters describe it, tiles are dealt
 // round-robin) or a batch of grids (BATCH = true: `grids` describes them,
 // each CTA takes a contiguous run of the batch's tiles, and the MMA warp
 // rebuilds its B matrices when the run crosses into the next grid, after
 // the MMAs of the previous tile have completed).
-template <class F, bool BATCH, bool ROWS1D = false>
+template <class F, bool BATCH, int MODE = kModeGrid>
 __global__ void __launch_bounds__(kThreads<F>, 1)
     k2d_tc(const __grid_constant__ CUtensorMap tmap, typename F::Out *__restrict__ out, int m, int n,
            long long ld, int tiles_x, int tiles, int map_x, int map_y, typename F::Digits sw, WaitCfg wc,
-           const TcGrid<F> *__restrict__ grids, int ngrids)
+           const TcGrid<F> *__restrict__ grids, int ngrids, const __grid_constant__ StepArgs sa)
 {
+    constexpr bool ROWS1D = MODE == kModeRows1d, STEPS = MODE == kModeSteps;
+    static_assert(!BATCH || MODE == kModeGrid, "batches run one sweep of 7x7 grids");
     constexpr int D = F::kDigits;
     using SM = Smem<F>;
     extern __shared__ unsigned char smem_raw[];
@@ -401,6 +504,13 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             uint4 v[PER];
             float vmax = 0.f;   // split: largest |hi|
             unsigned emax = 0;  // FP64: largest biased exponent
+            int x0 = 0, y0 = 0;
+            bool edge = false;  // kModeSteps: the window reaches past the halo of one point
+            if constexpr (STEPS) {
+                int g;
+                tile_at(it, g, x0, y0);
+                edge = x0 == 0 || y0 == 0 || x0 + ST_X - 4 > n + 1 || y0 + ST_Y - 3 > m + 1;
+            }
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 const int idx = st + q * kSliceThreads;
@@ -412,6 +522,14 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                         v[q] = S.stage[idx - 4 * (idx / PAIRS)];
                     else
                         v[q] = S.stage[idx];
+                    // Points past the halo meet zero weights in every output
+                    // kept, but must not set the tile's scale either.
+                    if (STEPS && edge) {
+                        const int yy = y0 - 3 + idx / PAIRS, xx = x0 - 4 + 2 * (idx % PAIRS);
+                        const bool row = yy >= -1 && yy <= m;
+                        if (!row || xx < -1 || xx > n) v[q].x = v[q].y = 0u;
+                        if (!row || xx + 1 < -1 || xx + 1 > n) v[q].z = v[q].w = 0u;
+                    }
                     if constexpr (F::kF64)
                         emax = max(emax, max((v[q].y >> 20) & 0x7FFu, (v[q].w >> 20) & 0x7FFu));
                     else
@@ -458,8 +576,8 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 for (int q = 0; q < PER; ++q) {
                     const int idx = st + q * kSliceThreads;
                     if (idx < NPAIR) {
-                        const unsigned long long ya = f64_biased_fixed(v[q].x, v[q].y, ex);
-                        const unsigned long long yb = f64_biased_fixed(v[q].z, v[q].w, ex);
+                        const unsigned long long ya = f64_biased_fixed<STEPS>(v[q].x, v[q].y, ex);
+                        const unsigned long long yb = f64_biased_fixed<STEPS>(v[q].z, v[q].w, ex);
                         unsigned *dst = dst0 + idx;
                         dst[0 * (PL / 2)] = f64_digit_pair<0>(ya, yb);
                         dst[1 * (PL / 2)] = f64_digit_pair<1>(ya, yb);
@@ -501,6 +619,15 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         const int mrow = 32 * quarter + lane;
         const int er = mrow >> 3, eb = mrow & 7;
         const unsigned lane_bits = (unsigned)(32 * quarter) << 16;
+        if constexpr (STEPS) {
+            const int fw = (warp - kWarpEpi0) * (int)gridDim.x + (int)blockIdx.x, fn = F::kEpiWarps * (int)gridDim.x;
+            pdl_wait();
+            if (sa.steps == 3)
+                frame_steps<3>(sa, out, m, n, ld, fw, fn);
+            else if (sa.steps == 2)
+                frame_steps<2>(sa, out, m, n, ld, fw, fn);
+        }
+        const int frame = STEPS ? sa.steps - 1 : 0;
         for (int it = 0; it < my_tiles; ++it) {
             const int buf = it & 1, use = it >> 1;
             if (!wait(bar2(S.acc_full, buf), use & 1)) break;
@@ -535,6 +662,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 }
                 const int yy = y0 + R * er + rho;
                 if (yy >= o_m) continue;
+                if (STEPS && (yy < frame || yy >= o_m - frame)) continue;
                 if constexpr (F::kF64) {
                     // value = T 2^c with T from the levels (f64_combine) and
                     // c = (input scale) + (weight scale) - 1080.
@@ -547,6 +675,12 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                                                       : f64_from_fixed(f64_combine(lv), c);
                     }
                     double *o = reinterpret_cast<double *>(o_base) + (long long)yy * o_ld + xb;
+                    if (STEPS && (xb < frame || xb + 8 > o_n - frame)) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (xb + j >= frame && xb + j < o_n - frame) o[j] = res[j];
+                        continue;
+                    }
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
                         if (xb + j + 1 < o_n)
@@ -595,17 +729,18 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-template <class F, bool BATCH, bool ROWS1D = false>
+template <class F, bool BATCH, int MODE = kModeGrid>
 cudaError_t set_smem_attr()
 {
     static const cudaError_t err = cudaFuncSetAttribute(
-        k2d_tc<F, BATCH, ROWS1D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(Smem<F>) + 128));
+        k2d_tc<F, BATCH, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(Smem<F>) + 128));
     return err;
 }
 
-template <class F>
+template <class F, int MODE = kModeGrid>
 cudaError_t launch_tc(const GridView &g, const typename F::Digits &digits, long long origin, long long elements,
-                      const void *in_base, void *out_base, const WaitCfg &wc, cudaStream_t st)
+                      const void *in_base, void *out_base, const WaitCfg &wc, cudaStream_t st,
+                      const StepArgs &sa = StepArgs{})
 {
     const long long ld = g.pitch[0];
     CUtensorMap map;
@@ -613,17 +748,17 @@ cudaError_t launch_tc(const GridView &g, const typename F::Digits &digits, long 
     cudaError_t e = encode_split_window_map(&map, reinterpret_cast<const float2 *>(in_base), ld, elements / ld,
                                             ST_X, ST_Y);
     if (e != cudaSuccess) return e;
-    if ((e = set_smem_attr<F, false>()) != cudaSuccess) return e;
+    if ((e = set_smem_attr<F, false, MODE>()) != cudaSuccess) return e;
     const int tiles_x = (int)((g.ext[1] + TX - 1) / TX);
     const int tiles = tiles_x * (int)((g.ext[0] + TY - 1) / TY);
     // One CTA per SM (its shared-memory footprint admits no second one, so
     // the TMEM allocation never waits).
     const int grid = std::min(tiles, device_sm_count());
     note_launch();
-    return launch_programmatic(k2d_tc<F, false>, grid, kThreads<F>, sizeof(Smem<F>) + 128, st, map,
+    return launch_programmatic(k2d_tc<F, false, MODE>, grid, kThreads<F>, sizeof(Smem<F>) + 128, st, map,
                                reinterpret_cast<typename F::Out *>(out_base) + origin, (int)g.ext[0],
                                (int)g.ext[1], ld, tiles_x, tiles, (int)(origin % ld), (int)(origin / ld), digits,
-                               wc, static_cast<const TcGrid<F> *>(nullptr), 0);
+                               wc, static_cast<const TcGrid<F> *>(nullptr), 0, sa);
 }
 
 template <class F>
@@ -665,7 +800,8 @@ cudaError_t launch_batch(const void *records, int ngrids, int total, const WaitC
     // so the set-up may read them before pdl_wait().
     return launch_programmatic(k2d_tc<F, true>, grid, kThreads<F>, sizeof(Smem<F>) + 128, st, unused,
                                static_cast<typename F::Out *>(nullptr), 0, 0, 0LL, 0, total, 0, 0,
-                               typename F::Digits{}, wc, reinterpret_cast<const TcGrid<F> *>(records), ngrids);
+                               typename F::Digits{}, wc, reinterpret_cast<const TcGrid<F> *>(records), ngrids,
+                               StepArgs{});
 }
 
 split::SliceWeights split_digits(const Weights &w) { return split::slice_weights(w); }
@@ -686,6 +822,19 @@ cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long 
 {
     return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base,
                              WaitCfg{wt.limit_ns, wt.skip_loads}, st);
+}
+
+cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
+                                 long long origin, long long elements, const double *in_base, double *out_base,
+                                 const TcWait &wt, cudaStream_t st)
+{
+    StepArgs sa{in_base + origin, steps, 0u, {}};
+    for (int t = 0; t < 9; ++t) {
+        sa.w[t] = w3x3.v[t];
+        if (w3x3.v[t] != 0.0) sa.taps |= 1u << t;
+    }
+    return launch_tc<FmtF64, kModeSteps>(g, f64_slice_weights(wT, 49, true), origin, elements, in_base, out_base,
+                                         WaitCfg{wt.limit_ns, wt.skip_loads}, st, sa);
 }
 
 cudaError_t launch_fp64_sweep_tc_rows1d(long long n, const Weights &w7, long long origin, long long elements,
@@ -710,14 +859,14 @@ cudaError_t launch_fp64_sweep_tc_rows1d(long long n, const Weights &w7, long lon
     cudaError_t e = encode_split_window_map(&map, reinterpret_cast<const float2 *>(in_base + origin - 4), TX,
                                             (elements - (origin - 4)) / TX, TX, kSpanRows);
     if (e != cudaSuccess) return e;
-    if ((e = set_smem_attr<FmtF64, false, true>()) != cudaSuccess) return e;
+    if ((e = set_smem_attr<FmtF64, false, kModeRows1d>()) != cudaSuccess) return e;
     const int tiles = (int)((rows + TY - 1) / TY);
     const int grid = std::min(tiles, device_sm_count());
     note_launch();
-    return launch_programmatic(k2d_tc<FmtF64, false, true>, grid, kThreads<FmtF64>, sizeof(Smem<FmtF64>) + 128, st,
+    return launch_programmatic(k2d_tc<FmtF64, false, kModeRows1d>, grid, kThreads<FmtF64>, sizeof(Smem<FmtF64>) + 128, st,
                                map, out_base + origin, (int)rows, TX, (long long)TX, 1, tiles, 0, 0,
                                f64_slice_weights(w7), WaitCfg{wt.limit_ns, wt.skip_loads},
-                               static_cast<const TcGrid<FmtF64> *>(nullptr), 0);
+                               static_cast<const TcGrid<FmtF64> *>(nullptr), 0, StepArgs{});
 }
 
 size_t tc_batch_record_bytes(bool fp64) { return fp64 ? sizeof(TcGrid<FmtF64>) : sizeof(TcGrid<FmtSplit>); }

@@ -72,7 +72,11 @@ typedef enum cs_semantics { CS_SEM_STEP = 0, CS_SEM_FUSED = 1 } cs_semantics;
  *                product and level sum is exact, inputs keep 52 bits below
  *                their 64x70 tile's largest value and weights 53 below the
  *                largest weight (relative error per sweep ~1e-16 of the
- *                tile's scale). Pin CS_ALGO_FP64_FMA for IEEE FP64 sums.
+ *                tile's scale). On 2D radius-1 plans of at least 64 tiles
+ *                of 64x64 that form takes three steps per launch (as one
+ *                7x7 kernel, the frame along the boundary step by step; a
+ *                run cut into calls of other lengths agrees to rounding, not
+ *                bitwise). Pin CS_ALGO_FP64_FMA for IEEE FP64 sums.
  * CS_PREC_SPLIT: grids stored as FP32 (hi, lo) pairs (8 bytes per point,
  *                about 48 significant bits); no FP64 arithmetic in the sweep.
  *                Dense 7x7 kernels contract exact 9-bit fixed-point slices
@@ -165,7 +169,8 @@ CS_API cs_status cs_plan_sweeps(const cs_plan *plan, long long steps, long long 
 /* The cs_algo the plan's last cs_run used (its tuner's choice under
  * CS_ALGO_AUTO); CS_ALGO_AUTO before the first run. */
 CS_API cs_status cs_plan_get_algo(const cs_plan *plan, int *algo);
-/* Steps per launch the plan's last cs_run used (temporal blocking; 1 = off). */
+/* Steps per launch the plan's last cs_run used (temporal blocking, or the
+ * several steps of an FP64 tcgen05 launch; 1 = off). */
 CS_API cs_status cs_plan_get_time_block(const cs_plan *plan, int *steps_per_launch);
 /* Rows per CTA tile of the FP64 FMA 2D kernel in the plan's last cs_run
  * (the tuner's choice under 0; 0 when another kernel ran). */

@@ -1,0 +1,115 @@
+"""Several steps per launch of the FP64 tcgen05 digit kernel (2D radius-1
+plans): three steps as one 7x7 sweep away from the boundary, the frame along it
+step by step. Compared with single steps in numpy. Bar: 1e-12 of the largest
+value, the FP64 paths' bar (a launch rounds at 2^-52 of its tile's largest
+value, and at most 40 launches run here)."""
+import numpy as np
+import pytest
+
+import convstencil_gb300 as cs
+from oracle import cs_oracle as O
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+TOL = 1e-12
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    cs.build()
+
+
+def dense_of(shape, w):
+    return O.star2d1r_to_dense(w).reshape(3, 3) if shape == "star2d1r" else w.reshape(3, 3)
+
+
+def steps_of(a, b, w, steps):
+    """(m+2) x (n+2) grids with halos, ping-pong as cs_run: returns the interior."""
+    a, b = a.copy(), b.copy()
+    m, n = a.shape[0] - 2, a.shape[1] - 2
+    for _ in range(steps):
+        b[1:-1, 1:-1] = sum(w[i, j] * a[i:i + m, j:j + n] for i in range(3) for j in range(3))
+        a, b = b, a
+    return a[1:-1, 1:-1]
+
+
+def run(plan, a, b, steps):
+    da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    in_b = plan.run(da, db, steps)
+    torch.cuda.synchronize()
+    assert cs.device_wait_timeouts() == 0
+    return (db if in_b else da).cpu().numpy()
+
+
+@pytest.mark.parametrize("shape,taps", [("star2d1r", 5), ("box2d1r", 9)])
+@pytest.mark.parametrize("ext", [(512, 512), (8, 4096), (4097, 9), (515, 577), (1023, 514)])
+@pytest.mark.parametrize("steps", [1, 2, 3, 4, 8, 40])
+def test_steps_equal_single_steps(shape, taps, ext, steps):
+    w = O.seeded_weights(taps, 7 + taps) - 0.04
+    p = cs.Plan(shape, ext, w)
+    p.set_option(cs.Option.ALGO, cs.Algo.FP64_TC)
+    x = O.splitmix_uniform(ext[0] * ext[1], 5 + ext[0]).reshape(ext) - 0.25
+    buf = p.pack(x)
+    got = run(p, buf, np.zeros_like(buf), steps)
+    assert p.algo == cs.Algo.FP64_TC and p.time_block == 3
+    ref = steps_of(np.pad(x, 1), np.zeros((ext[0] + 2, ext[1] + 2)), dense_of(shape, w), steps)
+    assert np.abs(p.unpack(got) - ref).max() <= TOL * np.abs(ref).max()
+    halo = np.ones(p.elements, bool)
+    halo[p.interior_index().reshape(-1)] = False
+    assert not got[halo].any(), "halo must stay zero"
+
+
+@pytest.mark.parametrize("steps", [2, 3, 5])
+def test_steps_read_each_buffers_halo_and_nothing_beyond(steps):
+    """A caller's layout with boundary values in both halos (each step reads
+    those of the buffer it reads) and huge values past the halo, which must
+    not reach any output, not even through a tile's scale."""
+    m, n, pad = 600, 520, 6
+    ld = n + 2 * pad
+    lay = {"dims": 2, "halo": 1, "extent": [m, n], "pitch": [ld, 1], "origin": pad * ld + pad,
+           "elements": (m + 2 * pad) * ld}
+    w = O.seeded_weights(9, 3)
+    p = cs.Plan("box2d1r", (m, n), w, layout=lay)
+    p.set_option(cs.Option.ALGO, cs.Algo.FP64_TC)
+    grids = []
+    for seed in (11, 12):
+        g = np.full((m + 2 * pad, ld), 1e200)
+        g[pad - 1:pad + m + 1, pad - 1:pad + n + 1] = O.splitmix_uniform((m + 2) * (n + 2), seed).reshape(m + 2, n + 2)
+        grids.append(g)
+    inner = [g[pad - 1:pad + m + 1, pad - 1:pad + n + 1] for g in grids]
+    ref = steps_of(inner[0], inner[1], w.reshape(3, 3), steps)
+    got = run(p, grids[0].reshape(-1), grids[1].reshape(-1), steps).reshape(m + 2 * pad, ld)
+    assert p.time_block == 3
+    assert np.abs(got[pad:pad + m, pad:pad + n] - ref).max() <= TOL * np.abs(ref).max()
+
+
+def test_small_grids_and_odd_buffers_keep_single_steps():
+    w = O.seeded_weights(9, 4)
+    p = cs.Plan("box2d1r", (448, 512), w)  # 56 tiles
+    p.set_option(cs.Option.ALGO, cs.Algo.FP64_TC)
+    x = O.splitmix_uniform(448 * 512, 6).reshape(448, 512)
+    run(p, p.pack(x), np.zeros(p.elements), 5)
+    assert p.time_block == 1
+    q = cs.Plan("box2d1r", (512, 512), w)
+    y = O.splitmix_uniform(512 * 512, 8).reshape(512, 512)
+    ref = steps_of(np.pad(y, 1), np.zeros((514, 514)), w.reshape(3, 3), 7)
+    a = torch.zeros(q.elements + 1, dtype=torch.float64, device="cuda")
+    b = torch.zeros_like(a)
+    a[1:] = torch.from_numpy(q.pack(y)).cuda()  # 8-byte aligned grids: no TMA
+    in_b = q.run(a[1:], b[1:], 7)
+    torch.cuda.synchronize()
+    assert q.time_block == 1
+    got = q.unpack((b if in_b else a)[1:].cpu().numpy())
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+def test_weights_out_of_range_keep_single_steps():
+    """Weights whose powers leave the FP64 range (here they would overflow)."""
+    w = O.seeded_weights(9, 4) * 2.0 ** 70
+    p = cs.Plan("box2d1r", (512, 512), w)
+    p.set_option(cs.Option.ALGO, cs.Algo.FP64_TC)
+    x = O.splitmix_uniform(512 * 512, 8).reshape(512, 512) * 2.0 ** -300
+    got = p.unpack(run(p, p.pack(x), np.zeros(p.elements), 3))
+    assert p.time_block == 1
+    ref = steps_of(np.pad(x, 1), np.zeros((514, 514)), w.reshape(3, 3), 3)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
