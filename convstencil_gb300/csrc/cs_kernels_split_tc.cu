@@ -116,6 +116,7 @@ template <class F>
 constexpr int kThreads = 32 * (kWarpEpi0 + F::kEpiWarps);  // 448 split, 576 FP64
 constexpr int kSliceThreads = 32 * kSliceWarps;
 constexpr int kSliceBarrier = 1;           // named barrier of the slicer warps
+constexpr int kBuildBarrier = 2;           // named barrier of the warps that build B
 
 constexpr int R = 4;                       // output rows per row group (N dimension)
 constexpr int G = 16;                      // row groups per tile (M = G x 8 blocks = 128)
@@ -125,6 +126,7 @@ constexpr int PL = ST_X * ST_Y;            // halves per digit plane (10,080 byt
 constexpr unsigned kRowBytes = ST_X * 2;   // 144
 constexpr int NOFF = R + 6;                // window row offsets per row group
 constexpr int NLV = 8 * R;                 // accumulator columns per level
+constexpr int kWz = 24;                    // halves per staged weight row: taps at 8 .. 14
 constexpr int kAccStride = 256;            // TMEM columns between the two accumulators
 constexpr int kTmemCols = 512;
 constexpr unsigned kStageBytes = ST_X * ST_Y * 8;  // 40,320 (8-byte points)
@@ -145,6 +147,7 @@ struct Smem {
     uint4 stage[NPAIR];                        // TMA destination: pairs of 8-byte points
     __half planes[2][D][PL];                   // digit planes, two tiles
     __half bmat[NOFF][NCOL * 16];              // B_i, K-major 8x16-byte core matrices
+    __half wz[D][7][kWz];                      // weight digits, rows padded with zeros
     unsigned long long stage_full, stage_empty;
     unsigned long long planes_full[2], planes_empty[2];
     unsigned long long acc_full[2], acc_empty[2];
@@ -190,19 +193,45 @@ struct alignas(128) TcGrid {
     typename F::Digits digits;
 };
 
-// B_i: N row nn = NLV e + 8 rho + c (digit e of w, output row rho of the
-// group, column c of the block), K index k; threads t0, t0 + nt, ... fill it.
+// The weight digits as B_i needs them: row ti of digit e at wz[e][ti][8 ..
+// 14], zeros around it. Threads t0, t0 + nt, ... fill it; a barrier of those
+// threads belongs between this and build_bmat.
 template <class F>
-__device__ __forceinline__ void build_bmat(Smem<F> &S, const typename F::Digits &sw, int t0, int nt)
+__device__ __forceinline__ void stage_digits(Smem<F> &S, const typename F::Digits &sw, int t0, int nt)
+{
+    for (int idx = t0; idx < F::kDigits * 7 * kWz; idx += nt) {
+        const int row = idx / kWz, j = idx - row * kWz - 8, e = row / 7, ti = row - 7 * e;
+        S.wz[e][ti][j + 8] = j >= 0 && j < 7 ? sw.d[e][ti * 7 + j] : __float2half(0.f);
+    }
+}
+
+// B_i: N row nn = NLV e + 8 rho + c (digit e of w, output row rho of the
+// group, column c of the block), K index k; threads t0, t0 + nt, ... fill it,
+// a 16-byte chunk of eight k at a time: chunk kh of a row holds
+// w_e[i - rho][8 kh - c - 1 ..], consecutive halves of the staged row. (One
+// half at a time, each from the kernel parameters at an address of its own,
+// the set-up took 16,500 cycles, 8 us of every launch; so it takes 4,000.
+// box2d3r 1024^2 on GB300: 20.9 us a launch before, 14.9 so.)
+template <class F>
+__device__ __forceinline__ void build_bmat(Smem<F> &S, int t0, int nt)
 {
     constexpr int NCOL = NLV * F::kDigits;
-    for (int idx = t0; idx < NOFF * NCOL * 16; idx += nt) {
-        const int i = idx / (NCOL * 16), rem = idx - i * (NCOL * 16);
-        const int nn = rem >> 4, k = rem & 15;
+    for (int idx = t0; idx < NOFF * NCOL * 2; idx += nt) {
+        const int i = idx / (NCOL * 2), rem = idx - i * (NCOL * 2);
+        const int nn = rem >> 1, kh = rem & 1;
         const int e = nn / NLV, rho = (nn % NLV) >> 3, c = nn & 7;
-        const int ti = i - rho, tj = k - c - 1;
-        const __half v = (ti >= 0 && ti < 7 && tj >= 0 && tj < 7) ? sw.d[e][ti * 7 + tj] : __float2half(0.f);
-        S.bmat[i][(nn >> 3) * 128 + (nn & 7) * 8 + (k >> 3) * 64 + (k & 7)] = v;
+        const int ti = i - rho;
+        __align__(16) __half v[8];
+        if (ti >= 0 && ti < 7) {
+            const __half *src = &S.wz[e][ti][8 * kh + 7 - c];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = src[k];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __float2half(0.f);
+        }
+        *reinterpret_cast<uint4 *>(&S.bmat[i][(nn >> 3) * 128 + (nn & 7) * 8 + kh * 64]) =
+            *reinterpret_cast<const uint4 *>(v);
     }
 }
 
@@ -234,72 +263,76 @@ constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
 // ready, from the same input, with the halo each single sweep would read. A
 // launch costs what one step on the 7x7 pipeline costs (its limit is the
 // digits, not the taps): box2d1r 2047 x 1531, 60 steps, GB300: 1818 us at a
-// step per launch, 744 at three; star2d1r 1024^2, 100 steps: 1295 us on the
-// FP64 FMA kernel (the FP64 pipe takes 10 us of each step's 13), 742 so.
+// step per launch, 639 at three; star2d1r 1024^2, 100 steps: 1295 us on the
+// FP64 FMA kernel (the FP64 pipe takes 10 us of each step's 13), 527 so.
+constexpr int kMaxSteps = 3;
 struct StepArgs {
     const double *in;  // interior point (0, 0) of the source
     int steps;         // T: 1, 2 or 3
     unsigned taps;     // bit t: weight t is not zero
+    int frame_cta;     // CTAs from this one on compute the frame
     double w[9];       // weights of one step
 };
 
 // One strip of the frame, by one warp: T steps for the T - 1 points next to
-// an edge, at positions l0 .. l0 + 31 - 2T along it. `edge` is the offset of
+// an edge, at positions l0 .. l0 + 25 along it. `edge` is the offset of
 // the edge's first point, `sa` the step away from the edge, `sl` the step
 // along it (`len` points, outputs before `end`); w and taps are the 3x3 weights turned the same
-// way. Lane l holds position l0 - T + l; neighbours along the edge come by
+// way. Lane l holds position l0 - 3 + l; neighbours along the edge come by
 // shuffles, and every level's outermost lanes fall out of use. A halo cell
 // keeps the value of the buffer that the sweep of its level would read.
-template <int T>
+// (The loops over levels and strips stay rolled: the code runs once or a few
+// times per launch, and unrolled its instruction fetches took most of 13,000
+// cycles, more than the first tile needs to reach the epilogue.)
 __device__ __forceinline__ void frame_strip(const double *__restrict__ in, double *__restrict__ out, long long edge,
-                                            long long sa, long long sl, int len, int l0, int end,
+                                            long long sa, long long sl, int len, int l0, int end, int steps,
                                             const double (&w)[9], unsigned taps)
 {
+    constexpr int T = kMaxSteps;
     const int lane = threadIdx.x & 31, p = l0 - T + lane;
     const bool inside = p >= 0 && p < len, halo = p == -1 || p == len;
     const long long at = edge + (long long)p * sl;
-    double u0[2 * T], u[2 * T], odd[2 * T - 1];  // row k of the strip is u[k + 1]; odd: halo cells of odd levels
+    double even[2 * T], odd[2 * T - 1], u[2 * T];  // row k of the strip is u[k + 1]
 #pragma unroll
-    for (int j = 0; j < 2 * T; ++j) u[j] = u0[j] = inside || halo ? in[at + (j - 1) * sa] : 0.0;
+    for (int j = 0; j < 2 * T; ++j) u[j] = even[j] = inside || halo ? in[at + (j - 1) * sa] : 0.0;
 #pragma unroll
     for (int j = 0; j < 2 * T - 1; ++j) odd[j] = halo || (inside && j == 0) ? out[at + (j - 1) * sa] : 0.0;
-#pragma unroll
-    for (int level = 1; level <= T; ++level) {
-        constexpr unsigned all = 0xffffffffu;
-        const int rows = 2 * T - 1 - level;  // rows 0 .. rows - 1 of this level
-        double v[2 * T];
+#pragma unroll 1
+    for (int level = 1; level <= steps; ++level) {
+        const int rows = 2 * steps - 1 - level;  // rows of this level that count
+        double v[2 * T - 2];
 #pragma unroll
         for (int k = 0; k < 2 * T - 2; ++k) v[k] = 0.0;
 #pragma unroll
         for (int j = 0; j < 2 * T; ++j) {
-            if (j > rows + 1) continue;
-            const double x[3] = {__shfl_up_sync(all, u[j], 1), u[j], __shfl_down_sync(all, u[j], 1)};
+            const double x[3] = {__shfl_up_sync(0xffffffffu, u[j], 1), u[j], __shfl_down_sync(0xffffffffu, u[j], 1)};
 #pragma unroll
             for (int t = 0; t < 9; ++t) {
                 const int k = j - t / 3;  // row k takes u[k + da] through weight row da
-                if (k >= 0 && k < rows && (taps >> t & 1u)) v[k] = fma(w[t], x[t % 3], v[k]);
+                if (k >= 0 && k < 2 * T - 2 && k < rows && (taps >> t & 1u)) v[k] = fma(w[t], x[t % 3], v[k]);
             }
         }
+        // the next level's input
+        u[0] = (level & 1) ? odd[0] : even[0];
 #pragma unroll
-        for (int k = -1; k < 2 * T - 2; ++k)
-            if (k < rows) {
-                const bool cell = halo || k < 0;  // a halo cell of the next level's input
-                u[k + 1] = cell ? ((level & 1) ? odd[k + 1] : u0[k + 1]) : inside ? v[k < 0 ? 0 : k] : 0.0;
-            }
+        for (int k = 0; k < 2 * T - 2; ++k) u[k + 1] = halo ? ((level & 1) ? odd[k + 1] : even[k + 1]) : inside ? v[k] : 0.0;
     }
     if (p < end && lane >= T && lane < 32 - T) {
 #pragma unroll
-        for (int k = 0; k < T - 1; ++k) out[at + k * sa] = u[k + 1];
+        for (int k = 0; k < T - 1; ++k)
+            if (k < steps - 1) out[at + k * sa] = u[k + 1];
     }
 }
 
 // The frame of an m x n grid, strip by strip, shared by `nwarps` warps.
-template <int T>
-__device__ __forceinline__ void frame_steps(const StepArgs &s, double *__restrict__ out, int m, int n, long long ld,
-                                            int warp, int nwarps)
+__device__ __noinline__ void frame_steps(const StepArgs &s, double *__restrict__ out, int m, int n, long long ld,
+                                         int warp, int nwarps)
 {
-    constexpr int F = T - 1, S = 32 - 2 * T;  // frame width, outputs per strip
+    constexpr int S = 32 - 2 * kMaxSteps;  // outputs per strip
+    const int F = s.steps - 1;             // frame width
+    if (F == 0) return;
     const int nx = (n + S - 1) / S, ny = (m - 2 * F + S - 1) / S;
+#pragma unroll 1
     for (int i = warp; i < 2 * (nx + ny); i += nwarps) {
         const bool horiz = i < 2 * nx;  // top and bottom rows, whole length
         const int q = horiz ? i : i - 2 * nx, cnt = horiz ? nx : ny;
@@ -314,10 +347,10 @@ __device__ __forceinline__ void frame_steps(const StepArgs &s, double *__restric
             w[t] = s.w[src];
             taps |= (s.taps >> src & 1u) << t;
         }
-        if (horiz)
-            frame_strip<T>(s.in, out, far ? (long long)(m - 1) * ld : 0, far ? -ld : ld, 1, n, l0, n, w, taps);
-        else  // the corners belong to the rows: columns end F short of them
-            frame_strip<T>(s.in, out, far ? n - 1 : 0, far ? -1 : 1, ld, m, l0, m - F, w, taps);
+        // columns end F short of the corners, which belong to the rows
+        frame_strip(s.in, out, far ? (horiz ? (long long)(m - 1) * ld : n - 1) : 0,
+                    horiz ? (far ? -ld : ld) : (far ? -1 : 1), horiz ? 1 : ld, horiz ? n : m, l0, horiz ? n : m - F,
+                    s.steps, w, taps);
     }
 }
 
@@ -393,6 +426,12 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         return mbar_wait(bar, parity, abort, &g_tc_wait_timeouts, limit);
     };
 
+    if (warp == kWarpTma) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_addr(&S.tmem)),
+                     "r"(kTmemCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
     int issued = 0, committed = 0;  // window loads issued / MMA batches committed (one thread each)
     if (tid == 0) {
         mbar_init(stage_full, 1);
@@ -411,23 +450,23 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             issued = 1;
         }
     }
-    if (warp == kWarpTma) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_addr(&S.tmem)),
-                     "r"(kTmemCols));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
     // B matrices of the first tile's grid (batch mode: the MMA warp rebuilds
-    // them whenever its run of tiles enters another grid).
+    // them whenever its run of tiles enters another grid), by every warp but
+    // the first, which may be waiting for the previous kernel's end.
+    constexpr int kBuilders = kThreads<F> - 32;
     int g_bmat = 0;
     if constexpr (BATCH) {
         if (my_tiles > 0) {
             int x0, y0;
             tile_at(0, g_bmat, x0, y0);
-            build_bmat<F>(S, grids[g_bmat].digits, tid, kThreads<F>);
+            if (warp != 0) stage_digits<F>(S, grids[g_bmat].digits, tid - 32, kBuilders);
         }
     } else {
-        build_bmat<F>(S, sw, tid, kThreads<F>);
+        if (warp != 0) stage_digits<F>(S, sw, tid - 32, kBuilders);
+    }
+    if (warp != 0) {
+        asm volatile("bar.sync %0, %1;" ::"n"(kBuildBarrier), "n"(kBuilders) : "memory");
+        build_bmat<F>(S, tid - 32, kBuilders);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
@@ -465,7 +504,9 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                         if (lane == 0 && it > 0) ok = wait(bar2(S.acc_full, (it - 1) & 1), ((it - 1) >> 1) & 1);
                         if (!__shfl_sync(0xffffffffu, ok, 0)) break;
                         tc_fence_after();
-                        build_bmat<F>(S, grids[g].digits, lane, 32);
+                        stage_digits<F>(S, grids[g].digits, lane, 32);
+                        __syncwarp();
+                        build_bmat<F>(S, lane, 32);
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         __syncwarp();
                     }
@@ -620,12 +661,11 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         const int er = mrow >> 3, eb = mrow & 7;
         const unsigned lane_bits = (unsigned)(32 * quarter) << 16;
         if constexpr (STEPS) {
-            const int fw = (warp - kWarpEpi0) * (int)gridDim.x + (int)blockIdx.x, fn = F::kEpiWarps * (int)gridDim.x;
-            pdl_wait();
-            if (sa.steps == 3)
-                frame_steps<3>(sa, out, m, n, ld, fw, fn);
-            else if (sa.steps == 2)
-                frame_steps<2>(sa, out, m, n, ld, fw, fn);
+            const int fc = (int)blockIdx.x - sa.frame_cta, fn = (int)gridDim.x - sa.frame_cta;
+            if (fc >= 0) {
+                pdl_wait();
+                frame_steps(sa, out, m, n, ld, (warp - kWarpEpi0) * fn + fc, F::kEpiWarps * fn);
+            }
         }
         const int frame = STEPS ? sa.steps - 1 : 0;
         for (int it = 0; it < my_tiles; ++it) {
@@ -828,7 +868,18 @@ cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Wei
                                  long long origin, long long elements, const double *in_base, double *out_base,
                                  const TcWait &wt, cudaStream_t st)
 {
-    StepArgs sa{in_base + origin, steps, 0u, {}};
+    StepArgs sa{in_base + origin, steps, 0u, 0, {}};
+    // The frame's strips go to the CTAs that have no tile in the last round,
+    // or to all CTAs where that is sooner. A strip keeps one of an SM's four
+    // FP64 pipes for about 9,000 cycles; an epilogue warp is idle that long
+    // before its first accumulator, and for a tile (6,500 cycles) more in a
+    // CTA that has one tile less (star2d1r 1024^2: 256 tiles, 104 CTAs with
+    // two and 48 with one, 158 strips).
+    const long long m = g.ext[0], n = g.ext[1];
+    const int tiles = (int)(((m + TY - 1) / TY) * ((n + TX - 1) / TX)), ctas = std::min(tiles, device_sm_count());
+    const long long strips = 2 * ((n + 25) / 26 + (m + 25) / 26), extra = tiles % ctas;
+    auto rounds = [&](long long c) { return (strips + 4 * c - 1) / (4 * c); };
+    if (extra > 0 && 9000 * rounds(ctas - extra) - 6500 < 9000 * rounds(ctas)) sa.frame_cta = (int)extra;
     for (int t = 0; t < 9; ++t) {
         sa.w[t] = w3x3.v[t];
         if (w3x3.v[t] != 0.0) sa.taps |= 1u << t;
