@@ -370,6 +370,15 @@ bool fp64_tc_ok(const cs_plan *p) { return p->prec == CS_PREC_FP64 && fp64_tc_ge
 bool fp64_tc3d_geometry_ok(const cs_plan *p) { return p->dims == 3 && p->radius == 1; }
 bool fp64_tc3d_ok(const cs_plan *p) { return p->prec == CS_PREC_FP64 && fp64_tc3d_geometry_ok(p); }
 
+// FP64 plans of 3D radius-3 stencils (the fused kernels) on tcgen05, whatever
+// their layout. As in 2D, grids smaller than the window stay on FP64 FMA. The
+// tuner's candidate only: FP64_TC pinned on such a plan stays refused.
+bool fp64_tc3d_r3_ok(const cs_plan *p)
+{
+    return p->prec == CS_PREC_FP64 && p->dims == 3 && p->radius == 3 && p->view.ext[0] >= 8 &&
+           p->view.ext[1] >= 8 && p->view.ext[2] >= 8;
+}
+
 // 1D plans of radius up to 3 on the 2D tcgen05 digit kernel through a row
 // view (launch_fp64_sweep_tc_rows1d): rows of 64 outputs, so the interior
 // must be a whole number of rows (at least 8), with an even origin, 4 points
@@ -411,6 +420,9 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
         if (algo == CS_ALGO_FP64_TC && fp64_tc3d_ok(p) && cs::split_tc3d_layout_ok(v, off, in_base, out_base))
             return cs::launch_fp64_sweep_tc3d(v, p->w, off, p->layout.elements, (const double *)in_base,
                                               (double *)out_base, p->wait, st);
+        if (algo == CS_ALGO_FP64_TC && fp64_tc3d_r3_ok(p))
+            return cs::launch_fp64_sweep_tc3d_r3(v, p->w, off, p->layout.elements, (const double *)in_base,
+                                                 (double *)out_base, p->wait, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc_ok(p) && fp64_tc_window_ok(v, off, in_base, out_base))
             return cs::launch_fp64_sweep_tc(v, p->w7, off, p->layout.elements, (const double *)in_base,
                                             (double *)out_base, p->wait, st);
@@ -508,7 +520,7 @@ cs_status choose_algo(cs_plan *p, const void *a, void *b, cudaStream_t st, int *
         cand[nc++] = CS_ALGO_SPLIT_MMA_TMA;
         cand[nc++] = CS_ALGO_SPLIT_FMA;
     } else {
-        const bool tc = fp64_tc_ok(p) || fp64_tc3d_ok(p) || fp64_tc1d_ok(p);
+        const bool tc = fp64_tc_ok(p) || fp64_tc3d_ok(p) || fp64_tc3d_r3_ok(p) || fp64_tc1d_ok(p);
         if ((p->algo == CS_ALGO_FP64_MMA && fp64_mma_ok(p)) || (p->algo == CS_ALGO_FP64_TC && tc)) {
             *out = p->algo;
             return CS_OK;
@@ -923,6 +935,8 @@ CS_API cs_status cs_device_wait_timeouts(unsigned *count, int reset)
     CS_CUDA(cs::split_tc_wait_timeouts(&b, reset != 0));
     unsigned c3 = 0;
     CS_CUDA(cs::split_tc3d_wait_timeouts(&c3, reset != 0));
+    b += c3;
+    CS_CUDA(cs::tc3d_r3_wait_timeouts(&c3, reset != 0));
     b += c3;
     *count = a + b;
     return CS_OK;

@@ -129,12 +129,18 @@ cudaError_t launch_split_sweep_tc3d(const GridView &g, const Weights &w, long lo
 cudaError_t launch_fp64_sweep_tc3d(const GridView &g, const Weights &w, long long origin, long long elements,
                                    const double *in_base, double *out_base, const TcWait &wait,
                                    cudaStream_t stream);
+// FP64 sweep of a 3D radius-3 kernel (343 weights, any pattern) on tcgen05
+// (cs_kernels_tc3d_r3.cu), any layout.
+cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long long origin, long long elements,
+                                      const double *in_base, double *out_base, const TcWait &wait,
+                                      cudaStream_t stream);
 int device_sm_count();
 // Bounded device-side waits that expired since the last reset (TMA/mma.sync
 // kernel, 2D and 3D tcgen05 kernels).
 cudaError_t split_wait_timeouts(unsigned *count, bool reset);
 cudaError_t split_tc_wait_timeouts(unsigned *count, bool reset);
 cudaError_t split_tc3d_wait_timeouts(unsigned *count, bool reset);
+cudaError_t tc3d_r3_wait_timeouts(unsigned *count, bool reset);
 // Whole-buffer conversions over n elements, and the in-place forms used by
 // the FP64 re-anchor sweeps ((hi, lo) pairs and FP64 values share a buffer
 // layout: 8 bytes per point).
