@@ -28,9 +28,13 @@
 //     two halves are the two TMEM blocks: one is drained while the other is
 //     being computed. (All seven taps in one N would need 384 columns, one
 //     block of the 512, and a wait for the epilogue after every plane.)
-//   * Bound: the MMA stream. 84 MMAs per plane and 1024 outputs at ~56 cycles
-//     allow about 68 G outputs/s; the FP64 pipe allows 1.5 (box), 8.3
-//     (octahedron).
+//   * Bound: the MMA stream and the shared memory it reads. An MMA reads 4 KB
+//     of A and N x 32 bytes of B, 60 cycles on average at 128 bytes a cycle;
+//     the 84 MMAs of a plane (1024 outputs) take 5,570 cycles with little else
+//     running and 7,260 of a plane's 8,350 beside the slicers and the epilogue
+//     (without the slicers' cutting the sweep runs 17 % faster, without the
+//     epilogue's arithmetic 8 %). GB300: 512^3 4.04 ms a sweep, 33 G
+//     outputs/s; the FP64 FMA kernel 1.5 (box), 8.3 (octahedron).
 //   * Roles (20 warps, five per scheduler, two of them idle, 96 registers):
 //     one loads windows (four stages), one thread issues the MMAs, two groups
 //     of four cut every second plane (ring of four digit-plane sets), eight
@@ -40,7 +44,8 @@
 //     16-byte aligned base); the window then starts 4 columns left of the
 //     tile, or 3 where the interior's first column is odd, so that its
 //     address is a multiple of 16 bytes. Other layouts (odd pitches) are
-//     loaded by the same warp with 8-byte cp.async.
+//     loaded by the same warp with 8-byte cp.async (its 50 copies a lane and
+//     plane hide behind the MMAs: 200 x 184 x 193 runs at the rate of its tiles).
 //
 // Every mbarrier wait is bounded (WaitCfg, 2 s by default); an expired wait is
 // counted in g_tc3d_r3_wait_timeouts and the CTA leaves as in the other
