@@ -188,7 +188,7 @@ bool selfconv(const double *w, int dims, int r, int steps, int R, double *out)
     const int k = 2 * r + 1, K = 2 * R + 1, n = ipow(k, dims), N = ipow(K, dims);
     double sum = 0.0;
     for (int i = 0; i < n; ++i) sum += std::fabs(w[i]);
-    if (!(sum > 0x1p-64 && sum < 0x1p64) || steps * r > R) return false;
+    if (steps * r > R || (steps > 1 && !(sum > 0x1p-64 && sum < 0x1p64))) return false;
     std::vector<double> h(N, 0.0), l(N, 0.0), h2(N), l2(N);
     const int c = dims == 2 ? R * K + R : R;
     h[c] = 1.0;
@@ -272,9 +272,12 @@ struct cs_plan {
     int dims, radius, pattern, steps_per_sweep;
     Weights w;
     Weights w7;  // 2D plans: w at the centre of a 7x7 (the 2D tcgen05 kernels' tap window)
-    // FP64 2D radius-1 plans: the 7x7 kernels of 1, 2 and 3 steps (launch_fp64_steps_tc)
+    // Kernels of several steps: FP64 2D radius-1 plans, the 7x7 ones of 1, 2 and
+    // 3 (launch_fp64_steps_tc); 1D plans, the 33 taps of 1 .. 16 / radius
+    // (launch_fp64_steps_tc_1d).
     Weights w_steps[3];
-    int max_steps = 1;  // steps per launch those allow
+    double w1_steps[16][33];
+    int max_steps = 0;  // steps per launch those allow (0: not even one)
     cs_layout layout;
     GridView view;
     int algo = CS_ALGO_AUTO;
@@ -379,23 +382,50 @@ bool fp64_tc3d_r3_ok(const cs_plan *p)
            p->view.ext[1] >= 8 && p->view.ext[2] >= 8;
 }
 
-// 1D plans of radius up to 3 on the 2D tcgen05 digit kernel through a row
-// view (launch_fp64_sweep_tc_rows1d): rows of 64 outputs, so the interior
-// must be a whole number of rows (at least 8), with an even origin, 4 points
-// of halo before it and 60 points of the array after it.
-bool fp64_tc1d_geometry_ok(const cs_plan *p)
+// FP64 1D plans on the tcgen05 digit kernel (rows of 32 outputs, a reach of
+// 16 points: launch_fp64_steps_tc_1d), whatever their layout. Pinning FP64_TC
+// keeps the conditions it had (fp64_tc1d_pin_ok); the tuner's candidate needs
+// no more than room for both ends of the grid.
+bool fp64_tc1d_geometry_ok(const cs_plan *p) { return p->dims == 1 && p->view.ext[0] >= 512 && p->max_steps >= 1; }
+bool fp64_tc1d_ok(const cs_plan *p) { return p->prec == CS_PREC_FP64 && fp64_tc1d_geometry_ok(p); }
+bool fp64_tc1d_pin_ok(const cs_plan *p)
 {
     const long long n = p->view.ext[0], o = p->layout.origin;
-    return p->dims == 1 && p->radius <= 3 && n % 64 == 0 && n >= 512 && o >= 4 && o % 2 == 0 &&
-           p->layout.elements >= o + n + 60;
+    return fp64_tc1d_ok(p) && p->radius <= 3 && n % 64 == 0 && o >= 4 && o % 2 == 0 && p->layout.elements >= o + n + 60;
 }
-bool fp64_tc1d_ok(const cs_plan *p) { return p->prec == CS_PREC_FP64 && fp64_tc1d_geometry_ok(p); }
 
 // Split plans of 3D radius-1 stencils (27 weights) also run on the tcgen05
 // slice kernel.
 bool split_tc3d_ok(const cs_plan *p)
 {
     return p->prec == CS_PREC_SPLIT && p->dims == 3 && p->radius == 1;
+}
+
+// Steps per launch of the tcgen05 digit kernel on this plan and these
+// buffers: 3 for FP64 2D radius-1 plans (three steps of a 3x3 kernel are one
+// 7x7 kernel, the kernel's tap window) from 64 tiles up. Smaller grids leave
+// most SMs without a tile, and a launch of ~12 us loses to single steps on
+// the FP64 FMA kernel (512^2, 64 tiles, is where three of those take as long).
+// FP64 1D plans take the most steps, an odd number, that reach at most 16
+// points, at any size.
+int fp64_steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base)
+{
+    if (p->dims == 1) return fp64_tc1d_ok(p) ? p->max_steps : 1;
+    if (p->max_steps < 2 || !fp64_tc_ok(p) || !fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base))
+        return 1;
+    const long long tiles = ((p->view.ext[0] + 63) / 64) * ((p->view.ext[1] + 63) / 64);
+    return tiles >= 64 ? p->max_steps : 1;
+}
+
+// `steps` (1 .. fp64_steps_per_launch) steps in one launch.
+cudaError_t launch_steps(const cs_plan *p, int steps, const void *in_base, void *out_base, cudaStream_t st)
+{
+    if (p->dims == 1)
+        return cs::launch_fp64_steps_tc_1d(p->view.ext[0], p->w1_steps[steps - 1], p->radius, p->w.v, steps,
+                                           p->layout.origin, (const double *)in_base, (double *)out_base, p->wait,
+                                           st);
+    return cs::launch_fp64_steps_tc(p->view, p->w_steps[steps - 1], p->w, steps, p->layout.origin,
+                                    p->layout.elements, (const double *)in_base, (double *)out_base, p->wait, st);
 }
 
 // One sweep over the slabs [row0, row0 + rows) of the slowest axis (rows of
@@ -413,10 +443,8 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
         const double *in = (const double *)in_base + off;
         double *out = (double *)out_base + off;
         if (algo == CS_ALGO_FP64_MMA) return cs::launch_fp64_mma_2d(v, p->w, in, out, st);
-        if (algo == CS_ALGO_FP64_TC && fp64_tc1d_ok(p) && row0 == 0 && rows == p->view.ext[0] &&
-            reinterpret_cast<uintptr_t>(in_base) % 16 == 0 && reinterpret_cast<uintptr_t>(out_base) % 16 == 0)
-            return cs::launch_fp64_sweep_tc_rows1d(rows, p->w7, p->layout.origin, p->layout.elements,
-                                                   (const double *)in_base, (double *)out_base, p->wait, st);
+        if (algo == CS_ALGO_FP64_TC && fp64_tc1d_ok(p) && row0 == 0 && rows == p->view.ext[0])
+            return launch_steps(p, 1, in_base, out_base, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc3d_ok(p) && cs::split_tc3d_layout_ok(v, off, in_base, out_base))
             return cs::launch_fp64_sweep_tc3d(v, p->w, off, p->layout.elements, (const double *)in_base,
                                               (double *)out_base, p->wait, st);
@@ -454,26 +482,6 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
     float2 *out = (float2 *)out_base + off;
     return cs::launch_split_sweep(v, p->radius, p->pattern, p->w, algo == CS_ALGO_SPLIT_MMA,
                                   in, out, st);
-}
-
-// Steps per launch of the tcgen05 digit kernel on this plan and these
-// buffers: 3 for FP64 2D radius-1 plans (three steps of a 3x3 kernel are one
-// 7x7 kernel, the kernel's tap window) from 64 tiles up. Smaller grids leave
-// most SMs without a tile, and a launch of ~12 us loses to single steps on
-// the FP64 FMA kernel (512^2, 64 tiles, is where three of those take as long).
-int fp64_steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base)
-{
-    if (p->max_steps < 2 || !fp64_tc_ok(p) || !fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base))
-        return 1;
-    const long long tiles = ((p->view.ext[0] + 63) / 64) * ((p->view.ext[1] + 63) / 64);
-    return tiles >= 64 ? p->max_steps : 1;
-}
-
-// `steps` (1 .. fp64_steps_per_launch) steps in one launch.
-cudaError_t launch_steps(const cs_plan *p, int steps, const void *in_base, void *out_base, cudaStream_t st)
-{
-    return cs::launch_fp64_steps_tc(p->view, p->w_steps[steps - 1], p->w, steps, p->layout.origin,
-                                    p->layout.elements, (const double *)in_base, (double *)out_base, p->wait, st);
 }
 
 cudaError_t launch_sweep(const cs_plan *p, int algo, const void *in_base, void *out_base, cudaStream_t st)
@@ -638,7 +646,7 @@ cs_status choose_time_block(cs_plan *p, int algo, const void *a, void *b, cudaSt
 // how many (*steps) and the kernel (*algo). Always when FP64_TC is pinned;
 // with AUTO where the time of ceil(sweeps / steps) such launches, measured
 // once per class of plan beside single sweeps of the chosen algorithm
-// (six steps each way, a -> b), is the shorter one. A caller that is capturing
+// (two launches, six sweeps, a -> b), is the shorter one. A caller that is capturing
 // its stream gets what is already known.
 cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long long sweeps, int *algo, int *steps)
 {
@@ -666,7 +674,7 @@ cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long
             CS_CUDA(cudaEventRecord(e[0], st));
             for (int i = 0; i < 6; ++i) CS_CUDA(launch_sweep(p, *algo, a, b, st));
             CS_CUDA(cudaEventRecord(e[1], st));
-            for (int i = 0; i < 6 / t; ++i) CS_CUDA(launch_steps(p, t, a, b, st));
+            for (int i = 0; i < 2; ++i) CS_CUDA(launch_steps(p, t, a, b, st));
             CS_CUDA(cudaEventRecord(e[2], st));
             CS_CUDA(cudaEventSynchronize(e[2]));
         }
@@ -674,7 +682,7 @@ cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long
         CS_CUDA(cudaEventElapsedTime(&ms.second, e[1], e[2]));
         for (auto &x : e) cudaEventDestroy(x);
         ms.first /= 6;
-        ms.second /= 6 / t;
+        ms.second /= 2;
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune_steps[key] = ms;
     }
@@ -755,10 +763,7 @@ cudaError_t fp64_anchor_sweep_fp64_in(const cs_plan *p, const void *src, void *d
         return launch_fp64_sweep_tc(p->view, p->w7, off, n, (const double *)src, (double *)dst, p->wait, st);
     if (fp64_tc3d_geometry_ok(p) && split_tc3d_layout_ok(p->view, off, src, dst))
         return launch_fp64_sweep_tc3d(p->view, p->w, off, n, (const double *)src, (double *)dst, p->wait, st);
-    if (fp64_tc1d_geometry_ok(p) && reinterpret_cast<uintptr_t>(src) % 16 == 0 &&
-        reinterpret_cast<uintptr_t>(dst) % 16 == 0)
-        return launch_fp64_sweep_tc_rows1d(p->view.ext[0], p->w7, off, n, (const double *)src, (double *)dst,
-                                           p->wait, st);
+    if (fp64_tc1d_geometry_ok(p)) return launch_steps(p, 1, src, dst, st);
     return launch_fp64_fma(p->view, p->radius, p->pattern, p->w, (const double *)src + off, (double *)dst + off, st);
 }
 
@@ -979,8 +984,6 @@ CS_API cs_status cs_plan_create(cs_plan **out, cs_shape shape, cs_semantics sem,
         const int k = 2 * p->radius + 1, o = 3 - p->radius;
         for (int i = 0; i < k; ++i)
             for (int j = 0; j < k; ++j) p->w7.v[(i + o) * 7 + j + o] = p->w.v[i * k + j];
-    } else if (p->dims == 1 && p->radius <= 3) {  // the taps in row 3 of the 7x7
-        for (int j = 0; j <= 2 * p->radius; ++j) p->w7.v[3 * 7 + 3 - p->radius + j] = p->w.v[j];
     }
     if (prec == CS_PREC_FP64 && p->dims == 2 && p->radius == 1) {
         bool ok = true;
@@ -989,6 +992,13 @@ CS_API cs_status cs_plan_create(cs_plan **out, cs_shape shape, cs_semantics sem,
             ok = ok && selfconv(p->w.v, 2, 1, t, 3, p->w_steps[t - 1].v);
         }
         if (ok) p->max_steps = 3;
+    } else if (p->dims == 1) {
+        for (int t = 1; t * p->radius <= cs::kTcReach1d; ++t) {
+            if (!selfconv(p->w.v, 1, p->radius, t, cs::kTcReach1d, p->w1_steps[t - 1])) break;
+            // an odd number: a launch then leaves the state in the buffer where
+            // single steps would, so each step still reads that one's halo
+            if (t % 2) p->max_steps = t;
+        }
     }
     if (layout) {
         const cs_layout &L = *layout;
@@ -1048,7 +1058,7 @@ CS_API cs_status cs_plan_set_option(cs_plan *p, cs_option opt, long long v)
             return fail(CS_ERR_INVALID_ARGUMENT, "FP64 algo needs an FP64 plan");
         if (v == CS_ALGO_FP64_MMA && !fp64_mma_ok(p))
             return fail(CS_ERR_UNSUPPORTED, "FP64 MMA serves 2D radius-3 dense FP64 plans only");
-        if (v == CS_ALGO_FP64_TC && !fp64_tc_ok(p) && !fp64_tc3d_ok(p) && !fp64_tc1d_ok(p))
+        if (v == CS_ALGO_FP64_TC && !fp64_tc_ok(p) && !fp64_tc3d_ok(p) && !fp64_tc1d_pin_ok(p))
             return fail(CS_ERR_UNSUPPORTED,
                         "FP64 tcgen05 serves 2D FP64 plans of radius up to 3 and at least 8x8 on even-aligned "
                         "layouts, 3D radius-1 FP64 plans and 1D FP64 plans of radius up to 3 whose length is a "

@@ -130,12 +130,24 @@ constexpr int kWz = 24;                    // halves per staged weight row: taps
 constexpr int kAccStride = 256;            // TMEM columns between the two accumulators
 constexpr int kTmemCols = 512;
 constexpr unsigned kStageBytes = ST_X * ST_Y * 8;  // 40,320 (8-byte points)
-// 1D row view: a tile's 70 window rows of 72 points lie in 71 array rows of 64
-constexpr int kSpanRows = ST_Y + 1;
-constexpr unsigned kSpanBytes = TX * kSpanRows * 8;  // 36,352
-static_assert(kSpanBytes <= kStageBytes, "the span fits the stage");
 constexpr int PAIRS = ST_X / 2, NPAIR = ST_Y * PAIRS;           // 36, 2,520
 constexpr int PER = (NPAIR + kSliceThreads - 1) / kSliceThreads;  // 10
+// 1D (kMode1d): a tile is 4096 outputs, 128 rows of 32; row m of A is the 64
+// points around output row m, read in four K steps. The window is 4096 + 32
+// points, 516 chunks of 8; chunk j sits in phase j % 4 at place j / 4, so the
+// rows' chunks of one K step (two phases, places m or m + 1) are core matrices
+// of consecutive 16-byte rows: the canonical non-swizzled layout again, each
+// point stored once.
+constexpr int kReach1d = kTcReach1d;                // points either side of an output: 16
+constexpr int kOut1d = 4096, kWin1d = kOut1d + 2 * kReach1d, NPAIR1D = kWin1d / 2;
+constexpr int kSteps1d = (32 + 2 * kReach1d) / 16;  // K steps
+// bytes between phases: 129 chunks, rounded so that the words a slicer warp
+// stores (16 per phase pair) fall into different banks
+constexpr int kPhase1d = 2080;
+constexpr unsigned kBytes1d = kWin1d * 8;
+static_assert(4 * kPhase1d <= PL * 2 && kBytes1d <= kStageBytes && NPAIR1D <= PER * kSliceThreads &&
+                  kPhase1d >= (kWin1d / 32) * 16 && kPhase1d / 4 % 32 == 8,
+              "the 1D window and digits fit the 2D buffers");
 static_assert(FmtSplit::kEpiWarps == 4 && FmtF64::kEpiWarps == 8 && R == 4,
               "one or two epilogue warps per TMEM lane quarter, R / (warps per quarter) rows each");
 
@@ -179,6 +191,21 @@ __device__ __forceinline__ void tile_mma(unsigned d_base, unsigned long long a0,
         tile_mma<D, I, DG + 1>(d_base, a0, b0);
     else if constexpr (I + 1 < NOFF)
         tile_mma<D, I + 1, 0>(d_base, a0, b0);
+}
+
+// The MMAs of one 1D tile: K step KK, input digit DG.
+template <int D, int KK, int DG>
+__device__ __forceinline__ void tile_mma_1d(unsigned d_base, unsigned long long a0, unsigned long long b0)
+{
+    constexpr unsigned long long a_off =
+        ((unsigned long long)DG * PL * 2 + (KK & 1) * 2 * kPhase1d + (KK >> 1) * 16) >> 4;
+    constexpr unsigned long long b_off = ((unsigned long long)KK * NLV * D * 16 * 2) >> 4;
+    mma_f16(d_base + (unsigned)(NLV * DG), a0 + a_off, b0 + b_off, instr_desc(NLV * (D - DG)),
+            (KK | DG) != 0 ? 1u : 0u);
+    if constexpr (DG + 1 < D)
+        tile_mma_1d<D, KK, DG + 1>(d_base, a0, b0);
+    else if constexpr (KK + 1 < kSteps1d)
+        tile_mma_1d<D, KK + 1, 0>(d_base, a0, b0);
 }
 
 // One grid of a batch (batch mode): its tensor map, output, sizes, tile
@@ -235,6 +262,37 @@ __device__ __forceinline__ void build_bmat(Smem<F> &S, int t0, int nt)
     }
 }
 
+// The same for 1D: the 33 taps of digit e at wz1[e][32 .. 64] (the rows of wz,
+// laid end to end), and B of K step kk: N row nn = 32 e + c (output c of a
+// row), tap 16 kk + k - c.
+constexpr int kWz1d = 96;
+static_assert(FmtF64::kDigits * kWz1d <= FmtF64::kDigits * 7 * kWz, "the 1D rows fit wz");
+template <class F>
+__device__ __forceinline__ void stage_digits_1d(Smem<F> &S, const typename F::Digits &sw, int t0, int nt)
+{
+    __half *wz = &S.wz[0][0][0];
+    for (int idx = t0; idx < F::kDigits * kWz1d; idx += nt) {
+        const int e = idx / kWz1d, j = idx - e * kWz1d - 32;
+        wz[idx] = j >= 0 && j <= 2 * kReach1d ? sw.d[e][j] : __float2half(0.f);
+    }
+}
+template <class F>
+__device__ __forceinline__ void build_bmat_1d(Smem<F> &S, int t0, int nt)
+{
+    constexpr int NCOL = NLV * F::kDigits;
+    const __half *wz = &S.wz[0][0][0];
+    for (int idx = t0; idx < kSteps1d * NCOL * 2; idx += nt) {
+        const int kk = idx / (NCOL * 2), rem = idx - kk * (NCOL * 2);
+        const int nn = rem >> 1, kh = rem & 1;
+        const __half *src = wz + (nn / NLV) * kWz1d + 32 + 16 * kk + 8 * kh - nn % NLV;
+        __align__(16) __half v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = src[k];
+        *reinterpret_cast<uint4 *>(&S.bmat[kk][(nn >> 3) * 128 + (nn & 7) * 8 + kh * 64]) =
+            *reinterpret_cast<const uint4 *>(v);
+    }
+}
+
 // Batch mode: the grid of global tile `tile` (last record whose tile_begin
 // is not above it).
 template <class F>
@@ -251,7 +309,7 @@ __device__ __forceinline__ int grid_of(const TcGrid<F> *grids, int ngrids, int t
 
 // What one launch computes.
 constexpr int kModeGrid = 0;    // one sweep of a 2D grid
-constexpr int kModeRows1d = 1;  // one sweep of a 1D grid, as rows of 64 outputs
+constexpr int kMode1d = 1;      // several steps of a 1D grid (FP64)
 constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
 
 // kModeSteps: T steps of a 3x3 stencil are one sweep of its T-fold
@@ -268,7 +326,9 @@ constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
 constexpr int kMaxSteps = 3;
 struct StepArgs {
     const double *in;  // interior point (0, 0) of the source
-    int steps;         // T: 1, 2 or 3
+    int steps;         // T
+    int radius;        // of one step
+    int aligned;       // 1D: the buffers and the interior are 16-byte aligned
     unsigned taps;     // bit t: weight t is not zero
     int frame_cta;     // CTAs from this one on compute the frame
     double w[9];       // weights of one step
@@ -354,6 +414,28 @@ __device__ __noinline__ void frame_steps(const StepArgs &s, double *__restrict__
     }
 }
 
+// The (T - 1) r outputs next to one end of a 1D grid (T r <= 16), by one warp:
+// lane l holds point l - r counted from that end, as frame_strip's lanes do.
+__device__ __noinline__ void frame_end_1d(const StepArgs &s, double *__restrict__ out, int n, bool left)
+{
+    const int lane = threadIdx.x & 31, r = s.radius, p = lane - r;
+    const long long at = left ? p : n - 1 - p;
+    const bool halo = p < 0;
+    const double even = s.in[at], odd = halo ? out[at] : 0.0;
+    double u = even;
+#pragma unroll 1
+    for (int level = 1; level <= s.steps; ++level) {
+        double v = 0.0;
+#pragma unroll 1
+        for (int t = 0; t <= 2 * r; ++t) {
+            const int d = left ? t - r : r - t;  // the tap's lane, towards the interior from this end
+            v = fma(s.w[t], __shfl_sync(0xffffffffu, u, (lane + d) & 31), v);
+        }
+        u = halo ? ((level & 1) ? odd : even) : v;
+    }
+    if (!halo && p < (s.steps - 1) * r) out[at] = u;
+}
+
 // One grid (BATCH = false: kernel parameters describe it, tiles are dealt
 // round-robin) or a batch of grids (BATCH = true: `grids` describes them,
 // each CTA takes a contiguous run of the batch's tiles, and the MMA warp
@@ -365,7 +447,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
            long long ld, int tiles_x, int tiles, int map_x, int map_y, typename F::Digits sw, WaitCfg wc,
            const TcGrid<F> *__restrict__ grids, int ngrids, const __grid_constant__ StepArgs sa)
 {
-    constexpr bool ROWS1D = MODE == kModeRows1d, STEPS = MODE == kModeSteps;
+    constexpr bool ONED = MODE == kMode1d, STEPS = MODE == kModeSteps;
     static_assert(!BATCH || MODE == kModeGrid, "batches run one sweep of 7x7 grids");
     constexpr int D = F::kDigits;
     using SM = Smem<F>;
@@ -408,13 +490,6 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             mx = grids[g].map_x;
             my = grids[g].map_y;
         }
-        if constexpr (ROWS1D) {
-            // 1D row view: the span of 71 array rows of 64 points from view
-            // row y0 - 3 (rows outside the map read as zero)
-            mbar_expect_tx(bar, kSpanBytes);
-            tma_load_2d(smem_addr(S.stage), map, 0, y0 - 3, bar);
-            return;
-        }
         mbar_expect_tx(bar, kStageBytes);
         tma_load_2d(smem_addr(S.stage), map, mx + x0 - 4, my + y0 - 3, bar);
     };
@@ -444,7 +519,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         }
         S.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (my_tiles > 0 && !wc.skip_loads) {  // the first window load overlaps the set-up below
+        if (!ONED && my_tiles > 0 && !wc.skip_loads) {  // the first window load overlaps the set-up below
             pdl_wait();
             load_window(0, stage_full);
             issued = 1;
@@ -462,11 +537,19 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             if (warp != 0) stage_digits<F>(S, grids[g_bmat].digits, tid - 32, kBuilders);
         }
     } else {
-        if (warp != 0) stage_digits<F>(S, sw, tid - 32, kBuilders);
+        if (warp != 0) {
+            if constexpr (ONED)
+                stage_digits_1d<F>(S, sw, tid - 32, kBuilders);
+            else
+                stage_digits<F>(S, sw, tid - 32, kBuilders);
+        }
     }
     if (warp != 0) {
         asm volatile("bar.sync %0, %1;" ::"n"(kBuildBarrier), "n"(kBuilders) : "memory");
-        build_bmat<F>(S, tid - 32, kBuilders);
+        if constexpr (ONED)
+            build_bmat_1d<F>(S, tid - 32, kBuilders);
+        else
+            build_bmat<F>(S, tid - 32, kBuilders);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
@@ -476,7 +559,38 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
 
     if (warp == kWarpTma) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0 && !wc.skip_loads) {
+        if constexpr (ONED) {
+            // A window inside the halo and 16-byte aligned is one bulk copy;
+            // others are copied in 8-byte pieces, with zeros past the halo.
+            pdl_wait();
+            bool ok = !wc.skip_loads;
+            for (int it = 0; it < my_tiles && ok; ++it) {
+                ok = lane != 0 || wait(stage_empty, (it & 1) ^ 1);
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) break;
+                const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d - kReach1d;
+                const unsigned dst = smem_addr(S.stage);
+                if (sa.aligned && x >= -sa.radius && x + kWin1d <= n + sa.radius) {
+                    if (lane == 0) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        mbar_expect_tx(stage_full, kBytes1d);
+                        bulk_load(dst, sa.in + x, kBytes1d, stage_full);
+                        issued = it + 1;
+                    }
+                } else {
+                    for (int i = lane; i < kWin1d; i += 32) {
+                        const bool take = x + i >= -sa.radius && x + i < n + sa.radius;
+                        cp_async8(dst + 8u * i, take ? sa.in + x + i : sa.in, take);
+                    }
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(stage_full);
+                        issued = it + 1;
+                    }
+                }
+            }
+        } else if (lane == 0 && !wc.skip_loads) {
             for (int it = issued; it < my_tiles; ++it) {
                 if (!wait(stage_empty, (it & 1) ^ 1)) break;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -486,8 +600,9 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         }
     } else if (warp == kWarpMma) {
         // ------------------------------------------------ MMA issuer
-        const unsigned long long a_desc_buf0 = smem_desc(smem_addr(S.planes[0][0]), 16, R * kRowBytes);
-        const unsigned long long a_desc_buf1 = smem_desc(smem_addr(S.planes[1][0]), 16, R * kRowBytes);
+        constexpr unsigned lbo = ONED ? kPhase1d : 16, sbo = ONED ? 128 : R * kRowBytes;
+        const unsigned long long a_desc_buf0 = smem_desc(smem_addr(S.planes[0][0]), lbo, sbo);
+        const unsigned long long a_desc_buf1 = smem_desc(smem_addr(S.planes[1][0]), lbo, sbo);
         const unsigned long long b_desc0 = smem_desc(smem_addr(S.bmat[0]), 128, 256);
         for (int it = 0; it < my_tiles; ++it) {
             const int buf = it & 1, use = it >> 1;
@@ -522,8 +637,12 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                     // core takes it, so nothing else sits between them: all
                     // MMAs are unrolled, each descriptor one add of a
                     // compile-time offset.
-                    tile_mma<D, 0, 0>(tmem + (unsigned)(kAccStride * buf), buf ? a_desc_buf1 : a_desc_buf0,
-                                      b_desc0);
+                    const unsigned d_base = tmem + (unsigned)(kAccStride * buf);
+                    const unsigned long long a0 = buf ? a_desc_buf1 : a_desc_buf0;
+                    if constexpr (ONED)
+                        tile_mma_1d<D, 0, 0>(d_base, a0, b_desc0);
+                    else
+                        tile_mma<D, 0, 0>(d_base, a0, b_desc0);
                     mma_commit(bar2(S.planes_empty, buf));  // planes may be overwritten
                     mma_commit(bar2(S.acc_full, buf));      // accumulator ready
                     committed = it + 1;
@@ -533,6 +652,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         }
     } else if (warp < kWarpEpi0) {
         // ------------------------------------------------ slicers
+        constexpr int kPairs = ONED ? NPAIR1D : NPAIR;
         const int st = tid - 32 * kWarpSlice0;
         const bool leader = st == 0;
         for (int it = 0; it < my_tiles; ++it) {
@@ -556,13 +676,8 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             for (int q = 0; q < PER; ++q) {
                 const int idx = st + q * kSliceThreads;
                 v[q] = make_uint4(0u, 0u, 0u, 0u);
-                if (idx < NPAIR) {
-                    // 1D row view: window row r (pairs 36 r ..) starts at pair
-                    // 32 r of the span, the 72 points from view row y0 - 3 + r
-                    if constexpr (ROWS1D)
-                        v[q] = S.stage[idx - 4 * (idx / PAIRS)];
-                    else
-                        v[q] = S.stage[idx];
+                if (idx < kPairs) {
+                    v[q] = S.stage[idx];
                     // Points past the halo meet zero weights in every output
                     // kept, but must not set the tile's scale either.
                     if (STEPS && edge) {
@@ -616,10 +731,12 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
 #pragma unroll
                 for (int q = 0; q < PER; ++q) {
                     const int idx = st + q * kSliceThreads;
-                    if (idx < NPAIR) {
-                        const unsigned long long ya = f64_biased_fixed<STEPS>(v[q].x, v[q].y, ex);
-                        const unsigned long long yb = f64_biased_fixed<STEPS>(v[q].z, v[q].w, ex);
-                        unsigned *dst = dst0 + idx;
+                    if (idx < kPairs) {
+                        const unsigned long long ya = f64_biased_fixed<STEPS || ONED>(v[q].x, v[q].y, ex);
+                        const unsigned long long yb = f64_biased_fixed<STEPS || ONED>(v[q].z, v[q].w, ex);
+                        // 1D: chunk idx / 4 in phase (idx / 4) % 4
+                        unsigned *dst = dst0 + (ONED ? (idx >> 2 & 3) * (kPhase1d / 4) + (idx >> 4) * 4 + (idx & 3)
+                                                     : idx);
                         dst[0 * (PL / 2)] = f64_digit_pair<0>(ya, yb);
                         dst[1 * (PL / 2)] = f64_digit_pair<1>(ya, yb);
                         dst[2 * (PL / 2)] = f64_digit_pair<2>(ya, yb);
@@ -667,7 +784,13 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 frame_steps(sa, out, m, n, ld, (warp - kWarpEpi0) * fn + fc, F::kEpiWarps * fn);
             }
         }
-        const int frame = STEPS ? sa.steps - 1 : 0;
+        if constexpr (ONED) {  // the ends, on the last CTA (no other has fewer tiles)
+            if (blockIdx.x == gridDim.x - 1 && warp < kWarpEpi0 + 2 && sa.steps > 1) {
+                pdl_wait();
+                frame_end_1d(sa, out, n, warp == kWarpEpi0);
+            }
+        }
+        const int frame = STEPS || ONED ? (sa.steps - 1) * sa.radius : 0;
         for (int it = 0; it < my_tiles; ++it) {
             const int buf = it & 1, use = it >> 1;
             if (!wait(bar2(S.acc_full, buf), use & 1)) break;
@@ -699,6 +822,28 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar2(S.acc_empty, buf));
+                }
+                if constexpr (ONED) {
+                    // outputs 32 mrow + 8 rho .. + 7 of the tile
+                    const int c = ex + ew - 1080;
+                    const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d + 32 * mrow + 8 * rho;
+                    double res[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float lv[6] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4][j], acc[5][j]};
+                        res[j] = ex == kNonFiniteTile ? __longlong_as_double(0x7FF8000000000000ll)
+                                                      : f64_from_fixed(f64_combine(lv), c);
+                    }
+                    if (sa.aligned && x >= frame && x + 8 <= n - frame) {
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2)
+                            *reinterpret_cast<double2 *>(out + x + j) = make_double2(res[j], res[j + 1]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (x + j >= frame && x + j < n - frame) out[x + j] = res[j];
+                    }
+                    continue;
                 }
                 const int yy = y0 + R * er + rho;
                 if (yy >= o_m) continue;
@@ -868,7 +1013,7 @@ cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Wei
                                  long long origin, long long elements, const double *in_base, double *out_base,
                                  const TcWait &wt, cudaStream_t st)
 {
-    StepArgs sa{in_base + origin, steps, 0u, 0, {}};
+    StepArgs sa{in_base + origin, steps, 1, 0, 0u, 0, {}};
     // The frame's strips go to the CTAs that have no tile in the last round,
     // or to all CTAs where that is sooner. A strip keeps one of an SM's four
     // FP64 pipes for about 9,000 cycles; an epilogue warp is idle that long
@@ -888,36 +1033,27 @@ cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Wei
                                          WaitCfg{wt.limit_ns, wt.skip_loads}, st, sa);
 }
 
-cudaError_t launch_fp64_sweep_tc_rows1d(long long n, const Weights &w7, long long origin, long long elements,
-                                        const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st)
+cudaError_t launch_fp64_steps_tc_1d(long long n, const double *taps, int radius, const double *w, int steps,
+                                    long long origin, const double *in_base, double *out_base, const TcWait &wt,
+                                    cudaStream_t st)
 {
-    // Row r of the view starts at point origin - 4 + 64 r and is 72 points
-    // wide: its outputs (columns 4..67) are the interior points
-    // origin + 64 r .. + 63, and columns 0..3 and 68..71 their neighbours on
-    // either side. The kernel sees an R x 64 grid (pitch 64); rows of the view
-    // overlap by 8 points, which a tensor map cannot describe, so a tile loads
-    // the span of 71 array rows of 64 points (from origin - 4, not
-    // overlapping) that holds its 70 window rows, and the slicers read window
-    // row r at point 64 r of the span. The taps sit in row 3 of the 7x7, so
-    // the window's other rows meet zero weights. The last tile's span reaches
-    // array row R (points origin + n - 4 .. origin + n + 59), so the array
-    // holds 60 points after the interior; the map covers its whole rows.
-    if (n % TX != 0 || n < 8 * TX || origin < 4 || origin % 2 != 0 || elements < origin + n + 60 ||
-        reinterpret_cast<uintptr_t>(in_base) % 16 != 0 || reinterpret_cast<uintptr_t>(out_base) % 16 != 0)
-        return cudaErrorInvalidValue;
-    const long long rows = n / TX;
-    CUtensorMap map;
-    cudaError_t e = encode_split_window_map(&map, reinterpret_cast<const float2 *>(in_base + origin - 4), TX,
-                                            (elements - (origin - 4)) / TX, TX, kSpanRows);
+    if (steps < 1 || steps * radius > kReach1d || n < 64) return cudaErrorInvalidValue;
+    cudaError_t e = set_smem_attr<FmtF64, false, kMode1d>();
     if (e != cudaSuccess) return e;
-    if ((e = set_smem_attr<FmtF64, false, kModeRows1d>()) != cudaSuccess) return e;
-    const int tiles = (int)((rows + TY - 1) / TY);
-    const int grid = std::min(tiles, device_sm_count());
+    Weights wT;
+    for (int i = 0; i < 49; ++i) wT.v[i] = i <= 2 * kReach1d ? taps[i] : 0.0;
+    StepArgs sa{in_base + origin, steps, radius, 0, 0u, 0, {}};
+    sa.aligned = origin % 2 == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0 &&
+                 reinterpret_cast<uintptr_t>(out_base) % 16 == 0;
+    for (int t = 0; t <= 2 * radius; ++t) sa.w[t] = w[t];
+    CUtensorMap unused;
+    std::memset(&unused, 0, sizeof unused);
+    const int tiles = (int)((n + kOut1d - 1) / kOut1d);
     note_launch();
-    return launch_programmatic(k2d_tc<FmtF64, false, kModeRows1d>, grid, kThreads<FmtF64>, sizeof(Smem<FmtF64>) + 128, st,
-                               map, out_base + origin, (int)rows, TX, (long long)TX, 1, tiles, 0, 0,
-                               f64_slice_weights(w7), WaitCfg{wt.limit_ns, wt.skip_loads},
-                               static_cast<const TcGrid<FmtF64> *>(nullptr), 0, StepArgs{});
+    return launch_programmatic(k2d_tc<FmtF64, false, kMode1d>, std::min(tiles, device_sm_count()), kThreads<FmtF64>,
+                               sizeof(Smem<FmtF64>) + 128, st, unused, out_base + origin, 1, (int)n, 0LL, 1, tiles, 0,
+                               0, f64_slice_weights(wT, 49, true), WaitCfg{wt.limit_ns, wt.skip_loads},
+                               static_cast<const TcGrid<FmtF64> *>(nullptr), 0, sa);
 }
 
 size_t tc_batch_record_bytes(bool fp64) { return fp64 ? sizeof(TcGrid<FmtF64>) : sizeof(TcGrid<FmtSplit>); }

@@ -157,12 +157,6 @@ __device__ __forceinline__ void tmem_ld4(unsigned taddr, float (&v)[4])
 // x 2^-k, k >= 0 (the low bits lie far below the result's last one).
 __device__ __forceinline__ long long shift_down(long long x, int k) { return x >> min(k, 63); }
 
-// 8 bytes from global to shared memory, or zeros.
-__device__ __forceinline__ void cp_async8(unsigned dst, const double *src, bool take)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(take ? 8 : 0) : "memory");
-}
-
 template <bool TMA>
 __global__ void __launch_bounds__(kThreads, 1)
     k3d_tc_r3(const __grid_constant__ CUtensorMap tmap, const double *__restrict__ in, double *__restrict__ out, int h,

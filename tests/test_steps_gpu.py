@@ -113,3 +113,56 @@ def test_weights_out_of_range_keep_single_steps():
     assert p.time_block == 1
     ref = steps_of(np.pad(x, 1), np.zeros((514, 514)), w.reshape(3, 3), 3)
     assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+def steps_1d(a, b, w, steps):
+    """1D grids with halos of the radius, ping-pong; returns the interior."""
+    a, b = a.copy(), b.copy()
+    r = len(w) // 2
+    n = a.size - 2 * r
+    for _ in range(steps):
+        b[r:-r] = sum(w[t] * a[t:t + n] for t in range(2 * r + 1))
+        a, b = b, a
+    return a[r:-r]
+
+
+@pytest.mark.parametrize("shape,taps,fused", [("1d1r", 3, 0), ("1d2r", 5, 0), ("1d1r", 7, 1)])
+@pytest.mark.parametrize("n", [512, 4096, 4160, 8192, 64 * 1231])
+@pytest.mark.parametrize("steps", [1, 2, 5, 8, 15, 16, 50])
+def test_1d_steps_equal_single_steps(shape, taps, fused, n, steps):
+    w = O.seeded_weights(taps, 7 + taps) - 0.03
+    p = cs.Plan(shape, (n,), w, semantics=cs.Semantics.FUSED if fused else cs.Semantics.STEP)
+    p.set_option(cs.Option.ALGO, cs.Algo.FP64_TC)
+    r = taps // 2
+    x = O.splitmix_uniform(n, 5 + n) - 0.25
+    buf = p.pack(x)
+    got = run(p, buf, np.zeros_like(buf), steps * (3 if fused else 1))
+    assert p.algo == cs.Algo.FP64_TC and p.time_block == {1: 15, 2: 7, 3: 5, 4: 3}[r]
+    ref = steps_1d(np.pad(x, r), np.zeros(n + 2 * r), w, steps)
+    assert np.abs(p.unpack(got) - ref).max() <= TOL * np.abs(ref).max()
+    halo = np.ones(p.elements, bool)
+    halo[p.interior_index().reshape(-1)] = False
+    assert not got[halo].any(), "halo must stay zero"
+
+
+@pytest.mark.parametrize("shape,taps,fused", [("1d1r", 3, 0), ("1d2r", 5, 0), ("1d1r", 7, 1), ("1d2r", 9, 1)])
+@pytest.mark.parametrize("n,pad", [(300_001, 9), (300_032, 8), (262_143, 4)])
+def test_1d_layouts_halos_and_nothing_beyond(shape, taps, fused, n, pad):
+    """Caller layouts of odd and even origin, boundary values in both halos and
+    huge values past them (AUTO: the tuner picks the tensor cores here)."""
+    r = taps // 2
+    w = O.seeded_weights(taps, 11)
+    lay = {"dims": 1, "halo": r, "extent": [n], "pitch": [1], "origin": pad, "elements": n + 2 * pad}
+    p = cs.Plan(shape, (n,), w, semantics=cs.Semantics.FUSED if fused else cs.Semantics.STEP, layout=lay)
+    grids = []
+    for seed in (21, 22):
+        g = np.full(n + 2 * pad, 1e200)
+        g[pad - r:pad + n + r] = O.splitmix_uniform(n + 2 * r, seed)
+        grids.append(g)
+    inner = [g[pad - r:pad + n + r] for g in grids]
+    per = {"1d1r": 3, "1d2r": 2}[shape] if fused else 1
+    sweeps = 43
+    ref = steps_1d(inner[0], inner[1], w, sweeps)
+    got = run(p, grids[0], grids[1], sweeps * per)
+    assert p.algo == cs.Algo.FP64_TC and p.time_block == {1: 15, 2: 7, 3: 5, 4: 3}[r]
+    assert np.abs(got[pad:pad + n] - ref).max() <= TOL * np.abs(ref).max()

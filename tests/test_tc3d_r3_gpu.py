@@ -32,17 +32,17 @@ def params_of(shape, seed, signed=False):
 
 
 def steps_of(a, b, d, sweeps):
-    """Padded grids (halo 3), ping-pong; long double sums; the final interior."""
-    a, b = a.astype(np.longdouble), b.astype(np.longdouble)
+    """Padded grids (halo 3), ping-pong; the final interior."""
+    a, b = a.copy(), b.copy()
     n = [s - 6 for s in a.shape]
     for _ in range(sweeps):
-        acc = np.zeros(n, np.longdouble)
+        acc = np.zeros(n)
         for t in np.ndindex(7, 7, 7):
             if d[t] != 0.0:
-                acc += np.longdouble(d[t]) * a[t[0]:t[0] + n[0], t[1]:t[1] + n[1], t[2]:t[2] + n[2]]
+                acc += d[t] * a[t[0]:t[0] + n[0], t[1]:t[1] + n[1], t[2]:t[2] + n[2]]
         b[3:-3, 3:-3, 3:-3] = acc
         a, b = b, a
-    return a[3:-3, 3:-3, 3:-3].astype(np.float64)
+    return a[3:-3, 3:-3, 3:-3]
 
 
 def layout_ref(e):
