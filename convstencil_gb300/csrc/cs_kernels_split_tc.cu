@@ -165,10 +165,9 @@ struct Smem {
     unsigned long long acc_full[2], acc_empty[2];
     unsigned tmem;                             // TMEM base column
     int abort;                                 // set by the first expired wait
-    int wait_ok[2];                            // slicer leader's wait results
     int scale_exp[4];                          // per-tile input scale, ring of 4
-    float red[kSliceWarps];                    // split: per-warp max |hi|
-    int redi[kSliceWarps];                     // FP64: per-warp max biased exponent
+    float red[2][kSliceWarps];                 // split: per-warp max |hi|, by tile parity
+    int redi[2][kSliceWarps];                  // FP64: per-warp max biased exponent
 };
 
 static_assert(sizeof(Smem<FmtF64>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 128 <= 232448,
@@ -657,40 +656,47 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         const bool leader = st == 0;
         for (int it = 0; it < my_tiles; ++it) {
             const int buf = it & 1, use = it >> 1;
-            // (a) window landed? One thread waits, the barrier shares the answer.
-            if (leader) S.wait_ok[0] = wait(stage_full, it & 1);
-            asm volatile("bar.sync %0, %1;" ::"n"(kSliceBarrier), "n"(kSliceThreads) : "memory");
-            if (!S.wait_ok[0]) break;
+            // (a) window landed? Every thread waits for itself; one barrier
+            // per tile, at (c), makes them agree to go on. (Before, one thread
+            // waited and three barriers shared its answers and the maxima.
+            // GB300, launch before and after: 1d2r 10,240,000 66.9 and 55.8
+            // us, box2d1r 8192^2 three steps 381 and 359, box2d3r 8192^2
+            // split 305 and 295; FP64, bound by the MMAs, 335 and 338.)
+            const bool landed = wait(stage_full, it & 1);
             // (b) window -> registers, then release the stage to the next load.
+            if constexpr (STEPS) {
+                // Points past the halo of one meet zero weights in every output
+                // kept, but must not set the tile's scale either: tiles at the
+                // boundary first zero them in the stage (a thread the points
+                // that it reads next).
+                int g, x0, y0;
+                tile_at(it, g, x0, y0);
+                if (x0 == 0 || y0 == 0 || x0 + ST_X - 4 > n + 1 || y0 + ST_Y - 3 > m + 1) {
+#pragma unroll 1
+                    for (int idx = st; idx < kPairs; idx += kSliceThreads) {
+                        const int yy = y0 - 3 + idx / PAIRS, xx = x0 - 4 + 2 * (idx % PAIRS);
+                        const bool row = yy >= -1 && yy <= m;
+                        uint4 w = S.stage[idx];
+                        if (!row || xx < -1 || xx > n) w.x = w.y = 0u;
+                        if (!row || xx + 1 < -1 || xx + 1 > n) w.z = w.w = 0u;
+                        S.stage[idx] = w;
+                    }
+                }
+            }
             uint4 v[PER];
             float vmax = 0.f;   // split: largest |hi|
             unsigned emax = 0;  // FP64: largest biased exponent
-            int x0 = 0, y0 = 0;
-            bool edge = false;  // kModeSteps: the window reaches past the halo of one point
-            if constexpr (STEPS) {
-                int g;
-                tile_at(it, g, x0, y0);
-                edge = x0 == 0 || y0 == 0 || x0 + ST_X - 4 > n + 1 || y0 + ST_Y - 3 > m + 1;
-            }
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 const int idx = st + q * kSliceThreads;
-                v[q] = make_uint4(0u, 0u, 0u, 0u);
-                if (idx < kPairs) {
-                    v[q] = S.stage[idx];
-                    // Points past the halo meet zero weights in every output
-                    // kept, but must not set the tile's scale either.
-                    if (STEPS && edge) {
-                        const int yy = y0 - 3 + idx / PAIRS, xx = x0 - 4 + 2 * (idx % PAIRS);
-                        const bool row = yy >= -1 && yy <= m;
-                        if (!row || xx < -1 || xx > n) v[q].x = v[q].y = 0u;
-                        if (!row || xx + 1 < -1 || xx + 1 > n) v[q].z = v[q].w = 0u;
-                    }
-                    if constexpr (F::kF64)
-                        emax = max(emax, max((v[q].y >> 20) & 0x7FFu, (v[q].w >> 20) & 0x7FFu));
-                    else
-                        vmax = fmaxf(vmax, fmaxf(fabsf(__uint_as_float(v[q].x)), fabsf(__uint_as_float(v[q].z))));
-                }
+                v[q] = idx < kPairs ? S.stage[idx] : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                if constexpr (F::kF64)
+                    emax = max(emax, max((v[q].y >> 20) & 0x7FFu, (v[q].w >> 20) & 0x7FFu));
+                else
+                    vmax = fmaxf(vmax, fmaxf(fabsf(__uint_as_float(v[q].x)), fabsf(__uint_as_float(v[q].z))));
             }
             if constexpr (F::kF64) {
                 emax = __reduce_max_sync(0xffffffffu, emax);
@@ -701,48 +707,47 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             __syncwarp();
             if (lane == 0) {
                 if constexpr (F::kF64)
-                    S.redi[warp - kWarpSlice0] = (int)emax;
+                    S.redi[buf][warp - kWarpSlice0] = (int)emax;
                 else
-                    S.red[warp - kWarpSlice0] = vmax;
+                    S.red[buf][warp - kWarpSlice0] = vmax;
                 mbar_arrive(stage_empty);
             }
-            // (c) planes of this buffer free (MMAs two tiles back done)?
-            if (leader) S.wait_ok[1] = wait(bar2(S.planes_empty, buf), (use & 1) ^ 1);
-            asm volatile("bar.sync %0, %1;" ::"n"(kSliceBarrier), "n"(kSliceThreads) : "memory");
-            const bool go = S.wait_ok[1];
+            // (c) planes of this buffer free (MMAs two tiles back done)? The
+            // barrier also publishes the maxima; their next tile's are in the
+            // other set, and the one after that comes after its barrier.
+            const bool free = landed && wait(bar2(S.planes_empty, buf), (use & 1) ^ 1);
+            if (bar_any(kSliceBarrier, kSliceThreads, !free)) break;
             int ex;
             if constexpr (F::kF64) {
-                int eb = S.redi[0];
+                int eb = S.redi[buf][0];
 #pragma unroll
-                for (int i = 1; i < kSliceWarps; ++i) eb = max(eb, S.redi[i]);
+                for (int i = 1; i < kSliceWarps; ++i) eb = max(eb, S.redi[buf][i]);
                 ex = max(eb, 1);
             } else {
-                vmax = S.red[0];
+                vmax = S.red[buf][0];
 #pragma unroll
-                for (int i = 1; i < kSliceWarps; ++i) vmax = fmaxf(vmax, S.red[i]);
+                for (int i = 1; i < kSliceWarps; ++i) vmax = fmaxf(vmax, S.red[buf][i]);
                 ex = split::tile_exponent(vmax);
             }
-            // (d) every slicer has read wait_ok[1] and the maxima before they are reused
-            asm volatile("bar.sync %0, %1;" ::"n"(kSliceBarrier), "n"(kSliceThreads) : "memory");
-            if (!go) break;
             if (leader) S.scale_exp[it & 3] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
             unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[buf][0][0]);
             if constexpr (F::kF64) {
+                constexpr bool EVEN = STEPS || ONED;
+                // 1D: chunk idx / 4 in phase (idx / 4) % 4
+                auto word = [&](int idx) {
+                    return dst0 + (ONED ? (idx >> 2 & 3) * (kPhase1d / 4) + (idx >> 4) * 4 + (idx & 3) : idx);
+                };
+                if (ex >= kFastExp) {
 #pragma unroll
-                for (int q = 0; q < PER; ++q) {
-                    const int idx = st + q * kSliceThreads;
-                    if (idx < kPairs) {
-                        const unsigned long long ya = f64_biased_fixed<STEPS || ONED>(v[q].x, v[q].y, ex);
-                        const unsigned long long yb = f64_biased_fixed<STEPS || ONED>(v[q].z, v[q].w, ex);
-                        // 1D: chunk idx / 4 in phase (idx / 4) % 4
-                        unsigned *dst = dst0 + (ONED ? (idx >> 2 & 3) * (kPhase1d / 4) + (idx >> 4) * 4 + (idx & 3)
-                                                     : idx);
-                        dst[0 * (PL / 2)] = f64_digit_pair<0>(ya, yb);
-                        dst[1 * (PL / 2)] = f64_digit_pair<1>(ya, yb);
-                        dst[2 * (PL / 2)] = f64_digit_pair<2>(ya, yb);
-                        dst[3 * (PL / 2)] = f64_digit_pair<3>(ya, yb);
-                        dst[4 * (PL / 2)] = f64_digit_pair<4>(ya, yb);
-                        dst[5 * (PL / 2)] = f64_digit_pair<5>(ya, yb);
+                    for (int q = 0; q < PER; ++q) {
+                        const int idx = st + q * kSliceThreads;
+                        if (idx < kPairs) f64_cut_fast<EVEN, PL / 2>(v[q], ex, word(idx));
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < PER; ++q) {
+                        const int idx = st + q * kSliceThreads;
+                        if (idx < kPairs) f64_cut_any<EVEN, PL / 2>(v[q], ex, word(idx));
                     }
                 }
             } else {
@@ -823,17 +828,30 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar2(S.acc_empty, buf));
                 }
-                if constexpr (ONED) {
-                    // outputs 32 mrow + 8 rho .. + 7 of the tile
+                double res[8];
+                if constexpr (F::kF64) {
+                    // value = T 2^c with T from the levels (f64_combine) and
+                    // c = (input scale) + (weight scale) - 1080.
                     const int c = ex + ew - 1080;
-                    const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d + 32 * mrow + 8 * rho;
-                    double res[8];
+                    long long t[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const float lv[6] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4][j], acc[5][j]};
-                        res[j] = ex == kNonFiniteTile ? __longlong_as_double(0x7FF8000000000000ll)
-                                                      : f64_from_fixed(f64_combine(lv), c);
+                        t[j] = f64_combine(lv);
                     }
+                    if (f64_scale_is_plain(c)) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) res[j] = f64_from_fixed_plain(t[j], c);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            res[j] = ex == kNonFiniteTile ? __longlong_as_double(0x7FF8000000000000ll)
+                                                          : f64_from_fixed(t[j], c);
+                    }
+                }
+                if constexpr (ONED) {
+                    // outputs 32 mrow + 8 rho .. + 7 of the tile
+                    const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d + 32 * mrow + 8 * rho;
                     if (sa.aligned && x >= frame && x + 8 <= n - frame) {
 #pragma unroll
                         for (int j = 0; j < 8; j += 2)
@@ -849,16 +867,6 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 if (yy >= o_m) continue;
                 if (STEPS && (yy < frame || yy >= o_m - frame)) continue;
                 if constexpr (F::kF64) {
-                    // value = T 2^c with T from the levels (f64_combine) and
-                    // c = (input scale) + (weight scale) - 1080.
-                    const int c = ex + ew - 1080;
-                    double res[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float lv[6] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4][j], acc[5][j]};
-                        res[j] = ex == kNonFiniteTile ? __longlong_as_double(0x7FF8000000000000ll)
-                                                      : f64_from_fixed(f64_combine(lv), c);
-                    }
                     double *o = reinterpret_cast<double *>(o_base) + (long long)yy * o_ld + xb;
                     if (STEPS && (xb < frame || xb + 8 > o_n - frame)) {
 #pragma unroll

@@ -145,10 +145,9 @@ struct Smem {
     unsigned long long blk_full[F::NBLK], blk_empty[F::NBLK];
     unsigned tmem;                             // TMEM base column
     int abort;                                 // set by the first expired wait
-    int wait_ok[kGroups][2];                   // slicer group leaders' wait results
     int scale_exp[kScaleRing];                 // input-plane scale exponents by plane sequence
-    float red[kGroups][kGroupWarps];           // split: per-warp max |hi|
-    int redi[kGroups][kGroupWarps];            // FP64: per-warp max biased exponent
+    float red[kGroups][2][kGroupWarps];           // split: per-warp max |hi|
+    int redi[kGroups][2][kGroupWarps];            // FP64: per-warp max biased exponent
 };
 static_assert(sizeof(Smem<F3F64>) + 128 <= 232448 && sizeof(Smem<F3Split>) + 128 <= 232448,
               "shared memory of one CTA must stay within 227 KB");
@@ -332,13 +331,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int p = 0; p < wi.zn + 2; ++p, ++q) {
                 if (q % kGroups != grp) continue;
                 const int sb = q % kStages, slot = q % NPL;
-                // (a) window landed? One thread waits, the barrier shares the answer.
-                if (leader) S.wait_ok[grp][0] = wait(bar(S.stage_full, sb), (q / kStages) & 1);
-                asm volatile("bar.sync %0, %1;" ::"r"(kSliceBarrier + grp), "n"(kGroupThreads) : "memory");
-                if (!S.wait_ok[grp][0]) {
-                    go = false;
-                    break;
-                }
+                // (a) window landed? Every thread waits for itself; one barrier
+                // per plane, at (c), makes the group agree to go on.
+                const bool landed = wait(bar(S.stage_full, sb), (q / kStages) & 1);
+                const int set = (q / kGroups) & 1;
                 // (b) window -> registers, then release the stage to the next load.
                 const uint4 *stg = S.stage[sb];
                 uint4 v[PER];
@@ -365,47 +361,45 @@ __global__ void __launch_bounds__(kThreads, 1)
                 __syncwarp();
                 if (lane == 0) {
                     if constexpr (F::kF64)
-                        S.redi[grp][gw] = (int)emax;
+                        S.redi[grp][set][gw] = (int)emax;
                     else
-                        S.red[grp][gw] = vmax;
+                        S.red[grp][set][gw] = vmax;
                     mbar_arrive(bar(S.stage_empty, sb));
                 }
                 // (c) digit-plane set free (the MMAs that read it are done)?
-                if (leader) S.wait_ok[grp][1] = wait(bar(S.planes_empty, slot), ((q / NPL) & 1) ^ 1);
-                asm volatile("bar.sync %0, %1;" ::"r"(kSliceBarrier + grp), "n"(kGroupThreads) : "memory");
-                go = S.wait_ok[grp][1];
+                // The barrier also publishes the maxima; the group's next
+                // plane's are in the other set.
+                const bool free = landed && wait(bar(S.planes_empty, slot), ((q / NPL) & 1) ^ 1);
+                go = !bar_any(kSliceBarrier + grp, kGroupThreads, !free);
+                if (!go) break;
                 int ex;
                 if constexpr (F::kF64) {
-                    int eb = S.redi[grp][0];
+                    int eb = S.redi[grp][set][0];
 #pragma unroll
-                    for (int i = 1; i < kGroupWarps; ++i) eb = max(eb, S.redi[grp][i]);
+                    for (int i = 1; i < kGroupWarps; ++i) eb = max(eb, S.redi[grp][set][i]);
                     ex = max(eb, 1);
                 } else {
-                    vmax = S.red[grp][0];
+                    vmax = S.red[grp][set][0];
 #pragma unroll
-                    for (int i = 1; i < kGroupWarps; ++i) vmax = fmaxf(vmax, S.red[grp][i]);
+                    for (int i = 1; i < kGroupWarps; ++i) vmax = fmaxf(vmax, S.red[grp][set][i]);
                     ex = split::tile_exponent(vmax);
                 }
-                // (d) every slicer of the group has read wait_ok and the maxima before they are reused
-                asm volatile("bar.sync %0, %1;" ::"r"(kSliceBarrier + grp), "n"(kGroupThreads) : "memory");
-                if (!go) break;
                 if (leader) S.scale_exp[q % kScaleRing] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
                 unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[slot][0][0]);
                 if constexpr (F::kF64) {
+                    if (ex >= kFastExp) {
 #pragma unroll
-                    for (int k = 0; k < PER; ++k) {
-                        const int u = st + k * kGroupThreads;
-                        if (u < NCUT) {
-                            const int idx = (u / NCUTX) * PAIRS + CUT0 + u % NCUTX;
-                            const unsigned long long ya = f64_biased_fixed(v[k].x, v[k].y, ex);
-                            const unsigned long long yb = f64_biased_fixed(v[k].z, v[k].w, ex);
-                            unsigned *dst = dst0 + idx;
-                            dst[0 * (PL / 2)] = f64_digit_pair<0>(ya, yb);
-                            dst[1 * (PL / 2)] = f64_digit_pair<1>(ya, yb);
-                            dst[2 * (PL / 2)] = f64_digit_pair<2>(ya, yb);
-                            dst[3 * (PL / 2)] = f64_digit_pair<3>(ya, yb);
-                            dst[4 * (PL / 2)] = f64_digit_pair<4>(ya, yb);
-                            dst[5 * (PL / 2)] = f64_digit_pair<5>(ya, yb);
+                        for (int k = 0; k < PER; ++k) {
+                            const int u = st + k * kGroupThreads;
+                            if (u < NCUT)
+                                f64_cut_fast<false, PL / 2>(v[k], ex, dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX);
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < PER; ++k) {
+                            const int u = st + k * kGroupThreads;
+                            if (u < NCUT)
+                                f64_cut_any<false, PL / 2>(v[k], ex, dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX);
                         }
                     }
                 } else {
@@ -510,11 +504,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                     add_part(a, ea, fa, na, acc, ex);
                     if (yy < m) {
                         double res[4];
+                        const int sc = ea + ew - 1080;
+                        if (!na && !fa && f64_scale_is_plain(sc)) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            res[c] = na ? __longlong_as_double(0x7FF8000000000000ll)
-                                 : fa ? __longlong_as_double(a[c])
-                                      : f64_from_fixed(a[c], ea + ew - 1080);
+                            for (int c = 0; c < 4; ++c) res[c] = f64_from_fixed_plain(a[c], sc);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 4; ++c)
+                                res[c] = na ? __longlong_as_double(0x7FF8000000000000ll)
+                                     : fa ? __longlong_as_double(a[c])
+                                          : f64_from_fixed(a[c], sc);
+                        }
                         double *op = out + (long long)(wi.zs + p - 2) * ldz + (long long)yy * ldy + xb;
 #pragma unroll
                         for (int c = 0; c < 4; c += 2) {

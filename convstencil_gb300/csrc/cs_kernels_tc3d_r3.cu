@@ -111,9 +111,8 @@ struct Smem {
     unsigned long long blk_full[2], blk_empty[2];
     unsigned tmem;
     int abort;
-    int wait_ok[kGroups][2];
     int scale_exp[kScaleRing];
-    int redi[kGroups][kGroupWarps];
+    int redi[kGroups][2][kGroupWarps];
 };
 static_assert(sizeof(Smem) + 128 <= 232448, "shared memory of one CTA must stay within 227 KB");
 static_assert(D * 49 * kWz * 2 <= (int)sizeof(Smem::planes), "the staged weights fit the digit planes");
@@ -316,13 +315,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int p = 0; p < wi.zn + 6; ++p, ++q) {
                 if (q % kGroups != grp) continue;
                 const int sb = q % kStages, slot = q % NPL;
-                // (a) window landed? One thread waits, the barrier shares the answer.
-                if (leader) S.wait_ok[grp][0] = wait(bar(S.stage_full, sb), (q / kStages) & 1);
-                asm volatile("bar.sync %0, %1;" ::"r"(kSliceBarrier + grp), "n"(kGroupThreads) : "memory");
-                if (!S.wait_ok[grp][0]) {
-                    go = false;
-                    break;
-                }
+                // (a) window landed? Every thread waits for itself; one barrier
+                // per plane, at (c), makes the group agree to go on.
+                const bool landed = wait(bar(S.stage_full, sb), (q / kStages) & 1);
+                const int set = (q / kGroups) & 1;
                 // (b) window -> registers, then release the stage to the next load.
                 const uint4 *stg = S.stage[sb];
                 uint4 v[PER];
@@ -345,34 +341,31 @@ __global__ void __launch_bounds__(kThreads, 1)
                 emax = __reduce_max_sync(0xffffffffu, emax);
                 __syncwarp();
                 if (lane == 0) {
-                    S.redi[grp][gw] = (int)emax;
+                    S.redi[grp][set][gw] = (int)emax;
                     mbar_arrive(bar(S.stage_empty, sb));
                 }
                 // (c) digit-plane set free (the MMAs that read it are done)?
-                if (leader) S.wait_ok[grp][1] = wait(bar(S.planes_empty, slot), ((q / NPL) & 1) ^ 1);
-                asm volatile("bar.sync %0, %1;" ::"r"(kSliceBarrier + grp), "n"(kGroupThreads) : "memory");
-                go = S.wait_ok[grp][1];
+                // The barrier also publishes the maxima; the group's next
+                // plane's are in the other set.
+                const bool free = landed && wait(bar(S.planes_empty, slot), ((q / NPL) & 1) ^ 1);
+                go = !bar_any(kSliceBarrier + grp, kGroupThreads, !free);
+                if (!go) break;
                 int ex = 1;
 #pragma unroll
-                for (int i = 0; i < kGroupWarps; ++i) ex = max(ex, S.redi[grp][i]);
-                // (d) every slicer of the group has read wait_ok and the maxima before they are reused
-                asm volatile("bar.sync %0, %1;" ::"r"(kSliceBarrier + grp), "n"(kGroupThreads) : "memory");
-                if (!go) break;
+                for (int i = 0; i < kGroupWarps; ++i) ex = max(ex, S.redi[grp][set][i]);
                 if (leader) S.scale_exp[q % kScaleRing] = ex == 2047 ? kNonFiniteTile : ex;
                 unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[slot][0][0]);
+                if (ex >= kFastExp) {
 #pragma unroll
-                for (int k = 0; k < PER; ++k) {
-                    const int u = st + k * kGroupThreads;
-                    if (u < NPAIR) {
-                        const unsigned long long ya = f64_biased_fixed<true>(v[k].x, v[k].y, ex);
-                        const unsigned long long yb = f64_biased_fixed<true>(v[k].z, v[k].w, ex);
-                        unsigned *dst = dst0 + u;
-                        dst[0 * (PL / 2)] = f64_digit_pair<0>(ya, yb);
-                        dst[1 * (PL / 2)] = f64_digit_pair<1>(ya, yb);
-                        dst[2 * (PL / 2)] = f64_digit_pair<2>(ya, yb);
-                        dst[3 * (PL / 2)] = f64_digit_pair<3>(ya, yb);
-                        dst[4 * (PL / 2)] = f64_digit_pair<4>(ya, yb);
-                        dst[5 * (PL / 2)] = f64_digit_pair<5>(ya, yb);
+                    for (int k = 0; k < PER; ++k) {
+                        const int u = st + k * kGroupThreads;
+                        if (u < NPAIR) f64_cut_fast<true, PL / 2>(v[k], ex, dst0 + u);
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) {
+                        const int u = st + k * kGroupThreads;
+                        if (u < NPAIR) f64_cut_any<true, PL / 2>(v[k], ex, dst0 + u);
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -457,10 +450,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!ok) break;
                 if (p >= 6 && yy < m) {  // output p - 6 of the column has all its taps
                     double res[4];
+                    const int sc = se[6] + sw.ew - 1080;
+                    if (!(bad & 0x7Fu) && f64_scale_is_plain(sc)) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        res[c] = (bad & 0x7Fu) ? __longlong_as_double(0x7FF8000000000000ll)
-                                               : f64_from_fixed(s[6][c], se[6] + sw.ew - 1080);
+                        for (int c = 0; c < 4; ++c) res[c] = f64_from_fixed_plain(s[6][c], sc);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            res[c] = (bad & 0x7Fu) ? __longlong_as_double(0x7FF8000000000000ll)
+                                                   : f64_from_fixed(s[6][c], sc);
+                    }
                     if (vec2 && xb + 3 < n) {
                         *reinterpret_cast<double2 *>(op) = make_double2(res[0], res[1]);
                         *reinterpret_cast<double2 *>(op + 2) = make_double2(res[2], res[3]);

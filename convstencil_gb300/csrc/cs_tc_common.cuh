@@ -133,6 +133,21 @@ __device__ __forceinline__ void mbar_arrive(unsigned bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// Named barrier of `threads` threads that also tells all of them whether any
+// came with `fail` set: a role whose threads wait on mbarriers one by one
+// decides with it, the same way in all of them, whether to go on.
+__device__ __forceinline__ bool bar_any(int id, int threads, bool fail)
+{
+    unsigned any;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %3, 0;\n"
+        " barrier.cta.red.or.pred.aligned q, %1, %2, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(any)
+        : "r"(id), "r"(threads), "r"((unsigned)fail)
+        : "memory");
+    return any != 0;
+}
+
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));

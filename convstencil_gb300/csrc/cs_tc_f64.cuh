@@ -86,6 +86,23 @@ __device__ __forceinline__ unsigned long long f64_biased_fixed(unsigned lo, unsi
     return (kF64Bias - neg) + (x ^ neg);  // kF64Bias + x, or kF64Bias - x = (kF64Bias + 1) + ~x
 }
 
+// The same for tiles whose largest biased exponent is at least kFastExp (all
+// but tiles of values below 2^-895): a zero or subnormal then shifts out
+// whether or not it is given the implicit bit, so neither needs a test, and
+// PTX defines a shift by more than 63 (C++ does not).
+constexpr int kFastExp = 128;
+template <bool EVEN = false>
+__device__ __forceinline__ unsigned long long f64_biased_fixed_fast(unsigned lo, unsigned hi, int eb1)
+{
+    const int sh = eb1 - (int)((hi >> 20) & 0x7FFu);
+    const unsigned long long mant = ((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+    unsigned long long t;
+    asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(mant), "r"(sh));
+    const unsigned up = EVEN ? (((unsigned)t & 2u) | (unsigned)sh) != 0u : 1u;
+    const unsigned long long x = (t + up) >> 1;
+    return (int)hi < 0 ? kF64Bias - x : kF64Bias + x;
+}
+
 // Digit k (0 = most significant) of two biased words, as an FP16 pair:
 // FP16 (1024 + u) has the bits 0x6400 | u, and (1024 + u) - 1280 = u - 256
 // is exact in FP16. (The top field is at most 384, so masking it is harmless.)
@@ -163,6 +180,42 @@ __device__ __forceinline__ double f64_from_fixed(long long t, int c)
     if (e == 0) return d;  // t == 0
     if (ne >= 1 && ne <= 2046) return __longlong_as_double(bits + ((long long)c << 52));
     return f64_from_fixed_rare(t, c);
+}
+
+// Whether every T != 0 times 2^c is a normal number (|T| < 2^63), and then its
+// value: no range tests per output.
+__device__ __forceinline__ bool f64_scale_is_plain(int c) { return c >= -1022 && c <= 960; }
+__device__ __forceinline__ double f64_from_fixed_plain(long long t, int c)
+{
+    const double d = __ll2double_rn(t);
+    const int hi = __double2hiint(d);
+    return __hiloint2double(hi != 0 ? hi + (c << 20) : 0, __double2loint(d));
+}
+
+// Cuts one pair of points (v: lo, hi words of both) into six digit planes
+// PW words apart.
+template <int PW>
+__device__ __forceinline__ void f64_cut_pair(unsigned long long ya, unsigned long long yb, unsigned *dst)
+{
+    dst[0 * PW] = f64_digit_pair<0>(ya, yb);
+    dst[1 * PW] = f64_digit_pair<1>(ya, yb);
+    dst[2 * PW] = f64_digit_pair<2>(ya, yb);
+    dst[3 * PW] = f64_digit_pair<3>(ya, yb);
+    dst[4 * PW] = f64_digit_pair<4>(ya, yb);
+    dst[5 * PW] = f64_digit_pair<5>(ya, yb);
+}
+template <bool EVEN, int PW>
+__device__ __forceinline__ void f64_cut_fast(const uint4 &v, int ex, unsigned *dst)
+{
+    f64_cut_pair<PW>(f64_biased_fixed_fast<EVEN>(v.x, v.y, ex), f64_biased_fixed_fast<EVEN>(v.z, v.w, ex), dst);
+}
+// Tiles of tiny values. (Inline although rare: as a call it made the compiler
+// keep the cutting loop's values where a call leaves them; the 3D radius-3
+// sweep took 586 us on 256^3, GB300, against 539 so.)
+template <bool EVEN, int PW>
+__device__ __forceinline__ void f64_cut_any(const uint4 &v, int ex, unsigned *dst)
+{
+    f64_cut_pair<PW>(f64_biased_fixed<EVEN>(v.x, v.y, ex), f64_biased_fixed<EVEN>(v.z, v.w, ex), dst);
 }
 
 // Marks a tile whose window holds an Inf or NaN (its outputs become NaN).
