@@ -260,7 +260,7 @@ std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int, int>, int> g_tune;      // -> algorithm
 std::map<std::tuple<int, int, int, int, int>, int> g_tune_tb;   // -> steps per launch (split FMA)
 std::map<std::tuple<int, int, int, int, int>, int> g_tune_rows; // -> FP64 FMA 2D tile rows
-// -> time of one sweep of the chosen algorithm and of one launch of several steps (FP64)
+// -> time of one launch of the chosen algorithm and of one tcgen05 launch of several steps
 std::map<std::tuple<int, int, int, int, int>, std::pair<float, float>> g_tune_steps;
 
 }  // namespace
@@ -272,9 +272,9 @@ struct cs_plan {
     int dims, radius, pattern, steps_per_sweep;
     Weights w;
     Weights w7;  // 2D plans: w at the centre of a 7x7 (the 2D tcgen05 kernels' tap window)
-    // Kernels of several steps: FP64 2D radius-1 plans, the 7x7 ones of 1, 2 and
-    // 3 (launch_fp64_steps_tc); 1D plans, the 33 taps of 1 .. 16 / radius
-    // (launch_fp64_steps_tc_1d).
+    // Kernels of several steps: 2D radius-1 plans, the 7x7 ones of 1, 2 and 3
+    // (launch_steps_tc); 1D plans, the 33 taps of 1 .. 16 / radius
+    // (launch_steps_tc_1d).
     Weights w_steps[3];
     double w1_steps[16][33];
     int max_steps = 0;  // steps per launch those allow (0: not even one)
@@ -383,7 +383,7 @@ bool fp64_tc3d_r3_ok(const cs_plan *p)
 }
 
 // FP64 1D plans on the tcgen05 digit kernel (rows of 32 outputs, a reach of
-// 16 points: launch_fp64_steps_tc_1d), whatever their layout. Pinning FP64_TC
+// 16 points: launch_steps_tc_1d), whatever their layout. Pinning FP64_TC
 // keeps the conditions it had (fp64_tc1d_pin_ok); the tuner's candidate needs
 // no more than room for both ends of the grid.
 bool fp64_tc1d_geometry_ok(const cs_plan *p) { return p->dims == 1 && p->view.ext[0] >= 512 && p->max_steps >= 1; }
@@ -402,30 +402,32 @@ bool split_tc3d_ok(const cs_plan *p)
 }
 
 // Steps per launch of the tcgen05 digit kernel on this plan and these
-// buffers: 3 for FP64 2D radius-1 plans (three steps of a 3x3 kernel are one
-// 7x7 kernel, the kernel's tap window) from 64 tiles up. Smaller grids leave
-// most SMs without a tile, and a launch of ~12 us loses to single steps on
-// the FP64 FMA kernel (512^2, 64 tiles, is where three of those take as long).
-// FP64 1D plans take the most steps, an odd number, that reach at most 16
-// points, at any size.
-int fp64_steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base)
+// buffers. 2D radius-1 plans: 3 (three steps of a 3x3 kernel are one 7x7
+// kernel, the kernel's tap window) from 64 tiles up; smaller grids leave most
+// SMs without a tile, and a launch of ~12 us loses to single steps (FP64 FMA;
+// 512^2, 64 tiles, is where three of those take as long) or to the
+// double-float kernel's four per launch. 1D plans: the most steps, an odd
+// number, that reach at most 16 points, FP64 at any size (the tuner decides),
+// split from 64 tiles of 4096 points up.
+int steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base)
 {
-    if (p->dims == 1) return fp64_tc1d_ok(p) ? p->max_steps : 1;
-    if (p->max_steps < 2 || !fp64_tc_ok(p) || !fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base))
+    const bool fp64 = p->prec == CS_PREC_FP64;
+    if (p->dims == 1) return fp64_tc1d_geometry_ok(p) && (fp64 || p->view.ext[0] > 63 * 4096) ? p->max_steps : 1;
+    if (p->max_steps < 2 || !fp64_tc_geometry_ok(p) ||
+        !fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base))
         return 1;
     const long long tiles = ((p->view.ext[0] + 63) / 64) * ((p->view.ext[1] + 63) / 64);
     return tiles >= 64 ? p->max_steps : 1;
 }
 
-// `steps` (1 .. fp64_steps_per_launch) steps in one launch.
-cudaError_t launch_steps(const cs_plan *p, int steps, const void *in_base, void *out_base, cudaStream_t st)
+// `steps` (1 .. steps_per_launch) steps in one launch, on FP64 or split grids.
+cudaError_t launch_steps(const cs_plan *p, bool fp64, int steps, const void *in_base, void *out_base, cudaStream_t st)
 {
     if (p->dims == 1)
-        return cs::launch_fp64_steps_tc_1d(p->view.ext[0], p->w1_steps[steps - 1], p->radius, p->w.v, steps,
-                                           p->layout.origin, (const double *)in_base, (double *)out_base, p->wait,
-                                           st);
-    return cs::launch_fp64_steps_tc(p->view, p->w_steps[steps - 1], p->w, steps, p->layout.origin,
-                                    p->layout.elements, (const double *)in_base, (double *)out_base, p->wait, st);
+        return cs::launch_steps_tc_1d(fp64, p->view.ext[0], p->w1_steps[steps - 1], p->radius, p->w.v, steps,
+                                      p->layout.origin, in_base, out_base, p->wait, st);
+    return cs::launch_steps_tc(fp64, p->view, p->w_steps[steps - 1], p->w, steps, p->layout.origin,
+                               p->layout.elements, in_base, out_base, p->wait, st);
 }
 
 // One sweep over the slabs [row0, row0 + rows) of the slowest axis (rows of
@@ -444,7 +446,7 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
         double *out = (double *)out_base + off;
         if (algo == CS_ALGO_FP64_MMA) return cs::launch_fp64_mma_2d(v, p->w, in, out, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc1d_ok(p) && row0 == 0 && rows == p->view.ext[0])
-            return launch_steps(p, 1, in_base, out_base, st);
+            return launch_steps(p, true, 1, in_base, out_base, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc3d_ok(p) && cs::split_tc3d_layout_ok(v, off, in_base, out_base))
             return cs::launch_fp64_sweep_tc3d(v, p->w, off, p->layout.elements, (const double *)in_base,
                                               (double *)out_base, p->wait, st);
@@ -642,17 +644,18 @@ cs_status choose_time_block(cs_plan *p, int algo, const void *a, void *b, cudaSt
     return CS_OK;
 }
 
-// Whether a run of `sweeps` sweeps takes several steps per launch, and then
-// how many (*steps) and the kernel (*algo). Always when FP64_TC is pinned;
-// with AUTO where the time of ceil(sweeps / steps) such launches, measured
-// once per class of plan beside single sweeps of the chosen algorithm
-// (two launches, six sweeps, a -> b), is the shorter one. A caller that is capturing
-// its stream gets what is already known.
-cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long long sweeps, int *algo, int *steps)
+// Whether a run of `sweeps` sweeps goes to the tcgen05 launches of several
+// steps (*steps > 0: how many each). Always when FP64_TC is pinned; with
+// nothing pinned where ceil(sweeps / steps) of them take less time than the
+// chosen algorithm's launches of tb sweeps, both measured once per class of
+// plan (a -> b). A caller that is capturing its stream gets what is known.
+cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long long sweeps, int algo, int tb,
+                       int *steps)
 {
-    *steps = 1;
-    const int t = fp64_steps_per_launch(p, a, b);
-    if (t < 2 || (p->algo != CS_ALGO_AUTO && p->algo != CS_ALGO_FP64_TC)) return CS_OK;
+    *steps = 0;
+    const bool fp64 = p->prec == CS_PREC_FP64;
+    const int t = steps_per_launch(p, a, b);
+    if (t < 2 || (p->algo != CS_ALGO_AUTO && p->algo != CS_ALGO_FP64_TC) || p->time_block > 0) return CS_OK;
     if (p->algo == CS_ALGO_FP64_TC) {
         *steps = t;
         return CS_OK;
@@ -668,28 +671,33 @@ cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         CS_CUDA(cudaStreamIsCapturing(st, &cap));
         if (cap != cudaStreamCaptureStatusNone) return CS_OK;
+        const int reps = 4;
         cudaEvent_t e[3];
         for (auto &x : e) CS_CUDA(cudaEventCreate(&x));
         for (int rep = 0; rep < 2; ++rep) {  // rep 0 warms up
             CS_CUDA(cudaEventRecord(e[0], st));
-            for (int i = 0; i < 6; ++i) CS_CUDA(launch_sweep(p, *algo, a, b, st));
+            for (int i = 0; i < reps; ++i) {
+                if (tb >= 2)
+                    CS_CUDA(cs::launch_split_sweep_tb(p->view, p->radius, p->pattern, tb, p->w,
+                                                      (const float2 *)a + p->layout.origin,
+                                                      (float2 *)b + p->layout.origin, st));
+                else
+                    CS_CUDA(launch_sweep(p, algo, a, b, st));
+            }
             CS_CUDA(cudaEventRecord(e[1], st));
-            for (int i = 0; i < 2; ++i) CS_CUDA(launch_steps(p, t, a, b, st));
+            for (int i = 0; i < reps; ++i) CS_CUDA(launch_steps(p, fp64, t, a, b, st));
             CS_CUDA(cudaEventRecord(e[2], st));
             CS_CUDA(cudaEventSynchronize(e[2]));
         }
         CS_CUDA(cudaEventElapsedTime(&ms.first, e[0], e[1]));
         CS_CUDA(cudaEventElapsedTime(&ms.second, e[1], e[2]));
         for (auto &x : e) cudaEventDestroy(x);
-        ms.first /= 6;
-        ms.second /= 2;
+        ms.first /= reps;
+        ms.second /= reps;
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune_steps[key] = ms;
     }
-    if (sweeps > 1 && ms.second * (float)((sweeps + t - 1) / t) < ms.first * (float)sweeps) {
-        *steps = t;
-        *algo = CS_ALGO_FP64_TC;
-    }
+    if (ms.second * (float)((sweeps + t - 1) / t) < ms.first * (float)((sweeps + tb - 1) / tb)) *steps = t;
     return CS_OK;
 }
 
@@ -763,7 +771,7 @@ cudaError_t fp64_anchor_sweep_fp64_in(const cs_plan *p, const void *src, void *d
         return launch_fp64_sweep_tc(p->view, p->w7, off, n, (const double *)src, (double *)dst, p->wait, st);
     if (fp64_tc3d_geometry_ok(p) && split_tc3d_layout_ok(p->view, off, src, dst))
         return launch_fp64_sweep_tc3d(p->view, p->w, off, n, (const double *)src, (double *)dst, p->wait, st);
-    if (fp64_tc1d_geometry_ok(p)) return launch_steps(p, 1, src, dst, st);
+    if (fp64_tc1d_geometry_ok(p)) return launch_steps(p, true, 1, src, dst, st);
     return launch_fp64_fma(p->view, p->radius, p->pattern, p->w, (const double *)src + off, (double *)dst + off, st);
 }
 
@@ -789,15 +797,17 @@ cs_status run_from(cs_plan *p, void *a, void *b, long long first_sweep, long lon
     long long sweeps = 0;
     cs_status s = cs_plan_sweeps(p, steps, &sweeps);
     if (s != CS_OK) return s;
-    int algo = CS_ALGO_FP64_FMA, tb = 1;
+    int algo = CS_ALGO_FP64_FMA, tb = 1, multi = 0;
     if (sweeps > 0) {
         s = choose_algo(p, a, b, st, &algo);
         if (s != CS_OK) return s;
         s = choose_time_block(p, algo, a, b, st, &tb);
         if (s != CS_OK) return s;
-        if (p->prec == CS_PREC_FP64) {
-            s = choose_steps(p, a, b, st, sweeps, &algo, &tb);
-            if (s != CS_OK) return s;
+        s = choose_steps(p, a, b, st, sweeps, algo, tb, &multi);
+        if (s != CS_OK) return s;
+        if (multi > 0) {
+            algo = p->prec == CS_PREC_FP64 ? CS_ALGO_FP64_TC : CS_ALGO_SPLIT_TC;
+            tb = multi;
         }
         int rows = 0;
         s = choose_tile_rows(p, algo, a, b, st, &rows);
@@ -811,7 +821,7 @@ cs_status run_from(cs_plan *p, void *a, void *b, long long first_sweep, long lon
     const long long off = p->layout.origin;
     // One launch of t sweeps from buf[c] to buf[c ^ 1] on stream `on`.
     auto one_launch = [&](int t, int c, cudaStream_t on) -> cudaError_t {
-        if (p->prec == CS_PREC_FP64 && tb >= 2) return launch_steps(p, t, buf[c], buf[c ^ 1], on);
+        if (multi > 0) return launch_steps(p, p->prec == CS_PREC_FP64, t, buf[c], buf[c ^ 1], on);
         if (t >= 2)
             return cs::launch_split_sweep_tb(p->view, p->radius, p->pattern, t, p->w,
                                              (const float2 *)buf[c] + off, (float2 *)buf[c ^ 1] + off, on);
@@ -985,7 +995,7 @@ CS_API cs_status cs_plan_create(cs_plan **out, cs_shape shape, cs_semantics sem,
         for (int i = 0; i < k; ++i)
             for (int j = 0; j < k; ++j) p->w7.v[(i + o) * 7 + j + o] = p->w.v[i * k + j];
     }
-    if (prec == CS_PREC_FP64 && p->dims == 2 && p->radius == 1) {
+    if (p->dims == 2 && p->radius == 1) {
         bool ok = true;
         for (int t = 1; t <= 3; ++t) {
             memset(p->w_steps[t - 1].v, 0, sizeof p->w_steps[t - 1].v);

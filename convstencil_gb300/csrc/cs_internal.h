@@ -81,11 +81,11 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
                                  const double *in_base, double *out_base, const TcWait &wait,
                                  cudaStream_t stream);
-// `steps` (1..3) steps of a 2D radius-1 FP64 grid in one launch: wT is the
-// 7x7 kernel of that many steps (selfconv7), w3x3 the weights of one.
-cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
-                                 long long origin, long long elements, const double *in_base, double *out_base,
-                                 const TcWait &wait, cudaStream_t stream);
+// `steps` (1..3) steps of a 2D radius-1 grid (FP64 or split) in one launch: wT
+// is the 7x7 kernel of that many steps, w3x3 the weights of one.
+cudaError_t launch_steps_tc(bool fp64, const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
+                            long long origin, long long elements, const void *in_base, void *out_base,
+                            const TcWait &wait, cudaStream_t stream);
 // Batches of 2D radius-3 grids on the tcgen05 kernels (split or FP64): one
 // device record per grid (tc_batch_record_bytes each, 128-byte aligned)
 // holding its tensor map over `in_base`, output, sizes, first tile and
@@ -102,13 +102,14 @@ cudaError_t launch_tc_batch(bool fp64, const void *records, int ngrids, int tota
 // 2D tensor map over a whole (hi, lo) buffer of `rows` x `ld` pairs, box_x x box_y tiles.
 cudaError_t encode_split_window_map(CUtensorMap *map, const float2 *base, long long ld, long long rows,
                                     unsigned box_x, unsigned box_y);
-// `steps` steps of a 1D FP64 grid of n >= 64 points in one launch of the
-// tcgen05 digit kernel, steps * radius <= kTcReach1d: taps are the 33 taps of
-// that many steps (the output's own at 16), w the 2 radius + 1 weights of one.
+// `steps` steps of a 1D grid (FP64 or split) of n >= 64 points in one launch
+// of the tcgen05 digit kernel, steps * radius <= kTcReach1d: taps are the 33
+// taps of that many steps (the output's own at 16), w the 2 radius + 1 weights
+// of one.
 constexpr int kTcReach1d = 16;
-cudaError_t launch_fp64_steps_tc_1d(long long n, const double *taps, int radius, const double *w, int steps,
-                                    long long origin, const double *in_base, double *out_base, const TcWait &wait,
-                                    cudaStream_t stream);
+cudaError_t launch_steps_tc_1d(bool fp64, long long n, const double *taps, int radius, const double *w, int steps,
+                               long long origin, const void *in_base, void *out_base, const TcWait &wait,
+                               cudaStream_t stream);
 // 3D tensor map: `planes` planes of pitch ldz, rows of pitch ld; box
 // box_x x box_y x 1.
 cudaError_t encode_split_window_map_3d(CUtensorMap *map, const float2 *base, long long ld, long long ldz,

@@ -65,6 +65,7 @@
 // leaves.
 #include "cs_internal.h"
 #include "cs_split_common.cuh"
+#include "cs_split_ff.cuh"
 #include "cs_tc_common.cuh"
 #include "cs_tc_f64.cuh"
 
@@ -99,6 +100,18 @@ struct FmtSplit {
     static constexpr int kEpiWarps = 4;
     using Out = float2;
     using Digits = split::SliceWeights;
+};
+
+// Split grids cut into six digits, for launches of several steps (radius-1 and
+// 1D stencils, whose single steps run in double-float arithmetic): the input
+// pairs keep 52 bits below their tile's largest value, more than the (hi, lo)
+// format holds, so a launch's error is the rounding of its results to pairs.
+struct FmtSplit6 {
+    static constexpr bool kF64 = false;
+    static constexpr int kDigits = 6;
+    static constexpr int kEpiWarps = 4;
+    using Out = float2;
+    using Digits = F64Weights;
 };
 
 struct FmtF64 {
@@ -170,7 +183,8 @@ struct Smem {
     int redi[2][kSliceWarps];                  // FP64: per-warp max biased exponent
 };
 
-static_assert(sizeof(Smem<FmtF64>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 128 <= 232448,
+static_assert(sizeof(Smem<FmtF64>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 128 <= 232448 &&
+                  sizeof(Smem<FmtSplit6>) + 128 <= 232448,
               "shared memory of one CTA must stay within 227 KB");
 
 // The MMAs of one tile: window row offset I, input digit DG. Descriptor
@@ -323,15 +337,47 @@ constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
 // step per launch, 639 at three; star2d1r 1024^2, 100 steps: 1295 us on the
 // FP64 FMA kernel (the FP64 pipe takes 10 us of each step's 13), 527 so.
 constexpr int kMaxSteps = 3;
+template <class F>
 struct StepArgs {
-    const double *in;  // interior point (0, 0) of the source
-    int steps;         // T
-    int radius;        // of one step
-    int aligned;       // 1D: the buffers and the interior are 16-byte aligned
-    unsigned taps;     // bit t: weight t is not zero
-    int frame_cta;     // CTAs from this one on compute the frame
-    double w[9];       // weights of one step
+    const typename F::Out *in;  // interior point (0, 0) of the source
+    int steps;                  // T
+    int radius;                 // of one step
+    int aligned;                // 1D: the buffers and the interior are 16-byte aligned
+    unsigned taps;              // bit t: weight t is not zero
+    int frame_cta;              // CTAs from this one on compute the frame
+    typename F::Out w[9];       // weights of one step
 };
+
+// The frame's arithmetic, that of single sweeps: FP64 FMA, or double-float.
+__device__ __forceinline__ void tap_acc(double &a, double w, double x) { a = fma(w, x, a); }
+// (ff::ff_tap's operations as intrinsics, which the compiler does not contract:
+// a product folded into the TwoSum that follows it would count its rounding
+// error twice.)
+__device__ __forceinline__ void tap_acc(float2 &a, float2 w, float2 x)
+{
+    const float p = __fmul_rn(w.x, x.x), ep = __fmaf_rn(w.x, x.x, -p);
+    const float s = __fadd_rn(a.x, p), bb = __fsub_rn(s, a.x);
+    const float q = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, bb)), __fsub_rn(p, bb));
+    a.y = __fmaf_rn(w.y, x.x, __fmaf_rn(w.x, x.y, __fadd_rn(__fadd_rn(a.y, q), ep)));
+    a.x = s;
+}
+__device__ __forceinline__ double tap_sum(double a) { return a; }
+__device__ __forceinline__ float2 tap_sum(float2 a) { return ff::ff_finish(a.x, a.y); }
+__device__ __forceinline__ double prev_lane(double x) { return __shfl_up_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ double next_lane(double x) { return __shfl_down_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ float2 prev_lane(float2 x)
+{
+    return make_float2(__shfl_up_sync(0xffffffffu, x.x, 1), __shfl_up_sync(0xffffffffu, x.y, 1));
+}
+__device__ __forceinline__ float2 next_lane(float2 x)
+{
+    return make_float2(__shfl_down_sync(0xffffffffu, x.x, 1), __shfl_down_sync(0xffffffffu, x.y, 1));
+}
+__device__ __forceinline__ double lane_of(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
+__device__ __forceinline__ float2 lane_of(float2 x, int src)
+{
+    return make_float2(__shfl_sync(0xffffffffu, x.x, src), __shfl_sync(0xffffffffu, x.y, src));
+}
 
 // One strip of the frame, by one warp: T steps for the T - 1 points next to
 // an edge, at positions l0 .. l0 + 25 along it. `edge` is the offset of
@@ -343,38 +389,40 @@ struct StepArgs {
 // (The loops over levels and strips stay rolled: the code runs once or a few
 // times per launch, and unrolled its instruction fetches took most of 13,000
 // cycles, more than the first tile needs to reach the epilogue.)
-__device__ __forceinline__ void frame_strip(const double *__restrict__ in, double *__restrict__ out, long long edge,
+template <class V>
+__device__ __forceinline__ void frame_strip(const V *__restrict__ in, V *__restrict__ out, long long edge,
                                             long long sa, long long sl, int len, int l0, int end, int steps,
-                                            const double (&w)[9], unsigned taps)
+                                            const V (&w)[9], unsigned taps)
 {
     constexpr int T = kMaxSteps;
     const int lane = threadIdx.x & 31, p = l0 - T + lane;
     const bool inside = p >= 0 && p < len, halo = p == -1 || p == len;
     const long long at = edge + (long long)p * sl;
-    double even[2 * T], odd[2 * T - 1], u[2 * T];  // row k of the strip is u[k + 1]
+    V even[2 * T], odd[2 * T - 1], u[2 * T];  // row k of the strip is u[k + 1]
 #pragma unroll
-    for (int j = 0; j < 2 * T; ++j) u[j] = even[j] = inside || halo ? in[at + (j - 1) * sa] : 0.0;
+    for (int j = 0; j < 2 * T; ++j) u[j] = even[j] = inside || halo ? in[at + (j - 1) * sa] : V{};
 #pragma unroll
-    for (int j = 0; j < 2 * T - 1; ++j) odd[j] = halo || (inside && j == 0) ? out[at + (j - 1) * sa] : 0.0;
+    for (int j = 0; j < 2 * T - 1; ++j) odd[j] = halo || (inside && j == 0) ? out[at + (j - 1) * sa] : V{};
 #pragma unroll 1
     for (int level = 1; level <= steps; ++level) {
         const int rows = 2 * steps - 1 - level;  // rows of this level that count
-        double v[2 * T - 2];
+        V v[2 * T - 2];
 #pragma unroll
-        for (int k = 0; k < 2 * T - 2; ++k) v[k] = 0.0;
+        for (int k = 0; k < 2 * T - 2; ++k) v[k] = V{};
 #pragma unroll
         for (int j = 0; j < 2 * T; ++j) {
-            const double x[3] = {__shfl_up_sync(0xffffffffu, u[j], 1), u[j], __shfl_down_sync(0xffffffffu, u[j], 1)};
+            const V x[3] = {prev_lane(u[j]), u[j], next_lane(u[j])};
 #pragma unroll
             for (int t = 0; t < 9; ++t) {
                 const int k = j - t / 3;  // row k takes u[k + da] through weight row da
-                if (k >= 0 && k < 2 * T - 2 && k < rows && (taps >> t & 1u)) v[k] = fma(w[t], x[t % 3], v[k]);
+                if (k >= 0 && k < 2 * T - 2 && k < rows && (taps >> t & 1u)) tap_acc(v[k], w[t], x[t % 3]);
             }
         }
         // the next level's input
         u[0] = (level & 1) ? odd[0] : even[0];
 #pragma unroll
-        for (int k = 0; k < 2 * T - 2; ++k) u[k + 1] = halo ? ((level & 1) ? odd[k + 1] : even[k + 1]) : inside ? v[k] : 0.0;
+        for (int k = 0; k < 2 * T - 2; ++k)
+            u[k + 1] = halo ? ((level & 1) ? odd[k + 1] : even[k + 1]) : inside ? tap_sum(v[k]) : V{};
     }
     if (p < end && lane >= T && lane < 32 - T) {
 #pragma unroll
@@ -384,20 +432,21 @@ __device__ __forceinline__ void frame_strip(const double *__restrict__ in, doubl
 }
 
 // The frame of an m x n grid, strip by strip, shared by `nwarps` warps.
-__device__ __noinline__ void frame_steps(const StepArgs &s, double *__restrict__ out, int m, int n, long long ld,
-                                         int warp, int nwarps)
+template <class F>
+__device__ __noinline__ void frame_steps(const StepArgs<F> &s, typename F::Out *__restrict__ out, int m, int n,
+                                         long long ld, int warp, int nwarps)
 {
     constexpr int S = 32 - 2 * kMaxSteps;  // outputs per strip
-    const int F = s.steps - 1;             // frame width
-    if (F == 0) return;
-    const int nx = (n + S - 1) / S, ny = (m - 2 * F + S - 1) / S;
+    const int fw = s.steps - 1;            // frame width
+    if (fw == 0) return;
+    const int nx = (n + S - 1) / S, ny = (m - 2 * fw + S - 1) / S;
 #pragma unroll 1
     for (int i = warp; i < 2 * (nx + ny); i += nwarps) {
         const bool horiz = i < 2 * nx;  // top and bottom rows, whole length
         const int q = horiz ? i : i - 2 * nx, cnt = horiz ? nx : ny;
         const bool far = q >= cnt;
-        const int l0 = (far ? q - cnt : q) * S + (horiz ? 0 : F);
-        double w[9];
+        const int l0 = (far ? q - cnt : q) * S + (horiz ? 0 : fw);
+        typename F::Out w[9];
         unsigned taps = 0;
 #pragma unroll
         for (int t = 0; t < 9; ++t) {
@@ -406,31 +455,33 @@ __device__ __noinline__ void frame_steps(const StepArgs &s, double *__restrict__
             w[t] = s.w[src];
             taps |= (s.taps >> src & 1u) << t;
         }
-        // columns end F short of the corners, which belong to the rows
+        // columns end fw short of the corners, which belong to the rows
         frame_strip(s.in, out, far ? (horiz ? (long long)(m - 1) * ld : n - 1) : 0,
-                    horiz ? (far ? -ld : ld) : (far ? -1 : 1), horiz ? 1 : ld, horiz ? n : m, l0, horiz ? n : m - F,
+                    horiz ? (far ? -ld : ld) : (far ? -1 : 1), horiz ? 1 : ld, horiz ? n : m, l0, horiz ? n : m - fw,
                     s.steps, w, taps);
     }
 }
 
 // The (T - 1) r outputs next to one end of a 1D grid (T r <= 16), by one warp:
 // lane l holds point l - r counted from that end, as frame_strip's lanes do.
-__device__ __noinline__ void frame_end_1d(const StepArgs &s, double *__restrict__ out, int n, bool left)
+template <class F>
+__device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out *__restrict__ out, int n, bool left)
 {
+    using V = typename F::Out;
     const int lane = threadIdx.x & 31, r = s.radius, p = lane - r;
     const long long at = left ? p : n - 1 - p;
     const bool halo = p < 0;
-    const double even = s.in[at], odd = halo ? out[at] : 0.0;
-    double u = even;
+    const V even = s.in[at], odd = halo ? out[at] : V{};
+    V u = even;
 #pragma unroll 1
     for (int level = 1; level <= s.steps; ++level) {
-        double v = 0.0;
+        V v{};
 #pragma unroll 1
         for (int t = 0; t <= 2 * r; ++t) {
             const int d = left ? t - r : r - t;  // the tap's lane, towards the interior from this end
-            v = fma(s.w[t], __shfl_sync(0xffffffffu, u, (lane + d) & 31), v);
+            tap_acc(v, s.w[t], lane_of(u, (lane + d) & 31));
         }
-        u = halo ? ((level & 1) ? odd : even) : v;
+        u = halo ? ((level & 1) ? odd : even) : tap_sum(v);
     }
     if (!halo && p < (s.steps - 1) * r) out[at] = u;
 }
@@ -444,7 +495,7 @@ template <class F, bool BATCH, int MODE = kModeGrid>
 __global__ void __launch_bounds__(kThreads<F>, 1)
     k2d_tc(const __grid_constant__ CUtensorMap tmap, typename F::Out *__restrict__ out, int m, int n,
            long long ld, int tiles_x, int tiles, int map_x, int map_y, typename F::Digits sw, WaitCfg wc,
-           const TcGrid<F> *__restrict__ grids, int ngrids, const __grid_constant__ StepArgs sa)
+           const TcGrid<F> *__restrict__ grids, int ngrids, const __grid_constant__ StepArgs<F> sa)
 {
     constexpr bool ONED = MODE == kMode1d, STEPS = MODE == kModeSteps;
     static_assert(!BATCH || MODE == kModeGrid, "batches run one sweep of 7x7 grids");
@@ -727,27 +778,28 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 vmax = S.red[buf][0];
 #pragma unroll
                 for (int i = 1; i < kSliceWarps; ++i) vmax = fmaxf(vmax, S.red[buf][i]);
-                ex = split::tile_exponent(vmax);
+                // six digits: |x| / 2^ex < 1/4, the top digit within 128
+                ex = split::tile_exponent(vmax) + (D == 6 ? 1 : 0);
             }
             if (leader) S.scale_exp[it & 3] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
             unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[buf][0][0]);
+            // 1D: chunk idx / 4 in phase (idx / 4) % 4
+            auto word = [](int idx) {
+                return ONED ? (idx >> 2 & 3) * (kPhase1d / 4) + (idx >> 4) * 4 + (idx & 3) : idx;
+            };
             if constexpr (F::kF64) {
                 constexpr bool EVEN = STEPS || ONED;
-                // 1D: chunk idx / 4 in phase (idx / 4) % 4
-                auto word = [&](int idx) {
-                    return dst0 + (ONED ? (idx >> 2 & 3) * (kPhase1d / 4) + (idx >> 4) * 4 + (idx & 3) : idx);
-                };
                 if (ex >= kFastExp) {
 #pragma unroll
                     for (int q = 0; q < PER; ++q) {
                         const int idx = st + q * kSliceThreads;
-                        if (idx < kPairs) f64_cut_fast<EVEN, PL / 2>(v[q], ex, word(idx));
+                        if (idx < kPairs) f64_cut_fast<EVEN, PL / 2>(v[q], ex, dst0 + word(idx));
                     }
                 } else {
 #pragma unroll
                     for (int q = 0; q < PER; ++q) {
                         const int idx = st + q * kSliceThreads;
-                        if (idx < kPairs) f64_cut_any<EVEN, PL / 2>(v[q], ex, word(idx));
+                        if (idx < kPairs) f64_cut_any<EVEN, PL / 2>(v[q], ex, dst0 + word(idx));
                     }
                 }
             } else {
@@ -755,14 +807,14 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
 #pragma unroll
                 for (int q = 0; q < PER; ++q) {
                     const int idx = st + q * kSliceThreads;
-                    if (idx < NPAIR) {
+                    if (idx < kPairs) {
                         split::f2x a, b, s2;
                         asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "r"(v[q].x), "r"(v[q].z));
                         asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(v[q].y), "r"(v[q].w));
                         asm("mov.b64 %0, {%1, %1};" : "=l"(s2) : "f"(to_digits));
                         unsigned wd[D];
                         split::slice_digit_pairs_x2(split::f2_mul(a, s2), split::f2_mul(b, s2), wd);
-                        unsigned *dst = dst0 + idx;
+                        unsigned *dst = dst0 + word(idx);
 #pragma unroll
                         for (int k = 0; k < D; ++k) dst[k * (PL / 2)] = wd[k];
                     }
@@ -778,23 +830,23 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         // er, block eb); warp h of a quarter (one warp per quarter split,
         // two FP64) stores rows kRowsPerWarp h .. of the group, columns
         // 8 eb .. 8 eb + 7.
-        const int quarter = warp & 3, h = (warp - kWarpEpi0) >> 2;
-        const int mrow = 32 * quarter + lane;
-        const int er = mrow >> 3, eb = mrow & 7;
-        const unsigned lane_bits = (unsigned)(32 * quarter) << 16;
         if constexpr (STEPS) {
             const int fc = (int)blockIdx.x - sa.frame_cta, fn = (int)gridDim.x - sa.frame_cta;
             if (fc >= 0) {
                 pdl_wait();
-                frame_steps(sa, out, m, n, ld, (warp - kWarpEpi0) * fn + fc, F::kEpiWarps * fn);
+                frame_steps<F>(sa, out, m, n, ld, (warp - kWarpEpi0) * fn + fc, F::kEpiWarps * fn);
             }
         }
         if constexpr (ONED) {  // the ends, on the last CTA (no other has fewer tiles)
             if (blockIdx.x == gridDim.x - 1 && warp < kWarpEpi0 + 2 && sa.steps > 1) {
                 pdl_wait();
-                frame_end_1d(sa, out, n, warp == kWarpEpi0);
+                frame_end_1d<F>(sa, out, n, warp == kWarpEpi0);
             }
         }
+        const int quarter = warp & 3, h = (warp - kWarpEpi0) >> 2;
+        const int mrow = 32 * quarter + lane;
+        const int er = mrow >> 3, eb = mrow & 7;
+        const unsigned lane_bits = (unsigned)(32 * quarter) << 16;
         const int frame = STEPS || ONED ? (sa.steps - 1) * sa.radius : 0;
         for (int it = 0; it < my_tiles; ++it) {
             const int buf = it & 1, use = it >> 1;
@@ -828,7 +880,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar2(S.acc_empty, buf));
                 }
-                double res[8];
+                typename F::Out res[8];
                 if constexpr (F::kF64) {
                     // value = T 2^c with T from the levels (f64_combine) and
                     // c = (input scale) + (weight scale) - 1080.
@@ -848,26 +900,42 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                             res[j] = ex == kNonFiniteTile ? __longlong_as_double(0x7FF8000000000000ll)
                                                           : f64_from_fixed(t[j], c);
                     }
+                } else {
+                    const float scale = ldexpf(1.0f, ex + ew - 2 * kDigitBits);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float h1, e1, h2, e2, hi, lo;
+                        two_sum(acc[0][j], acc[1][j] * 0x1p-9f, h1, e1);
+                        two_sum(h1, acc[2][j] * 0x1p-18f, h2, e2);
+                        float tail = acc[4][j] * 0x1p-36f;
+                        if constexpr (D == 6) tail = fmaf(acc[D - 1][j], 0x1p-45f, tail);
+                        tail = fmaf(acc[3][j], 0x1p-27f, tail);
+                        two_sum(h2, (e1 + e2) + tail, hi, lo);
+                        res[j] = make_float2(hi * scale, lo * scale);
+                    }
                 }
+                auto store2 = [](typename F::Out *o, typename F::Out u, typename F::Out v) {
+                    if constexpr (F::kF64)
+                        *reinterpret_cast<double2 *>(o) = make_double2(u, v);
+                    else
+                        *reinterpret_cast<float4 *>(o) = make_float4(u.x, u.y, v.x, v.y);
+                };
                 if constexpr (ONED) {
                     // outputs 32 mrow + 8 rho .. + 7 of the tile
                     const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d + 32 * mrow + 8 * rho;
                     if (sa.aligned && x >= frame && x + 8 <= n - frame) {
 #pragma unroll
-                        for (int j = 0; j < 8; j += 2)
-                            *reinterpret_cast<double2 *>(out + x + j) = make_double2(res[j], res[j + 1]);
+                        for (int j = 0; j < 8; j += 2) store2(out + x + j, res[j], res[j + 1]);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
                             if (x + j >= frame && x + j < n - frame) out[x + j] = res[j];
                     }
-                    continue;
-                }
-                const int yy = y0 + R * er + rho;
-                if (yy >= o_m) continue;
-                if (STEPS && (yy < frame || yy >= o_m - frame)) continue;
-                if constexpr (F::kF64) {
-                    double *o = reinterpret_cast<double *>(o_base) + (long long)yy * o_ld + xb;
+                } else {
+                    const int yy = y0 + R * er + rho;
+                    if (yy >= o_m) continue;
+                    if (STEPS && (yy < frame || yy >= o_m - frame)) continue;
+                    typename F::Out *o = o_base + (long long)yy * o_ld + xb;
                     if (STEPS && (xb < frame || xb + 8 > o_n - frame)) {
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
@@ -877,28 +945,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
                         if (xb + j + 1 < o_n)
-                            *reinterpret_cast<double2 *>(o + j) = make_double2(res[j], res[j + 1]);
-                        else if (xb + j < o_n)
-                            o[j] = res[j];
-                    }
-                } else {
-                    const float scale = ldexpf(1.0f, ex + ew - 2 * kDigitBits);
-                    float2 res[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float h1, e1, h2, e2, hi, lo;
-                        two_sum(acc[0][j], acc[1][j] * 0x1p-9f, h1, e1);
-                        two_sum(h1, acc[2][j] * 0x1p-18f, h2, e2);
-                        const float tail = fmaf(acc[3][j], 0x1p-27f, acc[4][j] * 0x1p-36f);
-                        two_sum(h2, (e1 + e2) + tail, hi, lo);
-                        res[j] = make_float2(hi * scale, lo * scale);
-                    }
-                    float2 *o = reinterpret_cast<float2 *>(o_base) + (long long)yy * o_ld + xb;
-#pragma unroll
-                    for (int j = 0; j < 8; j += 2) {
-                        if (xb + j + 1 < o_n)
-                            *reinterpret_cast<float4 *>(o + j) =
-                                make_float4(res[j].x, res[j].y, res[j + 1].x, res[j + 1].y);
+                            store2(o + j, res[j], res[j + 1]);
                         else if (xb + j < o_n)
                             o[j] = res[j];
                     }
@@ -933,7 +980,7 @@ cudaError_t set_smem_attr()
 template <class F, int MODE = kModeGrid>
 cudaError_t launch_tc(const GridView &g, const typename F::Digits &digits, long long origin, long long elements,
                       const void *in_base, void *out_base, const WaitCfg &wc, cudaStream_t st,
-                      const StepArgs &sa = StepArgs{})
+                      const StepArgs<F> &sa = StepArgs<F>{})
 {
     const long long ld = g.pitch[0];
     CUtensorMap map;
@@ -994,7 +1041,7 @@ cudaError_t launch_batch(const void *records, int ngrids, int total, const WaitC
     return launch_programmatic(k2d_tc<F, true>, grid, kThreads<F>, sizeof(Smem<F>) + 128, st, unused,
                                static_cast<typename F::Out *>(nullptr), 0, 0, 0LL, 0, total, 0, 0,
                                typename F::Digits{}, wc, reinterpret_cast<const TcGrid<F> *>(records), ngrids,
-                               StepArgs{});
+                               StepArgs<F>{});
 }
 
 split::SliceWeights split_digits(const Weights &w) { return split::slice_weights(w); }
@@ -1017,11 +1064,21 @@ cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long 
                              WaitCfg{wt.limit_ns, wt.skip_loads}, st);
 }
 
-cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
-                                 long long origin, long long elements, const double *in_base, double *out_base,
-                                 const TcWait &wt, cudaStream_t st)
+namespace {
+
+inline double step_weight(double w, double) { return w; }
+inline float2 step_weight(double w, float2)
 {
-    StepArgs sa{in_base + origin, steps, 1, 0, 0u, 0, {}};
+    const float h = (float)w;
+    return make_float2(h, (float)(w - (double)h));
+}
+
+template <class F>
+cudaError_t launch_steps_2d(const GridView &g, const Weights &wT, const Weights &w3x3, int steps, long long origin,
+                            long long elements, const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st)
+{
+    using Out = typename F::Out;
+    StepArgs<F> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, 1, 0, 0u, 0, {}};
     // The frame's strips go to the CTAs that have no tile in the last round,
     // or to all CTAs where that is sooner. A strip keeps one of an SM's four
     // FP64 pipes for about 9,000 cycles; an epilogue warp is idle that long
@@ -1034,34 +1091,53 @@ cudaError_t launch_fp64_steps_tc(const GridView &g, const Weights &wT, const Wei
     auto rounds = [&](long long c) { return (strips + 4 * c - 1) / (4 * c); };
     if (extra > 0 && 9000 * rounds(ctas - extra) - 6500 < 9000 * rounds(ctas)) sa.frame_cta = (int)extra;
     for (int t = 0; t < 9; ++t) {
-        sa.w[t] = w3x3.v[t];
+        sa.w[t] = step_weight(w3x3.v[t], Out{});
         if (w3x3.v[t] != 0.0) sa.taps |= 1u << t;
     }
-    return launch_tc<FmtF64, kModeSteps>(g, f64_slice_weights(wT, 49, true), origin, elements, in_base, out_base,
-                                         WaitCfg{wt.limit_ns, wt.skip_loads}, st, sa);
+    return launch_tc<F, kModeSteps>(g, f64_slice_weights(wT, 49, true), origin, elements, in_base, out_base,
+                                    WaitCfg{wt.limit_ns, wt.skip_loads}, st, sa);
 }
 
-cudaError_t launch_fp64_steps_tc_1d(long long n, const double *taps, int radius, const double *w, int steps,
-                                    long long origin, const double *in_base, double *out_base, const TcWait &wt,
-                                    cudaStream_t st)
+template <class F>
+cudaError_t launch_steps_1d(long long n, const double *taps, int radius, const double *w, int steps, long long origin,
+                            const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st)
 {
+    using Out = typename F::Out;
     if (steps < 1 || steps * radius > kReach1d || n < 64) return cudaErrorInvalidValue;
-    cudaError_t e = set_smem_attr<FmtF64, false, kMode1d>();
+    cudaError_t e = set_smem_attr<F, false, kMode1d>();
     if (e != cudaSuccess) return e;
     Weights wT;
     for (int i = 0; i < 49; ++i) wT.v[i] = i <= 2 * kReach1d ? taps[i] : 0.0;
-    StepArgs sa{in_base + origin, steps, radius, 0, 0u, 0, {}};
+    StepArgs<F> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, radius, 0, 0u, 0, {}};
     sa.aligned = origin % 2 == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0 &&
                  reinterpret_cast<uintptr_t>(out_base) % 16 == 0;
-    for (int t = 0; t <= 2 * radius; ++t) sa.w[t] = w[t];
+    for (int t = 0; t <= 2 * radius; ++t) sa.w[t] = step_weight(w[t], Out{});
     CUtensorMap unused;
     std::memset(&unused, 0, sizeof unused);
     const int tiles = (int)((n + kOut1d - 1) / kOut1d);
     note_launch();
-    return launch_programmatic(k2d_tc<FmtF64, false, kMode1d>, std::min(tiles, device_sm_count()), kThreads<FmtF64>,
-                               sizeof(Smem<FmtF64>) + 128, st, unused, out_base + origin, 1, (int)n, 0LL, 1, tiles, 0,
-                               0, f64_slice_weights(wT, 49, true), WaitCfg{wt.limit_ns, wt.skip_loads},
-                               static_cast<const TcGrid<FmtF64> *>(nullptr), 0, sa);
+    return launch_programmatic(k2d_tc<F, false, kMode1d>, std::min(tiles, device_sm_count()), kThreads<F>,
+                               sizeof(Smem<F>) + 128, st, unused, reinterpret_cast<Out *>(out_base) + origin, 1,
+                               (int)n, 0LL, 1, tiles, 0, 0, f64_slice_weights(wT, 49, true),
+                               WaitCfg{wt.limit_ns, wt.skip_loads}, static_cast<const TcGrid<F> *>(nullptr), 0, sa);
+}
+
+}  // namespace
+
+cudaError_t launch_steps_tc(bool fp64, const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
+                            long long origin, long long elements, const void *in_base, void *out_base,
+                            const TcWait &wt, cudaStream_t st)
+{
+    return fp64 ? launch_steps_2d<FmtF64>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st)
+                : launch_steps_2d<FmtSplit6>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st);
+}
+
+cudaError_t launch_steps_tc_1d(bool fp64, long long n, const double *taps, int radius, const double *w, int steps,
+                               long long origin, const void *in_base, void *out_base, const TcWait &wt,
+                               cudaStream_t st)
+{
+    return fp64 ? launch_steps_1d<FmtF64>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st)
+                : launch_steps_1d<FmtSplit6>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st);
 }
 
 size_t tc_batch_record_bytes(bool fp64) { return fp64 ? sizeof(TcGrid<FmtF64>) : sizeof(TcGrid<FmtSplit>); }

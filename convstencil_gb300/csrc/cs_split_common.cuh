@@ -105,13 +105,14 @@ __device__ __forceinline__ void slice_digits(float a, float b, float (&d)[kDigit
 // permute and a mask-and-or build both halves, and one FP16 subtraction of
 // 1536 leaves the digits exactly. Each lane of a pair instruction rounds as
 // the scalar one, so the digits equal slice_digits' (a zero digit is +0).
-__device__ __forceinline__ void slice_digit_pairs_x2(f2x a, f2x b, unsigned (&w)[kDigits])
+template <int N>
+__device__ __forceinline__ void slice_digit_pairs_x2(f2x a, f2x b, unsigned (&w)[N])
 {
     const f2x m2 = 0x4B4002004B400200ull;  // (M, M)
     const f2x r2 = 0x4400000044000000ull;  // (512, 512)
     const __half2 bias = __halves2half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600));  // 1536
 #pragma unroll
-    for (int k = 0; k < kDigits; ++k) {
+    for (int k = 0; k < N; ++k) {
         const f2x t = f2_add(f2_add(a, b), m2);
         unsigned t0, t1, u;
         asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t));
@@ -119,7 +120,7 @@ __device__ __forceinline__ void slice_digit_pairs_x2(f2x a, f2x b, unsigned (&w)
         u = (u & 0x03FF03FFu) | 0x64006400u;
         const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&u), bias);
         w[k] = *reinterpret_cast<const unsigned *>(&h);
-        if (k + 1 < kDigits) {
+        if (k + 1 < N) {
             a = f2_mul(f2_sub(a, f2_sub(t, m2)), r2);
             b = f2_mul(b, r2);
         }

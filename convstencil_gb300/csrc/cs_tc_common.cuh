@@ -221,7 +221,7 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigne
 }
 
 // 8 bytes from global to shared memory, or zeros.
-__device__ __forceinline__ void cp_async8(unsigned dst, const double *src, bool take)
+__device__ __forceinline__ void cp_async8(unsigned dst, const void *src, bool take)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(take ? 8 : 0) : "memory");
 }

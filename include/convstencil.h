@@ -81,8 +81,14 @@ typedef enum cs_semantics { CS_SEM_STEP = 0, CS_SEM_FUSED = 1 } cs_semantics;
  *                about 48 significant bits); no FP64 arithmetic in the sweep.
  *                Dense 7x7 kernels contract exact 9-bit fixed-point slices
  *                on FP16 tensor cores (FP32 accumulation is exact for them);
- *                other kernels use double-float FP32 arithmetic. Relative
- *                error per sweep ~1e-13. Inputs must be finite. */
+ *                other kernels use double-float FP32 arithmetic. 2D radius-1
+ *                and 1D plans of at least 64 tiles (64x64 or 4096 points)
+ *                also run on the tensor cores where the tuner measures it
+ *                faster, 3 to 15 steps per launch, with six digits per
+ *                operand: inputs keep 52 bits below their tile's largest
+ *                value, results are rounded to pairs once per launch. Relative
+ *                error per sweep ~1e-13. Inputs must be finite. Pin
+ *                CS_ALGO_SPLIT_FMA for double-float sums. */
 typedef enum cs_precision { CS_PREC_FP64 = 0, CS_PREC_SPLIT = 1 } cs_precision;
 
 /* Kernel family; CS_ALGO_AUTO lets the plan's tuner choose. */
@@ -123,7 +129,8 @@ typedef enum cs_option {
                                      (default 100, 0 = never) */
     CS_OPT_TIME_BLOCK = 3,        /* split double-float kernels, 2D radius 1 and 1D:
                                      steps fused per launch by temporal blocking
-                                     (0 = tuner picks 1..4, default; 1 = off) */
+                                     (0 = tuner picks 1..4, or a tensor-core launch of several
+                                     steps, default; 1 = off) */
     CS_OPT_TILE_ROWS = 6,         /* FP64 FMA 2D kernel: rows per CTA tile, 16 or 32 (0 = tuner,
                                      default: the first run times both; results do not depend on it) */
     CS_OPT_WAIT_LIMIT_US = 4,     /* bound of each device-side wait of the tcgen05 kernels, in

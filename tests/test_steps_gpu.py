@@ -166,3 +166,38 @@ def test_1d_layouts_halos_and_nothing_beyond(shape, taps, fused, n, pad):
     got = run(p, grids[0], grids[1], sweeps * per)
     assert p.algo == cs.Algo.FP64_TC and p.time_block == {1: 15, 2: 7, 3: 5, 4: 3}[r]
     assert np.abs(got[pad:pad + n] - ref).max() <= TOL * np.abs(ref).max()
+
+
+def run_split(plan, buf, steps):
+    raw = torch.from_numpy(buf).cuda()
+    a = torch.zeros(plan.elements * 2, dtype=torch.float32, device="cuda")
+    b = torch.zeros_like(a)
+    plan.split_from_fp64(raw, a)
+    in_b = plan.run(a, b, steps)
+    plan.split_to_fp64(b if in_b else a, raw)
+    torch.cuda.synchronize()
+    assert cs.device_wait_timeouts() == 0
+    return raw.cpu().numpy()
+
+
+@pytest.mark.parametrize("shape,taps,ext", [("star2d1r", 5, (1023, 1026)), ("box2d1r", 9, (900, 1101)),
+                                            ("star2d1r", 5, (4096, 4096)), ("1d1r", 3, (1_000_003,)),
+                                            ("1d2r", 5, (1_048_576,))])
+@pytest.mark.parametrize("steps", [3, 20, 107])
+def test_split_steps(shape, taps, ext, steps):
+    """Split plans under AUTO, re-anchor sweeps included, against FP64 single
+    steps: 1e-12 of the largest value (at most 36 launches, each rounding to
+    pairs of 48 bits, 3.6e-15), also where the tuner keeps the double-float
+    kernel (2^-44 per step)."""
+    w = O.seeded_weights(taps, 31)
+    p = cs.Plan(shape, ext, w, precision=cs.Precision.SPLIT)
+    x = O.splitmix_uniform(int(np.prod(ext)), 32).reshape(ext)
+    got = p.unpack(run_split(p, p.pack(x), steps))
+    if len(ext) == 2:
+        ref = steps_of(np.pad(x, 1), np.zeros((ext[0] + 2, ext[1] + 2)), dense_of(shape, w), steps)
+    else:
+        r = taps // 2
+        ref = steps_1d(np.pad(x, r), np.zeros(ext[0] + 2 * r), w, steps)
+    if np.prod(ext) >= 1 << 24:
+        assert p.algo == cs.Algo.SPLIT_TC and p.time_block == 3
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
