@@ -1813,6 +1813,13 @@ cs_status run_into(cs_plan *p, const void *in, void *out, void *scratch, long lo
     return CS_OK;
 }
 
+int plan_fix_fp64(cs_plan *p, bool tc)
+{
+    tc = tc && (fp64_tc_ok(p) || fp64_tc3d_ok(p) || fp64_tc3d_r3_ok(p) || fp64_tc1d_ok(p));
+    p->algo = tc ? CS_ALGO_FP64_TC : CS_ALGO_FP64_FMA;
+    return tc ? steps_per_launch(p, nullptr, nullptr) : 1;
+}
+
 cs_status set_error(cs_status s, const char *msg) { return fail(s, "%s", msg); }
 
 bool plan_facts(const cs_plan *p, PlanFacts *f)

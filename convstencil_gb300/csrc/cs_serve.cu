@@ -104,7 +104,7 @@ struct Request {
     cs_plan *plan = nullptr;
     cs_precision prec = CS_PREC_FP64;
     cs_layout layout{};
-    long long steps = 0, issued = 0, sweeps_per_step = 1;
+    long long steps = 0, issued = 0, sweeps_per_step = 1, sweeps_per_launch = 1;
     void *host = nullptr;  // pinned: packed input, later the packed FP64 result
     size_t host_cls = 0;
     void *d[2] = {nullptr, nullptr};
@@ -245,7 +245,10 @@ void advance(cs_server *s, Request *r)
         r->chunk_pending = false;
     }
     // Chunks are whole fused sweeps: a multiple of the plan's steps per sweep.
-    const long long full = std::max(1LL, s->cfg.chunk_steps / r->sweeps_per_step) * r->sweeps_per_step;
+    // For plans that take several sweeps per launch also whole launches, so
+    // the launches do not depend on the chunk length.
+    const long long unit = r->sweeps_per_step * r->sweeps_per_launch;
+    const long long full = std::max(1LL, s->cfg.chunk_steps / unit) * unit;
     if (r->small) {
         // All chunks now, back to back on the request's high-priority stream:
         // the same kernels and re-anchoring points as chunk-by-chunk issue,
@@ -265,7 +268,8 @@ void advance(cs_server *s, Request *r)
     const long long chunk = std::min(full, r->steps - r->issued);
     cs_status st = CS_OK;
     const bool graphable = s->cfg.use_graphs && chunk == full &&
-                           (chunk / r->sweeps_per_step) % 2 == 0 && r->prec == CS_PREC_FP64;
+                           (chunk / r->sweeps_per_step) % 2 == 0 && r->prec == CS_PREC_FP64 &&
+                           r->sweeps_per_launch == 1;  // an even number of launches
     if (graphable && r->graph && r->graph_steps == chunk) {
         st = cudaGraphLaunch(r->graph, r->stream) == cudaSuccess ? CS_OK : CS_ERR_CUDA;
     } else if (graphable && r->full_chunks >= 1) {
@@ -540,44 +544,40 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     if (st != CS_OK) return st;
     // A fixed kernel choice keeps results identical in any mix and keeps the
     // plan tuner (which times candidates synchronously) off the worker
-    // thread: the FP64 FMA kernels; for split precision the tcgen05 slice
-    // kernel where it applies (it falls back by itself on buffers it cannot
-    // use), else the double-float kernels with a fixed temporal block (their
-    // results do not depend on it).
+    // thread: the tcgen05 kernels from the sizes below up, else FP64 FMA or,
+    // for split precision, the double-float kernels with a fixed temporal
+    // block (their results do not depend on it).
+    // The lines between kernels are where single sweeps of both took as long
+    // (GB300, us per sweep, alone): split 7x7 256^2 8.4 mma.sync, 7.3 tcgen05;
+    // split box3d1r 64^3 10.6 double-float, 10.8 tcgen05, 96^3 18.7, 16.9;
+    // FP64 7x7 256^2 18.7 FMA, 9.5 tcgen05 (an FMA tile takes 14 us however
+    // few there are); box3d1r 32^3 10.6, 9.3; star3d1r 80^3 16.6, 17.5, 96^3
+    // 20.7, 20.5; star2d1r 512^2 6.4, 4.4 (three steps a launch). The fused
+    // 7x7x7 box costs 343 FMA per point, 171 us at 64^3 against 41; its
+    // octahedron 63, about as long at 64^3.
+    const bool box3d = d->shape == CS_SHAPE_BOX3D1R, in3d = box3d || d->shape == CS_SHAPE_STAR3D1R;
+    const bool in1d = d->shape == CS_SHAPE_1D1R || d->shape == CS_SHAPE_1D2R;
+    const bool fused = d->semantics == CS_SEM_FUSED;
+    double pts = 1;
+    for (int k = 0; k < (in3d ? 3 : in1d ? 1 : 2); ++k) pts *= (double)d->extent[k];
     if (d->precision == CS_PREC_SPLIT) {
-        int algo;
-        if (d->shape == CS_SHAPE_STAR3D1R || d->shape == CS_SHAPE_BOX3D1R) {
-            // 3D: the 27-point box on tcgen05 from about 128^3 points up
-            // (measured crossover), else the double-float kernels (the
-            // 7-point star always: its own kernel is faster).
-            const double pts = (double)d->extent[0] * (double)d->extent[1] * (double)d->extent[2];
-            algo = d->shape == CS_SHAPE_BOX3D1R && d->semantics == CS_SEM_STEP && pts >= 2.0e6
-                       ? CS_ALGO_SPLIT_TC
-                       : CS_ALGO_SPLIT_FMA;
-        } else {
-            // tcgen05 pays a fixed ~16 us per sweep (one 64 x 64 tile per CTA
-            // and SM, set-up of its weight matrices and TMEM); below about four
-            // tiles per SM the mma.sync slice kernel (~8 us floor) finishes sooner.
-            const long long tiles = ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64);
-            algo = tiles >= 4LL * s->sm_count ? CS_ALGO_SPLIT_TC : CS_ALGO_SPLIT_MMA;
-        }
+        // The 7-point star always has its own double-float kernel.
+        const int algo = in3d ? (box3d && !fused && pts >= 8.8e5 ? CS_ALGO_SPLIT_TC : CS_ALGO_SPLIT_FMA)
+                              : CS_ALGO_SPLIT_TC;
         if (cs_plan_set_option(r->plan, CS_OPT_ALGO, algo) != CS_OK)
             cs_plan_set_option(r->plan, CS_OPT_ALGO, CS_ALGO_SPLIT_FMA);
-        const int tb = (d->shape == CS_SHAPE_1D1R || d->shape == CS_SHAPE_1D2R) ? 4
-                       : d->shape == CS_SHAPE_STAR2D1R                           ? 3
-                                                                                 : 2;
+        const int tb = in1d ? 4 : d->shape == CS_SHAPE_STAR2D1R ? 3 : 2;
         cs_plan_set_option(r->plan, CS_OPT_TIME_BLOCK, tb);
     } else {
-        // FP64: 7x7 kernels of at least four 64 x 64 tiles per SM on the
-        // tcgen05 digit pipeline (same cost model as the split slices), the
-        // FP64 FMA kernels otherwise.
-        const long long tiles = ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64);
-        const bool r3_2d = (d->shape == CS_SHAPE_BOX2D3R || d->shape == CS_SHAPE_STAR2D3R ||
-                            (d->semantics == CS_SEM_FUSED &&
-                             (d->shape == CS_SHAPE_BOX2D1R || d->shape == CS_SHAPE_STAR2D1R)));
-        if (!(r3_2d && tiles >= 4LL * s->sm_count &&
-              cs_plan_set_option(r->plan, CS_OPT_ALGO, CS_ALGO_FP64_TC) == CS_OK))
-            cs_plan_set_option(r->plan, CS_OPT_ALGO, CS_ALGO_FP64_FMA);
+        bool tc;
+        if (in3d)
+            tc = pts >= (fused ? (box3d ? 3.2e4 : 2.6e5) : (box3d ? 3.2e4 : 8.8e5));
+        else if (in1d)
+            tc = pts >= 2.6e5;
+        else  // radius 3 any size, radius 1 from 64 tiles
+            tc = fused || d->shape == CS_SHAPE_BOX2D3R || d->shape == CS_SHAPE_STAR2D3R ||
+                 ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64) >= 64;
+        r->sweeps_per_launch = cs::plan_fix_fp64(r->plan, tc);
     }
     // The FP64 FMA 2D kernel's tile rows: fixed here (the plan tuner would
     // time both on the worker thread); results do not depend on them.
