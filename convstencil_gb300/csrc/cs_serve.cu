@@ -463,29 +463,61 @@ void worker_main(cs_server *s)
 }
 
 // Packs a dense interior (row-major) into the plan's layout, zero halo.
-void pack(const cs_layout &L, const double *interior, double *buf)
+// fn(lo, hi) over [0, n) in up to `most` threads, the caller's among them. A
+// thread that cannot be started leaves its part to the caller.
+template <class Fn>
+void in_threads(long long n, long long most, const Fn &fn)
 {
-    memset(buf, 0, L.bytes);
-    const long long nx = L.extent[L.dims - 1];
-    const long long rows = L.dims == 1 ? 1 : L.dims == 2 ? L.extent[0] : L.extent[0] * L.extent[1];
-    for (long long r = 0; r < rows; ++r) {
-        long long off = L.origin;
-        if (L.dims == 2) off += r * L.pitch[0];
-        if (L.dims == 3) off += (r / L.extent[1]) * L.pitch[0] + (r % L.extent[1]) * L.pitch[1];
-        memcpy(buf + off, interior + r * nx, nx * sizeof(double));
+    const long long t = std::max(1LL, std::min({n, most, 8LL, (long long)std::thread::hardware_concurrency()}));
+    std::vector<std::thread> ths;
+    long long own = n / t;  // the caller's share; a failed thread's is added
+    std::vector<std::pair<long long, long long>> left;
+    for (long long i = 1; i < t; ++i) {
+        const long long lo = n * i / t, hi = n * (i + 1) / t;
+        try {
+            ths.emplace_back([&fn, lo, hi] { fn(lo, hi); });
+        } catch (...) {
+            left.push_back({lo, hi});
+        }
     }
+    fn(0, own);
+    for (const auto &p : left) fn(p.first, p.second);
+    for (auto &th : ths) th.join();
 }
 
-void unpack(const cs_layout &L, const double *buf, double *interior)
+// The rows of a layout between a dense interior and a padded buffer. Grids
+// above a few MB are copied by several threads: one moves 8 GB/s (result
+// arrays also take their page faults here), the link to the GPU 200.
+long long row_offset(const cs_layout &L, long long r)
+{
+    if (L.dims == 2) return L.origin + r * L.pitch[0];
+    if (L.dims == 3) return L.origin + (r / L.extent[1]) * L.pitch[0] + (r % L.extent[1]) * L.pitch[1];
+    return L.origin;
+}
+long long row_count(const cs_layout &L) { return L.dims == 1 ? 1 : L.dims == 2 ? L.extent[0] : L.extent[0] * L.extent[1]; }
+constexpr size_t kBytesPerThread = 1 << 20;
+
+void pack(const cs_layout &L, const double *interior, double *buf, long long threads)
+{
+    const long long nx = L.extent[L.dims - 1], rows = row_count(L);
+    in_threads(rows, threads, [&](long long lo, long long hi) {
+        long long end = lo == 0 ? 0 : row_offset(L, lo - 1) + nx;  // zeros up to each row, and after the last
+        for (long long r = lo; r < hi; ++r) {
+            const long long off = row_offset(L, r);
+            memset(buf + end, 0, (off - end) * sizeof(double));
+            memcpy(buf + off, interior + r * nx, nx * sizeof(double));
+            end = off + nx;
+        }
+        if (hi == rows) memset(buf + end, 0, (L.elements - end) * sizeof(double));
+    });
+}
+
+void unpack(const cs_layout &L, const double *buf, double *interior, long long threads)
 {
     const long long nx = L.extent[L.dims - 1];
-    const long long rows = L.dims == 1 ? 1 : L.dims == 2 ? L.extent[0] : L.extent[0] * L.extent[1];
-    for (long long r = 0; r < rows; ++r) {
-        long long off = L.origin;
-        if (L.dims == 2) off += r * L.pitch[0];
-        if (L.dims == 3) off += (r / L.extent[1]) * L.pitch[0] + (r % L.extent[1]) * L.pitch[1];
-        memcpy(interior + r * nx, buf + off, nx * sizeof(double));
-    }
+    in_threads(row_count(L), threads, [&](long long lo, long long hi) {
+        for (long long r = lo; r < hi; ++r) memcpy(interior + r * nx, buf + row_offset(L, r), nx * sizeof(double));
+    });
 }
 
 }  // namespace
@@ -535,7 +567,8 @@ namespace {
 
 // Everything a request needs before it is queued: plan, kernel choice,
 // packed host copy of its input (no server lock held).
-cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_ptr<Request> &out)
+cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_ptr<Request> &out,
+                          long long threads = 8)
 {
     if (!d || !d->interior_in || !d->weights || d->steps < 0) return CS_ERR_INVALID_ARGUMENT;
     auto r = std::make_unique<Request>();
@@ -631,7 +664,8 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
         cs_plan_destroy(r->plan);
         return CS_ERR_OUT_OF_MEMORY;
     }
-    pack(r->layout, d->interior_in, (double *)r->host);
+    pack(r->layout, d->interior_in, (double *)r->host,
+         std::min(threads, (long long)(r->layout.bytes / kBytesPerThread)));
     out = std::move(r);
     return CS_OK;
 }
@@ -686,13 +720,32 @@ CS_API cs_status cs_server_submit_many(cs_server *s, const cs_request_desc *reqs
 {
     if (!s || !reqs || !ids || count < 1) return CS_ERR_INVALID_ARGUMENT;
     std::vector<std::unique_ptr<Request>> rs(count);
+    // Prepared by several threads, one request each at a time.
+    double bytes = 0;
     for (int i = 0; i < count; ++i) {
-        const cs_status st = prepare_request(s, &reqs[i], rs[i]);
-        if (st != CS_OK) {
-            for (auto &r : rs) discard(s, r);
-            return st;
-        }
+        double b = sizeof(double);
+        for (int k = 0; k < 3; ++k) b *= (double)std::max(1LL, reqs[i].extent[k]);
+        bytes += b;
     }
+    std::atomic<int> next{0};
+    std::vector<cs_status> sts(count, CS_OK);
+    std::vector<std::string> errs(count);
+    in_threads(std::min(8, count), (long long)std::min(8.0, bytes / (double)kBytesPerThread),
+               [&](long long, long long) {
+                   int own = 0;
+                   cudaGetDevice(&own);
+                   if (own != s->device) cudaSetDevice(s->device);
+                   for (int i; (i = next.fetch_add(1)) < count;) {
+                       sts[i] = prepare_request(s, &reqs[i], rs[i], 1);
+                       if (sts[i] != CS_OK) errs[i] = cs_last_error();
+                   }
+                   if (own != s->device) cudaSetDevice(own);
+               });
+    for (int i = 0; i < count; ++i)
+        if (sts[i] != CS_OK) {
+            for (auto &r : rs) discard(s, r);
+            return cs::set_error(sts[i], errs[i].c_str());
+        }
     std::lock_guard<std::mutex> lk(s->mu);  // one lock: the worker sees all of them at once
     for (int i = 0; i < count; ++i) ids[i] = enqueue(s, std::move(rs[i]));
     s->cv_work.notify_one();
@@ -714,13 +767,19 @@ CS_API cs_status cs_server_wait(cs_server *s, long long id, double *interior_out
         if (s->cv_done.wait_until(lk, deadline) == std::cv_status::timeout && !r->retired)
             return CS_ERR_TIMEOUT;
     }
-    cs_status st = r->status;
-    if (r->state == State::Done && interior_out) unpack(r->layout, (const double *)r->host, interior_out);
-    if (latency_seconds) *latency_seconds = r->t_done - r->t_submit;
-    if (r->done_ev) cudaEventDestroy(r->done_ev);
-    s->pinned.put(r->host, r->host_cls);
-    cs_plan_destroy(r->plan);
-    s->all.erase(it);
+    // The request is this call's alone from here on: the worker may go on
+    // while the result is copied.
+    std::unique_ptr<Request> done = std::move(s->all.find(id)->second);
+    s->all.erase(id);
+    lk.unlock();
+    const cs_status st = done->status;
+    if (done->state == State::Done && interior_out)
+        unpack(done->layout, (const double *)done->host, interior_out,
+               (long long)(done->layout.bytes / kBytesPerThread));
+    if (latency_seconds) *latency_seconds = done->t_done - done->t_submit;
+    if (done->done_ev) cudaEventDestroy(done->done_ev);
+    s->pinned.put(done->host, done->host_cls);
+    cs_plan_destroy(done->plan);
     return st;
 }
 
