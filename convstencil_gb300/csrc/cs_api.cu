@@ -495,13 +495,17 @@ int size_class(const cs_plan *p)
 {
     long long pts = 1;
     for (int d = 0; d < p->dims; ++d) pts *= p->view.ext[d];
-    int c = 0;
+    int c = 0;  // log2
     while (pts > 1) {
-        pts >>= 2;
+        pts >>= 1;
         ++c;
     }
     return c;
 }
+
+// Launches of a candidate that the tuner times back to back: on small grids
+// several, since a single one is mostly its start.
+int tune_launches(const cs_plan *p) { return size_class(p) <= 20 ? 6 : 1; }
 
 // Picks the algorithm for a plan. With CS_ALGO_AUTO and more than one
 // candidate, the first sweep of the first run is timed once per candidate
@@ -561,11 +565,12 @@ cs_status choose_algo(cs_plan *p, const void *a, void *b, cudaStream_t st, int *
     cudaEvent_t e0, e1;
     CS_CUDA(cudaEventCreate(&e0));
     CS_CUDA(cudaEventCreate(&e1));
+    const int reps = tune_launches(p);
     for (int rep = 0; rep < 2; ++rep) {  // rep 0 warms up
         for (int ci = 0; ci < nc; ++ci) {
             const int c = cand[ci];
             CS_CUDA(cudaEventRecord(e0, st));
-            CS_CUDA(launch_sweep(p, c, a, b, st));
+            for (int i = 0; i < reps; ++i) CS_CUDA(launch_sweep(p, c, a, b, st));
             CS_CUDA(cudaEventRecord(e1, st));
             CS_CUDA(cudaEventSynchronize(e1));
             float ms = 0.f;
@@ -701,9 +706,9 @@ cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long
     return CS_OK;
 }
 
-// Tile rows of the FP64 FMA 2D kernel (16 or 32 rows per CTA tile): with
-// tile_rows 0 the first run times both once on a -> b (bitwise the same
-// sweep) and remembers the faster for plans of the same class.
+// Tile of the FP64 FMA 2D kernel (16 or 32 rows of 64 columns, or 16 rows of
+// 8): with tile_rows 0 the first run times them once on a -> b (bitwise the same
+// sweep) and remembers the fastest for plans of the same class.
 cs_status choose_tile_rows(cs_plan *p, int algo, const void *a, void *b, cudaStream_t st, int *out)
 {
     *out = 0;
@@ -728,11 +733,15 @@ cs_status choose_tile_rows(cs_plan *p, int algo, const void *a, void *b, cudaStr
     float best = 1e30f;
     int best_rows = 32;
     for (int rep = 0; rep < 2; ++rep) {
-        for (int rows : {16, 32}) {
+        for (int rows : {cs::kSmallTile, 16, 32}) {
+            // small tiles: not where there are many times as many as SMs
+            if (rows == cs::kSmallTile && p->view.ext[0] * p->view.ext[1] > (1 << 20)) continue;
             CS_CUDA(cudaEventRecord(e0, st));
-            cudaError_t e = cs::launch_fp64_fma(p->view, p->radius, p->pattern, p->w, (const double *)a + off,
-                                                (double *)b + off, st, rows);
-            if (e != cudaSuccess) return cuda_fail(e, "tile-rows tuning launch");
+            for (int i = 0; i < tune_launches(p); ++i) {
+                cudaError_t e = cs::launch_fp64_fma(p->view, p->radius, p->pattern, p->w, (const double *)a + off,
+                                                    (double *)b + off, st, rows);
+                if (e != cudaSuccess) return cuda_fail(e, "tile-rows tuning launch");
+            }
             CS_CUDA(cudaEventRecord(e1, st));
             CS_CUDA(cudaEventSynchronize(e1));
             float ms = 0.f;
@@ -1142,7 +1151,7 @@ CS_API cs_status cs_plan_get_algo(const cs_plan *p, int *algo)
 CS_API cs_status cs_plan_get_tile_rows(const cs_plan *p, int *rows)
 {
     if (!p || !rows) return fail(CS_ERR_INVALID_ARGUMENT, "NULL argument");
-    *rows = p->active_rows;
+    *rows = std::abs(p->active_rows);  // kSmallTile has 16 rows too
     return CS_OK;
 }
 

@@ -18,7 +18,16 @@
 //    K row covers an 8x10 input window: 20 DMMA per 64 outputs = 80 FMA per
 //    point. Still more FP64 work than the FMA form (49 per point), so the
 //    plan's tuner only picks it if it measures faster.
+//
+// Grids of at most one CTA per SM are launched with the programmatic stream
+// serialization attribute: the CTAs are scheduled while the previous sweep
+// finishes and wait for it (pdl_wait) before their first access. Larger ones
+// are not: scheduled among the previous sweep's CTAs they spread unevenly over
+// the SMs (box2d3r 192^2 on 288 small tiles, GB300: 9.5 us a sweep against
+// 6.1), except the small tiles of radius 1, whose FP64 work is short (star2d1r
+// 384^2, 1152 of them: 3.8 us against 5.3).
 #include "cs_internal.h"
+#include "cs_tc_common.cuh"
 
 #include <algorithm>
 
@@ -60,6 +69,8 @@ __global__ void __launch_bounds__(256) k1d_fma(const double *__restrict__ in,
 {
     constexpr int T = 1024;
     __shared__ double s[T + 2 * R];
+    tc::pdl_allow_dependents();
+    tc::pdl_wait();
     const long long x0 = (long long)blockIdx.x * T;
     for (int i = threadIdx.x; i < T + 2 * R; i += blockDim.x) {
         const long long gx = x0 - R + i;
@@ -92,6 +103,8 @@ __global__ void __launch_bounds__(256) k2d_fma(const double *__restrict__ in,
     constexpr int SX = TX + 2 * R, SY = TY + 2 * R;
     __shared__ double s[SY * SX];
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    tc::pdl_allow_dependents();
+    tc::pdl_wait();
     for (int idx = threadIdx.x; idx < SY * SX; idx += blockDim.x) {
         const int sy = idx / SX, sx = idx - sy * SX;
         const int gy = y0 - R + sy, gx = x0 - R + sx;
@@ -128,6 +141,40 @@ __global__ void __launch_bounds__(256) k2d_fma(const double *__restrict__ in,
     }
 }
 
+// The same sums on tiles of 16 rows and 8 columns, one output a thread: for
+// grids of so few points that the tiles above would leave most SMs idle. A
+// 64-column tile of a 49-tap kernel takes 15 us however small the grid (it
+// keeps four quarter-SM FP64 pipes busy, 77 cycles a warp FMA; box2d3r 96 x
+// 130, GB300: 18 of 152 SMs, 17.1 us a sweep); here it is 102 tiles, 4.1 us.
+// Up to 2^20 points the tuner measures both (star2d1r 512^2 4.9 and 6.1 us).
+template <int R, int P>
+__global__ void __launch_bounds__(128) k2d_fma_small(const double *__restrict__ in, double *__restrict__ out, int m,
+                                                     int n, long long ld, WK<(2 * R + 1) * (2 * R + 1)> w)
+{
+    constexpr int K = 2 * R + 1, TX = 8, TY = 16, WX = TX + 2 * R, SY = TY + 2 * R;
+    constexpr int SX = 24;  // two rows of a half-warp fall into different banks
+    __shared__ double s[SY * SX];
+    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    tc::pdl_allow_dependents();
+    tc::pdl_wait();
+#pragma unroll
+    for (int q = 0; q < (SY * WX + 127) / 128; ++q) {
+        const int idx = threadIdx.x + 128 * q, sy = idx / WX, sx = idx - sy * WX;
+        const int gy = y0 - R + sy, gx = x0 - R + sx;
+        if (idx < SY * WX) s[sy * SX + sx] = (gy < m + R && gx < n + R) ? __ldg(in + (long long)gy * ld + gx) : 0.0;
+    }
+    __syncthreads();
+    const int c = threadIdx.x & 7, g = threadIdx.x >> 3;
+    double acc = 0.0;
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (tap2<P, R>(i, j)) acc = fma(w.v[i * K + j], s[(g + i) * SX + c + j], acc);
+    const int y = y0 + g, x = x0 + c;
+    if (y < m && x < n) out[(long long)y * ld + x] = acc;
+}
+
 // ---------------------------------------------------------------- 3D
 // CTA column of 16 x 32 outputs marching ZC planes in z; a ring of 2R+1
 // input planes (with halo) lives in shared memory.
@@ -146,6 +193,8 @@ __global__ void __launch_bounds__(256) k3d_fma(const double *__restrict__ in,
     constexpr int K = 2 * R + 1, TX = 32, TY = 16;
     constexpr int SX = TX + 2 * R, SY = TY + 2 * R, PL = SX * SY;
     extern __shared__ double ring[];
+    tc::pdl_allow_dependents();
+    tc::pdl_wait();
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * zc;
     const int zend = min(z0 + zc, h);
 
@@ -205,6 +254,8 @@ __global__ void __launch_bounds__(256) k2d_mma(const double *__restrict__ in,
 {
     constexpr int R = 3, TX = 64, TY = 32, SX = TX + 2 * R + 2, SY = TY + 2 * R, KS = 20;
     __shared__ double s[SY * SX];
+    tc::pdl_allow_dependents();
+    tc::pdl_wait();
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     for (int idx = threadIdx.x; idx < SY * (TX + 2 * R); idx += blockDim.x) {
         const int sy = idx / (TX + 2 * R), sx = idx - sy * (TX + 2 * R);
@@ -251,6 +302,15 @@ WK<K> pack(const Weights &w)
 
 unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
+// Overlapping the previous sweep's end (`always`, or at most one CTA per SM).
+template <typename... Exp, typename... Act>
+cudaError_t launch(bool always, void (*kernel)(Exp...), dim3 grid, int block, size_t smem, cudaStream_t st,
+                   Act &&...args)
+{
+    const bool overlap = always || (long long)grid.x * grid.y * grid.z <= device_sm_count();
+    return tc::launch_overlapped(overlap, kernel, grid, block, smem, st, std::forward<Act>(args)...);
+}
+
 // Planes per CTA of the z-marching 3D kernels: 32 on large grids; fewer on
 // small ones, so that the grid still gives every SM several CTAs (a CTA
 // marches its planes one after another, so a small grid with 32-plane
@@ -264,26 +324,27 @@ int z_chunk(const GridView &g)
 }
 
 
-// Rows per CTA tile: 16 (4 per thread) or 32 (8 per thread); 0 picks 16 on
-// grids too small to give every SM several 32-row tiles. Both tile shapes sum
-// every point's taps in the same order, so results do not depend on it.
+// Rows per CTA tile: 16 (4 per thread) or 32 (8 per thread) of 64 columns, or
+// kSmallTile: 16 of 8 columns; 0 picks that up to 2^18 points and 16 on grids
+// too small to give every SM several 32-row tiles. All tile shapes sum every point's taps in the
+// same order, so results do not depend on it.
 template <int R, int P>
 cudaError_t go2d(const GridView &g, const Weights &w, const double *in, double *out, int tile_rows,
                  cudaStream_t st)
 {
     constexpr int K = 2 * R + 1;
     const unsigned gx = ceil_div(g.ext[1], 64);
+    if (tile_rows == 0 && g.ext[0] * g.ext[1] <= 1 << 18) tile_rows = kSmallTile;
     if (tile_rows == 0) tile_rows = (long long)gx * ceil_div(g.ext[0], 32) < 6LL * device_sm_count() ? 16 : 32;
-    if (tile_rows == 16) {
-        dim3 grid(gx, ceil_div(g.ext[0], 16));
-        k2d_fma<R, P, 4><<<grid, 256, 0, st>>>(in, out, (int)g.ext[0], (int)g.ext[1], g.pitch[0],
-                                                pack<K * K>(w));
-    } else {
-        dim3 grid(gx, ceil_div(g.ext[0], 32));
-        k2d_fma<R, P, 8><<<grid, 256, 0, st>>>(in, out, (int)g.ext[0], (int)g.ext[1], g.pitch[0],
-                                                pack<K * K>(w));
-    }
-    return cudaGetLastError();
+    const int m = (int)g.ext[0], n = (int)g.ext[1];
+    if (tile_rows == kSmallTile)
+        return launch(R == 1, k2d_fma_small<R, P>, dim3(ceil_div(n, 8), ceil_div(m, 16)), 128, 0, st, in, out,
+                                       m, n, g.pitch[0], pack<K * K>(w));
+    if (tile_rows == 16)
+        return launch(false, k2d_fma<R, P, 4>, dim3(gx, ceil_div(m, 16)), 256, 0, st, in, out, m, n,
+                                       g.pitch[0], pack<K * K>(w));
+    return launch(false, k2d_fma<R, P, 8>, dim3(gx, ceil_div(m, 32)), 256, 0, st, in, out, m, n, g.pitch[0],
+                                   pack<K * K>(w));
 }
 
 template <int R, int P>
@@ -295,19 +356,16 @@ cudaError_t go3d(const GridView &g, const Weights &w, const double *in, double *
     static_assert(smem <= 48 * 1024, "3D ring exceeds the default shared-memory window");
     const int zc = z_chunk(g);
     dim3 grid(ceil_div(g.ext[2], 32), ceil_div(g.ext[1], 16), ceil_div(g.ext[0], zc));
-    k3d_fma<R, P><<<grid, 256, smem, st>>>(in, out, (int)g.ext[0], (int)g.ext[1],
-                                            (int)g.ext[2], g.pitch[1], g.pitch[0], zc,
-                                            pack<K * K * K>(w));
-    return cudaGetLastError();
+    return launch(false, k3d_fma<R, P>, grid, 256, smem, st, in, out, (int)g.ext[0], (int)g.ext[1],
+                                   (int)g.ext[2], g.pitch[1], g.pitch[0], zc, pack<K * K * K>(w));
 }
 
 template <int R>
 cudaError_t go1d(const GridView &g, const Weights &w, const double *in, double *out,
                  cudaStream_t st)
 {
-    dim3 grid(ceil_div(g.ext[0], 1024));
-    k1d_fma<R><<<grid, 256, 0, st>>>(in, out, g.ext[0], pack<2 * R + 1>(w));
-    return cudaGetLastError();
+    return launch(false, k1d_fma<R>, dim3(ceil_div(g.ext[0], 1024)), 256, 0, st, in, out, g.ext[0],
+                                   pack<2 * R + 1>(w));
 }
 
 }  // namespace
@@ -365,9 +423,8 @@ cudaError_t launch_fp64_mma_2d(const GridView &g, const Weights &w, const double
 {
     note_launch();
     dim3 grid(ceil_div(g.ext[1], 64), ceil_div(g.ext[0], 32));
-    k2d_mma<<<grid, 256, 0, st>>>(in, out, (int)g.ext[0], (int)g.ext[1], g.pitch[0],
-                                  pack<49>(w));
-    return cudaGetLastError();
+    return launch(false, k2d_mma, grid, 256, 0, st, in, out, (int)g.ext[0], (int)g.ext[1], g.pitch[0],
+                                   pack<49>(w));
 }
 
 }  // namespace cs

@@ -43,14 +43,14 @@ __device__ __forceinline__ void pdl_allow_dependents()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Launches a sweep kernel with the programmatic stream serialization
-// attribute (see pdl_wait).
+// Launches a sweep kernel, with the programmatic stream serialization
+// attribute (see pdl_wait) where `overlap` is set.
 template <typename... Exp, typename... Act>
-cudaError_t launch_programmatic(void (*kernel)(Exp...), int grid, int block, size_t smem, cudaStream_t st,
-                                Act &&...args)
+cudaError_t launch_overlapped(bool overlap, void (*kernel)(Exp...), dim3 grid, int block, size_t smem,
+                              cudaStream_t st, Act &&...args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -58,8 +58,14 @@ cudaError_t launch_programmatic(void (*kernel)(Exp...), int grid, int block, siz
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...);
+}
+template <typename... Exp, typename... Act>
+cudaError_t launch_programmatic(void (*kernel)(Exp...), int grid, int block, size_t smem, cudaStream_t st,
+                                Act &&...args)
+{
+    return launch_overlapped(true, kernel, dim3((unsigned)grid), block, smem, st, std::forward<Act>(args)...);
 }
 
 __device__ __forceinline__ unsigned smem_addr(const void *p)
