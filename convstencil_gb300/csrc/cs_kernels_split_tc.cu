@@ -605,7 +605,9 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = S.tmem;
+    // All 512 columns are this CTA's, so they start at column 0: as a constant
+    // it costs the MMA thread no move into a uniform register per MMA.
+    const unsigned tmem = 0;
 
     if (warp == kWarpTma) {
         // ------------------------------------------------ TMA producer
@@ -678,27 +680,24 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                     g_bmat = g;
                 }
             }
-            int ok = 1;
-            if (lane == 0) {
-                ok = wait(bar2(S.planes_full, buf), use & 1) && wait(bar2(S.acc_empty, buf), (use & 1) ^ 1);
-                if (ok) {
-                    tc_fence_after();
-                    // The issuing thread stalls on every MMA until the tensor
-                    // core takes it, so nothing else sits between them: all
-                    // MMAs are unrolled, each descriptor one add of a
-                    // compile-time offset.
-                    const unsigned d_base = tmem + (unsigned)(kAccStride * buf);
-                    const unsigned long long a0 = buf ? a_desc_buf1 : a_desc_buf0;
-                    if constexpr (ONED)
-                        tile_mma_1d<D, 0, 0>(d_base, a0, b_desc0);
-                    else
-                        tile_mma<D, 0, 0>(d_base, a0, b_desc0);
-                    mma_commit(bar2(S.planes_empty, buf));  // planes may be overwritten
-                    mma_commit(bar2(S.acc_full, buf));      // accumulator ready
-                    committed = it + 1;
-                }
+            if (!__all_sync(0xffffffffu, wait(bar2(S.planes_full, buf), use & 1) &&
+                                             wait(bar2(S.acc_empty, buf), (use & 1) ^ 1)))
+                break;
+            tc_fence_after();
+            if (elect_one()) {
+                // The issuing thread stalls on every MMA until the tensor core
+                // takes it, so nothing else sits between them: all MMAs are
+                // unrolled, each descriptor one add of a compile-time offset.
+                const unsigned d_base = tmem + (unsigned)(kAccStride * buf);
+                const unsigned long long a0 = buf ? a_desc_buf1 : a_desc_buf0;
+                if constexpr (ONED)
+                    tile_mma_1d<D, 0, 0>(d_base, a0, b_desc0);
+                else
+                    tile_mma<D, 0, 0>(d_base, a0, b_desc0);
+                mma_commit(bar2(S.planes_empty, buf));  // planes may be overwritten
+                mma_commit(bar2(S.acc_full, buf));      // accumulator ready
             }
-            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+            committed = it + 1;
         }
     } else if (warp < kWarpEpi0) {
         // ------------------------------------------------ slicers
@@ -966,7 +965,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == kWarpTma)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kTmemCols));
 }
 
 template <class F, bool BATCH, int MODE = kModeGrid>

@@ -271,7 +271,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = S.tmem;
+    // All 512 columns are this CTA's, so they start at column 0: as a constant
+    // it costs the MMA thread no move into a uniform register per MMA.
+    const unsigned tmem = 0;
 
     if (warp == kWarpTma) {
         // ------------------------------------------------ TMA producer
@@ -297,22 +299,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         const unsigned long long a_desc0 = smem_desc(smem_addr(S.planes[0][0]), 16, kRowBytes);
         constexpr unsigned long long kSetUnits = (unsigned long long)D * PL * 2 / 16;
         const unsigned long long b_desc0 = smem_desc(smem_addr(S.bmat[0]), 128, 256);
-        if (lane == 0) {
-            int q = 0;
-            bool ok = true;
-            for (int item = first; item < items && ok; item += step) {
-                const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
-                for (int p = 0; p < wi.zn + 2; ++p, ++q) {
-                    const int slot = q % NPL, blk = q % NBLK;
-                    if (!(ok = wait(bar(S.planes_full, slot), (q / NPL) & 1) &&
-                               wait(bar(S.blk_empty, blk), ((q / NBLK) & 1) ^ 1)))
-                        break;
-                    tc_fence_after();
+        int q = 0;
+        bool ok = true;
+        for (int item = first; item < items && ok; item += step) {
+            const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
+            for (int p = 0; p < wi.zn + 2; ++p, ++q) {
+                const int slot = q % NPL, blk = q % NBLK;
+                if (!(ok = __all_sync(0xffffffffu, wait(bar(S.planes_full, slot), (q / NPL) & 1) &&
+                                                       wait(bar(S.blk_empty, blk), ((q / NBLK) & 1) ^ 1))))
+                    break;
+                tc_fence_after();
+                if (elect_one()) {
                     plane_mma<F, 0, 0>(tmem + (unsigned)(NCOL * blk), a_desc0 + kSetUnits * slot, b_desc0);
                     mma_commit(bar(S.blk_full, blk));       // block ready for the epilogue
                     mma_commit(bar(S.planes_empty, slot));  // digit planes may be overwritten
-                    committed = q + 1;
                 }
+                committed = q + 1;
             }
         }
     } else if ((kSliceMask >> warp) & 1u) {
@@ -690,7 +692,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == kWarpTma)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kTmemCols));
 }
 
 }  // namespace

@@ -30,16 +30,18 @@
 //     block of the 512, and a wait for the epilogue after every plane.)
 //   * Bound: the MMA stream and the shared memory it reads. An MMA reads 4 KB
 //     of A and N x 32 bytes of B, 60 cycles on average at 128 bytes a cycle;
-//     the 84 MMAs of a plane (1024 outputs) take 5,570 cycles with little else
-//     running and 7,260 of a plane's 8,350 beside the slicers and the epilogue
-//     (without the slicers' cutting the sweep runs 17 % faster, without the
-//     epilogue's arithmetic 8 %). GB300: 512^3 4.04 ms a sweep, 33 G
-//     outputs/s; the FP64 FMA kernel 1.5 (box), 8.3 (octahedron).
-//   * Roles (20 warps, five per scheduler, two of them idle, 96 registers):
-//     one loads windows (four stages), one thread issues the MMAs, two groups
-//     of four cut every second plane (ring of four digit-plane sets), eight
-//     drain the blocks and keep the seven running sums of four columns each.
-//     No slicer shares the MMA thread's scheduler.
+//     issued from registers the compiler knows to be uniform (elect_one, the
+//     TMEM base a constant) the 84 MMAs of a plane (1024 outputs) take 5,500
+//     cycles, of 6,100 per plane (issued under lane == 0: 7,260 of 8,350).
+//   * Roles (27 warps, seven per scheduler, one idle, 72 registers): one loads
+//     windows (four stages), one thread issues the MMAs, two groups of four
+//     cut every second plane (ring of four digit-plane sets), sixteen drain
+//     the blocks and keep the seven running sums of two columns each. No
+//     slicer shares the MMA thread's scheduler. (Eight draining four columns:
+//     7,000 cycles a plane, mostly waiting for their own TMEM loads, longer
+//     than the MMAs.) GB300, box 256^3: 545 us a sweep with lane == 0 and
+//     eight, 466 with elect_one, 398 with sixteen: 42 G outputs/s; the FP64
+//     FMA kernel 1.5 (box), 8.3 (octahedron).
 //   * Windows arrive by TMA where the layout allows it (even pitches,
 //     16-byte aligned base); the window then starts 4 columns left of the
 //     tile, or 3 where the interior's first column is odd, so that its
@@ -74,13 +76,12 @@ struct Weights7 {
 };
 
 constexpr int kGroups = 2, kGroupWarps = 4, kGroupThreads = 32 * kGroupWarps;
-constexpr int kEpiWarps = 8;
+constexpr int kEpiWarps = 16;
 constexpr int kWarpTma = 1, kWarpMma = 5;
-constexpr unsigned kEpiMask = (1u << 0) | (1u << 2) | (1u << 3) | (1u << 4) | (1u << 6) | (1u << 7) | (1u << 9) |
-                              (1u << 13);
-constexpr unsigned kSliceMask = (1u << 8) | (1u << 10) | (1u << 11) | (1u << 12) | (1u << 14) | (1u << 15) |
-                                (1u << 16) | (1u << 18);
-constexpr int kWarps = 20, kThreads = 32 * kWarps;  // warps 17 and 19 idle
+constexpr unsigned kEpiMask = 0x0000DDDDu | (1u << 9) | (1u << 13) | (1u << 17) | (1u << 21);
+constexpr unsigned kSliceMask = (1u << 16) | (1u << 18) | (1u << 19) | (1u << 20) | (1u << 22) | (1u << 23) |
+                                (1u << 24) | (1u << 26);
+constexpr int kWarps = 27, kThreads = 32 * kWarps;  // warp 25 idle
 static_assert(__builtin_popcount(kSliceMask) == kGroups * kGroupWarps && __builtin_popcount(kEpiMask) == kEpiWarps &&
                   (kSliceMask & kEpiMask) == 0 &&
                   ((kSliceMask | kEpiMask) & ((1u << kWarpTma) | (1u << kWarpMma))) == 0 &&
@@ -143,14 +144,12 @@ __device__ __forceinline__ Item item_of(int item, int tiles_x, int tiles_y, int 
     return Item{(rem - ty * tiles_x) * TX, ty * TY, chunk * zc, min(zc, h - chunk * zc)};
 }
 
-__device__ __forceinline__ void tmem_ld4(unsigned taddr, float (&v)[4])
+__device__ __forceinline__ void tmem_ld2(unsigned taddr, float (&v)[2])
 {
-    unsigned r[4];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(taddr));
+    unsigned r[2];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
+    for (int j = 0; j < 2; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 // x 2^-k, k >= 0 (the low bits lie far below the result's last one).
@@ -229,7 +228,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = S.tmem;
+    // All 512 columns are this CTA's, so they start at column 0: as a constant
+    // it costs the MMA thread no move into a uniform register per MMA.
+    const unsigned tmem = 0;
 
     if (warp == kWarpTma) {
         // ------------------------------------------------ window loads
@@ -276,27 +277,30 @@ __global__ void __launch_bounds__(kThreads, 1)
         const unsigned long long a_desc0 = smem_desc(smem_addr(S.planes[0][0]), 16, kRowBytes);
         constexpr unsigned long long kSetUnits = (unsigned long long)D * PL * 2 / 16;
         const unsigned long long b_desc0 = smem_desc(smem_addr(S.bmat[0][0]), 128, 256);
-        if (lane == 0) {
-            int q = 0;
-            bool ok = true;
-            for (int item = first; item < items && ok; item += step) {
-                const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
-                for (int p = 0; p < wi.zn + 6; ++p, ++q) {
-                    const int slot = q % NPL;
-                    const unsigned long long a = a_desc0 + kSetUnits * slot;
-                    if (!(ok = wait(bar(S.planes_full, slot), (q / NPL) & 1) && wait(bar(S.blk_empty, 0), (q & 1) ^ 1)))
-                        break;
-                    tc_fence_after();
+        int q = 0;
+        bool ok = true;
+        for (int item = first; item < items && ok; item += step) {
+            const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
+            for (int p = 0; p < wi.zn + 6; ++p, ++q) {
+                const int slot = q % NPL;
+                const unsigned long long a = a_desc0 + kSetUnits * slot;
+                if (!(ok = __all_sync(0xffffffffu, wait(bar(S.planes_full, slot), (q / NPL) & 1) &&
+                                                       wait(bar(S.blk_empty, 0), (q & 1) ^ 1))))
+                    break;
+                tc_fence_after();
+                if (elect_one()) {
                     half_mma<0, 0, 0>(tmem, a, b_desc0);
                     mma_commit(bar(S.blk_full, 0));
-                    committed = 2 * q + 1;
-                    if (!(ok = wait(bar(S.blk_empty, 1), (q & 1) ^ 1))) break;
-                    tc_fence_after();
+                }
+                committed = 2 * q + 1;
+                if (!(ok = __all_sync(0xffffffffu, wait(bar(S.blk_empty, 1), (q & 1) ^ 1)))) break;
+                tc_fence_after();
+                if (elect_one()) {
                     half_mma<1, 0, 0>(tmem + kBlkStride, a, b_desc0);
                     mma_commit(bar(S.blk_full, 1));
                     mma_commit(bar(S.planes_empty, slot));  // digit planes may be overwritten
-                    committed = 2 * q + 2;
                 }
+                committed = 2 * q + 2;
             }
         }
     } else if ((kSliceMask >> warp) & 1u) {
@@ -380,23 +384,23 @@ __global__ void __launch_bounds__(kThreads, 1)
         // columns 8 eb + 4 hh .. + 3. s[dz] is the running sum of the output
         // whose z tap dz the current input plane is, in units of its largest
         // plane exponent so far, se[dz] (the same in every thread).
-        const int quarter = warp & 3, hh = (warp >> 2) & 1;
+        const int quarter = warp & 3, hh = quarter == 1 ? (warp - 9) >> 2 : warp >> 2;
         const int mrow = 32 * quarter + lane;
         const int er = mrow >> 3, eb = mrow & 7;
-        const unsigned taddr = tmem + ((unsigned)(32 * quarter) << 16) + 4u * hh;
+        const unsigned taddr = tmem + ((unsigned)(32 * quarter) << 16) + 2u * hh;
         int q = 0;
         bool ok = true;
         for (int item = first; item < items && ok; item += step) {
             const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
-            const int xb = wi.x0 + 8 * eb + 4 * hh, yy = wi.y0 + er;
+            const int xb = wi.x0 + 8 * eb + 2 * hh, yy = wi.y0 + er;
             double *op = out + (long long)(wi.zs - 6) * ldz + (long long)yy * ldy + xb;
-            long long s[7][4];
+            long long s[7][2];
             int se[7];
 #pragma unroll
             for (int dz = 0; dz < 7; ++dz) {
                 se[dz] = 1;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) s[dz][c] = 0;
+                for (int c = 0; c < 2; ++c) s[dz][c] = 0;
             }
             unsigned bad = 0;  // bit k: the plane k back holds an Inf or NaN
             for (int p = 0; p < wi.zn + 6; ++p, ++q, op += ldz) {
@@ -413,66 +417,65 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                     for (int dl = 0; dl < (hz ? 3 : 4); ++dl) {
                         const int dz = 4 * hz + dl;
-                        float acc[D][4];
+                        float acc[D][2];
 #pragma unroll
-                        for (int L = 0; L < D; ++L) tmem_ld4(taddr + kBlkStride * hz + NLV * L + 8 * dl, acc[L]);
+                        for (int L = 0; L < D; ++L) tmem_ld2(taddr + kBlkStride * hz + NLV * L + 8 * dl, acc[L]);
                         tmem_wait_ld();
                         if (dl == (hz ? 2 : 3)) {  // block drained: hand it back
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) mbar_arrive(bar(S.blk_empty, hz));
                         }
-                        long long t[4];
+                        long long t[2];
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
+                        for (int c = 0; c < 2; ++c) {
                             const float lv[6] = {acc[0][c], acc[1][c], acc[2][c], acc[3][c], acc[4][c], acc[5][c]};
                             t[c] = f64_combine(lv);
                         }
                         if (dz == 0) {
                             se[0] = ex;
 #pragma unroll
-                            for (int c = 0; c < 4; ++c) s[0][c] = t[c];
+                            for (int c = 0; c < 2; ++c) s[0][c] = t[c];
                         } else {
                             if (ex != se[dz]) {
                                 const int up = max(ex - se[dz], 0), down = max(se[dz] - ex, 0);
 #pragma unroll
-                                for (int c = 0; c < 4; ++c) {
+                                for (int c = 0; c < 2; ++c) {
                                     s[dz][c] = shift_down(s[dz][c], up);
                                     t[c] = shift_down(t[c], down);
                                 }
                                 se[dz] += up;
                             }
 #pragma unroll
-                            for (int c = 0; c < 4; ++c) s[dz][c] += t[c];
+                            for (int c = 0; c < 2; ++c) s[dz][c] += t[c];
                         }
                     }
                 }
                 if (!ok) break;
                 if (p >= 6 && yy < m) {  // output p - 6 of the column has all its taps
-                    double res[4];
+                    double res[2];
                     const int sc = se[6] + sw.ew - 1080;
                     if (!(bad & 0x7Fu) && f64_scale_is_plain(sc)) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) res[c] = f64_from_fixed_plain(s[6][c], sc);
+                        for (int c = 0; c < 2; ++c) res[c] = f64_from_fixed_plain(s[6][c], sc);
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
+                        for (int c = 0; c < 2; ++c)
                             res[c] = (bad & 0x7Fu) ? __longlong_as_double(0x7FF8000000000000ll)
                                                    : f64_from_fixed(s[6][c], sc);
                     }
-                    if (vec2 && xb + 3 < n) {
+                    if (vec2 && xb + 1 < n) {
                         *reinterpret_cast<double2 *>(op) = make_double2(res[0], res[1]);
-                        *reinterpret_cast<double2 *>(op + 2) = make_double2(res[2], res[3]);
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
+                        for (int c = 0; c < 2; ++c)
                             if (xb + c < n) op[c] = res[c];
                     }
                 }
 #pragma unroll
                 for (int dz = 6; dz > 0; --dz) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) s[dz][c] = s[dz - 1][c];
+                    for (int c = 0; c < 2; ++c) s[dz][c] = s[dz - 1][c];
                     se[dz] = se[dz - 1];
                 }
             }
@@ -491,7 +494,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == kWarpTma)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kTmemCols));
 }
 
 // Digits of the 343 weights: as f64_slice_weights with the sum kept, and a

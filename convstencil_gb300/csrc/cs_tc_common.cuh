@@ -181,6 +181,20 @@ __host__ __device__ constexpr unsigned instr_desc(int n)
     return (1u << 4) | ((unsigned)(n >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
 }
 
+// One thread of a converged warp, the same one every time. The MMA warp walks
+// its loop as a whole and issues under this: under lane == 0 the compiler must
+// move every descriptor of every MMA from a thread's registers to the uniform
+// ones the instruction takes, and the issuing thread, not the tensor core, set
+// the pace (GB300, cycles per MMA beside the other roles, before and after:
+// 3D radius 1 106 and 80, radius 3 86 and 65; split box3d1r 512^3 930 and 750
+// us a sweep, box2d3r 8192^2 FP64 337 and 327).
+__device__ __forceinline__ bool elect_one()
+{
+    unsigned leader;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(leader));
+    return leader != 0;
+}
+
 __device__ __forceinline__ void mma_f16(unsigned d_tmem, unsigned long long a, unsigned long long b,
                                         unsigned idesc, unsigned accumulate)
 {
