@@ -273,10 +273,10 @@ struct cs_plan {
     Weights w;
     Weights w7;  // 2D plans: w at the centre of a 7x7 (the 2D tcgen05 kernels' tap window)
     // Kernels of several steps: 2D radius-1 plans, the 7x7 ones of 1, 2 and 3
-    // (launch_steps_tc); 1D plans, the 33 taps of 1 .. 16 / radius
+    // (launch_steps_tc); 1D plans, the 49 taps of 1 .. 24 / radius
     // (launch_steps_tc_1d).
     Weights w_steps[3];
-    double w1_steps[16][33];
+    double w1_steps[cs::kTcReach1d][2 * cs::kTcReach1d + 1];
     int max_steps = 0;  // steps per launch those allow (0: not even one)
     cs_layout layout;
     GridView view;
@@ -383,7 +383,7 @@ bool fp64_tc3d_r3_ok(const cs_plan *p)
 }
 
 // FP64 1D plans on the tcgen05 digit kernel (rows of 32 outputs, a reach of
-// 16 points: launch_steps_tc_1d), whatever their layout. Pinning FP64_TC
+// 24 points: launch_steps_tc_1d), whatever their layout. Pinning FP64_TC
 // keeps the conditions it had (fp64_tc1d_pin_ok); the tuner's candidate needs
 // no more than room for both ends of the grid.
 bool fp64_tc1d_geometry_ok(const cs_plan *p) { return p->dims == 1 && p->view.ext[0] >= 512 && p->max_steps >= 1; }
@@ -407,7 +407,7 @@ bool split_tc3d_ok(const cs_plan *p)
 // SMs without a tile, and a launch of ~12 us loses to single steps (FP64 FMA;
 // 512^2, 64 tiles, is where three of those take as long) or to the
 // double-float kernel's four per launch. 1D plans: the most steps, an odd
-// number, that reach at most 16 points, FP64 at any size (the tuner decides),
+// number, that reach at most 24 points, FP64 at any size (the tuner decides),
 // split from 64 tiles of 4096 points up.
 int steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base)
 {

@@ -105,10 +105,10 @@ cudaError_t launch_tc_batch(bool fp64, const void *records, int ngrids, int tota
 cudaError_t encode_split_window_map(CUtensorMap *map, const float2 *base, long long ld, long long rows,
                                     unsigned box_x, unsigned box_y);
 // `steps` steps of a 1D grid (FP64 or split) of n >= 64 points in one launch
-// of the tcgen05 digit kernel, steps * radius <= kTcReach1d: taps are the 33
-// taps of that many steps (the output's own at 16), w the 2 radius + 1 weights
+// of the tcgen05 digit kernel, steps * radius <= kTcReach1d: taps are the 49
+// taps of that many steps (the output's own at 24), w the 2 radius + 1 weights
 // of one.
-constexpr int kTcReach1d = 16;
+constexpr int kTcReach1d = 24;
 cudaError_t launch_steps_tc_1d(bool fp64, long long n, const double *taps, int radius, const double *w, int steps,
                                long long origin, const void *in_base, void *out_base, const TcWait &wait,
                                cudaStream_t stream);

@@ -94,10 +94,13 @@ using namespace tc;
 // kernel, so its light recombination runs on four warps (8192^2 on GB300:
 // 192 -> 204 GStencil/s against eight); the FP64 recombination (integer
 // operations) needs eight (120 GStencil/s on four, 169 on eight).
+// kCols: columns drained at a time. Four leave the FP64 kernels' registers
+// free of spills (three-step 8192^2 launch, GB300: 370 us with eight, 359 with
+// four; with twelve or sixteen slicer warps, 80 or 72 registers, 403 and 420).
 struct FmtSplit {
     static constexpr bool kF64 = false;
     static constexpr int kDigits = split::kDigits;  // 5
-    static constexpr int kEpiWarps = 4;
+    static constexpr int kEpiWarps = 4, kSliceWarps = 8, kCols = 8;
     using Out = float2;
     using Digits = split::SliceWeights;
 };
@@ -109,7 +112,7 @@ struct FmtSplit {
 struct FmtSplit6 {
     static constexpr bool kF64 = false;
     static constexpr int kDigits = 6;
-    static constexpr int kEpiWarps = 4;
+    static constexpr int kEpiWarps = 4, kSliceWarps = 8, kCols = 8;
     using Out = float2;
     using Digits = F64Weights;
 };
@@ -117,17 +120,16 @@ struct FmtSplit6 {
 struct FmtF64 {
     static constexpr bool kF64 = true;
     static constexpr int kDigits = 6;
-    static constexpr int kEpiWarps = 8;
+    static constexpr int kEpiWarps = 8, kSliceWarps = 8, kCols = 4;
     using Out = double;
     using Digits = F64Weights;
 };
 
 // Warp roles.
-constexpr int kSliceWarps = 8;
-constexpr int kWarpTma = 0, kWarpMma = 1, kWarpSlice0 = 2, kWarpEpi0 = kWarpSlice0 + kSliceWarps;
+constexpr int kWarpTma = 0, kWarpMma = 1, kWarpSlice0 = 2;
 template <class F>
-constexpr int kThreads = 32 * (kWarpEpi0 + F::kEpiWarps);  // 448 split, 576 FP64
-constexpr int kSliceThreads = 32 * kSliceWarps;
+constexpr int kThreads = 32 * (kWarpSlice0 + F::kSliceWarps + F::kEpiWarps);  // 448 split, 576 FP64
+constexpr int kMaxSliceWarps = 8;
 constexpr int kSliceBarrier = 1;           // named barrier of the slicer warps
 constexpr int kBuildBarrier = 2;           // named barrier of the warps that build B
 
@@ -144,22 +146,26 @@ constexpr int kAccStride = 256;            // TMEM columns between the two accum
 constexpr int kTmemCols = 512;
 constexpr unsigned kStageBytes = ST_X * ST_Y * 8;  // 40,320 (8-byte points)
 constexpr int PAIRS = ST_X / 2, NPAIR = ST_Y * PAIRS;           // 36, 2,520
-constexpr int PER = (NPAIR + kSliceThreads - 1) / kSliceThreads;  // 10
-// 1D (kMode1d): a tile is 4096 outputs, 128 rows of 32; row m of A is the 64
-// points around output row m, read in four K steps. The window is 4096 + 32
-// points, 516 chunks of 8; chunk j sits in phase j % 4 at place j / 4, so the
-// rows' chunks of one K step (two phases, places m or m + 1) are core matrices
+// 1D (kMode1d): a tile is 4096 outputs, 128 rows of 32; row m of A is the 80
+// points around output row m, read in five K steps. The window is 4096 + 48
+// points, 518 chunks of 8; chunk j sits in phase j % 4 at place j / 4, so the
+// rows' chunks of one K step (two phases, places m .. m + 2) are core matrices
 // of consecutive 16-byte rows: the canonical non-swizzled layout again, each
-// point stored once.
-constexpr int kReach1d = kTcReach1d;                // points either side of an output: 16
+// point stored once. The reach is the largest whose 2 * 24 + 1 taps keep the
+// level sums exact, as the 49 of a 7x7 do (with a reach of 16, four K steps,
+// a launch took the same time, set by the slicers, for two thirds of the
+// steps: 1d2r 10,240,000 x 100, GB300, 852 us, so 597).
+constexpr int kReach1d = kTcReach1d;                // points either side of an output: 24
 constexpr int kOut1d = 4096, kWin1d = kOut1d + 2 * kReach1d, NPAIR1D = kWin1d / 2;
 constexpr int kSteps1d = (32 + 2 * kReach1d) / 16;  // K steps
-// bytes between phases: 129 chunks, rounded so that the words a slicer warp
-// stores (16 per phase pair) fall into different banks
+// bytes between phases: 130 chunks; the words a slicer warp stores (16 per
+// phase pair) then fall into different banks
 constexpr int kPhase1d = 2080;
 constexpr unsigned kBytes1d = kWin1d * 8;
-static_assert(4 * kPhase1d <= PL * 2 && kBytes1d <= kStageBytes && NPAIR1D <= PER * kSliceThreads &&
-                  kPhase1d >= (kWin1d / 32) * 16 && kPhase1d / 4 % 32 == 8,
+constexpr int kFrame1d = 2 * kReach1d;              // points of an end computed step by step (frame_end_1d)
+static_assert(2 * kReach1d + 1 <= 49, "level sums are exact for 49 taps");
+static_assert(4 * kPhase1d <= PL * 2 && kBytes1d <= kStageBytes && NPAIR1D <= NPAIR &&
+                  kPhase1d >= (kWin1d + 31) / 32 * 16 && kPhase1d / 4 % 32 == 8,
               "the 1D window and digits fit the 2D buffers");
 static_assert(FmtSplit::kEpiWarps == 4 && FmtF64::kEpiWarps == 8 && R == 4,
               "one or two epilogue warps per TMEM lane quarter, R / (warps per quarter) rows each");
@@ -176,11 +182,12 @@ struct Smem {
     unsigned long long stage_full, stage_empty;
     unsigned long long planes_full[2], planes_empty[2];
     unsigned long long acc_full[2], acc_empty[2];
+    unsigned long long ends[2][2][kFrame1d];   // 1D: the two ends, two levels
     unsigned tmem;                             // TMEM base column
     int abort;                                 // set by the first expired wait
     int scale_exp[4];                          // per-tile input scale, ring of 4
-    float red[2][kSliceWarps];                 // split: per-warp max |hi|, by tile parity
-    int redi[2][kSliceWarps];                  // FP64: per-warp max biased exponent
+    float red[2][kMaxSliceWarps];                 // split: per-warp max |hi|, by tile parity
+    int redi[2][kMaxSliceWarps];                  // FP64: per-warp max biased exponent
 };
 
 static_assert(sizeof(Smem<FmtF64>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 128 <= 232448 &&
@@ -275,10 +282,10 @@ __device__ __forceinline__ void build_bmat(Smem<F> &S, int t0, int nt)
     }
 }
 
-// The same for 1D: the 33 taps of digit e at wz1[e][32 .. 64] (the rows of wz,
+// The same for 1D: the 49 taps of digit e at wz1[e][32 .. 80] (the rows of wz,
 // laid end to end), and B of K step kk: N row nn = 32 e + c (output c of a
 // row), tap 16 kk + k - c.
-constexpr int kWz1d = 96;
+constexpr int kWz1d = 112;
 static_assert(FmtF64::kDigits * kWz1d <= FmtF64::kDigits * 7 * kWz, "the 1D rows fit wz");
 template <class F>
 __device__ __forceinline__ void stage_digits_1d(Smem<F> &S, const typename F::Digits &sw, int t0, int nt)
@@ -373,12 +380,6 @@ __device__ __forceinline__ float2 next_lane(float2 x)
 {
     return make_float2(__shfl_down_sync(0xffffffffu, x.x, 1), __shfl_down_sync(0xffffffffu, x.y, 1));
 }
-__device__ __forceinline__ double lane_of(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
-__device__ __forceinline__ float2 lane_of(float2 x, int src)
-{
-    return make_float2(__shfl_sync(0xffffffffu, x.x, src), __shfl_sync(0xffffffffu, x.y, src));
-}
-
 // One strip of the frame, by one warp: T steps for the T - 1 points next to
 // an edge, at positions l0 .. l0 + 25 along it. `edge` is the offset of
 // the edge's first point, `sa` the step away from the edge, `sl` the step
@@ -462,28 +463,33 @@ __device__ __noinline__ void frame_steps(const StepArgs<F> &s, typename F::Out *
     }
 }
 
-// The (T - 1) r outputs next to one end of a 1D grid (T r <= 16), by one warp:
-// lane l holds point l - r counted from that end, as frame_strip's lanes do.
+// The (T - 1) r outputs next to one end of a 1D grid (T r <= 24), by one warp:
+// points -r .. 2 T r - r - 1 counted from that end, two per lane, in `buf`
+// (level l's in buf[l % 2]); every level's last r points fall out of use.
 template <class F>
-__device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out *__restrict__ out, int n, bool left)
+__device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out *__restrict__ out, int n, bool left,
+                                          typename F::Out (*buf)[kFrame1d])
 {
     using V = typename F::Out;
-    const int lane = threadIdx.x & 31, r = s.radius, p = lane - r;
-    const long long at = left ? p : n - 1 - p;
-    const bool halo = p < 0;
-    const V even = s.in[at], odd = halo ? out[at] : V{};
-    V u = even;
+    const int lane = threadIdx.x & 31, r = s.radius, points = 2 * s.steps * r;
+    auto at = [&](int i) { return (long long)(left ? i - r : n - 1 - (i - r)); };  // point i - r from this end
+    for (int i = lane; i < points; i += 32) {
+        buf[0][i] = s.in[at(i)];
+        if (i < r) buf[1][i] = out[at(i)];  // the halo that odd levels read
+    }
+    __syncwarp();
 #pragma unroll 1
     for (int level = 1; level <= s.steps; ++level) {
-        V v{};
+        const V *u = buf[(level & 1) ^ 1];
+        for (int i = r + lane; i < points - level * r; i += 32) {
+            V v{};
 #pragma unroll 1
-        for (int t = 0; t <= 2 * r; ++t) {
-            const int d = left ? t - r : r - t;  // the tap's lane, towards the interior from this end
-            tap_acc(v, s.w[t], lane_of(u, (lane + d) & 31));
+            for (int t = 0; t <= 2 * r; ++t) tap_acc(v, s.w[left ? t : 2 * r - t], u[i - r + t]);
+            buf[level & 1][i] = tap_sum(v);
         }
-        u = halo ? ((level & 1) ? odd : even) : tap_sum(v);
+        __syncwarp();
     }
-    if (!halo && p < (s.steps - 1) * r) out[at] = u;
+    for (int i = r + lane; i < s.steps * r; i += 32) out[at(i)] = buf[s.steps & 1][i];
 }
 
 // One grid (BATCH = false: kernel parameters describe it, tiles are dealt
@@ -499,7 +505,9 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
 {
     constexpr bool ONED = MODE == kMode1d, STEPS = MODE == kModeSteps;
     static_assert(!BATCH || MODE == kModeGrid, "batches run one sweep of 7x7 grids");
-    constexpr int D = F::kDigits;
+    constexpr int D = F::kDigits, kSliceWarps = F::kSliceWarps, kSliceThreads = 32 * kSliceWarps;
+    constexpr int kWarpEpi0 = kWarpSlice0 + kSliceWarps;
+    constexpr int PER = (NPAIR + kSliceThreads - 1) / kSliceThreads;  // pairs of points a slicer holds
     using SM = Smem<F>;
     extern __shared__ unsigned char smem_raw[];
     SM &S = *reinterpret_cast<SM *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
@@ -839,7 +847,8 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         if constexpr (ONED) {  // the ends, on the last CTA (no other has fewer tiles)
             if (blockIdx.x == gridDim.x - 1 && warp < kWarpEpi0 + 2 && sa.steps > 1) {
                 pdl_wait();
-                frame_end_1d<F>(sa, out, n, warp == kWarpEpi0);
+                frame_end_1d<F>(sa, out, n, warp == kWarpEpi0,
+                                reinterpret_cast<typename F::Out(*)[kFrame1d]>(S.ends[warp - kWarpEpi0][0]));
             }
         }
         const int quarter = warp & 3, h = (warp - kWarpEpi0) >> 2;
@@ -866,43 +875,45 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             const int ex = S.scale_exp[it & 3];
             const int xb = x0 + 8 * eb;
             constexpr int kRowsPerWarp = R * 4 / F::kEpiWarps;  // 4 split, 2 FP64
+            constexpr int C = F::kCols, kPasses = kRowsPerWarp * 8 / C;
 #pragma unroll 1
-            for (int pass = 0; pass < kRowsPerWarp; ++pass) {
-                const int rho = kRowsPerWarp * h + pass;
-                float acc[D][8];
+            for (int pass = 0; pass < kPasses; ++pass) {
+                const int rho = kRowsPerWarp * h + pass * C / 8;
+                const int c0 = pass * C % 8;  // first of the C columns of this pass
+                float acc[D][C];
 #pragma unroll
                 for (int L = 0; L < D; ++L)
-                    tmem_ld8(tmem + lane_bits + (unsigned)(kAccStride * buf + NLV * L + 8 * rho), acc[L]);
+                    tmem_ldc(tmem + lane_bits + (unsigned)(kAccStride * buf + NLV * L + 8 * rho + c0), acc[L]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (pass == kRowsPerWarp - 1) {  // accumulator drained: hand it back to the MMA warp
+                if (pass == kPasses - 1) {  // accumulator drained: hand it back to the MMA warp
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar2(S.acc_empty, buf));
                 }
-                typename F::Out res[8];
+                typename F::Out res[C];
                 if constexpr (F::kF64) {
                     // value = T 2^c with T from the levels (f64_combine) and
                     // c = (input scale) + (weight scale) - 1080.
                     const int c = ex + ew - 1080;
-                    long long t[8];
+                    long long t[C];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < C; ++j) {
                         const float lv[6] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4][j], acc[5][j]};
                         t[j] = f64_combine(lv);
                     }
                     if (f64_scale_is_plain(c)) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) res[j] = f64_from_fixed_plain(t[j], c);
+                        for (int j = 0; j < C; ++j) res[j] = f64_from_fixed_plain(t[j], c);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
+                        for (int j = 0; j < C; ++j)
                             res[j] = ex == kNonFiniteTile ? __longlong_as_double(0x7FF8000000000000ll)
                                                           : f64_from_fixed(t[j], c);
                     }
                 } else {
                     const float scale = ldexpf(1.0f, ex + ew - 2 * kDigitBits);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    for (int j = 0; j < C; ++j) {
                         float h1, e1, h2, e2, hi, lo;
                         two_sum(acc[0][j], acc[1][j] * 0x1p-9f, h1, e1);
                         two_sum(h1, acc[2][j] * 0x1p-18f, h2, e2);
@@ -921,31 +932,31 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 };
                 if constexpr (ONED) {
                     // outputs 32 mrow + 8 rho .. + 7 of the tile
-                    const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d + 32 * mrow + 8 * rho;
-                    if (sa.aligned && x >= frame && x + 8 <= n - frame) {
+                    const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d + 32 * mrow + 8 * rho + c0;
+                    if (sa.aligned && x >= frame && x + C <= n - frame) {
 #pragma unroll
-                        for (int j = 0; j < 8; j += 2) store2(out + x + j, res[j], res[j + 1]);
+                        for (int j = 0; j < C; j += 2) store2(out + x + j, res[j], res[j + 1]);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
+                        for (int j = 0; j < C; ++j)
                             if (x + j >= frame && x + j < n - frame) out[x + j] = res[j];
                     }
                 } else {
-                    const int yy = y0 + R * er + rho;
+                    const int yy = y0 + R * er + rho, xc = xb + c0;
                     if (yy >= o_m) continue;
                     if (STEPS && (yy < frame || yy >= o_m - frame)) continue;
-                    typename F::Out *o = o_base + (long long)yy * o_ld + xb;
-                    if (STEPS && (xb < frame || xb + 8 > o_n - frame)) {
+                    typename F::Out *o = o_base + (long long)yy * o_ld + xc;
+                    if (STEPS && (xc < frame || xc + C > o_n - frame)) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (xb + j >= frame && xb + j < o_n - frame) o[j] = res[j];
+                        for (int j = 0; j < C; ++j)
+                            if (xc + j >= frame && xc + j < o_n - frame) o[j] = res[j];
                         continue;
                     }
 #pragma unroll
-                    for (int j = 0; j < 8; j += 2) {
-                        if (xb + j + 1 < o_n)
+                    for (int j = 0; j < C; j += 2) {
+                        if (xc + j + 1 < o_n)
                             store2(o + j, res[j], res[j + 1]);
-                        else if (xb + j < o_n)
+                        else if (xc + j < o_n)
                             o[j] = res[j];
                     }
                 }
@@ -1106,7 +1117,7 @@ cudaError_t launch_steps_1d(long long n, const double *taps, int radius, const d
     cudaError_t e = set_smem_attr<F, false, kMode1d>();
     if (e != cudaSuccess) return e;
     Weights wT;
-    for (int i = 0; i < 49; ++i) wT.v[i] = i <= 2 * kReach1d ? taps[i] : 0.0;
+    for (int i = 0; i < 49; ++i) wT.v[i] = taps[i];
     StepArgs<F> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, radius, 0, 0u, 0, {}};
     sa.aligned = origin % 2 == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0 &&
                  reinterpret_cast<uintptr_t>(out_base) % 16 == 0;

@@ -210,7 +210,16 @@ __device__ __forceinline__ void mma_commit(unsigned bar)
                  : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld8(unsigned taddr, float (&v)[8])
+__device__ __forceinline__ void tmem_ldc(unsigned taddr, float (&v)[4])
+{
+    unsigned r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
+}
+__device__ __forceinline__ void tmem_ldc(unsigned taddr, float (&v)[8])
 {
     unsigned r[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"

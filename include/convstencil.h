@@ -84,7 +84,7 @@ typedef enum cs_semantics { CS_SEM_STEP = 0, CS_SEM_FUSED = 1 } cs_semantics;
  *                other kernels use double-float FP32 arithmetic. 2D radius-1
  *                and 1D plans of at least 64 tiles (64x64 or 4096 points)
  *                also run on the tensor cores where the tuner measures it
- *                faster, 3 to 15 steps per launch, with six digits per
+ *                faster, 3 to 23 steps per launch, with six digits per
  *                operand: inputs keep 52 bits below their tile's largest
  *                value, results are rounded to pairs once per launch. Relative
  *                error per sweep ~1e-13. Inputs must be finite. Pin
