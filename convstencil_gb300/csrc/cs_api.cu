@@ -960,8 +960,6 @@ CS_API cs_status cs_device_wait_timeouts(unsigned *count, int reset)
     unsigned c3 = 0;
     CS_CUDA(cs::split_tc3d_wait_timeouts(&c3, reset != 0));
     b += c3;
-    CS_CUDA(cs::tc3d_r3_wait_timeouts(&c3, reset != 0));
-    b += c3;
     *count = a + b;
     return CS_OK;
 }

@@ -142,7 +142,8 @@ int device_sm_count();
 cudaError_t split_wait_timeouts(unsigned *count, bool reset);
 cudaError_t split_tc_wait_timeouts(unsigned *count, bool reset);
 cudaError_t split_tc3d_wait_timeouts(unsigned *count, bool reset);
-cudaError_t tc3d_r3_wait_timeouts(unsigned *count, bool reset);
+// Device address of the 3D kernels' counter, which the radius-3 ones share.
+cudaError_t tc3d_wait_counter(unsigned **counter);
 // Whole-buffer conversions over n elements, and the in-place forms used by
 // the FP64 re-anchor sweeps ((hi, lo) pairs and FP64 values share a buffer
 // layout: 8 bytes per point).

@@ -759,6 +759,11 @@ cudaError_t launch_fp64_sweep_tc3d(const GridView &g, const Weights &w, long lon
     return launch_tc3d<F3F64>(g, f64_slice_weights(w, 27), origin, elements, in_base, out_base, wt, st);
 }
 
+cudaError_t tc3d_wait_counter(unsigned **counter)
+{
+    return cudaGetSymbolAddress((void **)counter, g_tc3d_wait_timeouts);
+}
+
 cudaError_t split_tc3d_wait_timeouts(unsigned *count, bool reset)
 {
     cudaError_t e = cudaMemcpyFromSymbol(count, g_tc3d_wait_timeouts, sizeof(unsigned));

@@ -50,8 +50,8 @@
 //     plane hide behind the MMAs: 200 x 184 x 193 runs at the rate of its tiles).
 //
 // Every mbarrier wait is bounded (WaitCfg, 2 s by default); an expired wait is
-// counted in g_tc3d_r3_wait_timeouts and the CTA leaves as in the other
-// tcgen05 kernels.
+// counted beside those of the radius-1 kernels (one counter, so that the
+// synchronous runs read no further one) and the CTA leaves as in those.
 #include "cs_internal.h"
 #include "cs_split_common.cuh"
 #include "cs_tc_common.cuh"
@@ -60,8 +60,6 @@
 #include <algorithm>
 
 namespace cs {
-
-__device__ unsigned int g_tc3d_r3_wait_timeouts;
 
 namespace {
 
@@ -159,7 +157,8 @@ template <bool TMA>
 __global__ void __launch_bounds__(kThreads, 1)
     k3d_tc_r3(const __grid_constant__ CUtensorMap tmap, const double *__restrict__ in, double *__restrict__ out, int h,
               int m, int n, long long ldy, long long ldz, int tiles_x, int tiles_y, int zc, int items, int map_x,
-              int map_y, int map_z, int left, int vec2, const __grid_constant__ Weights7 sw, WaitCfg wc)
+              int map_y, int map_z, int left, int vec2, const __grid_constant__ Weights7 sw, WaitCfg wc,
+              unsigned *timeouts)
 {
     extern __shared__ unsigned char smem_raw[];
     Smem &S = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
@@ -168,8 +167,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     volatile int *abort = &S.abort;
     auto bar = [](unsigned long long *b, int i) { return smem_addr(&b[i]); };
     const unsigned long long limit = wc.limit_ns;
-    auto wait = [abort, limit](unsigned b, unsigned parity) {
-        return mbar_wait(b, parity, abort, &g_tc3d_r3_wait_timeouts, limit);
+    auto wait = [abort, limit, timeouts](unsigned b, unsigned parity) {
+        return mbar_wait(b, parity, abort, timeouts, limit);
     };
     const int first = blockIdx.x, step = gridDim.x;
 
@@ -488,9 +487,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     if (warp == kWarpTma && lane == 0)
         for (int l = max(0, issued - kStages); l < issued; ++l)
-            mbar_drain(bar(S.stage_full, l % kStages), (l / kStages) & 1, &g_tc3d_r3_wait_timeouts);
+            mbar_drain(bar(S.stage_full, l % kStages), (l / kStages) & 1, timeouts);
     if (warp == kWarpMma && lane == 0 && committed > 0)
-        mbar_drain(bar(S.blk_full, (committed - 1) & 1), ((committed - 1) / 2) & 1, &g_tc3d_r3_wait_timeouts);
+        mbar_drain(bar(S.blk_full, (committed - 1) & 1), ((committed - 1) / 2) & 1, timeouts);
     __syncthreads();
     tc_fence_after();
     if (warp == kWarpTma)
@@ -543,6 +542,9 @@ cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long 
                                                          elements / ldz, ST_X, ST_Y);
         if (e != cudaSuccess) return e;
     }
+    unsigned *timeouts = nullptr;
+    const cudaError_t ce = tc3d_wait_counter(&timeouts);
+    if (ce != cudaSuccess) return ce;
     const size_t smem = sizeof(Smem) + 128;
     auto kernel = tma ? k3d_tc_r3<true> : k3d_tc_r3<false>;
     static const cudaError_t attr[2] = {
@@ -566,15 +568,7 @@ cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long 
     return launch_programmatic(kernel, std::min(items, sms), kThreads, smem, st, map, in_base + origin,
                                out_base + origin, h, m, n, ldy, ldz, tiles_x, tiles_y, zc, items, map_x,
                                (int)((origin % ldz) / ldy), (int)(origin / ldz), left, vec2 ? 1 : 0, slice_weights7(w),
-                               WaitCfg{wt.limit_ns, wt.skip_loads});
-}
-
-cudaError_t tc3d_r3_wait_timeouts(unsigned *count, bool reset)
-{
-    cudaError_t e = cudaMemcpyFromSymbol(count, g_tc3d_r3_wait_timeouts, sizeof(unsigned));
-    if (e != cudaSuccess || !reset) return e;
-    const unsigned zero = 0;
-    return cudaMemcpyToSymbol(g_tc3d_r3_wait_timeouts, &zero, sizeof(unsigned));
+                               WaitCfg{wt.limit_ns, wt.skip_loads}, timeouts);
 }
 
 }  // namespace cs
