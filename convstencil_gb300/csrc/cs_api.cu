@@ -350,6 +350,11 @@ bool fp64_tc_geometry_ok(const cs_plan *p)
            cs::split_mma_layout_ok(p->view, p->layout.origin);
 }
 
+bool tc_bases_ok(const void *in_base, const void *out_base)
+{
+    return reinterpret_cast<uintptr_t>(in_base) % 16 == 0 && reinterpret_cast<uintptr_t>(out_base) % 16 == 0;
+}
+
 // Buffers and layout the 2D FP64 tcgen05 sweep can read by TMA: even pitch
 // and interior column (the window's first column, 4 to the left of a tile,
 // must be 16-byte aligned), 16-byte aligned bases. Window rows and columns
@@ -359,11 +364,19 @@ bool fp64_tc_geometry_ok(const cs_plan *p)
 bool fp64_tc_window_ok(const GridView &v, long long off, const void *in_base, const void *out_base)
 {
     const long long ld = v.pitch[0];
-    return v.dims == 2 && ld % 2 == 0 && (off % ld) % 2 == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0 &&
-           reinterpret_cast<uintptr_t>(out_base) % 16 == 0;
+    return v.dims == 2 && ld % 2 == 0 && (off % ld) % 2 == 0 && tc_bases_ok(in_base, out_base);
 }
 
-bool fp64_tc_ok(const cs_plan *p) { return p->prec == CS_PREC_FP64 && fp64_tc_geometry_ok(p); }
+// Pinning FP64_TC wants that geometry; the tuner's candidate also runs on odd
+// pitches and first columns (ODD_FIGURES).
+bool fp64_tc_pin_ok(const cs_plan *p) { return p->prec == CS_PREC_FP64 && fp64_tc_geometry_ok(p); }
+bool fp64_tc_ok(const cs_plan *p)
+{
+    const cs_layout &L = p->layout;
+    return fp64_tc_pin_ok(p) ||
+           (p->prec == CS_PREC_FP64 && p->dims == 2 && p->radius <= 3 && p->view.ext[0] >= 8 &&
+            p->view.ext[1] >= 8 && L.origin / L.pitch[0] + L.extent[0] + p->radius <= L.elements / L.pitch[0]);
+}
 
 // FP64 plans of 3D radius-1 stencils run on the 3D tcgen05 digit pipeline
 // (the same work items as the split 3D kernel, six digits per point). The
@@ -413,9 +426,10 @@ int steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base
 {
     const bool fp64 = p->prec == CS_PREC_FP64;
     if (p->dims == 1) return fp64_tc1d_geometry_ok(p) && (fp64 || p->view.ext[0] > 63 * 4096) ? p->max_steps : 1;
-    if (p->max_steps < 2 || !fp64_tc_geometry_ok(p) ||
-        !fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base))
-        return 1;
+    const bool ok = fp64 ? fp64_tc_ok(p) && tc_bases_ok(in_base, out_base)
+                         : fp64_tc_geometry_ok(p) &&
+                               fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base);
+    if (p->max_steps < 2 || !ok) return 1;
     const long long tiles = ((p->view.ext[0] + 63) / 64) * ((p->view.ext[1] + 63) / 64);
     return tiles >= 64 ? p->max_steps : 1;
 }
@@ -427,7 +441,8 @@ cudaError_t launch_steps(const cs_plan *p, bool fp64, int steps, const void *in_
         return cs::launch_steps_tc_1d(fp64, p->view.ext[0], p->w1_steps[steps - 1], p->radius, p->w.v, steps,
                                       p->layout.origin, in_base, out_base, p->wait, st);
     return cs::launch_steps_tc(fp64, p->view, p->w_steps[steps - 1], p->w, steps, p->layout.origin,
-                               p->layout.elements, in_base, out_base, p->wait, st);
+                               p->layout.elements, in_base, out_base, p->wait, st,
+                               fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base));
 }
 
 // One sweep over the slabs [row0, row0 + rows) of the slowest axis (rows of
@@ -453,9 +468,10 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
         if (algo == CS_ALGO_FP64_TC && fp64_tc3d_r3_ok(p))
             return cs::launch_fp64_sweep_tc3d_r3(v, p->w, off, p->layout.elements, (const double *)in_base,
                                                  (double *)out_base, p->wait, st);
-        if (algo == CS_ALGO_FP64_TC && fp64_tc_ok(p) && fp64_tc_window_ok(v, off, in_base, out_base))
+        if (algo == CS_ALGO_FP64_TC && fp64_tc_ok(p) && tc_bases_ok(in_base, out_base))
             return cs::launch_fp64_sweep_tc(v, p->w7, off, p->layout.elements, (const double *)in_base,
-                                            (double *)out_base, p->wait, st);
+                                            (double *)out_base, p->wait, st,
+                                            fp64_tc_window_ok(v, off, in_base, out_base) ? 0 : p->radius);
         return cs::launch_fp64_fma(v, p->radius, p->pattern, p->w, in, out, st, p->active_rows);
     }
     // The tensor-core split kernels store float4 (two points) at even element
@@ -1075,7 +1091,7 @@ CS_API cs_status cs_plan_set_option(cs_plan *p, cs_option opt, long long v)
             return fail(CS_ERR_INVALID_ARGUMENT, "FP64 algo needs an FP64 plan");
         if (v == CS_ALGO_FP64_MMA && !fp64_mma_ok(p))
             return fail(CS_ERR_UNSUPPORTED, "FP64 MMA serves 2D radius-3 dense FP64 plans only");
-        if (v == CS_ALGO_FP64_TC && !fp64_tc_ok(p) && !fp64_tc3d_ok(p) && !fp64_tc1d_pin_ok(p))
+        if (v == CS_ALGO_FP64_TC && !fp64_tc_pin_ok(p) && !fp64_tc3d_ok(p) && !fp64_tc1d_pin_ok(p))
             return fail(CS_ERR_UNSUPPORTED,
                         "FP64 tcgen05 serves 2D FP64 plans of radius up to 3 and at least 8x8 on even-aligned "
                         "layouts, 3D radius-1 FP64 plans and 1D FP64 plans of radius up to 3 whose length is a "

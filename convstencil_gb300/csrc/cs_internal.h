@@ -80,14 +80,17 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 // The same pipeline on FP64 grids (2D dense 7x7): six exact 9-bit digits per
 // operand cut from the FP64 bits by integer operations, exact FP32 level sums
 // on tcgen05, integer recombination to FP64. Layout conditions as above.
+// radius not 0: any pitch and first column (whole rows of the halo in the
+// buffer), points past a halo of `radius` read as zero.
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
                                  const double *in_base, double *out_base, const TcWait &wait,
-                                 cudaStream_t stream);
+                                 cudaStream_t stream, int radius = 0);
 // `steps` (1..3) steps of a 2D radius-1 grid (FP64 or split) in one launch: wT
-// is the 7x7 kernel of that many steps, w3x3 the weights of one.
+// is the 7x7 kernel of that many steps, w3x3 the weights of one. tma false
+// (FP64): as a radius above.
 cudaError_t launch_steps_tc(bool fp64, const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
                             long long origin, long long elements, const void *in_base, void *out_base,
-                            const TcWait &wait, cudaStream_t stream);
+                            const TcWait &wait, cudaStream_t stream, bool tma);
 // Batches of 2D radius-3 grids on the tcgen05 kernels (split or FP64): one
 // device record per grid (tc_batch_record_bytes each, 128-byte aligned)
 // holding its tensor map over `in_base`, output, sizes, first tile and
@@ -101,9 +104,10 @@ cudaError_t tc_batch_fill_record(bool fp64, void *rec, const GridView &g, const 
                                  int digits_id, int *tiles);
 cudaError_t launch_tc_batch(bool fp64, const void *records, int ngrids, int total_tiles, const TcWait &wait,
                             cudaStream_t stream);
-// 2D tensor map over a whole (hi, lo) buffer of `rows` x `ld` pairs, box_x x box_y tiles.
+// 2D tensor map over a whole (hi, lo) buffer of `rows` x `ld` pairs, box_x x box_y
+// tiles; row: points of a row that the map covers, 0 for all ld.
 cudaError_t encode_split_window_map(CUtensorMap *map, const float2 *base, long long ld, long long rows,
-                                    unsigned box_x, unsigned box_y);
+                                    unsigned box_x, unsigned box_y, long long row = 0);
 // `steps` steps of a 1D grid (FP64 or split) of n >= 64 points in one launch
 // of the tcgen05 digit kernel, steps * radius <= kTcReach1d: taps are the 49
 // taps of that many steps (the output's own at 24), w the 2 radius + 1 weights

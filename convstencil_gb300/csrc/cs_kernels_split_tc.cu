@@ -146,6 +146,9 @@ constexpr int kAccStride = 256;            // TMEM columns between the two accum
 constexpr int kTmemCols = 512;
 constexpr unsigned kStageBytes = ST_X * ST_Y * 8;  // 40,320 (8-byte points)
 constexpr int PAIRS = ST_X / 2, NPAIR = ST_Y * PAIRS;           // 36, 2,520
+// Windows of odd layouts (OddRows): a spare pair per row, even and odd rows apart.
+constexpr int kOddRow = 8 * ST_X + 16, kOddHalf = (ST_Y / 2 * kOddRow + 127) / 128 * 128;  // bytes
+constexpr int kStageF64 = (kOddHalf + ST_Y / 2 * kOddRow) / 16;
 // 1D (kMode1d): a tile is 4096 outputs, 128 rows of 32; row m of A is the 80
 // points around output row m, read in five K steps. The window is 4096 + 48
 // points, 518 chunks of 8; chunk j sits in phase j % 4 at place j / 4, so the
@@ -175,7 +178,7 @@ struct Smem {
     static constexpr int D = F::kDigits;
     static constexpr int NCOL = NLV * D;       // level L at NLV * L
     static_assert(NCOL <= kAccStride, "an accumulator must fit between the two TMEM bases");
-    uint4 stage[NPAIR];                        // TMA destination: pairs of 8-byte points
+    uint4 stage[F::kF64 ? kStageF64 : NPAIR];  // windows: pairs of 8-byte points
     __half planes[2][D][PL];                   // digit planes, two tiles
     __half bmat[NOFF][NCOL * 16];              // B_i, K-major 8x16-byte core matrices
     __half wz[D][7][kWz];                      // weight digits, rows padded with zeros
@@ -344,6 +347,22 @@ constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
 // step per launch, 639 at three; star2d1r 1024^2, 100 steps: 1295 us on the
 // FP64 FMA kernel (the FP64 pipe takes 10 us of each step's 13), 527 so.
 constexpr int kMaxSteps = 3;
+
+// Grids of odd pitch or odd first column, whose rows are not all 16-byte
+// aligned: the rows of each parity have a map of their own, its pitch two rows
+// and its base a 16-byte boundary at the first of them or one point before it.
+// A window's even and odd rows come by one load each, from the even column at
+// or before the window's first, so that they may lie one point late in the
+// stage. (GB300, 8192^2 box2d3r: ODD_BOX us a sweep, one point at a time by
+// cp.async 570 from one warp and 607 from the slicers, row by row 508 by bulk
+// copies; 6237 on FP64 FMA, 326 on an even layout. The output's 8-byte stores
+// alone cost 60 of those us.)
+struct OddRows {
+    CUtensorMap map[2];  // rows 0, 2, .. and 1, 3, .. of a window
+    int x[2], y[2];      // where tile (0, 0)'s window starts in them
+    unsigned late[2];    // points by which its rows are late
+};
+
 template <class F>
 struct StepArgs {
     const typename F::Out *in;  // interior point (0, 0) of the source
@@ -353,6 +372,7 @@ struct StepArgs {
     unsigned taps;              // bit t: weight t is not zero
     int frame_cta;              // CTAs from this one on compute the frame
     typename F::Out w[9];       // weights of one step
+    OddRows rows;               // odd layouts
 };
 
 // The frame's arithmetic, that of single sweeps: FP64 FMA, or double-float.
@@ -497,14 +517,14 @@ __device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out 
 // each CTA takes a contiguous run of the batch's tiles, and the MMA warp
 // rebuilds its B matrices when the run crosses into the next grid, after
 // the MMAs of the previous tile have completed).
-template <class F, bool BATCH, int MODE = kModeGrid>
+template <class F, bool BATCH, int MODE = kModeGrid, bool ODD = false>
 __global__ void __launch_bounds__(kThreads<F>, 1)
     k2d_tc(const __grid_constant__ CUtensorMap tmap, typename F::Out *__restrict__ out, int m, int n,
            long long ld, int tiles_x, int tiles, int map_x, int map_y, typename F::Digits sw, WaitCfg wc,
            const TcGrid<F> *__restrict__ grids, int ngrids, const __grid_constant__ StepArgs<F> sa)
 {
     constexpr bool ONED = MODE == kMode1d, STEPS = MODE == kModeSteps;
-    static_assert(!BATCH || MODE == kModeGrid, "batches run one sweep of 7x7 grids");
+    static_assert(!BATCH || (MODE == kModeGrid && !ODD), "batches run one sweep of 7x7 grids");
     constexpr int D = F::kDigits, kSliceWarps = F::kSliceWarps, kSliceThreads = 32 * kSliceWarps;
     constexpr int kWarpEpi0 = kWarpSlice0 + kSliceWarps;
     constexpr int PER = (NPAIR + kSliceThreads - 1) / kSliceThreads;  // pairs of points a slicer holds
@@ -548,8 +568,15 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             mx = grids[g].map_x;
             my = grids[g].map_y;
         }
-        mbar_expect_tx(bar, kStageBytes);
-        tma_load_2d(smem_addr(S.stage), map, mx + x0 - 4, my + y0 - 3, bar);
+        const int x = mx + x0 - 4, y = my + y0 - 3;
+        if constexpr (ODD) {
+            mbar_expect_tx(bar, ST_Y * kOddRow);
+            tma_load_2d(smem_addr(S.stage), &sa.rows.map[0], sa.rows.x[0] + x0, sa.rows.y[0] + y0 / 2, bar);
+            tma_load_2d(smem_addr(S.stage) + kOddHalf, &sa.rows.map[1], sa.rows.x[1] + x0, sa.rows.y[1] + y0 / 2, bar);
+        } else {
+            mbar_expect_tx(bar, kStageBytes);
+            tma_load_2d(smem_addr(S.stage), map, x, y, bar);
+        }
     };
     volatile int *abort = &S.abort;
     const unsigned stage_full = smem_addr(&S.stage_full), stage_empty = smem_addr(&S.stage_empty);
@@ -712,6 +739,15 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         constexpr int kPairs = ONED ? NPAIR1D : NPAIR;
         const int st = tid - 32 * kWarpSlice0;
         const bool leader = st == 0;
+        auto stage_pair = [&](int idx) {  // pair idx of a 2D window
+            if constexpr (ODD) {
+                const int row = idx / PAIRS, half = row & 1;
+                return reinterpret_cast<uint2 *>(S.stage) + half * (kOddHalf / 8) + (row >> 1) * (kOddRow / 8) +
+                       2 * (idx % PAIRS) + (half ? sa.rows.late[1] : sa.rows.late[0]);
+            } else {
+                return reinterpret_cast<uint2 *>(S.stage + idx);
+            }
+        };
         for (int it = 0; it < my_tiles; ++it) {
             const int buf = it & 1, use = it >> 1;
             // (a) window landed? Every thread waits for itself; one barrier
@@ -722,32 +758,53 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             // split 305 and 295; FP64, bound by the MMAs, 335 and 338.)
             const bool landed = wait(stage_full, it & 1);
             // (b) window -> registers, then release the stage to the next load.
-            if constexpr (STEPS) {
-                // Points past the halo of one meet zero weights in every output
-                // kept, but must not set the tile's scale either: tiles at the
+            if constexpr (STEPS || ODD) {
+                // Points past the halo meet zero weights in every output kept,
+                // but must not set the tile's scale either: tiles at the
                 // boundary first zero them in the stage (a thread the points
                 // that it reads next).
+                const int r = STEPS ? 1 : sa.radius;
                 int g, x0, y0;
                 tile_at(it, g, x0, y0);
-                if (x0 == 0 || y0 == 0 || x0 + ST_X - 4 > n + 1 || y0 + ST_Y - 3 > m + 1) {
+                if (x0 - 4 < -r || y0 - 3 < -r || x0 + ST_X - 4 >= n + r || y0 + ST_Y - 3 >= m + r) {
 #pragma unroll 1
                     for (int idx = st; idx < kPairs; idx += kSliceThreads) {
                         const int yy = y0 - 3 + idx / PAIRS, xx = x0 - 4 + 2 * (idx % PAIRS);
-                        const bool row = yy >= -1 && yy <= m;
-                        uint4 w = S.stage[idx];
-                        if (!row || xx < -1 || xx > n) w.x = w.y = 0u;
-                        if (!row || xx + 1 < -1 || xx + 1 > n) w.z = w.w = 0u;
-                        S.stage[idx] = w;
+                        const bool row = yy >= -r && yy < m + r;
+                        uint2 *at = stage_pair(idx);
+                        if (!row || xx < -r || xx >= n + r) at[0] = make_uint2(0u, 0u);
+                        if (!row || xx + 1 < -r || xx + 1 >= n + r) at[1] = make_uint2(0u, 0u);
                     }
                 }
             }
             uint4 v[PER];
             float vmax = 0.f;   // split: largest |hi|
             unsigned emax = 0;  // FP64: largest biased exponent
+            if constexpr (!ODD) {
 #pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int idx = st + q * kSliceThreads;
-                v[q] = idx < kPairs ? S.stage[idx] : make_uint4(0u, 0u, 0u, 0u);
+                for (int q = 0; q < PER; ++q) {
+                    const int idx = st + q * kSliceThreads;
+                    v[q] = idx < kPairs ? S.stage[idx] : make_uint4(0u, 0u, 0u, 0u);
+                }
+            } else {
+                // pair q of this thread lies 7 q rows and 4 q pairs on, or one row more
+                static_assert(kSliceThreads == 7 * PAIRS + 4 && PER <= 10);
+                unsigned u = st;
+                asm volatile("" : "+r"(u));  // what follows is not kept in registers over a tile
+                const unsigned row0 = u / PAIRS, col0 = u % PAIRS, at0 = smem_addr(S.stage) + 16 * col0;
+#pragma unroll
+                for (int q = 0; q < PER; ++q) {
+                    v[q] = make_uint4(0u, 0u, 0u, 0u);
+                    if (st + q * kSliceThreads < kPairs) {
+                        const unsigned next = col0 + 4 * q >= PAIRS ? 1u : 0u, row = row0 + 7 * q + next;
+                        const unsigned at = at0 + 64 * q - next * (16 * PAIRS) + (row >> 1) * kOddRow +
+                                            ((row & 1) ? kOddHalf + 8 * sa.rows.late[1] : 8 * sa.rows.late[0]);
+                        asm volatile("ld.shared.v2.b32 {%0, %1}, [%4];\n\tld.shared.v2.b32 {%2, %3}, [%4 + 8];"
+                                     : "=r"(v[q].x), "=r"(v[q].y), "=r"(v[q].z), "=r"(v[q].w)
+                                     : "r"(at)
+                                     : "memory");
+                    }
+                }
             }
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
@@ -795,7 +852,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 return ONED ? (idx >> 2 & 3) * (kPhase1d / 4) + (idx >> 4) * 4 + (idx & 3) : idx;
             };
             if constexpr (F::kF64) {
-                constexpr bool EVEN = STEPS || ONED;
+                constexpr bool EVEN = STEPS || ONED || ODD;
                 if (ex >= kFastExp) {
 #pragma unroll
                     for (int q = 0; q < PER; ++q) {
@@ -952,6 +1009,23 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                             if (xc + j >= frame && xc + j < o_n - frame) o[j] = res[j];
                         continue;
                     }
+                    if constexpr (ODD) {  // all rows of a warp start on the same side of a 16-byte boundary
+                        const int late = (int)(reinterpret_cast<unsigned long long>(o) >> 3 & 1);
+                        if (xc + C > o_n) {
+#pragma unroll
+                            for (int j = 0; j < C; ++j)
+                                if (xc + j < o_n) o[j] = res[j];
+                        } else if (late) {
+                            o[0] = res[0];
+#pragma unroll
+                            for (int j = 1; j + 1 < C; j += 2) store2(o + j, res[j], res[j + 1]);
+                            o[C - 1] = res[C - 1];
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < C; j += 2) store2(o + j, res[j], res[j + 1]);
+                        }
+                        continue;
+                    }
 #pragma unroll
                     for (int j = 0; j < C; j += 2) {
                         if (xc + j + 1 < o_n)
@@ -979,36 +1053,52 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kTmemCols));
 }
 
-template <class F, bool BATCH, int MODE = kModeGrid>
+template <class F, bool BATCH, int MODE = kModeGrid, bool ODD = false>
 cudaError_t set_smem_attr()
 {
     static const cudaError_t err = cudaFuncSetAttribute(
-        k2d_tc<F, BATCH, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(Smem<F>) + 128));
+        k2d_tc<F, BATCH, MODE, ODD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(Smem<F>) + 128));
     return err;
 }
 
-template <class F, int MODE = kModeGrid>
+template <class F, int MODE = kModeGrid, bool ODD = false>
 cudaError_t launch_tc(const GridView &g, const typename F::Digits &digits, long long origin, long long elements,
                       const void *in_base, void *out_base, const WaitCfg &wc, cudaStream_t st,
                       const StepArgs<F> &sa = StepArgs<F>{})
 {
     const long long ld = g.pitch[0];
-    CUtensorMap map;
-    // The map copies 8-byte points whatever they hold ((hi, lo) pairs or FP64).
-    cudaError_t e = encode_split_window_map(&map, reinterpret_cast<const float2 *>(in_base), ld, elements / ld,
-                                            ST_X, ST_Y);
+    CUtensorMap map = {};
+    StepArgs<F> args = sa;
+    cudaError_t e = cudaSuccess;
+    // The maps copy 8-byte points whatever they hold ((hi, lo) pairs or FP64).
+    const float2 *points = reinterpret_cast<const float2 *>(in_base);
+    if constexpr (ODD) {
+        const long long rows = elements / ld, x = origin % ld - 4, y = origin / ld - 3;
+        const int first = (int)(y & 1), late = (int)(ld & 1);  // rows 1, 3, .. of an odd pitch: one point late
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+            const int q = k ^ first, shift = q * late;
+            const long long start = x + shift;
+            args.rows.x[k] = (int)(start - (start & 1));
+            args.rows.late[k] = (unsigned)(start & 1);
+            args.rows.y[k] = (int)((y + k - q) / 2);
+            e = encode_split_window_map(&args.rows.map[k], points + q * ld - shift, 2 * ld, (rows + 1 - q) / 2,
+                                        ST_X + 2, ST_Y / 2, ld + shift);
+        }
+    } else {
+        e = encode_split_window_map(&map, points, ld, elements / ld, ST_X, ST_Y);
+    }
     if (e != cudaSuccess) return e;
-    if ((e = set_smem_attr<F, false, MODE>()) != cudaSuccess) return e;
+    if ((e = set_smem_attr<F, false, MODE, ODD>()) != cudaSuccess) return e;
     const int tiles_x = (int)((g.ext[1] + TX - 1) / TX);
     const int tiles = tiles_x * (int)((g.ext[0] + TY - 1) / TY);
     // One CTA per SM (its shared-memory footprint admits no second one, so
     // the TMEM allocation never waits).
     const int grid = std::min(tiles, device_sm_count());
     note_launch();
-    return launch_programmatic(k2d_tc<F, false, MODE>, grid, kThreads<F>, sizeof(Smem<F>) + 128, st, map,
+    return launch_programmatic(k2d_tc<F, false, MODE, ODD>, grid, kThreads<F>, sizeof(Smem<F>) + 128, st, map,
                                reinterpret_cast<typename F::Out *>(out_base) + origin, (int)g.ext[0],
                                (int)g.ext[1], ld, tiles_x, tiles, (int)(origin % ld), (int)(origin / ld), digits,
-                               wc, static_cast<const TcGrid<F> *>(nullptr), 0, sa);
+                               wc, static_cast<const TcGrid<F> *>(nullptr), 0, args);
 }
 
 template <class F>
@@ -1068,10 +1158,14 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 }
 
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
-                                 const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st)
+                                 const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st, int radius)
 {
-    return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base,
-                             WaitCfg{wt.limit_ns, wt.skip_loads}, st);
+    const WaitCfg wc{wt.limit_ns, wt.skip_loads};
+    if (radius == 0) return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base, wc, st);
+    StepArgs<FmtF64> sa{};
+    sa.in = in_base + origin;
+    sa.radius = radius;
+    return launch_tc<FmtF64, kModeGrid, true>(g, f64_slice_weights(w, 49, true), origin, elements, in_base, out_base, wc, st, sa);
 }
 
 namespace {
@@ -1085,7 +1179,8 @@ inline float2 step_weight(double w, float2)
 
 template <class F>
 cudaError_t launch_steps_2d(const GridView &g, const Weights &wT, const Weights &w3x3, int steps, long long origin,
-                            long long elements, const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st)
+                            long long elements, const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st,
+                            bool tma)
 {
     using Out = typename F::Out;
     StepArgs<F> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, 1, 0, 0u, 0, {}};
@@ -1104,8 +1199,11 @@ cudaError_t launch_steps_2d(const GridView &g, const Weights &wT, const Weights 
         sa.w[t] = step_weight(w3x3.v[t], Out{});
         if (w3x3.v[t] != 0.0) sa.taps |= 1u << t;
     }
-    return launch_tc<F, kModeSteps>(g, f64_slice_weights(wT, 49, true), origin, elements, in_base, out_base,
-                                    WaitCfg{wt.limit_ns, wt.skip_loads}, st, sa);
+    const F64Weights digits = f64_slice_weights(wT, 49, true);
+    const WaitCfg wc{wt.limit_ns, wt.skip_loads};
+    if constexpr (F::kF64)
+        if (!tma) return launch_tc<F, kModeSteps, true>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
+    return launch_tc<F, kModeSteps>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
 }
 
 template <class F>
@@ -1136,10 +1234,10 @@ cudaError_t launch_steps_1d(long long n, const double *taps, int radius, const d
 
 cudaError_t launch_steps_tc(bool fp64, const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
                             long long origin, long long elements, const void *in_base, void *out_base,
-                            const TcWait &wt, cudaStream_t st)
+                            const TcWait &wt, cudaStream_t st, bool tma)
 {
-    return fp64 ? launch_steps_2d<FmtF64>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st)
-                : launch_steps_2d<FmtSplit6>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st);
+    return fp64 ? launch_steps_2d<FmtF64>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, tma)
+                : launch_steps_2d<FmtSplit6>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, true);
 }
 
 cudaError_t launch_steps_tc_1d(bool fp64, long long n, const double *taps, int radius, const double *w, int steps,

@@ -313,11 +313,11 @@ int device_sm_count()
 }
 
 cudaError_t encode_split_window_map(CUtensorMap *map, const float2 *base, long long ld, long long rows,
-                                    unsigned box_x, unsigned box_y)
+                                    unsigned box_x, unsigned box_y, long long row)
 {
     auto encode = encode_fn();
     if (!encode) return cudaErrorNotSupported;
-    cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)rows};
+    cuuint64_t dims[2] = {(cuuint64_t)(row > 0 ? row : ld), (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)(ld * sizeof(float2))};
     cuuint32_t box[2] = {box_x, box_y};
     cuuint32_t estr[2] = {1, 1};
