@@ -157,7 +157,7 @@ constexpr int kStageF64 = (kOddHalf + ST_Y / 2 * kOddRow) / 16;
 // point stored once. The reach is the largest whose 2 * 24 + 1 taps keep the
 // level sums exact, as the 49 of a 7x7 do (with a reach of 16, four K steps,
 // a launch took the same time, set by the slicers, for two thirds of the
-// steps: 1d2r 10,240,000 x 100, GB300, 852 us, so 597).
+// steps: 1d2r 10,240,000 x 100, GB300, 852 us, so 597 then).
 constexpr int kReach1d = kTcReach1d;                // points either side of an output: 24
 constexpr int kOut1d = 4096, kWin1d = kOut1d + 2 * kReach1d, NPAIR1D = kWin1d / 2;
 constexpr int kSteps1d = (32 + 2 * kReach1d) / 16;  // K steps
@@ -353,7 +353,7 @@ constexpr int kMaxSteps = 3;
 // and its base a 16-byte boundary at the first of them or one point before it.
 // A window's even and odd rows come by one load each, from the even column at
 // or before the window's first, so that they may lie one point late in the
-// stage. (GB300, 8192^2 box2d3r: ODD_BOX us a sweep, one point at a time by
+// stage. (GB300, 8192^2 box2d3r: 412 us a sweep, one point at a time by
 // cp.async 570 from one warp and 607 from the slicers, row by row 508 by bulk
 // copies; 6237 on FP64 FMA, 326 on an even layout. The output's 8-byte stores
 // alone cost 60 of those us.)
@@ -988,9 +988,16 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                         *reinterpret_cast<float4 *>(o) = make_float4(u.x, u.y, v.x, v.y);
                 };
                 if constexpr (ONED) {
-                    // outputs 32 mrow + 8 rho .. + 7 of the tile
+                    // Outputs 32 mrow + 8 rho .. + 7 of the tile: every lane's
+                    // store has a line of its own, so it is 32 bytes where the
+                    // grid allows them. (GB300, launch of 10,240,000 x 11 steps
+                    // with 16 and 32 bytes: FP64 58.0 and 55.8 us, split 61.8
+                    // and 53.7. In 2D, whose lanes share lines, no difference.)
                     const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d + 32 * mrow + 8 * rho + c0;
-                    if (sa.aligned && x >= frame && x + C <= n - frame) {
+                    if (reinterpret_cast<unsigned long long>(out) % 32 == 0 && x >= frame && x + C <= n - frame) {
+#pragma unroll
+                        for (int j = 0; j < C; j += 4) store_32(out + x + j, res + j);
+                    } else if (sa.aligned && x >= frame && x + C <= n - frame) {
 #pragma unroll
                         for (int j = 0; j < C; j += 2) store2(out + x + j, res[j], res[j + 1]);
                     } else {

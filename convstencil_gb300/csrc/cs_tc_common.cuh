@@ -249,6 +249,17 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigne
                  : "memory");
 }
 
+// Four 8-byte points to a 32-byte boundary.
+template <class T>
+__device__ __forceinline__ void store_32(T *dst, const T *v)
+{
+    static_assert(sizeof(T) == 8);
+    unsigned long long w[4];
+    memcpy(w, v, sizeof w);
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "l"(w[0]), "l"(w[1]), "l"(w[2]), "l"(w[3])
+                 : "memory");
+}
+
 // 8 bytes from global to shared memory, or zeros.
 __device__ __forceinline__ void cp_async8(unsigned dst, const void *src, bool take)
 {
