@@ -22,13 +22,16 @@
 //     (0..2) is the same descriptor started i rows lower.
 //   * Input plane P feeds output planes P+1, P and P-1 as their z taps
 //     dz = 0, 1, 2, and its MMAs serve all three at once: column n of B_i is
-//     (weight digit e, tap plane dz, column c), n = 32 e + 8 dz + c, with
-//     B[k][n] = w_e[dz][i][k - c - 3] (n with dz = 3 is zero padding that
-//     keeps every level 32 columns wide). For input digit d one MMA with
-//     N = 32 (5 - d) feeds levels d..4 of the plane's TMEM block: 3 row
-//     offsets x 5 digits = 15 MMAs per input plane and 1024 outputs.
-//   * Each input plane has its own 160-column TMEM block (ring of three,
-//     columns 0, 160, 320), so every plane keeps its own scale. The epilogue
+//     (weight digit e, tap plane dz, column c), n = 24 e + 8 dz + c, with
+//     B[k][n] = w_e[dz][i][k - c - 3]. For input digit d one MMA with
+//     N = 24 (5 - d), rounded up to 16s, feeds levels d..4 of the plane's TMEM
+//     block: 3 row offsets x 5 digits = 15 MMAs per input plane and 1024
+//     outputs.
+//   * Each input plane has its own 128-column TMEM block (ring of four), so
+//     every plane keeps its own scale. (Levels of 32 columns, one in four of
+//     them padding, took rings of three and, FP64, of two; GB300, us a sweep:
+//     split 128^3 20.8 and 19.8, 512^3 740 and 734; FP64 512^3 1112 and 1107.) The
+//     epilogue
 //     reads a block once, as soon as its MMAs are done, hands it back, and
 //     adds its three tap-plane parts to the running sums of output planes
 //     P+1 (dz = 0), P (dz = 1) and P-1 (dz = 2, its last: stored). Parts of
@@ -66,21 +69,30 @@ using split::slice_digits;
 using split::two_sum;
 using namespace tc;
 
-// Number formats: split (FP32 (hi, lo) grids, five digits, a ring of three
-// 160-column TMEM blocks) and FP64 (FP64 grids, six digits cut with integer
-// operations as in the 2D kernel, a ring of two 192-column blocks: three do
-// not fit in the 512 columns).
+// Number formats: split (FP32 (hi, lo) grids, five digits, a ring of four
+// 128-column TMEM blocks) and FP64 (FP64 grids, six digits cut with integer
+// operations as in the 2D kernel, a ring of three 160-column blocks).
+//
+// FP64 is bound by its epilogue (GB300, star3d1r 512^3: 2,400 cycles a plane of
+// 1024 outputs, of which the epilogue waits 160; 1,590 with its arithmetic left
+// out). The conversions to FP64, 64 cycles a warp on a scheduler's FP64 unit,
+// are a third of it: without them 1,690. Not faster: conversions by integer
+// operations (1200 us a sweep against 1112; that pipe is the slicers'),
+// interleaved with the other parts (1104 to 1170), two columns a step with the
+// next ones' loads in flight (1277), all three parts loaded first with 112
+// registers for the epilogue by setmaxnreg (1287; split 826 against 738),
+// sixteen epilogue warps (1171 against 1126).
 struct F3Split {
     static constexpr bool kF64 = false;
     static constexpr int D = split::kDigits;  // 5
-    static constexpr int NBLK = 3;
+    static constexpr int NBLK = 4;
     using Out = float2;
     using Digits = SliceWeights;
 };
 struct F3F64 {
     static constexpr bool kF64 = true;
     static constexpr int D = 6;
-    static constexpr int NBLK = 2;
+    static constexpr int NBLK = 3;
     using Out = double;
     using Digits = F64Weights;
 };
@@ -115,9 +127,15 @@ constexpr int ST_X = TX + 8, ST_Y = TY + 2;  // window: columns x0-4 .. x0+67, r
 constexpr int PL = ST_X * ST_Y;              // halves per digit plane (2,592 bytes)
 constexpr unsigned kRowBytes = ST_X * 2;     // 144
 constexpr int NOFF = 3;                      // window row offsets
-constexpr int NLV = 32;                      // TMEM columns per level: 4 tap planes (3 + padding) x 8
+constexpr int NLV = 24;                      // TMEM columns per level: 3 tap planes x 8
+// N of an MMA that feeds `levels` levels: M = 128 wants multiples of 16, so odd
+// counts take 8 columns more, of a level that does not exist; they lie behind
+// the block's last level and are not read.
+__host__ __device__ constexpr int mma_n(int levels) { return (NLV * levels + 15) / 16 * 16; }
 template <class F>
-constexpr int kNcol = NLV * F::D;            // columns per input-plane block: 160 split, 192 FP64
+constexpr int kNcol = mma_n(F::D);           // rows of B_i: 128 split, 144 FP64
+template <class F>
+constexpr int kBlk = F::kF64 ? 160 : 128;    // TMEM columns from one input plane's block to the next
 constexpr int kTmemCols = 512;
 constexpr int kStages = 2 * kGroups;         // TMA window buffers (two per slicer group)
 constexpr int NPL = 7;                       // digit-plane sets (ring); also keeps one CTA per SM
@@ -130,7 +148,7 @@ constexpr unsigned kStageBytes = ST_X * ST_Y * 8;  // 10,368 (8-byte points)
 // zero weights, so they only need to be finite).
 constexpr int PAIRS = ST_X / 2, CUT0 = 1, NCUTX = 34, NCUT = ST_Y * NCUTX;  // 36, 612
 constexpr int PER = (NCUT + kGroupThreads - 1) / kGroupThreads;            // 5
-static_assert(F3Split::NBLK * kNcol<F3Split> <= kTmemCols && F3F64::NBLK * kNcol<F3F64> <= kTmemCols,
+static_assert(F3Split::NBLK * kBlk<F3Split> <= kTmemCols && F3F64::NBLK * kBlk<F3F64> <= kTmemCols,
               "TMEM blocks exceed the allocation");
 static_assert(kEpiWarps == 8, "two epilogue warps per TMEM lane quarter, four columns each");
 static_assert(kStageBytes % 128 == 0, "TMA destinations stay 128-byte aligned");
@@ -163,7 +181,7 @@ __device__ __forceinline__ void plane_mma(unsigned d_base, unsigned long long a,
     constexpr unsigned long long b_off = ((unsigned long long)I * NCOL * 16 * 2) >> 4;
     static_assert(((unsigned long long)D * PL * 2 + I * kRowBytes) % 16 == 0 && (NCOL * 16 * 2) % 16 == 0,
                   "descriptor offsets must be 16-byte multiples");
-    mma_f16(d_base + (unsigned)(NLV * D), a + a_off, b0 + b_off, instr_desc(NLV * (F::D - D)),
+    mma_f16(d_base + (unsigned)(NLV * D), a + a_off, b0 + b_off, instr_desc(mma_n(F::D - D)),
             (I | D) != 0 ? 1u : 0u);
     if constexpr (D + 1 < F::D)
         plane_mma<F, I, D + 1>(d_base, a, b0);
@@ -255,18 +273,28 @@ __global__ void __launch_bounds__(kThreads, 1)
                      "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    // B_i: N row nn = NLV e + 8 dz + c (digit e of w, z tap dz, column c of
-    // the block; dz = 3 is padding), K index k.
-    for (int idx = tid; idx < NOFF * NCOL * 16; idx += kThreads) {
-        const int i = idx / (NCOL * 16), rem = idx - i * (NCOL * 16);
-        const int nn = rem >> 4, k = rem & 15;
-        const int e = nn / NLV, dz = (nn % NLV) >> 3, c = nn & 7;
-        const int tj = k - c - 3;
-        const __half v = (dz < 3 && tj >= 0 && tj < 3) ? sw.d[e][(dz * 3 + i) * 3 + tj] : __float2half(0.f);
-        S.bmat[i][(nn >> 3) * 128 + (nn & 7) * 8 + (k >> 3) * 64 + (k & 7)] = v;
+    // B_i: N row nn = NLV e + 8 dz + c (digit e of w, z tap dz, column c of the
+    // block), K index k; a thread takes 8 k at a time. (One at a time, and
+    // the planes zeroed by words: GB300, 64^3 12.7 us a sweep FP64 and 10.6 split,
+    // so 10.2 and 8.0.)
+    for (int idx = tid; idx < NOFF * NCOL * 2; idx += kThreads) {
+        const int i = idx / (NCOL * 2), rem = idx - i * (NCOL * 2), kc = rem / NCOL, nn = rem - kc * NCOL;
+        const int e = nn / NLV, dz = nn % NLV >> 3, c = nn & 7;
+        unsigned long long lo = 0, hi = 0;
+#pragma unroll
+        for (int tj = 0; tj < 3; ++tj) {
+            const int k = c + 3 + tj - 8 * kc;
+            if (e >= D || k < 0 || k >= 8) continue;
+            const unsigned long long v = __half_as_ushort(sw.d[e][(dz * 3 + i) * 3 + tj]);
+            if (k < 4)
+                lo |= v << 16 * k;
+            else
+                hi |= v << 16 * (k - 4);
+        }
+        *reinterpret_cast<ulonglong2 *>(&S.bmat[i][(nn >> 3) * 128 + (nn & 7) * 8 + kc * 64]) = make_ulonglong2(lo, hi);
     }
-    for (int i = tid; i < NPL * D * PL / 2; i += kThreads)
-        reinterpret_cast<unsigned *>(&S.planes[0][0][0])[i] = 0u;
+    for (int i = tid; i < NPL * D * PL / 8; i += kThreads)
+        reinterpret_cast<uint4 *>(&S.planes[0][0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
@@ -310,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     break;
                 tc_fence_after();
                 if (elect_one()) {
-                    plane_mma<F, 0, 0>(tmem + (unsigned)(NCOL * blk), a_desc0 + kSetUnits * slot, b_desc0);
+                    plane_mma<F, 0, 0>(tmem + (unsigned)(kBlk<F> * blk), a_desc0 + kSetUnits * slot, b_desc0);
                     mma_commit(bar(S.blk_full, blk));       // block ready for the epilogue
                     mma_commit(bar(S.planes_empty, slot));  // digit planes may be overwritten
                 }
@@ -458,38 +486,43 @@ __global__ void __launch_bounds__(kThreads, 1)
             int ea = 0, eb2 = 0;
             bool fa = false, fb = false, na = false, nb = false;
             const int ew = sw.ew;
-            auto part_t = [](const float (&acc)[D][4], long long (&t)[4]) {
+            // Integer sums start at -3 kRawBias, so that they are right once
+            // all three parts are in; `left` parts are missing before this one.
+            auto add_raw = [](long long (&sm)[4], const float (&acc)[D][4]) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float lv[6] = {acc[0][c], acc[1][c], acc[2][c], acc[3][c], acc[4][c], acc[5][c]};
-                    t[c] = f64_combine_small(lv);  // one z tap: every level below 2^22
+                for (int c = 0; c < 4; c += 2) {
+                    const float u[6] = {acc[0][c], acc[1][c], acc[2][c], acc[3][c], acc[4][c], acc[5][c]};
+                    const float v[6] = {acc[0][c + 1], acc[1][c + 1], acc[2][c + 1],
+                                        acc[3][c + 1], acc[4][c + 1], acc[5][c + 1]};
+                    f64_add_raw2(u, v, sm[c], sm[c + 1]);
                 }
             };
             auto add_part = [&](long long (&sm)[4], int &se, bool &fl, bool &nf, const float (&acc)[D][4],
-                                int ex) {
+                                int ex, int left) {
                 if (nf) return;
                 if (ex == kNonFiniteTile) {
                     nf = true;
                     return;
                 }
-                long long t[4];
-                part_t(acc, t);
                 if (!fl && ex == se) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) sm[c] += t[c];
+                    add_raw(sm, acc);
                     return;
                 }
                 if (!fl) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) sm[c] = __double_as_longlong(f64_from_fixed(sm[c], se + ew - 1080));
+                    for (int c = 0; c < 4; ++c)
+                        sm[c] = __double_as_longlong(f64_from_fixed((long long)((unsigned long long)sm[c] + left * kRawBias), se + ew - 1080));
                     fl = true;
                 }
+                const long long none = (long long)(0 - kRawBias);
+                long long t[4] = {none, none, none, none};
+                add_raw(t, acc);
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
                     sm[c] = __double_as_longlong(__longlong_as_double(sm[c]) + f64_from_fixed(t[c], ex + ew - 1080));
             };
             auto load_part = [&](int q, int dz, float (&acc)[D][4]) {
-                const unsigned col = (unsigned)(NCOL * (q % NBLK) + 8 * dz + 4 * hh);
+                const unsigned col = (unsigned)(kBlk<F> * (q % NBLK) + 8 * dz + 4 * hh);
 #pragma unroll
                 for (int L = 0; L < D; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
                 tmem_wait_ld();
@@ -503,7 +536,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // z tap 2 of output p - 2: its last part; store.
                 load_part(q, 2, acc);
                 if (p >= 2) {
-                    add_part(a, ea, fa, na, acc, ex);
+                    add_part(a, ea, fa, na, acc, ex, 1);
                     if (yy < m) {
                         double res[4];
                         const int sc = ea + ew - 1080;
@@ -529,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
                 // z tap 1 of output p - 1.
                 load_part(q, 1, acc);
-                if (p >= 1 && p - 1 < wi.zn) add_part(b, eb2, fb, nb, acc, ex);
+                if (p >= 1 && p - 1 < wi.zn) add_part(b, eb2, fb, nb, acc, ex, 2);
                 // z tap 0 of output p: its first part. The block is then
                 // drained and handed back.
                 load_part(q, 0, acc);
@@ -537,14 +570,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(S.blk_empty, q % NBLK));
 #pragma unroll
-                for (int c = 0; c < 4; ++c) a[c] = b[c];  // rotate: p - 1 becomes p - 2, p starts
+                for (int c = 0; c < 4; ++c) {  // rotate: p - 1 becomes p - 2, p starts
+                    a[c] = b[c];
+                    b[c] = (long long)(0 - 3 * kRawBias);
+                }
                 ea = eb2;
                 fa = fb;
                 na = nb;
                 eb2 = ex;
                 fb = false;
                 nb = ex == kNonFiniteTile;
-                if (!nb) part_t(acc, b);
+                if (!nb) add_raw(b, acc);
             }
             q0 += wi.zn + 2;
         }
@@ -614,7 +650,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             };
             auto load_part = [&](int q, int dz, float (&acc)[D][4]) {
-                const unsigned col = (unsigned)(NCOL * (q % NBLK) + 8 * dz + 4 * hh);
+                const unsigned col = (unsigned)(kBlk<F> * (q % NBLK) + 8 * dz + 4 * hh);
 #pragma unroll
                 for (int L = 0; L < D; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
                 tmem_wait_ld();

@@ -135,28 +135,40 @@ __device__ __forceinline__ long long f64_combine(const float (&lv)[6])
     return t;
 }
 
-// f64_combine for level sums below 2^22 in magnitude (one z tap of a 3D
-// input plane: 9 taps, so level L sums at most 9 * 5 * 2^16 < 2^22): the
-// integers come out of the FP32 sums by one addition of 1.5 * 2^23 (exact in
-// that range: the sum lands in [2^23, 2^24), where the spacing is 1, and its
-// low mantissa bits are 2^22 + S) and one integer subtraction, instead of
-// the conversion unit's __float2int_rn (16 per clock per SM, three parts per
-// 3D output). Same T as f64_combine.
-__device__ __forceinline__ int f32_small_int(float s)
+// f64_combine for two outputs whose level sums are below 2^22 in magnitude
+// (one z tap of a 3D input plane: 9 taps, so level L sums at most 9 * 5 * 2^16 <
+// 2^22), added to their running 64-bit sums: an FP32 addition of 1.5 * 2^23
+// (exact in that range: the sum lands in [2^23, 2^24), where the spacing is 1)
+// leaves kRaw + S in the bits of S's float, and the multiply-adds take those
+// bits as they are. Every call therefore adds kRawBias too (modulo 2^64; kRaw is
+// a multiple of 8, so level 5's shift leaves it whole), which the caller takes
+// off once per sum. (GB300, star3d1r 512^3: 1128 us a sweep with the bias taken
+// off every level, 1112 so.)
+constexpr unsigned kRaw = 0x4B400000u;
+constexpr unsigned long long kRawBias = (kRaw >> 3) + (unsigned long long)kRaw * ((1u << 6) + (1u << 15) + (1u << 24)) +
+                                        ((unsigned long long)(kRaw * 1026u) << 32);
+__device__ __forceinline__ void f64_add_raw2(const float (&u)[6], const float (&v)[6], long long &su, long long &sv)
 {
-    return __float_as_int(__fadd_rn(s, 12582912.0f)) - 0x4B400000;
-}
-__device__ __forceinline__ long long f64_combine_small(const float (&lv)[6])
-{
-    long long t = (long long)(f32_small_int(lv[5]) >> 3);
-    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(f32_small_int(lv[4])), "r"(1 << 6));
-    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(f32_small_int(lv[3])), "r"(1 << 15));
-    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(f32_small_int(lv[2])), "r"(1 << 24));
-    unsigned tl, th;
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(tl), "=r"(th) : "l"(t));
-    th += (unsigned)(f32_small_int(lv[1]) * 2 + f32_small_int(lv[0]) * 1024);
-    asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "r"(tl), "r"(th));
-    return t;
+    int a[6], b[6];
+#pragma unroll
+    for (int L = 0; L < 6; ++L) {
+        unsigned long long x;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(u[L]), "f"(v[L]));
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(0x4B4000004B400000ull));
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(a[L]), "=r"(b[L]) : "l"(x));
+    }
+    auto sum = [](const int (&r)[6], long long &t) {
+        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[5] >> 3), "r"(1));
+        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[4]), "r"(1 << 6));
+        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[3]), "r"(1 << 15));
+        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[2]), "r"(1 << 24));
+        unsigned tl, th;
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(tl), "=r"(th) : "l"(t));
+        th += (unsigned)r[1] * 2u + (unsigned)r[0] * 1024u;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "r"(tl), "r"(th));
+    };
+    sum(a, su);
+    sum(b, sv);
 }
 
 // Results outside the normal FP64 range (subnormal or overflowing): FP64
