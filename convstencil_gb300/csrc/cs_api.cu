@@ -298,27 +298,12 @@ struct cs_plan {
     std::mutex host_mu;
     void *host_bufs[2] = {nullptr, nullptr};
     size_t host_bytes = 0;
-    // The band schedule of host-buffer runs on the tcgen05 batch kernel
-    // (host_run_banded): the device records of every distinct set of
-    // band-sweeps, kept for the bands, sweeps and grids they were made for.
-    struct BandSet {
-        long long rec;  // first record in the table
-        int count, tiles;
-    };
-    struct BandTable {
-        int bands = 0, algo = -1;
-        long long sweeps = 0;
-        const void *d0 = nullptr, *d1 = nullptr;
-        void *tab = nullptr;
-        std::vector<BandSet> sets;  // one per set, in launch order
-    } band;
     ~cs_plan()
     {
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
         if (capture_stream) cudaStreamDestroy(capture_stream);
         for (void *b : host_bufs)
             if (b) cudaFree(b);
-        if (band.tab) cudaFree(band.tab);
     }
 };
 
@@ -1218,150 +1203,59 @@ struct DevBuf {
     }
 };
 
-// in_elems doubles from host_in into buffer 0 (buffer 1 zero), `sweeps`
-// sweeps, then out_elems doubles from result + out_offset to host_out.
 // Host-buffer run with the copies overlapped: the grid goes to the device in
-// row bands (slabs of the slowest axis) on one stream while the sweeps run
-// as a wavefront over the bands on another (sweep s of band k once sweep
-// s - 1 of bands k - 1 .. k + 1 is done, band k + 1 of the input having
-// arrived for the first sweep), and each band goes back as soon as its last
-// sweep is done. Launches are issued diagonal by diagonal on one stream, so
-// sweep s of band k always precedes sweep s + 1 of band k - 1, which
-// overwrites rows that it reads. Used when the kernel is known without a
-// timing run, no temporal blocking and no re-anchor sweep is involved, and
-// the whole grid goes both ways.
-// Whether the band-sweeps of a host-buffer run go to the tcgen05 batch
-// kernel: 2D split plans on SPLIT_TC (the 2D radius-3 tile geometry). On
-// GB300, 20 sweeps of 8192^2 with the copies: 10.3 ms in 32 bands of batched
-// sets against 11.7 in 8 bands of one launch each; FP64 plans gain nothing
-// from the batches (12.1 against 11.9 ms), whose kernel runs 5 % slower than
-// the one-grid kernel, and keep one launch per band-sweep.
-bool band_batch_ok(const cs_plan *p, int algo)
-{
-    return p->prec == CS_PREC_SPLIT && algo == CS_ALGO_SPLIT_TC && p->radius == 3 && fp64_tc_geometry_ok(p);
-}
-
-// `kept`: the run uses the plan's kept grids (batched sets allowed).
-bool banded_ok(cs_plan *p, long long sweeps, bool kept, int *algo, int *bands)
+// bands of slabs (of the slowest axis) on one stream while the sweeps of what
+// has arrived run on another, and slabs go back as soon as their last sweep is
+// done. Used when the kernel is known without a timing run, no temporal
+// blocking and no re-anchor sweep is involved, and the whole grid goes both
+// ways.
+bool banded_ok(cs_plan *p, long long sweeps, int *algo, int *bands)
 {
     if (p->dims < 2 || sweeps < 1) return false;
     if (p->prec == CS_PREC_SPLIT && cs::split_tb_supported(p->dims, p->radius, p->pattern) && p->time_block != 1)
         return false;
     if (p->prec == CS_PREC_SPLIT && p->reanchor > 0 && sweeps >= p->reanchor) return false;
     if (choose_algo(p, nullptr, nullptr, nullptr, algo, false) != CS_OK || *algo < 0) return false;
-    const long long slabs = p->view.ext[0];
-    if (kept && band_batch_ok(p, *algo)) {
-        *bands = (int)std::min<long long>(32, slabs / 256);  // one batch launch per set
-    } else {
-        const long long per = p->dims == 2 ? 1024 : 64;  // slabs per band at least
-        *bands = (int)std::min<long long>(8, slabs / per);
-    }
+    // The copies take 2 bytes / kLinkRate, of which b bands leave one b-th to
+    // wait for; a cut costs every sweep a launch and, in 3D, the window planes
+    // of its neighbours. The sum is least at the b below. (GB300, ms in 1, 2, 3,
+    // 4, 6, 8 bands: FP64 box2d3r 4096^2 x 5 sweeps 1.91 1.48 1.38 1.35 1.30 1.33, x 20
+    // 3.24 2.79 2.81 2.81 2.97 3.34, x 60 6.77 7.03 7.20 7.38 8.04 9.28; 8192^2 x 20
+    // 12.1 9.46 8.83 8.48 8.60 8.90; 2048^2 x 20 0.99 1.15 1.22 1.34 1.56 1.83;
+    // box3d1r 512^3 x 10 22.1 16.8 15.6 14.5 14.2 14.3; fused box3d1r 200 x 184 x 192 x
+    // 10 2.56 2.77 2.92 3.08 3.49 3.81.)
+    constexpr double kLinkRate = 205e3;  // bytes per us each way, pinned host buffers
+    const double cut_us = p->dims == 3 && p->radius > 1 ? 20.0 : 6.0;
+    const double best = std::sqrt(2.0 * (double)p->layout.bytes / kLinkRate / (cut_us * (double)sweeps));
+    const long long least = p->dims == 2 ? 128 : 16;  // slabs per band
+    *bands = (int)std::min({best, 6.0, (double)(p->view.ext[0] / least)});
+    // Bands take one step per launch: not where a launch of several saves more
+    // (star2d1r 4096^2 x 20: 2.15 ms whole, 2.79 in bands).
+    if (steps_per_launch(p, nullptr, nullptr) > 1 && sweeps > 12) return false;
     return *bands >= 2;
 }
 
-// Band-sweep (k, s) is sweep s (0-based) of the interior slabs of band k: it
-// reads level s of bands k-1 .. k+1 (grid s % 2) and writes level s+1 of band
-// k (grid (s+1) % 2). Its inputs come from (k-1, s-1), (k, s-1), (k+1, s-1),
-// and the level s-1 it overwrites was last read by the same three, so with
-// c = 2s + k every dependency points from set c to sets c-1, c-2, c-3: the
-// band-sweeps of one set are independent (neighbouring bands are never in
-// the same set, and bands are taller than the halo), and the sets in order
-// c = 0, 1, ... form a wavefront that starts on the first bands while later
-// ones are still arriving. Set c needs band c + 1 on the device when c < K.
-struct BandMember {
-    int k;
-    long long s;
-};
-static std::vector<BandMember> band_set(int bands, long long sweeps, long long c)
-{
-    std::vector<BandMember> m;
-    for (long long sw = std::max(0LL, (c - bands + 2) / 2); sw <= std::min(sweeps - 1, c / 2); ++sw) {
-        const long long k = c - 2 * sw;
-        if (k >= 0 && k < bands) m.push_back({(int)k, sw});
-    }
-    return m;
-}
-
-// The batch records of every set (sets whose members have the same bands
-// and grid parities share them: in the middle of a long run the pattern
-// repeats every four sets), uploaded once per bands, sweeps and grids.
-static cs_status band_table(cs_plan *p, int algo, int bands, long long sweeps, void *const d[2],
-                            const std::vector<long long> &b)
-{
-    auto &T = p->band;
-    if (T.tab && T.bands == bands && T.sweeps == sweeps && T.algo == algo && T.d0 == d[0] && T.d1 == d[1])
-        return CS_OK;
-    if (T.tab) cudaFree(T.tab), T.tab = nullptr;
-    T.sets.clear();
-    const bool fp64 = p->prec == CS_PREC_FP64;
-    const size_t rb = cs::tc_batch_record_bytes(fp64);
-    std::vector<unsigned char> rec;
-    std::map<std::vector<long long>, cs_plan::BandSet> seen;
-    const long long nsets = 2 * (sweeps - 1) + bands;
-    for (long long c = 0; c < nsets; ++c) {
-        const auto mem = band_set(bands, sweeps, c);
-        std::vector<long long> sig;
-        for (const auto &x : mem) sig.push_back(2 * x.k + (x.s & 1));
-        auto it = seen.find(sig);
-        if (it == seen.end()) {
-            cs_plan::BandSet bs{(long long)(rec.size() / rb), (int)mem.size(), 0};
-            for (const auto &x : mem) {
-                GridView v = p->view;
-                v.ext[0] = b[x.k + 1] - b[x.k];
-                const long long off = p->layout.origin + b[x.k] * p->view.pitch[0];
-                rec.resize(rec.size() + rb);
-                int tiles = 0;
-                const cudaError_t e = cs::tc_batch_fill_record(fp64, rec.data() + rec.size() - rb, v, p->w, off,
-                                                               p->layout.elements, d[x.s & 1], d[(x.s + 1) & 1],
-                                                               bs.tiles, 0, &tiles);
-                if (e != cudaSuccess) return fail(CS_ERR_CUDA, "band record: %s", cudaGetErrorString(e));
-                bs.tiles += tiles;
-            }
-            it = seen.emplace(sig, bs).first;
-        }
-        T.sets.push_back(it->second);
-    }
-    CS_CUDA(cudaMalloc(&T.tab, rec.size()));
-    CS_CUDA(cudaMemcpy(T.tab, rec.data(), rec.size(), cudaMemcpyHostToDevice));
-    T.bands = bands;
-    T.sweeps = sweeps;
-    T.algo = algo;
-    T.d0 = d[0];
-    T.d1 = d[1];
-    return CS_OK;
-}
-
-// `kept`: d are the plan's kept grids and the caller holds host_mu, so the
-// plan's cached band records (p->band) may be used and rebuilt; a call on
-// grids of its own (another thread holds the kept ones) launches its
-// band-sweeps one by one and leaves the cache alone.
+// Group g of the sweeps takes level s (1 .. sweeps) of the slabs from
+// g height - align s up to the next group's: it reads nothing that a later
+// group computes or that is still arriving (align >= radius), and overwrites
+// nothing that one still reads, so a group runs all its levels in a row. Every
+// cut is a multiple of the kernels' tiles, so that the tiles see the windows of
+// a whole sweep. (As a wavefront of one sweep per band the first sweeps waited
+// for most of the copy in and the last band's end for most of the copy out;
+// GB300, that and so: FP64 box2d3r 4096^2 x 20 sweeps 3.48 and 2.80 ms, 8192^2 11.9
+// and 8.9; split on the batch kernel, a launch for all independent
+// band-sweeps, 2.95 and 2.59, 9.27 and 8.65.)
 cs_status host_run_banded(cs_plan *p, int algo, int bands, const double *host_in, double *host_out,
-                          long long sweeps, void *const d[2], bool kept, double *loop_seconds)
+                          long long sweeps, void *const d[2], double *loop_seconds)
 {
     const long long ld0 = p->view.pitch[0];        // elements per slab
     const long long total = p->layout.elements / ld0;  // slabs in the buffer, halo included
     const long long first = p->layout.origin / ld0;    // halo slabs before the interior
     const long long slabs = p->view.ext[0];
     const long long align = p->dims == 2 ? 64 : 8;
-    std::vector<long long> b(bands + 1);  // interior slab boundaries of the bands
-    for (int k = 0; k <= bands; ++k) b[k] = std::min(slabs, (slabs * k / bands + align - 1) / align * align);
-    b[bands] = slabs;
-    std::vector<long long> c(bands + 1);  // buffer slab boundaries of the copy chunks
-    for (int k = 0; k <= bands; ++k) c[k] = k == 0 ? 0 : k == bands ? total : first + b[k];
-    // The tcgen05 batch kernel takes a whole set per launch when every band
-    // meets its layout conditions; otherwise each band-sweep is a launch.
-    bool batch = kept && band_batch_ok(p, algo) && reinterpret_cast<uintptr_t>(d[0]) % 16 == 0 &&
-                 reinterpret_cast<uintptr_t>(d[1]) % 16 == 0;
-    for (int k = 0; k < bands && batch; ++k) {
-        GridView v = p->view;
-        v.ext[0] = b[k + 1] - b[k];
-        const long long off = p->layout.origin + b[k] * ld0;
-        batch = cs::split_tma_layout_ok(v, off, d[0]) && cs::split_tma_layout_ok(v, off, d[1]);
-    }
-    if (batch) {
-        const cs_status st = band_table(p, algo, bands, sweeps, d, b);
-        if (st != CS_OK) return st;
-    }
+    const long long height = ((slabs + bands - 1) / bands + align - 1) / align * align;
+    std::vector<long long> c(bands + 1);  // buffer slab boundaries of the copies in
+    for (int k = 0; k <= bands; ++k) c[k] = k == 0 ? 0 : k == bands ? total : first + std::min(slabs, height * k);
     struct Streams {
         cudaStream_t s[3] = {nullptr, nullptr, nullptr};
         std::vector<cudaEvent_t> ev;
@@ -1374,9 +1268,9 @@ cs_status host_run_banded(cs_plan *p, int algo, int bands, const double *host_in
     } S;
     for (auto &x : S.s) CS_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
     cudaStream_t sc = S.s[0], sh = S.s[1], sd = S.s[2];
-    S.ev.resize(2 * bands + 2);
+    S.ev.resize(bands + 3);
     for (auto &e : S.ev) CS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDefault));
-    cudaEvent_t *in_ev = S.ev.data(), *out_ev = S.ev.data() + bands, e0 = S.ev[2 * bands], e1 = S.ev[2 * bands + 1];
+    cudaEvent_t *in_ev = S.ev.data(), out_ev = S.ev[bands], e0 = S.ev[bands + 1], e1 = S.ev[bands + 2];
     const size_t slab_bytes = (size_t)ld0 * sizeof(double);
     CS_CUDA(cudaMemsetAsync(d[1], 0, (size_t)p->layout.bytes, sc));  // the second grid's halo reads as zero
     // The copies in go back to back on their own stream; a split plan's band
@@ -1401,51 +1295,31 @@ cs_status host_run_banded(cs_plan *p, int algo, int bands, const double *host_in
         return CS_OK;
     };
     void *f = d[sweeps & 1];  // final grid
-    const bool fp64 = p->prec == CS_PREC_FP64;
-    const size_t rb = batch ? cs::tc_batch_record_bytes(fp64) : 0;
-    auto band_done = [&](int k) -> cs_status {  // band k is final: back to the host now
-        const long long cnt = (c[k + 1] - c[k]) * ld0;
-        char *src = (char *)f + c[k] * slab_bytes;
+    auto slabs_done = [&](long long from, long long to) -> cs_status {  // final: back to the host now
+        const long long cnt = (to - from) * ld0;
+        char *src = (char *)f + from * slab_bytes;
         if (p->prec == CS_PREC_SPLIT) CS_CUDA(cs::launch_split_to_fp64_inplace(cnt, src, sc));
-        CS_CUDA(cudaEventRecord(out_ev[k], sc));
-        CS_CUDA(cudaStreamWaitEvent(sd, out_ev[k], 0));
-        CS_CUDA(cudaMemcpyAsync(host_out + c[k] * ld0, src, (size_t)cnt * sizeof(double), cudaMemcpyDeviceToHost, sd));
+        CS_CUDA(cudaEventRecord(out_ev, sc));  // (a wait that was enqueued keeps the event's record of that time)
+        CS_CUDA(cudaStreamWaitEvent(sd, out_ev, 0));
+        CS_CUDA(cudaMemcpyAsync(host_out + from * ld0, src, (size_t)cnt * sizeof(double), cudaMemcpyDeviceToHost, sd));
         return CS_OK;
     };
-    if (batch) {
-        // One batch launch per set c = 2s + k (band_set).
-        const long long nsets = 2 * (sweeps - 1) + bands;
-        for (long long set = 0; set < nsets; ++set) {
-            if (set < bands) {
-                const cs_status st = arrive((int)std::min<long long>(set + 1, bands - 1));
-                if (st != CS_OK) return st;
-            }
-            const cs_plan::BandSet &bs = p->band.sets[set];
-            CS_CUDA(cs::launch_tc_batch(fp64, (const char *)p->band.tab + bs.rec * rb, bs.count, bs.tiles, p->wait,
-                                        sc));
-            for (const auto &x : band_set(bands, sweeps, set))
-                if (x.s == sweeps - 1) {
-                    const cs_status st = band_done(x.k);
-                    if (st != CS_OK) return st;
-                }
+    const long long groups = (slabs + align * sweeps + height - 1) / height;
+    long long sent = 0;  // buffer slabs on their way back
+    for (long long g = 0; g < groups; ++g) {
+        const cs_status st = arrive((int)std::min<long long>(g, bands - 1));
+        if (st != CS_OK) return st;
+        long long hi = 0;
+        for (long long sw = 1; sw <= sweeps; ++sw) {
+            const long long lo = std::max(0LL, g * height - align * sw);
+            hi = std::min(slabs, (g + 1) * height - align * sw);
+            if (hi > lo) CS_CUDA(launch_sweep_rows(p, algo, d[(sw - 1) & 1], d[sw & 1], lo, hi - lo, sc));
         }
-    } else {
-        // One launch per band-sweep, diagonal by diagonal (d = k + s): a
-        // topological order too, with (k, s) launched before (k - 1, s + 1),
-        // which overwrites the rows it reads; (k, 0) waits for bands k, k + 1.
-        for (long long diag = 0; diag < bands + sweeps - 1; ++diag) {
-            for (long long sw = std::max(0LL, diag - (bands - 1)); sw <= std::min(sweeps - 1, diag); ++sw) {
-                const int k = (int)(diag - sw);
-                if (sw == 0) {
-                    const cs_status st = arrive(std::min(k + 1, bands - 1));
-                    if (st != CS_OK) return st;
-                }
-                CS_CUDA(launch_sweep_rows(p, algo, d[sw & 1], d[(sw + 1) & 1], b[k], b[k + 1] - b[k], sc));
-                if (sw == sweeps - 1) {
-                    const cs_status st = band_done(k);
-                    if (st != CS_OK) return st;
-                }
-            }
+        const long long end = hi == slabs ? total : first + hi;
+        if (hi > 0 && end > sent) {
+            const cs_status done = slabs_done(sent, end);
+            if (done != CS_OK) return done;
+            sent = end;
         }
     }
     CS_CUDA(cudaEventRecord(e1, sc));
@@ -1458,6 +1332,8 @@ cs_status host_run_banded(cs_plan *p, int algo, int bands, const double *host_in
     return CS_OK;
 }
 
+// in_elems doubles from host_in into buffer 0 (buffer 1 zero), `sweeps`
+// sweeps, then out_elems doubles from result + out_offset to host_out.
 cs_status host_run(cs_plan *p, const double *host_in, size_t in_elems, double *host_out,
                    size_t out_offset, size_t out_elems, long long steps, double *loop_seconds)
 {
@@ -1490,11 +1366,11 @@ cs_status host_run(cs_plan *p, const double *host_in, size_t in_elems, double *h
     }
     const bool whole = in_elems * elem_bytes == bytes;
     int balgo = 0, bands = 0;
-    if (whole && out_offset == 0 && out_elems == (size_t)n && banded_ok(p, sweeps, kept.owns_lock(), &balgo, &bands)) {
+    if (whole && out_offset == 0 && out_elems == (size_t)n && banded_ok(p, sweeps, &balgo, &bands)) {
         unsigned w0 = 0, w1 = 0;
         s = cs_device_wait_timeouts(&w0, 0);
         if (s != CS_OK) return s;
-        s = host_run_banded(p, balgo, bands, host_in, host_out, sweeps, d, kept.owns_lock(), loop_seconds);
+        s = host_run_banded(p, balgo, bands, host_in, host_out, sweeps, d, loop_seconds);
         if (s != CS_OK) return s;
         p->last_algo = balgo;
         p->last_time_block = 1;
