@@ -235,6 +235,38 @@ __global__ void __launch_bounds__(256) k3d_fma(const double *__restrict__ in,
     }
 }
 
+// Radius 1: an output a thread and no shared memory. Its 7 or 27 loads are all
+// in flight together, where the march above waits for a plane at a time; the
+// neighbours' come from L1. On large grids both are bound by the FP64 pipes, so
+// this one takes every size, overlapped with the previous sweep's end. (GB300, us a
+// sweep, the march and this: 7 points 32^3 5.9 and 2.5, 64^3 10.5 and 5.9, 128^3 39.1
+// and 30.0, 256^3 274 and 227; 27 points 8.7 and 5.6, 22.7 and 16.3, 123 and 111,
+// 933 and 863. Two and four planes a thread are no faster on large grids and
+// slower on small ones: 7 points 64^3 7.9 and 10.6.)
+template <int P>
+__global__ void __launch_bounds__(128) k3d_fma1(const double *__restrict__ in, double *__restrict__ out, int m, int n,
+                                                long long ldy, long long ldz, unsigned gx, unsigned gy, WK<27> w)
+{
+    const unsigned rest = blockIdx.x / gx;  // one grid axis: the others end at 65,535
+    const int x = (int)(blockIdx.x - rest * gx) * 32 + (threadIdx.x & 31);
+    const int z = (int)(rest / gy), y = (int)(rest - z * gy) * 4 + (threadIdx.x >> 5);
+    tc::pdl_allow_dependents();
+    tc::pdl_wait();
+    if (x >= n || y >= m) return;
+    const long long at = (long long)z * ldz + (long long)y * ldy + x;
+    const double *src = in + at;
+    double v[27];
+#pragma unroll
+    for (int t = 0; t < 27; ++t)
+        if (tap3<P, 1>(t / 9, t / 3 % 3, t % 3))
+            v[t] = __ldg(src + (t / 9 - 1) * ldz + (t / 3 % 3 - 1) * ldy + (t % 3 - 1));
+    double acc = 0.0;
+#pragma unroll
+    for (int t = 0; t < 27; ++t)
+        if (tap3<P, 1>(t / 9, t / 3 % 3, t % 3)) acc = fma(w.v[t], v[t], acc);
+    out[at] = acc;
+}
+
 // ---------------------------------------------------------------- 2D FP64 MMA
 // mma.sync.m8n8k4.f64: A 8x4 (row), B 4x8 (col), C 8x8. Lane l holds
 // A[l/4][l%4], B[l%4][l/4], C[l/4][2(l%4)], C[l/4][2(l%4)+1].
@@ -347,6 +379,14 @@ cudaError_t go2d(const GridView &g, const Weights &w, const double *in, double *
                                    pack<K * K>(w));
 }
 
+template <int P>
+cudaError_t go3d_r1(const GridView &g, const Weights &w, const double *in, double *out, cudaStream_t st)
+{
+    const unsigned gx = ceil_div(g.ext[2], 32), gy = ceil_div(g.ext[1], 4);
+    return launch(true, k3d_fma1<P>, dim3((unsigned)(g.ext[0] * gx * gy)), 128, 0, st, in, out, (int)g.ext[1],
+                  (int)g.ext[2], g.pitch[1], g.pitch[0], gx, gy, pack<27>(w));
+}
+
 template <int R, int P>
 cudaError_t go3d(const GridView &g, const Weights &w, const double *in, double *out,
                  cudaStream_t st)
@@ -406,8 +446,8 @@ cudaError_t launch_fp64_fma(const GridView &g, int R, int P, const Weights &w, c
         }
     } else if (g.dims == 3) {
         if (R == 1) {
-            if (P == PAT_STAR) return go3d<1, PAT_STAR>(g, w, in, out, st);
-            return go3d<1, PAT_DENSE>(g, w, in, out, st);
+            if (P == PAT_STAR) return go3d_r1<PAT_STAR>(g, w, in, out, st);
+            return go3d_r1<PAT_DENSE>(g, w, in, out, st);
         }
         if (R == 3) {
             if (P == PAT_STAR) return go3d<3, PAT_STAR>(g, w, in, out, st);

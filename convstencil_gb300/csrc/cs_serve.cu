@@ -582,10 +582,11 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     // block (their results do not depend on it).
     // The lines between kernels are where single sweeps of both took as long
     // (GB300, us per sweep, alone): split 7x7 256^2 8.4 mma.sync, 7.3 tcgen05;
-    // split box3d1r 64^3 10.6 double-float, 10.8 tcgen05, 96^3 18.7, 16.9;
-    // FP64 7x7 256^2 18.7 FMA, 9.5 tcgen05 (an FMA tile takes 14 us however
-    // few there are); box3d1r 32^3 10.6, 9.3; star3d1r 80^3 16.6, 17.5, 96^3
-    // 20.7, 20.5; star2d1r 512^2 6.4, 4.4 (three steps a launch). The fused
+    // split box3d1r 64^3 10.5 double-float, 8.0 tcgen05, 96^3 18.7, 13.3 (its five
+    // digits err by up to twice as much as double-float, so smaller requests
+    // keep that); FP64 7x7 256^2 18.7 FMA, 9.5 tcgen05 (an FMA tile takes 14 us however few there
+    // are); box3d1r 32^3 5.7, 8.4, 48^3 12.3, 8.9; star3d1r 96^3 13.5, 18.4, 128^3
+    // 29.8, 29.0; star2d1r 512^2 6.4, 4.4 (three steps a launch). The fused
     // 7x7x7 box costs 343 FMA per point, 171 us at 64^3 against 41; its
     // octahedron 63, about as long at 64^3.
     const bool box3d = d->shape == CS_SHAPE_BOX3D1R, in3d = box3d || d->shape == CS_SHAPE_STAR3D1R;
@@ -604,7 +605,7 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     } else {
         bool tc;
         if (in3d)
-            tc = pts >= (fused ? (box3d ? 3.2e4 : 2.6e5) : (box3d ? 3.2e4 : 8.8e5));
+            tc = pts >= (fused ? (box3d ? 3.2e4 : 2.6e5) : (box3d ? 6e4 : 2e6));
         else if (in1d)
             tc = pts >= 2.6e5;
         else  // radius 3 any size, radius 1 from 64 tiles
