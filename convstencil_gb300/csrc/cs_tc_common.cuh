@@ -80,11 +80,15 @@ __device__ __forceinline__ unsigned long long globaltimer()
     return t;
 }
 
+// A waiting warp sleeps up to 2 us at a time: with the default limit the waits
+// of the slicers and the producer take more of the others' issue slots and
+// shared-memory cycles (GB300, us a launch: box2d3r 8192^2 327 and 319, split
+// box3d1r 512^3 732 and 724).
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity)
 {
     unsigned ok;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n"
         " selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
