@@ -354,17 +354,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int grp = sidx / kGroupWarps, gw = sidx % kGroupWarps;
         const int st = 32 * gw + lane;
         const bool leader = st == 0;
-        int q = 0;
-        bool go = true;
-        for (int item = first; item < items && go; item += step) {
-            const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
-            for (int p = 0; p < wi.zn + 2; ++p, ++q) {
-                if (q % kGroups != grp) continue;
-                const int sb = q % kStages, slot = q % NPL;
+        // Of a sequence of planes that runs through all items the group takes
+        // numbers grp + kGroups j, with `slot` and `lap` their remainder by NPL
+        // and the parity of the quotient.
+        int slot = grp, lap = 0;
+        long long planes = 0;  // of all items of this CTA
+        for (int item = first; item < items; item += step) planes += item_of(item, tiles_x, tiles_y, zc, h).zn + 2;
+        {
+            const int own = (int)((planes - grp + kGroups - 1) / kGroups);
+            for (int j = 0; j < own; ++j) {
+                const int q = grp + kGroups * j, set = j & 1, sb = grp + kGroups * set;
                 // (a) window landed? Every thread waits for itself; one barrier
                 // per plane, at (c), makes the group agree to go on.
-                const bool landed = wait(bar(S.stage_full, sb), (q / kStages) & 1);
-                const int set = (q / kGroups) & 1;
+                const bool landed = wait(bar(S.stage_full, sb), (j >> 1) & 1);
                 // (b) window -> registers, then release the stage to the next load.
                 const uint4 *stg = S.stage[sb];
                 uint4 v[PER];
@@ -399,9 +401,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // (c) digit-plane set free (the MMAs that read it are done)?
                 // The barrier also publishes the maxima; the group's next
                 // plane's are in the other set.
-                const bool free = landed && wait(bar(S.planes_empty, slot), ((q / NPL) & 1) ^ 1);
-                go = !bar_any(kSliceBarrier + grp, kGroupThreads, !free);
-                if (!go) break;
+                const bool free = landed && wait(bar(S.planes_empty, slot), lap ^ 1);
+                if (bar_any(kSliceBarrier + grp, kGroupThreads, !free)) break;
                 int ex;
                 if constexpr (F::kF64) {
                     int eb = S.redi[grp][set][0];
@@ -414,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     for (int i = 1; i < kGroupWarps; ++i) vmax = fmaxf(vmax, S.red[grp][set][i]);
                     ex = split::tile_exponent(vmax);
                 }
-                if (leader) S.scale_exp[q % kScaleRing] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
+                if (leader) S.scale_exp[(unsigned)q % kScaleRing] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
                 unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[slot][0][0]);
                 if constexpr (F::kF64) {
                     if (ex >= kFastExp) {
@@ -451,6 +452,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(S.planes_full, slot));
+                slot += kGroups;
+                if (slot >= NPL) {
+                    slot -= NPL;
+                    lap ^= 1;
+                }
             }
         }
     } else if ((kEpiMask >> warp) & 1u) {
@@ -468,12 +474,27 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int mrow = 32 * quarter + lane;
         const int er = mrow >> 3, eb = mrow & 7;
         const unsigned lane_bits = (unsigned)(32 * quarter) << 16;
+        unsigned q = 0;    // input plane, of a sequence through all items
+        int blk = 0, full = 0;  // its TMEM block, and the parity of its turn
+        auto release = [&] {  // the block is drained: hand it back
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(S.blk_empty, blk));
+        };
+        auto next = [&] {
+            ++q;
+            if (++blk == NBLK) {
+                blk = 0;
+                full ^= 1;
+            }
+        };
         if constexpr (F::kF64) {
-        int q0 = 0;  // first input plane of the item
         bool ok = true;
         for (int item = first; item < items && ok; item += step) {
             const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
             const int xb = wi.x0 + 8 * eb + 4 * hh, yy = wi.y0 + er;
+            const bool whole = yy < m && xb + 3 < n;
+            typename F::Out *op = out + (long long)(wi.zs - 2) * ldz + (long long)yy * ldy + xb;  // plane p - 2
             // Running sums of outputs p - 2 (a) and p - 1 (b). A part's six
             // level sums combine into one 64-bit integer T (value T 2^c,
             // c = plane exponent + ew - 1080, as in the 2D kernel); while every
@@ -521,20 +542,51 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int c = 0; c < 4; ++c)
                     sm[c] = __double_as_longlong(__longlong_as_double(sm[c]) + f64_from_fixed(t[c], ex + ew - 1080));
             };
-            auto load_part = [&](int q, int dz, float (&acc)[D][4]) {
-                const unsigned col = (unsigned)(kBlk<F> * (q % NBLK) + 8 * dz + 4 * hh);
+            auto load_part = [&](int dz, float (&acc)[D][4]) {
+                const unsigned col = (unsigned)(kBlk<F> * blk + 8 * dz + 4 * hh);
 #pragma unroll
                 for (int L = 0; L < D; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
                 tmem_wait_ld();
             };
-            for (int p = 0; p < wi.zn + 2; ++p) {
-                const int q = q0 + p;
-                if (!(ok = wait(bar(S.blk_full, q % NBLK), (q / NBLK) & 1))) break;
+            for (int p = 0; p < wi.zn + 2; ++p, op += ldz, next()) {
+                if (!(ok = wait(bar(S.blk_full, blk), full))) break;
                 tc_fence_after();
                 const int ex = S.scale_exp[q % kScaleRing];
                 float acc[D][4];
+                // The usual plane: every sum it goes to has its exponent, and
+                // nothing rare is under way. (All of this is the same in the
+                // whole CTA: the loads want full warps.)
+                const int sc_q = ex + ew - 1080;
+                if (ex == ea && ex == eb2 && p >= 2 && p <= wi.zn && !(fa | fb | na | nb) &&
+                    ex != kNonFiniteTile && f64_scale_is_plain(sc_q)) {
+                    load_part(2, acc);
+                    add_raw(a, acc);
+                    double res[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) res[c] = f64_from_fixed_plain(a[c], sc_q);
+                    if (whole) {
+                        *reinterpret_cast<double2 *>(op) = make_double2(res[0], res[1]);
+                        *reinterpret_cast<double2 *>(op + 2) = make_double2(res[2], res[3]);
+                    } else if (yy < m) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            if (xb + c < n) op[c] = res[c];
+                    }
+                    __syncwarp();
+                    load_part(1, acc);
+                    add_raw(b, acc);
+                    load_part(0, acc);
+                    release();
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        a[c] = b[c];
+                        b[c] = (long long)(0 - 3 * kRawBias);
+                    }
+                    add_raw(b, acc);
+                    continue;
+                }
                 // z tap 2 of output p - 2: its last part; store.
-                load_part(q, 2, acc);
+                load_part(2, acc);
                 if (p >= 2) {
                     add_part(a, ea, fa, na, acc, ex, 1);
                     if (yy < m) {
@@ -550,7 +602,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                                      : fa ? __longlong_as_double(a[c])
                                           : f64_from_fixed(a[c], sc);
                         }
-                        double *op = out + (long long)(wi.zs + p - 2) * ldz + (long long)yy * ldy + xb;
 #pragma unroll
                         for (int c = 0; c < 4; c += 2) {
                             if (xb + c + 1 < n)
@@ -561,14 +612,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 }
                 // z tap 1 of output p - 1.
-                load_part(q, 1, acc);
+                load_part(1, acc);
                 if (p >= 1 && p - 1 < wi.zn) add_part(b, eb2, fb, nb, acc, ex, 2);
                 // z tap 0 of output p: its first part. The block is then
                 // drained and handed back.
-                load_part(q, 0, acc);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(S.blk_empty, q % NBLK));
+                load_part(0, acc);
+                release();
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {  // rotate: p - 1 becomes p - 2, p starts
                     a[c] = b[c];
@@ -582,14 +631,16 @@ __global__ void __launch_bounds__(kThreads, 1)
                 nb = ex == kNonFiniteTile;
                 if (!nb) add_raw(b, acc);
             }
-            q0 += wi.zn + 2;
         }
         } else {
-        int q0 = 0;  // first input plane of the item
+        float scale = 0.f;  // 2^scale_e
+        int scale_e = -(1 << 20);
         bool ok = true;
         for (int item = first; item < items && ok; item += step) {
             const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
             const int xb = wi.x0 + 8 * eb + 4 * hh, yy = wi.y0 + er;
+            const bool whole = yy < m && xb + 3 < n;
+            typename F::Out *op = out + (long long)(wi.zs - 2) * ldz + (long long)yy * ldy + xb;  // plane p - 2
             // Running sums of outputs p - 2 (a) and p - 1 (b). While every
             // part added to a sum had the same plane scale (2^ea, 2^eb2), the
             // sum is kept as level sums: S0, S1, S2 exact (three parts of at
@@ -649,20 +700,65 @@ __global__ void __launch_bounds__(kThreads, 1)
                     sm[0][c] = s2;
                 }
             };
-            auto load_part = [&](int q, int dz, float (&acc)[D][4]) {
-                const unsigned col = (unsigned)(kBlk<F> * (q % NBLK) + 8 * dz + 4 * hh);
+            auto load_part = [&](int dz, float (&acc)[D][4]) {
+                const unsigned col = (unsigned)(kBlk<F> * blk + 8 * dz + 4 * hh);
 #pragma unroll
                 for (int L = 0; L < D; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
                 tmem_wait_ld();
             };
-            for (int p = 0; p < wi.zn + 2; ++p) {
-                const int q = q0 + p;
-                if (!(ok = wait(bar(S.blk_full, q % NBLK), (q / NBLK) & 1))) break;
+            for (int p = 0; p < wi.zn + 2; ++p, op += ldz, next()) {
+                if (!(ok = wait(bar(S.blk_full, blk), full))) break;
                 tc_fence_after();
                 const int ex = S.scale_exp[q % kScaleRing];
                 float acc[D][4];
+                // The usual plane: every sum it goes to has its scale.
+                if (ex == ea && ex == eb2 && p >= 2 && p <= wi.zn && !(fa | fb)) {
+                    if (ex != scale_e) {
+                        scale_e = ex;
+                        scale = ldexpf(1.0f, ex + sw.ew - 2 * kDigitBits);
+                    }
+                    load_part(2, acc);
+                    float2 res[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float s0 = a[0][c] + acc[0][c], s1 = a[1][c] + acc[1][c], s2 = a[2][c] + acc[2][c];
+                        const float s3 = a[3][c] + tail(acc[3][c], acc[4][c]);
+                        float h1, e1, h2, e2, hi, lo;
+                        two_sum(s0, s1 * 0x1p-9f, h1, e1);
+                        two_sum(h1, s2 * 0x1p-18f, h2, e2);
+                        two_sum(h2, (e1 + e2) + s3, hi, lo);
+                        res[c] = make_float2(hi * scale, lo * scale);
+                    }
+                    if (whole) {
+                        *reinterpret_cast<float4 *>(op) = make_float4(res[0].x, res[0].y, res[1].x, res[1].y);
+                        *reinterpret_cast<float4 *>(op + 2) = make_float4(res[2].x, res[2].y, res[3].x, res[3].y);
+                    } else if (yy < m) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            if (xb + c < n) op[c] = res[c];
+                    }
+                    __syncwarp();
+                    load_part(1, acc);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        a[0][c] = b[0][c] + acc[0][c];
+                        a[1][c] = b[1][c] + acc[1][c];
+                        a[2][c] = b[2][c] + acc[2][c];
+                        a[3][c] = b[3][c] + tail(acc[3][c], acc[4][c]);
+                    }
+                    load_part(0, acc);
+                    release();
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        b[0][c] = acc[0][c];
+                        b[1][c] = acc[1][c];
+                        b[2][c] = acc[2][c];
+                        b[3][c] = tail(acc[3][c], acc[4][c]);
+                    }
+                    continue;
+                }
                 // z tap 2 of output p - 2: its last part; store.
-                load_part(q, 2, acc);
+                load_part(2, acc);
                 if (p >= 2) {
                     add_part(a, ea, fa, acc, ex);
                     if (!fa) to_pair(a);
@@ -675,7 +771,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                             two_sum(a[0][c], a[1][c], hi, lo);
                             res[c] = make_float2(hi * scale, lo * scale);
                         }
-                        float2 *op = out + (long long)(wi.zs + p - 2) * ldz + (long long)yy * ldy + xb;
 #pragma unroll
                         for (int c = 0; c < 4; c += 2) {
                             if (xb + c + 1 < n)
@@ -687,14 +782,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 }
                 // z tap 1 of output p - 1.
-                load_part(q, 1, acc);
+                load_part(1, acc);
                 if (p >= 1 && p - 1 < wi.zn) add_part(b, eb2, fb, acc, ex);
                 // z tap 0 of output p: its first part. The block is then
                 // drained and handed back.
-                load_part(q, 0, acc);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar(S.blk_empty, q % NBLK));
+                load_part(0, acc);
+                release();
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {  // rotate: p - 1 becomes p - 2, p starts
 #pragma unroll
@@ -709,7 +802,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                 eb2 = ex;
                 fb = false;
             }
-            q0 += wi.zn + 2;
         }
         }
     }
