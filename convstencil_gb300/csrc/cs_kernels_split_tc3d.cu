@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint4 *stg = S.stage[sb];
                 uint4 v[PER];
                 float vmax = 0.f;   // split: largest |hi|
-                unsigned emax = 0;  // FP64: largest biased exponent
+                unsigned emax = 0;  // FP64: largest upper word without its sign, then biased exponent
 #pragma unroll
                 for (int k = 0; k < PER; ++k) {
                     const int u = st + k * kGroupThreads;
@@ -379,13 +379,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (u < NCUT) {
                         v[k] = stg[(u / NCUTX) * PAIRS + CUT0 + u % NCUTX];
                         if constexpr (F::kF64)
-                            emax = max(emax, max((v[k].y >> 20) & 0x7FFu, (v[k].w >> 20) & 0x7FFu));
+                            emax = max(emax, max(v[k].y & 0x7FFFFFFFu, v[k].w & 0x7FFFFFFFu));
                         else
                             vmax = fmaxf(vmax, fmaxf(fabsf(__uint_as_float(v[k].x)), fabsf(__uint_as_float(v[k].z))));
                     }
                 }
                 if constexpr (F::kF64) {
-                    emax = __reduce_max_sync(0xffffffffu, emax);
+                    emax = __reduce_max_sync(0xffffffffu, emax) >> 20;
                 } else {
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
