@@ -22,10 +22,11 @@
 //     (0..6) starts i plane rows lower.
 //   * Input plane P feeds outputs P .. P - 6 (counted from the column's first)
 //     as their z taps 0 .. 6. The taps go to N in two halves, dz 0..3 and
-//     4..6: column n of B_{half,i} is (digit e, dz % 4, column c), n = 32 e +
-//     8 (dz % 4) + c, and one MMA with N = 32 (6 - d) feeds levels d..5, so a
-//     half is 7 row offsets x 6 digits = 42 MMAs into 192 TMEM columns. The
-//     two halves are the two TMEM blocks: one is drained while the other is
+//     4..6: column n of B_{half,i} is (digit e, dz % 4, column c), n = 32 e
+//     (24 e) + 8 (dz % 4) + c, and one MMA with N = 32 (24) x (6 - d) feeds levels
+//     d..5, so a half is 7 row offsets x 6 digits = 42 MMAs into 192 (144) TMEM
+//     columns. (With the second half padded to 32 a level: 200 x 184 x 192, GB300,
+//     185 us a sweep, so 177.) The two halves are the two TMEM blocks: one is drained while the other is
 //     being computed. (All seven taps in one N would need 384 columns, one
 //     block of the 512, and a wait for the epilogue after every plane.)
 //   * Bound: the MMA stream and the shared memory it reads. An MMA reads 4 KB
@@ -91,7 +92,12 @@ constexpr int TX = 64, TY = 16;              // output tile
 constexpr int ST_X = TX + 8, ST_Y = TY + 6;  // window: 72 columns, rows y0-3 .. y0+18
 constexpr int PL = ST_X * ST_Y;              // halves per digit plane
 constexpr unsigned kRowBytes = ST_X * 2;     // 144
-constexpr int NOFF = 7, NLV = 32, NCOL = NLV * D;  // 192 columns per half
+constexpr int NOFF = 7, NCOL = 32 * D;       // rows of B: 192, and 144 of the second half
+// TMEM columns per level: four tap planes x 8, three in the second half; and N
+// of an MMA that feeds `levels` levels (M = 128 wants multiples of 16; the 8
+// columns of an odd count lie behind the block's last level and are not read).
+__host__ __device__ constexpr int nlv(int half) { return half ? 24 : 32; }
+__host__ __device__ constexpr int mma_n(int half, int levels) { return (nlv(half) * levels + 15) / 16 * 16; }
 constexpr int kBlkStride = 256, kTmemCols = 512;
 constexpr int kStages = 4, NPL = 4;
 constexpr int kScaleRing = 32;               // planes in flight stay below it
@@ -122,7 +128,7 @@ __device__ __forceinline__ void half_mma(unsigned d_base, unsigned long long a, 
     constexpr unsigned long long a_off = ((unsigned long long)DG * PL * 2 + I * kRowBytes) >> 4;
     constexpr unsigned long long b_off = ((unsigned long long)(HZ * NOFF + I) * NCOL * 16 * 2) >> 4;
     static_assert(((unsigned long long)DG * PL * 2 + I * kRowBytes) % 16 == 0, "descriptor offsets");
-    mma_f16(d_base + (unsigned)(NLV * DG), a + a_off, b0 + b_off, instr_desc(NLV * (D - DG)),
+    mma_f16(d_base + (unsigned)(nlv(HZ) * DG), a + a_off, b0 + b_off, instr_desc(mma_n(HZ, D - DG)),
             (I | DG) != 0 ? 1u : 0u);
     if constexpr (DG + 1 < D)
         half_mma<HZ, I, DG + 1>(d_base, a, b0);
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                      "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    // B_{half,i}: N row nn = 32 e + 8 dzl + c, K index k, tap column tj = k - c
+    // B_{half,i}: N row nn = 32 e (24 e) + 8 dzl + c, K index k, tap column tj = k - c
     // - (left - 3). The weight rows are staged first, padded with zeros (row
     // (e, dz, ti) by one warp: uniform parameter reads), then written in
     // 16-byte chunks of eight k, consecutive halves of a staged row.
@@ -215,11 +221,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int hi = idx / (NCOL * 2), rem = idx - hi * (NCOL * 2);
         const int hz = hi / NOFF, i = hi - hz * NOFF;
         const int nn = rem >> 1, kh = rem & 1;
-        const int e = nn / NLV, dz = 4 * hz + ((nn % NLV) >> 3), c = nn & 7;
+        const int e = nn / nlv(hz), dz = 4 * hz + ((nn % nlv(hz)) >> 3), c = nn & 7;
         __align__(16) __half v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            v[k] = dz < 7 ? wz[(e * 49 + dz * 7 + i) * kWz + 8 * kh + 11 - left - c + k] : __float2half(0.f);
+            v[k] = e < D ? wz[(e * 49 + dz * 7 + i) * kWz + 8 * kh + 11 - left - c + k] : __float2half(0.f);
         *reinterpret_cast<uint4 *>(&S.bmat[hz][i][(nn >> 3) * 128 + (nn & 7) * 8 + kh * 64]) =
             *reinterpret_cast<const uint4 *>(v);
     }
@@ -338,10 +344,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                             if (!row || xx < -3 || xx > n + 2) v[k].x = v[k].y = 0u;
                             if (!row || xx + 1 < -3 || xx + 1 > n + 2) v[k].z = v[k].w = 0u;
                         }
-                        emax = max(emax, max((v[k].y >> 20) & 0x7FFu, (v[k].w >> 20) & 0x7FFu));
+                        emax = max(emax, max(v[k].y & 0x7FFFFFFFu, v[k].w & 0x7FFFFFFFu));
                     }
                 }
-                emax = __reduce_max_sync(0xffffffffu, emax);
+                emax = __reduce_max_sync(0xffffffffu, emax) >> 20;
                 __syncwarp();
                 if (lane == 0) {
                     S.redi[grp][set][gw] = (int)emax;
@@ -418,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         const int dz = 4 * hz + dl;
                         float acc[D][2];
 #pragma unroll
-                        for (int L = 0; L < D; ++L) tmem_ld2(taddr + kBlkStride * hz + NLV * L + 8 * dl, acc[L]);
+                        for (int L = 0; L < D; ++L) tmem_ld2(taddr + kBlkStride * hz + nlv(hz) * L + 8 * dl, acc[L]);
                         tmem_wait_ld();
                         if (dl == (hz ? 2 : 3)) {  // block drained: hand it back
                             tc_fence_before();
