@@ -219,6 +219,14 @@ __device__ __forceinline__ void tmem_ld4(unsigned taddr, float (&v)[4])
     for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
 }
 
+// The larger, or NaN where one is.
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // Recombines five exact level sums (level L in units of 2^-9L) into a
 // double-float pair.
 __device__ __forceinline__ void recombine(const float (&acc)[split::kDigits], float &hi, float &lo)
@@ -381,14 +389,22 @@ __global__ void __launch_bounds__(kThreads, 1)
                         if constexpr (F::kF64)
                             emax = max(emax, max(v[k].y & 0x7FFFFFFFu, v[k].w & 0x7FFFFFFFu));
                         else
-                            vmax = fmaxf(vmax, fmaxf(fabsf(__uint_as_float(v[k].x)), fabsf(__uint_as_float(v[k].z))));
+                            vmax = max_nan(vmax, max_nan(fabsf(__uint_as_float(v[k].x)), fabsf(__uint_as_float(v[k].z))));
                     }
                 }
                 if constexpr (F::kF64) {
                     emax = __reduce_max_sync(0xffffffffu, emax) >> 20;
                 } else {
+                    vmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(vmax)));
+                    if (!(vmax <= 3.402823466e38f)) {  // an Inf or a NaN: the largest of the numbers, with a sign
+                        vmax = 0.f;
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+                        for (int k = 0; k < PER; ++k)
+                            vmax = fmaxf(vmax, fmaxf(fabsf(__uint_as_float(v[k].x)), fabsf(__uint_as_float(v[k].z))));
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+                        vmax = -vmax;
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) {
@@ -404,15 +420,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const bool free = landed && wait(bar(S.planes_empty, slot), lap ^ 1);
                 if (bar_any(kSliceBarrier + grp, kGroupThreads, !free)) break;
                 int ex;
+                bool finite = true;  // split: no Inf or NaN in the plane
                 if constexpr (F::kF64) {
                     int eb = S.redi[grp][set][0];
 #pragma unroll
                     for (int i = 1; i < kGroupWarps; ++i) eb = max(eb, S.redi[grp][set][i]);
                     ex = max(eb, 1);
                 } else {
-                    vmax = S.red[grp][set][0];
+                    vmax = 0.f;
 #pragma unroll
-                    for (int i = 1; i < kGroupWarps; ++i) vmax = fmaxf(vmax, S.red[grp][set][i]);
+                    for (int i = 0; i < kGroupWarps; ++i) {
+                        const float w = S.red[grp][set][i];
+                        vmax = fmaxf(vmax, fabsf(w));
+                        finite = finite && __float_as_int(w) >= 0;
+                    }
                     ex = split::tile_exponent(vmax);
                 }
                 if (leader) S.scale_exp[(unsigned)q % kScaleRing] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
@@ -435,17 +456,35 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 } else {
                     const float to_digits = ldexpf(1.0f, kDigitBits - ex);
+                    if (finite) {
+                        split::f2x s2;
+                        asm("mov.b64 %0, {%1, %1};" : "=l"(s2) : "f"(to_digits));
 #pragma unroll
-                    for (int k = 0; k < PER; ++k) {
-                        const int u = st + k * kGroupThreads;
-                        if (u < NCUT) {
-                            const int idx = (u / NCUTX) * PAIRS + CUT0 + u % NCUTX;
-                            float d0[D], d1[D];
-                            slice_digits(__uint_as_float(v[k].x) * to_digits, __uint_as_float(v[k].y) * to_digits, d0);
-                            slice_digits(__uint_as_float(v[k].z) * to_digits, __uint_as_float(v[k].w) * to_digits, d1);
-                            unsigned *dst = dst0 + idx;
+                        for (int k = 0; k < PER; ++k) {
+                            const int u = st + k * kGroupThreads;
+                            if (u < NCUT) {
+                                split::f2x a, b;
+                                asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "r"(v[k].x), "r"(v[k].z));
+                                asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(v[k].y), "r"(v[k].w));
+                                unsigned wd[D];
+                                split::slice_digit_pairs_x2(split::f2_mul(a, s2), split::f2_mul(b, s2), wd);
+                                unsigned *dst = dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX;
 #pragma unroll
-                            for (int dg = 0; dg < D; ++dg) dst[dg * (PL / 2)] = split::pack_h2(d0[dg], d1[dg]);
+                                for (int dg = 0; dg < D; ++dg) dst[dg * (PL / 2)] = wd[dg];
+                            }
+                        }
+                    } else {  // digits of an Inf or NaN are NaN here
+#pragma unroll
+                        for (int k = 0; k < PER; ++k) {
+                            const int u = st + k * kGroupThreads;
+                            if (u < NCUT) {
+                                float d0[D], d1[D];
+                                slice_digits(__uint_as_float(v[k].x) * to_digits, __uint_as_float(v[k].y) * to_digits, d0);
+                                slice_digits(__uint_as_float(v[k].z) * to_digits, __uint_as_float(v[k].w) * to_digits, d1);
+                                unsigned *dst = dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX;
+#pragma unroll
+                                for (int dg = 0; dg < D; ++dg) dst[dg * (PL / 2)] = split::pack_h2(d0[dg], d1[dg]);
+                            }
                         }
                     }
                 }
