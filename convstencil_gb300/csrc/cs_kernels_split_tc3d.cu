@@ -73,15 +73,13 @@ using namespace tc;
 // 128-column TMEM blocks) and FP64 (FP64 grids, six digits cut with integer
 // operations as in the 2D kernel, a ring of three 160-column blocks).
 //
-// FP64 is bound by its epilogue (GB300, star3d1r 512^3: 2,400 cycles a plane of
-// 1024 outputs, of which the epilogue waits 160; 1,590 with its arithmetic left
-// out). The conversions to FP64, 64 cycles a warp on a scheduler's FP64 unit,
-// are a third of it: without them 1,690. Not faster: conversions by integer
-// operations (1200 us a sweep against 1112; that pipe is the slicers'),
-// interleaved with the other parts (1104 to 1170), two columns a step with the
-// next ones' loads in flight (1277), all three parts loaded first with 112
-// registers for the epilogue by setmaxnreg (1287; split 826 against 738),
-// sixteen epilogue warps (1171 against 1126).
+// FP64 is bound by its epilogue and the slicers' integer operations: 155
+// instructions an output, 0.6 of the schedulers' slots (GB300, star3d1r 512^3, 861
+// us a sweep). Not faster: conversions to FP64 by integer operations (1200 us
+// against 1112 then), two columns a step with the next ones' loads in flight
+// (1277), all three parts loaded first with 112 registers for the epilogue by
+// setmaxnreg (1287; split 826 against 738), sixteen epilogue warps (1171 against
+// 1126), two planes per loop iteration (930 against 897, spills).
 struct F3Split {
     static constexpr bool kF64 = false;
     static constexpr int D = split::kDigits;  // 5
@@ -581,10 +579,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int c = 0; c < 4; ++c)
                     sm[c] = __double_as_longlong(__longlong_as_double(sm[c]) + f64_from_fixed(t[c], ex + ew - 1080));
             };
-            auto load_part = [&](int dz, float (&acc)[D][4]) {
+            auto load_issue = [&](int dz, float (&acc)[D][4]) {
                 const unsigned col = (unsigned)(kBlk<F> * blk + 8 * dz + 4 * hh);
 #pragma unroll
                 for (int L = 0; L < D; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
+            };
+            auto load_part = [&](int dz, float (&acc)[D][4]) {
+                load_issue(dz, acc);
                 tmem_wait_ld();
             };
             for (int p = 0; p < wi.zn + 2; ++p, op += ldz, next()) {
@@ -598,11 +599,28 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int sc_q = ex + ew - 1080;
                 if (ex == ea && ex == eb2 && p >= 2 && p <= wi.zn && !(fa | fb | na | nb) &&
                     ex != kNonFiniteTile && f64_scale_is_plain(sc_q)) {
+                    load_part(1, acc);
+                    add_raw(b, acc);
                     load_part(2, acc);
                     add_raw(a, acc);
+                    // The conversions, 64 cycles each on the FP64 unit, run
+                    // beside the last part's load and sum (one after the other
+                    // before the store: star3d1r 512^3, GB300, 897 us, so 861).
+                    load_issue(0, acc);
+                    long long d[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) d[c] = f64_bits_of(a[c]);
+                    tmem_wait_ld();
+                    release();
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        a[c] = b[c];
+                        b[c] = (long long)(0 - 3 * kRawBias);
+                    }
+                    add_raw(b, acc);
                     double res[4];
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) res[c] = f64_from_fixed_plain(a[c], sc_q);
+                    for (int c = 0; c < 4; ++c) res[c] = f64_scaled(d[c], sc_q);
                     if (whole) {
                         *reinterpret_cast<double2 *>(op) = make_double2(res[0], res[1]);
                         *reinterpret_cast<double2 *>(op + 2) = make_double2(res[2], res[3]);
@@ -612,16 +630,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                             if (xb + c < n) op[c] = res[c];
                     }
                     __syncwarp();
-                    load_part(1, acc);
-                    add_raw(b, acc);
-                    load_part(0, acc);
-                    release();
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        a[c] = b[c];
-                        b[c] = (long long)(0 - 3 * kRawBias);
-                    }
-                    add_raw(b, acc);
                     continue;
                 }
                 // z tap 2 of output p - 2: its last part; store.

@@ -204,11 +204,21 @@ __device__ __forceinline__ double f64_from_fixed(long long t, int c)
 // Whether every T != 0 times 2^c is a normal number (|T| < 2^63), and then its
 // value: no range tests per output.
 __device__ __forceinline__ bool f64_scale_is_plain(int c) { return c >= -1022 && c <= 960; }
+// f64_bits_of converts where it is written, f64_scaled does the rest.
+__device__ __forceinline__ long long f64_bits_of(long long t)
+{
+    double d;
+    asm volatile("cvt.rn.f64.s64 %0, %1;" : "=d"(d) : "l"(t));
+    return __double_as_longlong(d);
+}
+__device__ __forceinline__ double f64_scaled(long long bits, int c)
+{
+    const int hi = (int)(bits >> 32);
+    return __hiloint2double(hi != 0 ? hi + (c << 20) : 0, (int)bits);
+}
 __device__ __forceinline__ double f64_from_fixed_plain(long long t, int c)
 {
-    const double d = __ll2double_rn(t);
-    const int hi = __double2hiint(d);
-    return __hiloint2double(hi != 0 ? hi + (c << 20) : 0, __double2loint(d));
+    return f64_scaled(__double_as_longlong(__ll2double_rn(t)), c);
 }
 
 // Cuts one pair of points (v: lo, hi words of both) into six digit planes
