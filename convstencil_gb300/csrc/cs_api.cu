@@ -563,6 +563,14 @@ cs_status choose_algo(cs_plan *p, const void *a, void *b, cudaStream_t st, int *
         *out = -1;
         return CS_OK;
     }
+    // A caller that is capturing its stream cannot have one either: the first
+    // candidate, as on plans that have no other.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CS_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        *out = cand[0];
+        return CS_OK;
+    }
     float best_ms = 1e30f;
     int best = cand[0];
     cudaEvent_t e0, e1;
