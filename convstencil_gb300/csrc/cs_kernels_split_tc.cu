@@ -24,6 +24,15 @@
 //     dropped levels >= 6 weigh below 2^-48 of (tile max x largest weight)
 //     in the worst case (about 2^-53 for data without adversarial digits).
 //
+//   * split with six digits (FmtSplit6): the launches of several steps, below,
+//     of split plans, whose errors would otherwise grow with the steps' weights.
+//
+// Modes (MODE): one sweep of a 2D grid (kModeGrid); three steps of a radius-1
+// 2D grid as one sweep of its three times self-convolved kernel, the frame two
+// points wide computed step by step (kModeSteps); up to 23 steps of a 1D grid
+// (kMode1d). BATCH: many grids in one launch. ODD: grids whose rows TMA cannot
+// address one by one (OddRows).
+//
 // Mapping onto tcgen05 (M = 128, K = 16, N = 32 per level):
 //   * A CTA owns a 64 x 64 output tile: 16 row groups of 4 rows, 8 blocks
 //     of 8 columns. Its input window (70 x 72 points, columns x0-4 ..
@@ -49,15 +58,20 @@
 //     accepts it, so the MMAs are unrolled with compile-time descriptor
 //     offsets (measured on GB300: 56 cycles per MMA for the split N =
 //     160..32 sequence, 70 with the descriptors computed in the loop).
-//   * One persistent CTA per SM (about 188 KB of shared memory split, 218 KB
+//   * One persistent CTA per SM (about 188 KB of shared memory split, 219 KB
 //     FP64) with warp roles joined by mbarriers: one warp issues the TMA
 //     window loads, one thread issues the MMAs (tcgen05.mma issue blocks
 //     while the tensor core is busy, so it must not sit in anyone else's
 //     barrier), eight warps read a window into registers, release the stage
 //     to the next load and cut the digit planes, and four (split) or eight
-//     (FP64) warps drain the accumulators, recombine and store. Two accumulators (TMEM columns 0 and
-//     256) and two sets of digit planes let slicing of tile t+1, the MMAs of
-//     tile t and the stores of tile t-1 run at the same time.
+//     (FP64) warps drain the accumulators, recombine and store. Two
+//     accumulators (TMEM columns 0 and 256) and two sets of digit planes let
+//     slicing of tile t+1, the MMAs of tile t and the stores of tile t-1 run at
+//     the same time.
+//   * Bound: the shared memory that the MMAs read (354 KB of operands a tile
+//     split, 455 KB FP64, at 128 bytes a cycle 2,770 and 3,560 cycles) beside
+//     the slicers' and the TMA unit's ~120 KB. GB300, 8192^2: split 291 us a
+//     sweep, FP64 320, three steps of radius 1 353.
 //
 // Every mbarrier wait is bounded (WaitCfg, 2 s by default). An expired wait
 // is counted in g_tc_wait_timeouts; the CTA then waits, again bounded, for
@@ -344,8 +358,8 @@ constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
 // ready, from the same input, with the halo each single sweep would read. A
 // launch costs what one step on the 7x7 pipeline costs (its limit is the
 // digits, not the taps): box2d1r 2047 x 1531, 60 steps, GB300: 1818 us at a
-// step per launch, 639 at three; star2d1r 1024^2, 100 steps: 1295 us on the
-// FP64 FMA kernel (the FP64 pipe takes 10 us of each step's 13), 527 so.
+// step per launch, 525 at three; star2d1r 1024^2, 100 steps: 1295 us on the
+// FP64 FMA kernel (the FP64 pipe takes 10 us of each step's 13), 478 so.
 constexpr int kMaxSteps = 3;
 
 // Grids of odd pitch or odd first column, whose rows are not all 16-byte

@@ -116,7 +116,7 @@ typedef enum cs_algo {
                              plans, box and star (an output's three plane parts are added as exact
                              integers when their plane exponents agree, in FP64 otherwise), and 1D
                              FP64 plans of radius up to 3 whose length is a multiple of 64 (at
-                             least 512) with 4 halo points either side (as rows of 64 outputs) */
+                             least 512) with 4 halo points either side */
 } cs_algo;
 
 typedef enum cs_option {
@@ -222,13 +222,11 @@ CS_API cs_status cs_split_to_fp64(const cs_plan *plan, const void *src, double *
  * device grid (converted to (hi, lo) in place for split plans), runs, copies
  * the result (FP64) to host_out. Synchronous. When the kernel is known
  * without a timing run (pinned, or tuned earlier for this kind of plan), the
- * grid has at least two bands (256 rows for split 7x7 plans on the tensor
- * cores, else 1024 rows in 2D or 64 planes in 3D), and no temporal blocking
- * or re-anchor sweep is involved, the copies overlap the sweeps: the grid
- * moves in bands, the sweeps run as a wavefront over the bands already there,
- * and each band returns after its last sweep (results bitwise those of
- * whole-grid sweeps). The two device grids are
- * allocated by the plan's first call and kept for its later calls until
+ * copies take long enough for that to pay and no temporal blocking or
+ * re-anchor sweep is involved, the copies of 2D and 3D grids overlap the
+ * sweeps: the grid moves in bands, the sweeps of a band run as soon as it is
+ * there, and rows return after their last sweep (results bitwise those of
+ * whole-grid sweeps). The two device grids are allocated by the plan's first call and kept for its later calls until
  * cs_plan_destroy (a call that finds them in use by another thread allocates
  * and frees its own). Returns CS_ERR_TIMEOUT (result incomplete) if a
  * bounded device-side wait expired during the call. */
