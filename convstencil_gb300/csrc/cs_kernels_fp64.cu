@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(128) k2d_fma_small(const double *__restrict__ 
 }
 
 // ---------------------------------------------------------------- 3D
-// CTA column of 16 x 32 outputs marching ZC planes in z; a ring of 2R+1
+// Radius 3: CTA column of 16 x 32 outputs marching ZC planes in z; a ring of 2R+1
 // input planes (with halo) lives in shared memory.
 template <int R>
 constexpr int k3d_smem_bytes()

@@ -70,7 +70,7 @@
 //     the same time.
 //   * Bound: the shared memory that the MMAs read (354 KB of operands a tile
 //     split, 455 KB FP64, at 128 bytes a cycle 2,770 and 3,560 cycles) beside
-//     the slicers' and the TMA unit's ~120 KB. GB300, 8192^2: split 291 us a
+//     the slicers' and the TMA unit's ~120 KB. GB300, 8192^2: split 282 us a
 //     sweep, FP64 320, three steps of radius 1 353.
 //
 // Every mbarrier wait is bounded (WaitCfg, 2 s by default). An expired wait

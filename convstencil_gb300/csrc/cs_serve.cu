@@ -582,9 +582,10 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     // block (their results do not depend on it).
     // The lines between kernels are where single sweeps of both took as long
     // (GB300, us per sweep, alone): split 7x7 256^2 8.4 mma.sync, 7.3 tcgen05;
-    // split box3d1r 64^3 10.5 double-float, 8.0 tcgen05, 96^3 18.7, 13.3 (its five
-    // digits err by up to twice as much as double-float, so smaller requests
-    // keep that); FP64 7x7 256^2 18.7 FMA, 9.5 tcgen05 (an FMA tile takes 14 us however few there
+    // split box3d1r 64^3 10.5 double-float, 8.0 tcgen05, 96^3 18.7, 13.3 (but its
+    // five digits err more than double-float, 1.7e-12 against 1e-14 in the norm
+    // after tens of sweeps, so requests below 2e6 points keep that); FP64 7x7
+    // 256^2 18.7 FMA, 9.5 tcgen05 (an FMA tile takes 14 us however few there
     // are); box3d1r 32^3 5.7, 8.4, 48^3 12.3, 8.9; star3d1r 96^3 13.5, 18.4, 128^3
     // 29.8, 29.0; star2d1r 512^2 6.4, 4.4 (three steps a launch). The fused
     // 7x7x7 box costs 343 FMA per point, 171 us at 64^3 against 41; its
@@ -596,7 +597,7 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     for (int k = 0; k < (in3d ? 3 : in1d ? 1 : 2); ++k) pts *= (double)d->extent[k];
     if (d->precision == CS_PREC_SPLIT) {
         // The 7-point star always has its own double-float kernel.
-        const int algo = in3d ? (box3d && !fused && pts >= 8.8e5 ? CS_ALGO_SPLIT_TC : CS_ALGO_SPLIT_FMA)
+        const int algo = in3d ? (box3d && !fused && pts >= 2e6 ? CS_ALGO_SPLIT_TC : CS_ALGO_SPLIT_FMA)
                               : CS_ALGO_SPLIT_TC;
         if (cs_plan_set_option(r->plan, CS_OPT_ALGO, algo) != CS_OK)
             cs_plan_set_option(r->plan, CS_OPT_ALGO, CS_ALGO_SPLIT_FMA);
