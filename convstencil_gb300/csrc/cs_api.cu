@@ -9,6 +9,7 @@
 // streams can run different stencils at once), no lookup tables exist (the
 // kernels index their tiles directly), and every failure is a status code.
 #include "../../include/convstencil.h"
+#include "cs_host_bands.h"
 #include "cs_internal.h"
 #include "cs_plan_internal.h"
 
@@ -1243,32 +1244,26 @@ bool banded_ok(cs_plan *p, long long sweeps, int *algo, int *bands)
     return *bands >= 2;
 }
 
-// Group g of the sweeps takes level s (1 .. sweeps) of the slabs from
-// g height - align s up to the next group's: it reads nothing that a later
-// group computes or that is still arriving (align >= radius), and overwrites
-// nothing that one still reads, so a group runs all its levels in a row. Every
-// cut is a multiple of the kernels' tiles, so that the tiles see the windows of
-// a whole sweep. (As a wavefront of one sweep per band the first sweeps waited
-// for most of the copy in and the last band's end for most of the copy out;
+// The launches and copies of host_bands (which says why they may run in that
+// order). (As a wavefront of one sweep per band the first sweeps waited for
+// most of the copy in and the last band's end for most of the copy out;
 // GB300, that and so: FP64 box2d3r 4096^2 x 20 sweeps 3.48 and 2.80 ms, 8192^2 11.9
 // and 8.9; split on the batch kernel, a launch for all independent
 // band-sweeps, 2.95 and 2.59, 9.27 and 8.65.)
 cs_status host_run_banded(cs_plan *p, int algo, int bands, const double *host_in, double *host_out,
                           long long sweeps, void *const d[2], double *loop_seconds)
 {
-    const long long ld0 = p->view.pitch[0];        // elements per slab
-    const long long total = p->layout.elements / ld0;  // slabs in the buffer, halo included
-    const long long first = p->layout.origin / ld0;    // halo slabs before the interior
-    const long long slabs = p->view.ext[0];
-    const long long align = p->dims == 2 ? 64 : 8;
-    const long long height = ((slabs + bands - 1) / bands + align - 1) / align * align;
-    std::vector<long long> c(bands + 1);  // buffer slab boundaries of the copies in
-    for (int k = 0; k <= bands; ++k) c[k] = k == 0 ? 0 : k == bands ? total : first + std::min(slabs, height * k);
+    const cs::HostBands plan = cs::host_bands(p->layout, p->radius, bands, sweeps);
+    const std::vector<long long> &c = plan.chunk;
+    const int chunks = (int)c.size() - 1;
     struct Streams {
         cudaStream_t s[3] = {nullptr, nullptr, nullptr};
         std::vector<cudaEvent_t> ev;
         ~Streams()
         {
+            // (after an error too no copy to or from the caller's arrays goes on)
+            for (cudaStream_t x : s)
+                if (x) cudaStreamSynchronize(x);
             for (cudaEvent_t e : ev) cudaEventDestroy(e);
             for (cudaStream_t x : s)
                 if (x) cudaStreamDestroy(x);
@@ -1276,63 +1271,41 @@ cs_status host_run_banded(cs_plan *p, int algo, int bands, const double *host_in
     } S;
     for (auto &x : S.s) CS_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
     cudaStream_t sc = S.s[0], sh = S.s[1], sd = S.s[2];
-    S.ev.resize(bands + 3);
+    S.ev.resize(chunks + 3);
     for (auto &e : S.ev) CS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDefault));
-    cudaEvent_t *in_ev = S.ev.data(), out_ev = S.ev[bands], e0 = S.ev[bands + 1], e1 = S.ev[bands + 2];
-    const size_t slab_bytes = (size_t)ld0 * sizeof(double);
+    cudaEvent_t *in_ev = S.ev.data(), out_ev = S.ev[chunks], e0 = S.ev[chunks + 1], e1 = S.ev[chunks + 2];
     CS_CUDA(cudaMemsetAsync(d[1], 0, (size_t)p->layout.bytes, sc));  // the second grid's halo reads as zero
-    // The copies in go back to back on their own stream; a split plan's band
+    // The copies in go back to back on their own stream; a split plan's chunk
     // is converted to (hi, lo) on the sweep stream just before its first use
     // (on the copy stream, each conversion held up the next copy while the
     // sweep kernel filled the SMs: 8192^2 in 4.1 ms instead of 2.6).
-    for (int k = 0; k < bands; ++k) {
-        const long long cnt = (c[k + 1] - c[k]) * ld0;
-        char *dst = (char *)d[0] + c[k] * slab_bytes;
-        CS_CUDA(cudaMemcpyAsync(dst, host_in + c[k] * ld0, (size_t)cnt * sizeof(double), cudaMemcpyHostToDevice, sh));
+    for (int k = 0; k < chunks; ++k) {
+        CS_CUDA(cudaMemcpyAsync((double *)d[0] + c[k], host_in + c[k], (size_t)(c[k + 1] - c[k]) * sizeof(double),
+                                cudaMemcpyHostToDevice, sh));
         CS_CUDA(cudaEventRecord(in_ev[k], sh));
     }
     CS_CUDA(cudaEventRecord(e0, sc));
-    int arrived = 0;  // bands copied and converted, as the sweep stream sees them
-    auto arrive = [&](int upto) -> cs_status {  // bands 0 .. upto on the device, converted
-        for (; arrived <= upto; ++arrived) {
+    int arrived = 0;  // chunks copied and converted, as the sweep stream sees them
+    void *f = d[sweeps & 1];  // final grid
+    for (const cs::HostBands::Op &op : plan.ops) {
+        for (; arrived < op.chunks; ++arrived) {
             CS_CUDA(cudaStreamWaitEvent(sc, in_ev[arrived], 0));
             if (p->prec == CS_PREC_SPLIT)
-                CS_CUDA(cs::launch_fp64_to_split_inplace((c[arrived + 1] - c[arrived]) * ld0,
-                                                         (char *)d[0] + c[arrived] * slab_bytes, sc));
+                CS_CUDA(cs::launch_fp64_to_split_inplace(c[arrived + 1] - c[arrived], (double *)d[0] + c[arrived], sc));
         }
-        return CS_OK;
-    };
-    void *f = d[sweeps & 1];  // final grid
-    auto slabs_done = [&](long long from, long long to) -> cs_status {  // final: back to the host now
-        const long long cnt = (to - from) * ld0;
-        char *src = (char *)f + from * slab_bytes;
+        if (op.kind == cs::HostBands::Op::kSweep) {
+            CS_CUDA(launch_sweep_rows(p, algo, d[(op.level - 1) & 1], d[op.level & 1], op.from, op.to - op.from, sc));
+            continue;
+        }
+        const long long cnt = op.to - op.from;  // final: back to the host now
+        double *src = (double *)f + op.from;
         if (p->prec == CS_PREC_SPLIT) CS_CUDA(cs::launch_split_to_fp64_inplace(cnt, src, sc));
         CS_CUDA(cudaEventRecord(out_ev, sc));  // (a wait that was enqueued keeps the event's record of that time)
         CS_CUDA(cudaStreamWaitEvent(sd, out_ev, 0));
-        CS_CUDA(cudaMemcpyAsync(host_out + from * ld0, src, (size_t)cnt * sizeof(double), cudaMemcpyDeviceToHost, sd));
-        return CS_OK;
-    };
-    const long long groups = (slabs + align * sweeps + height - 1) / height;
-    long long sent = 0;  // buffer slabs on their way back
-    for (long long g = 0; g < groups; ++g) {
-        const cs_status st = arrive((int)std::min<long long>(g, bands - 1));
-        if (st != CS_OK) return st;
-        long long hi = 0;
-        for (long long sw = 1; sw <= sweeps; ++sw) {
-            const long long lo = std::max(0LL, g * height - align * sw);
-            hi = std::min(slabs, (g + 1) * height - align * sw);
-            if (hi > lo) CS_CUDA(launch_sweep_rows(p, algo, d[(sw - 1) & 1], d[sw & 1], lo, hi - lo, sc));
-        }
-        const long long end = hi == slabs ? total : first + hi;
-        if (hi > 0 && end > sent) {
-            const cs_status done = slabs_done(sent, end);
-            if (done != CS_OK) return done;
-            sent = end;
-        }
+        CS_CUDA(cudaMemcpyAsync(host_out + op.from, src, (size_t)cnt * sizeof(double), cudaMemcpyDeviceToHost, sd));
     }
     CS_CUDA(cudaEventRecord(e1, sc));
-    CS_CUDA(cudaStreamSynchronize(sd));
-    CS_CUDA(cudaStreamSynchronize(sc));
+    for (cudaStream_t x : {sh, sd, sc}) CS_CUDA(cudaStreamSynchronize(x));
     float ms = 0.f;
     CS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     if (loop_seconds) *loop_seconds = ms * 1e-3;
