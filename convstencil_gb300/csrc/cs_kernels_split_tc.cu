@@ -510,12 +510,12 @@ __device__ __noinline__ void frame_steps(const StepArgs<F> &s, typename F::Out *
 // points -r .. 2 T r - r - 1 counted from that end, two per lane, in `buf`
 // (level l's in buf[l % 2]); every level's last r points fall out of use.
 template <class F>
-__device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out *__restrict__ out, int n, bool left,
+__device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out *__restrict__ out, long long n, bool left,
                                           typename F::Out (*buf)[kFrame1d])
 {
     using V = typename F::Out;
     const int lane = threadIdx.x & 31, r = s.radius, points = 2 * s.steps * r;
-    auto at = [&](int i) { return (long long)(left ? i - r : n - 1 - (i - r)); };  // point i - r from this end
+    auto at = [&](int i) { return left ? i - r : n - 1 - (i - r); };  // point i - r from this end
     for (int i = lane; i < points; i += 32) {
         buf[0][i] = s.in[at(i)];
         if (i < r) buf[1][i] = out[at(i)];  // the halo that odd levels read
@@ -674,13 +674,14 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             // others are copied in 8-byte pieces, with zeros past the halo.
             pdl_wait();
             bool ok = !wc.skip_loads;
+            const long long end = (long long)n + sa.radius;  // (2^31 and more for the longest arrays)
             for (int it = 0; it < my_tiles && ok; ++it) {
                 ok = lane != 0 || wait(stage_empty, (it & 1) ^ 1);
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) break;
                 const long long x = (long long)(blockIdx.x + it * gridDim.x) * kOut1d - kReach1d;
                 const unsigned dst = smem_addr(S.stage);
-                if (sa.aligned && x >= -sa.radius && x + kWin1d <= n + sa.radius) {
+                if (sa.aligned && x >= -sa.radius && x + kWin1d <= end) {
                     if (lane == 0) {
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         mbar_expect_tx(stage_full, kBytes1d);
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                     }
                 } else {
                     for (int i = lane; i < kWin1d; i += 32) {
-                        const bool take = x + i >= -sa.radius && x + i < n + sa.radius;
+                        const bool take = x + i >= -sa.radius && x + i < end;
                         cp_async8(dst + 8u * i, take ? sa.in + x + i : sa.in, take);
                     }
                     asm volatile("cp.async.wait_all;" ::: "memory");
