@@ -12,6 +12,7 @@
 #include "cs_host_bands.h"
 #include "cs_internal.h"
 #include "cs_plan_internal.h"
+#include "cs_selfconv.h"
 
 #include <algorithm>
 #include <atomic>
@@ -176,48 +177,6 @@ int classify(const Weights &w, int dims, int r)
     if (star) return cs::PAT_STAR;
     if (diamond) return r == 1 ? cs::PAT_STAR : cs::PAT_DIAMOND;
     return cs::PAT_DENSE;
-}
-
-// Kernel of `steps` steps of a (2r+1)^dims kernel (dims 1 or 2) at the centre
-// of a (2R+1)^dims array: the self-convolution, every sum carried in two
-// doubles (products by fma, sums by TwoSum) and rounded once at the end, what
-// rounding leaves of one weight carried to the next so that their sum keeps
-// its value (see f64_slice_weights). False when the weights' size could
-// take a power of them out of range (such plans keep single steps).
-bool selfconv(const double *w, int dims, int r, int steps, int R, double *out)
-{
-    const int k = 2 * r + 1, K = 2 * R + 1, n = ipow(k, dims), N = ipow(K, dims);
-    double sum = 0.0;
-    for (int i = 0; i < n; ++i) sum += std::fabs(w[i]);
-    if (steps * r > R || (steps > 1 && !(sum > 0x1p-64 && sum < 0x1p64))) return false;
-    std::vector<double> h(N, 0.0), l(N, 0.0), h2(N), l2(N);
-    const int c = dims == 2 ? R * K + R : R;
-    h[c] = 1.0;
-    for (int s = 0; s < steps; ++s) {
-        std::fill(h2.begin(), h2.end(), 0.0);
-        std::fill(l2.begin(), l2.end(), 0.0);
-        for (int i = 0; i < N; ++i) {
-            if (h[i] == 0.0 && l[i] == 0.0) continue;
-            for (int t = 0; t < n; ++t) {
-                if (w[t] == 0.0) continue;
-                const int j = i + (dims == 2 ? (t / k - r) * K + t % k - r : t - r);
-                const double p = h[i] * w[t], pe = std::fma(h[i], w[t], -p) + l[i] * w[t];
-                const double a = h2[j] + p, b = a - h2[j];
-                l2[j] += (h2[j] - (a - b)) + (p - b) + pe;
-                h2[j] = a;
-            }
-        }
-        h.swap(h2);
-        l.swap(l2);
-    }
-    double carry = 0.0;
-    for (int i = 0; i < N; ++i) {
-        out[i] = 0.0;
-        if (h[i] == 0.0 && l[i] == 0.0) continue;
-        out[i] = h[i] + (l[i] + carry);
-        carry += (h[i] - out[i]) + l[i];
-    }
-    return true;
 }
 
 long long round_up(long long v, long long a) { return (v + a - 1) / a * a; }
@@ -1018,12 +977,12 @@ CS_API cs_status cs_plan_create(cs_plan **out, cs_shape shape, cs_semantics sem,
         bool ok = true;
         for (int t = 1; t <= 3; ++t) {
             memset(p->w_steps[t - 1].v, 0, sizeof p->w_steps[t - 1].v);
-            ok = ok && selfconv(p->w.v, 2, 1, t, 3, p->w_steps[t - 1].v);
+            ok = ok && cs::selfconv(p->w.v, 2, 1, t, 3, p->w_steps[t - 1].v);
         }
         if (ok) p->max_steps = 3;
     } else if (p->dims == 1) {
         for (int t = 1; t * p->radius <= cs::kTcReach1d; ++t) {
-            if (!selfconv(p->w.v, 1, p->radius, t, cs::kTcReach1d, p->w1_steps[t - 1])) break;
+            if (!cs::selfconv(p->w.v, 1, p->radius, t, cs::kTcReach1d, p->w1_steps[t - 1])) break;
             // an odd number: a launch then leaves the state in the buffer where
             // single steps would, so each step still reads that one's halo
             if (t % 2) p->max_steps = t;
