@@ -240,6 +240,7 @@ struct cs_plan {
     int max_steps = 0;  // steps per launch those allow (0: not even one)
     cs_layout layout;
     GridView view;
+    bool rows_whole = false;  // halo_in_rows
     int algo = CS_ALGO_AUTO;
     int last_algo = CS_ALGO_AUTO;  // kernel family the last cs_run used
     int time_block = 0;            // split FMA: steps per launch (0 = tuner)
@@ -268,6 +269,23 @@ struct cs_plan {
 };
 
 namespace {
+
+// Whether the layout's rows (and planes) hold the halo: none of its columns in
+// a neighbouring row, none of its rows in a neighbouring plane, none in a row
+// or plane that the buffer's end cuts short. TMA maps are made of whole rows
+// and planes and read zeros elsewhere, so plans for which it does not hold run
+// on the kernels that address their points one by one.
+bool halo_in_rows(const cs_layout &L, int r)
+{
+    if (L.dims == 1) return true;
+    const long long ld = L.pitch[L.dims - 2], n = L.extent[L.dims - 1], x = L.origin % ld;
+    if (x < r || x + n + r > ld) return false;
+    if (L.dims == 3) {
+        const long long y = L.origin % L.pitch[0] / ld;
+        if (y < r || y + L.extent[1] + r > L.pitch[0] / ld) return false;
+    }
+    return L.origin / L.pitch[0] + L.extent[0] + r <= L.elements / L.pitch[0];
+}
 
 bool fp64_mma_ok(const cs_plan *p)
 {
@@ -319,10 +337,8 @@ bool fp64_tc_window_ok(const GridView &v, long long off, const void *in_base, co
 bool fp64_tc_pin_ok(const cs_plan *p) { return p->prec == CS_PREC_FP64 && fp64_tc_geometry_ok(p); }
 bool fp64_tc_ok(const cs_plan *p)
 {
-    const cs_layout &L = p->layout;
-    return fp64_tc_pin_ok(p) ||
-           (p->prec == CS_PREC_FP64 && p->dims == 2 && p->radius <= 3 && p->view.ext[0] >= 8 &&
-            p->view.ext[1] >= 8 && L.origin / L.pitch[0] + L.extent[0] + p->radius <= L.elements / L.pitch[0]);
+    return p->prec == CS_PREC_FP64 && p->dims == 2 && p->radius <= 3 && p->view.ext[0] >= 8 && p->view.ext[1] >= 8 &&
+           p->rows_whole;
 }
 
 // FP64 plans of 3D radius-1 stencils run on the 3D tcgen05 digit pipeline
@@ -374,7 +390,7 @@ int steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base
     const bool fp64 = p->prec == CS_PREC_FP64;
     if (p->dims == 1) return fp64_tc1d_geometry_ok(p) && (fp64 || p->view.ext[0] > 63 * 4096) ? p->max_steps : 1;
     const bool ok = fp64 ? fp64_tc_ok(p) && tc_bases_ok(in_base, out_base)
-                         : fp64_tc_geometry_ok(p) &&
+                         : fp64_tc_geometry_ok(p) && p->rows_whole &&
                                fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base);
     if (p->max_steps < 2 || !ok) return 1;
     const long long tiles = ((p->view.ext[0] + 63) / 64) * ((p->view.ext[1] + 63) / 64);
@@ -409,12 +425,13 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
         if (algo == CS_ALGO_FP64_MMA) return cs::launch_fp64_mma_2d(v, p->w, in, out, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc1d_ok(p) && row0 == 0 && rows == p->view.ext[0])
             return launch_steps(p, true, 1, in_base, out_base, st);
-        if (algo == CS_ALGO_FP64_TC && fp64_tc3d_ok(p) && cs::split_tc3d_layout_ok(v, off, in_base, out_base))
+        if (algo == CS_ALGO_FP64_TC && fp64_tc3d_ok(p) && p->rows_whole &&
+            cs::split_tc3d_layout_ok(v, off, in_base, out_base))
             return cs::launch_fp64_sweep_tc3d(v, p->w, off, p->layout.elements, (const double *)in_base,
                                               (double *)out_base, p->wait, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc3d_r3_ok(p))
             return cs::launch_fp64_sweep_tc3d_r3(v, p->w, off, p->layout.elements, (const double *)in_base,
-                                                 (double *)out_base, p->wait, st);
+                                                 (double *)out_base, p->rows_whole, p->wait, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc_ok(p) && tc_bases_ok(in_base, out_base))
             return cs::launch_fp64_sweep_tc(v, p->w7, off, p->layout.elements, (const double *)in_base,
                                             (double *)out_base, p->wait, st,
@@ -427,13 +444,13 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
     // (8-byte accesses only) runs.
     const bool out16 = (reinterpret_cast<uintptr_t>(out_base) % 16) == 0;
     if (p->dims == 3) {
-        if (algo == CS_ALGO_SPLIT_TC && split_tc3d_ok(p) &&
+        if (algo == CS_ALGO_SPLIT_TC && split_tc3d_ok(p) && p->rows_whole &&
             cs::split_tc3d_layout_ok(v, off, in_base, out_base))
             return cs::launch_split_sweep_tc3d(v, p->w, off, p->layout.elements,
                                                (const float2 *)in_base, (float2 *)out_base, p->wait, st);
         algo = CS_ALGO_SPLIT_FMA;
     }
-    const bool tma_ok = out16 && cs::split_tma_layout_ok(v, off, in_base);
+    const bool tma_ok = out16 && p->rows_whole && cs::split_tma_layout_ok(v, off, in_base);
     if (algo == CS_ALGO_SPLIT_TC && tma_ok)
         return cs::launch_split_sweep_tc(v, p->w, off, p->layout.elements,
                                          (const float2 *)in_base, (float2 *)out_base, p->wait, st);
@@ -747,9 +764,9 @@ namespace cs {
 cudaError_t fp64_anchor_sweep_fp64_in(const cs_plan *p, const void *src, void *dst, cudaStream_t st)
 {
     const long long n = p->layout.elements, off = p->layout.origin;
-    if (fp64_tc_geometry_ok(p) && fp64_tc_window_ok(p->view, off, src, dst))
+    if (fp64_tc_geometry_ok(p) && p->rows_whole && fp64_tc_window_ok(p->view, off, src, dst))
         return launch_fp64_sweep_tc(p->view, p->w7, off, n, (const double *)src, (double *)dst, p->wait, st);
-    if (fp64_tc3d_geometry_ok(p) && split_tc3d_layout_ok(p->view, off, src, dst))
+    if (fp64_tc3d_geometry_ok(p) && p->rows_whole && split_tc3d_layout_ok(p->view, off, src, dst))
         return launch_fp64_sweep_tc3d(p->view, p->w, off, n, (const double *)src, (double *)dst, p->wait, st);
     if (fp64_tc1d_geometry_ok(p)) return launch_steps(p, true, 1, src, dst, st);
     return launch_fp64_fma(p->view, p->radius, p->pattern, p->w, (const double *)src + off, (double *)dst + off, st);
@@ -1014,6 +1031,7 @@ CS_API cs_status cs_plan_create(cs_plan **out, cs_shape shape, cs_semantics sem,
     } else {
         native_layout(si.dims, p->radius, extent, p->layout);
     }
+    p->rows_whole = halo_in_rows(p->layout, p->radius);
     p->view.dims = si.dims;
     for (int d = 0; d < 3; ++d) {
         p->view.ext[d] = d < si.dims ? p->layout.extent[d] : 1;
@@ -1674,6 +1692,7 @@ bool plan_facts(const cs_plan *p, PlanFacts *f)
     f->view = p->view;
     f->origin = p->layout.origin;
     f->elements = p->layout.elements;
+    f->rows_whole = p->rows_whole;
     f->reanchor = p->reanchor;
     f->algo = p->algo;
     f->w = &p->w;

@@ -435,7 +435,7 @@ cs_status batch_create_ex(cs_batch **out, cs_plan *const *plans, void *const *a,
     // 16-byte aligned buffers run on the tcgen05 kernels (split or FP64).
     bt->tc = allow_tc && !sweeps && bt->dims == 2 && bt->radius == 3;
     for (int i = 0; bt->tc && i < count; ++i)
-        bt->tc = f[i].view.ext[0] >= 8 && f[i].view.ext[1] >= 8 &&
+        bt->tc = f[i].view.ext[0] >= 8 && f[i].view.ext[1] >= 8 && f[i].rows_whole &&
                  cs::split_tma_layout_ok(f[i].view, f[i].origin, a[i]) &&
                  cs::split_tma_layout_ok(f[i].view, f[i].origin, b[i]) &&
                  reinterpret_cast<uintptr_t>(a[i]) % 16 == 0 && reinterpret_cast<uintptr_t>(b[i]) % 16 == 0;

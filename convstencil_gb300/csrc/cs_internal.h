@@ -136,9 +136,10 @@ cudaError_t launch_fp64_sweep_tc3d(const GridView &g, const Weights &w, long lon
                                    const double *in_base, double *out_base, const TcWait &wait,
                                    cudaStream_t stream);
 // FP64 sweep of a 3D radius-3 kernel (343 weights, any pattern) on tcgen05
-// (cs_kernels_tc3d_r3.cu), any layout.
+// (cs_kernels_tc3d_r3.cu), any layout. rows_whole: whole rows and planes of the
+// buffer hold the halo, as the windows' tensor map wants.
 cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long long origin, long long elements,
-                                      const double *in_base, double *out_base, const TcWait &wait,
+                                      const double *in_base, double *out_base, bool rows_whole, const TcWait &wait,
                                       cudaStream_t stream);
 int device_sm_count();
 // Bounded device-side waits that expired since the last reset (TMA/mma.sync

@@ -44,9 +44,9 @@
 //     eight, 466 with elect_one, 398 with sixteen: 42 G outputs/s; the FP64
 //     FMA kernel 1.5 (box), 8.3 (octahedron).
 //   * Windows arrive by TMA where the layout allows it (even pitches,
-//     16-byte aligned base); the window then starts 4 columns left of the
+//     16-byte aligned base, the halo in whole rows and planes); the window then starts 4 columns left of the
 //     tile, or 3 where the interior's first column is odd, so that its
-//     address is a multiple of 16 bytes. Other layouts (odd pitches) are
+//     address is a multiple of 16 bytes. Other layouts (odd pitches among them) are
 //     loaded by the same warp with 8-byte cp.async (its 50 copies a lane and
 //     plane hide behind the MMAs: 200 x 184 x 193 runs at the rate of its tiles).
 //
@@ -535,10 +535,11 @@ Weights7 slice_weights7(const Weights &w)
 }  // namespace
 
 cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long long origin, long long elements,
-                                      const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st)
+                                      const double *in_base, double *out_base, bool rows_whole, const TcWait &wt,
+                                      cudaStream_t st)
 {
     const long long ldy = g.pitch[1], ldz = g.pitch[0];
-    const bool tma = ldy % 2 == 0 && ldz % ldy == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0;
+    const bool tma = rows_whole && ldy % 2 == 0 && ldz % ldy == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0;
     const int map_x = (int)(origin % ldy);
     const int left = tma && map_x % 2 != 0 ? 3 : 4;  // the window's address stays a multiple of 16 bytes
     const bool vec2 = ldy % 2 == 0 && ldz % 2 == 0 && origin % 2 == 0 && reinterpret_cast<uintptr_t>(out_base) % 16 == 0;

@@ -14,6 +14,7 @@ struct PlanFacts {
     cs_precision prec;
     GridView view;
     long long origin, elements;
+    bool rows_whole;     // whole rows and planes of the layout hold the halo (TMA maps want that)
     long long reanchor;  // split: FP64 re-anchor interval in sweeps (0 = never)
     int algo;            // the pinned cs_algo (CS_ALGO_AUTO: the tuner's)
     const Weights *w;
