@@ -487,6 +487,16 @@ int size_class(const cs_plan *p)
 // several, since a single one is mostly its start.
 int tune_launches(const cs_plan *p) { return size_class(p) <= 20 ? 6 : 1; }
 
+// A caller that is capturing its stream cannot have a timing run: what is not
+// measured yet then takes a default, and stays unmeasured.
+cs_status is_capturing(cudaStream_t st, bool *yes)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CS_CUDA(cudaStreamIsCapturing(st, &cap));
+    *yes = cap != cudaStreamCaptureStatusNone;
+    return CS_OK;
+}
+
 // Picks the algorithm for a plan. With CS_ALGO_AUTO and more than one
 // candidate, the first sweep of the first run is timed once per candidate
 // (every candidate computes the same sweep a -> b, so the extra work changes
@@ -540,11 +550,10 @@ cs_status choose_algo(cs_plan *p, const void *a, void *b, cudaStream_t st, int *
         *out = -1;
         return CS_OK;
     }
-    // A caller that is capturing its stream cannot have one either: the first
-    // candidate, as on plans that have no other.
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CS_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) {
+    bool capturing = false;
+    const cs_status known = is_capturing(st, &capturing);
+    if (known != CS_OK) return known;
+    if (capturing) {  // as on plans that have no other candidate
         *out = cand[0];
         return CS_OK;
     }
@@ -602,6 +611,9 @@ cs_status choose_time_block(cs_plan *p, int algo, const void *a, void *b, cudaSt
             return CS_OK;
         }
     }
+    bool capturing = false;
+    const cs_status known = is_capturing(st, &capturing);
+    if (known != CS_OK || capturing) return known;
     const long long off = p->layout.origin;
     const float2 *in = (const float2 *)a + off;
     float2 *o = (float2 *)b + off;
@@ -661,9 +673,9 @@ cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long
         if (it != g_tune_steps.end()) ms = it->second;
     }
     if (ms.second == 0.f) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        CS_CUDA(cudaStreamIsCapturing(st, &cap));
-        if (cap != cudaStreamCaptureStatusNone) return CS_OK;
+        bool capturing = false;
+        const cs_status known = is_capturing(st, &capturing);
+        if (known != CS_OK || capturing) return known;
         const int reps = 4;
         cudaEvent_t e[3];
         for (auto &x : e) CS_CUDA(cudaEventCreate(&x));
@@ -714,6 +726,9 @@ cs_status choose_tile_rows(cs_plan *p, int algo, const void *a, void *b, cudaStr
             return CS_OK;
         }
     }
+    bool capturing = false;
+    const cs_status known = is_capturing(st, &capturing);
+    if (known != CS_OK || capturing) return known;
     const long long off = p->layout.origin;
     cudaEvent_t e0, e1;
     CS_CUDA(cudaEventCreate(&e0));
