@@ -799,8 +799,9 @@ cudaError_t fp64_anchor_sweep(const cs_plan *p, void *src, void *dst, cudaStream
 // cs_run with the sweeps numbered from first_sweep: split plans run sweep k
 // in FP64 when (k + 1) is a multiple of the re-anchor interval, so a run cut
 // into chunks (the server) re-anchors where one whole run would.
+// single: one step per launch of the tcgen05 kernels.
 cs_status run_from(cs_plan *p, void *a, void *b, long long first_sweep, long long steps, cudaStream_t st,
-                   int *result_in_b)
+                   int *result_in_b, bool single)
 {
     if (!p || !a || !b) return fail(CS_ERR_INVALID_ARGUMENT, "NULL plan or buffer");
     if (a == b) return fail(CS_ERR_INVALID_ARGUMENT, "ping-pong buffers must differ");
@@ -815,7 +816,7 @@ cs_status run_from(cs_plan *p, void *a, void *b, long long first_sweep, long lon
         if (s != CS_OK) return s;
         s = choose_time_block(p, algo, a, b, st, &tb);
         if (s != CS_OK) return s;
-        s = choose_steps(p, a, b, st, sweeps, algo, tb, &multi);
+        if (!single) s = choose_steps(p, a, b, st, sweeps, algo, tb, &multi);
         if (s != CS_OK) return s;
         if (multi > 0) {
             algo = p->prec == CS_PREC_FP64 ? CS_ALGO_FP64_TC : CS_ALGO_SPLIT_TC;
@@ -1207,16 +1208,16 @@ struct DevBuf {
 // Host-buffer run with the copies overlapped: the grid goes to the device in
 // bands of slabs (of the slowest axis) on one stream while the sweeps of what
 // has arrived run on another, and slabs go back as soon as their last sweep is
-// done. Used when the kernel is known without a timing run, no temporal
-// blocking and no re-anchor sweep is involved, and the whole grid goes both
-// ways.
-bool banded_ok(cs_plan *p, long long sweeps, int *algo, int *bands)
+// done. Used when no temporal blocking and no re-anchor sweep is involved, the
+// whole grid goes both ways and the kernel is known without a timing run.
+// The number of bands that pays, whether or not the kernel is known yet: 0 or
+// at least 2.
+int bands_that_pay(const cs_plan *p, long long sweeps)
 {
-    if (p->dims < 2 || sweeps < 1) return false;
+    if (p->dims < 2 || sweeps < 1) return 0;
     if (p->prec == CS_PREC_SPLIT && cs::split_tb_supported(p->dims, p->radius, p->pattern) && p->time_block != 1)
-        return false;
-    if (p->prec == CS_PREC_SPLIT && p->reanchor > 0 && sweeps >= p->reanchor) return false;
-    if (choose_algo(p, nullptr, nullptr, nullptr, algo, false) != CS_OK || *algo < 0) return false;
+        return 0;
+    if (p->prec == CS_PREC_SPLIT && p->reanchor > 0 && sweeps >= p->reanchor) return 0;
     // The copies take 2 bytes / kLinkRate, of which b bands leave one b-th to
     // wait for; a cut costs every sweep a launch and, in 3D, the window planes
     // of its neighbours. The sum is least at the b below. (GB300, ms in 1, 2, 3,
@@ -1229,11 +1230,11 @@ bool banded_ok(cs_plan *p, long long sweeps, int *algo, int *bands)
     const double cut_us = p->dims == 3 && p->radius > 1 ? 20.0 : 6.0;
     const double best = std::sqrt(2.0 * (double)p->layout.bytes / kLinkRate / (cut_us * (double)sweeps));
     const long long least = p->dims == 2 ? 128 : 16;  // slabs per band
-    *bands = (int)std::min({best, 6.0, (double)(p->view.ext[0] / least)});
+    const int bands = (int)std::min({best, 6.0, (double)(p->view.ext[0] / least)});
     // Bands take one step per launch: not where a launch of several saves more
     // (star2d1r 4096^2 x 20: 2.15 ms whole, 2.79 in bands).
-    if (steps_per_launch(p, nullptr, nullptr) > 1 && sweeps > 12) return false;
-    return *bands >= 2;
+    if (steps_per_launch(p, nullptr, nullptr) > 1 && sweeps > 12) return 0;
+    return bands >= 2 ? bands : 0;
 }
 
 // The launches and copies of host_bands (which says why they may run in that
@@ -1338,8 +1339,13 @@ cs_status host_run(cs_plan *p, const double *host_in, size_t in_elems, double *h
         d[1] = own[1].p;
     }
     const bool whole = in_elems * elem_bytes == bytes;
-    int balgo = 0, bands = 0;
-    if (whole && out_offset == 0 && out_elems == (size_t)n && banded_ok(p, sweeps, &balgo, &bands)) {
+    int balgo = -1;
+    const int bands = whole && out_offset == 0 && out_elems == (size_t)n ? bands_that_pay(p, sweeps) : 0;
+    if (bands > 0) {
+        s = choose_algo(p, nullptr, nullptr, nullptr, &balgo, false);
+        if (s != CS_OK) return s;
+    }
+    if (balgo >= 0) {
         unsigned w0 = 0, w1 = 0;
         s = cs_device_wait_timeouts(&w0, 0);
         if (s != CS_OK) return s;
@@ -1372,7 +1378,9 @@ cs_status host_run(cs_plan *p, const double *host_in, size_t in_elems, double *h
     CS_CUDA(cudaEventCreate(&e1));
     CS_CUDA(cudaEventRecord(e0, nullptr));
     int in_b = 0;
-    s = cs_run(p, d[0], d[1], steps, nullptr, &in_b);
+    // A run that the next call of its kind makes in bands, once the kernel is
+    // known, takes one step per launch too: the same bits from call to call.
+    s = cs::run_from(p, d[0], d[1], 0, steps, nullptr, &in_b, bands > 0);
     if (s != CS_OK) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);

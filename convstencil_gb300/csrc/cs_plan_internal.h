@@ -27,9 +27,10 @@ cs_status set_error(cs_status s, const char *msg);
 int plan_fix_fp64(cs_plan *p, bool tc);
 
 // cs_run with the sweeps numbered from first_sweep (so chunked runs take
-// their FP64 re-anchor sweeps at the same global sweep counts).
+// their FP64 re-anchor sweeps at the same global sweep counts); single: one
+// step per launch of the tcgen05 kernels.
 cs_status run_from(cs_plan *p, void *a, void *b, long long first_sweep, long long steps, cudaStream_t st,
-                   int *result_in_b);
+                   int *result_in_b, bool single = false);
 // One FP64 re-anchor sweep of a split plan: (hi, lo) state in src -> dst.
 cudaError_t fp64_anchor_sweep(const cs_plan *p, void *src, void *dst, cudaStream_t st);
 
