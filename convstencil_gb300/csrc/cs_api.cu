@@ -435,7 +435,8 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
         if (algo == CS_ALGO_FP64_TC && fp64_tc_ok(p) && tc_bases_ok(in_base, out_base))
             return cs::launch_fp64_sweep_tc(v, p->w7, off, p->layout.elements, (const double *)in_base,
                                             (double *)out_base, p->wait, st,
-                                            fp64_tc_window_ok(v, off, in_base, out_base) ? 0 : p->radius);
+                                            fp64_tc_window_ok(v, off, in_base, out_base) ? 0 : p->radius, row0,
+                                            p->view.ext[0] - row0 - rows);
         return cs::launch_fp64_fma(v, p->radius, p->pattern, p->w, in, out, st, p->active_rows);
     }
     // The tensor-core split kernels store float4 (two points) at even element

@@ -81,10 +81,11 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 // operand cut from the FP64 bits by integer operations, exact FP32 level sums
 // on tcgen05, integer recombination to FP64. Layout conditions as above.
 // radius not 0: any pitch and first column (whole rows of the halo in the
-// buffer), points past a halo of `radius` read as zero.
+// buffer), points past a halo of `radius` read as zero; the grid goes on for
+// `above` and `below` rows before and after the ones swept.
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
                                  const double *in_base, double *out_base, const TcWait &wait,
-                                 cudaStream_t stream, int radius = 0);
+                                 cudaStream_t stream, int radius = 0, long long above = 0, long long below = 0);
 // `steps` (1..3) steps of a 2D radius-1 grid (FP64 or split) in one launch: wT
 // is the 7x7 kernel of that many steps, w3x3 the weights of one. tma false
 // (FP64): as a radius above.

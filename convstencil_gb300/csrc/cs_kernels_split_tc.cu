@@ -396,6 +396,7 @@ struct StepArgs {
     int frame_cta;              // CTAs from this one on compute the frame
     typename F::Out w[9];       // weights of one step
     OddRows rows;               // odd layouts
+    int above, below;           // odd layouts: rows of the grid before and after the ones swept
 };
 
 // The frame's arithmetic, that of single sweeps: FP64 FMA, or double-float.
@@ -788,13 +789,16 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 // boundary first zero them in the stage (a thread the points
                 // that it reads next).
                 const int r = STEPS ? 1 : sa.radius;
+                // (A band's neighbouring rows are in, so that its tiles see the
+                // windows, and take the scales, of a whole sweep.)
+                const int top = STEPS ? -r : -r - sa.above, bottom = STEPS ? m + r : m + r + sa.below;
                 int g, x0, y0;
                 tile_at(it, g, x0, y0);
-                if (x0 - 4 < -r || y0 - 3 < -r || x0 + ST_X - 4 >= n + r || y0 + ST_Y - 3 >= m + r) {
+                if (x0 - 4 < -r || y0 - 3 < top || x0 + ST_X - 4 >= n + r || y0 + ST_Y - 3 >= bottom) {
 #pragma unroll 1
                     for (int idx = st; idx < kPairs; idx += kSliceThreads) {
                         const int yy = y0 - 3 + idx / PAIRS, xx = x0 - 4 + 2 * (idx % PAIRS);
-                        const bool row = yy >= -r && yy < m + r;
+                        const bool row = yy >= top && yy < bottom;
                         uint2 *at = stage_pair(idx);
                         if (!row || xx < -r || xx >= n + r) at[0] = make_uint2(0u, 0u);
                         if (!row || xx + 1 < -r || xx + 1 >= n + r) at[1] = make_uint2(0u, 0u);
@@ -1191,13 +1195,16 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 }
 
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
-                                 const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st, int radius)
+                                 const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st, int radius,
+                                 long long above, long long below)
 {
     const WaitCfg wc{wt.limit_ns, wt.skip_loads};
     if (radius == 0) return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base, wc, st);
     StepArgs<FmtF64> sa{};
     sa.in = in_base + origin;
     sa.radius = radius;
+    sa.above = (int)std::min(above, 3LL);
+    sa.below = (int)std::min(below, 3LL);
     return launch_tc<FmtF64, kModeGrid, true>(g, f64_slice_weights(w, 49, true), origin, elements, in_base, out_base, wc, st, sa);
 }
 
