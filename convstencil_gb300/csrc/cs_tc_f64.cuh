@@ -66,23 +66,35 @@ constexpr unsigned long long kF64Bias = 256ull * ((1ull << 54) - 1) / 511;
 // biased exponent is eb1 (at least 1): X = round(x / 2^(eb1 - 1074)), so
 // |X| <= 2^52, returned as 2 (X + kF64Bias), whose lowest bit says nothing. The
 // shift is clamped at 63: any mantissa (< 2^53) shifted by 55 or more rounds to
-// 0 as it should. Values of
-// the largest exponent lose one bit, so half of them are ties. EVEN rounds
-// those to even; half up adds a quarter unit to every such value on average,
-// the same way each sweep (30 steps of a 9-point average of uniform data,
-// 520 x 512, against quad precision: 3.7e-15 half up and one step per launch,
-// 5.9e-16 to even and three), and costs three instructions less per point.
+// 0 as it should.
+// EVEN rounds ties to even. They are frequent: half of the values of the largest
+// exponent (which lose one bit), a quarter of those of the next, 2^-(sh + 1) of
+// those sh below. Half up adds a quarter unit to every value of the largest
+// exponent on average, an eighth to the next, the same way each sweep (30
+// steps of a 9-point average of uniform data, 520 x 512, against quad
+// precision: 3.7e-15 half up and one step per launch), and costs less.
+// f64_ties_down: takes one unit off a mantissa (lo its lower word) whose last
+// bit kept, number sh + 1, is clear: ties then round down, which is to even, and
+// nothing else changes. (Of the lower word only: bits of the upper one are
+// reached from sh = 31, where a value in 2^32 is a tie. To even at sh = 0 alone,
+// 100 steps of star2d1r 1024^2 erred by 1.2e-15, so by 5.7e-16; GB300, box2d1r
+// 2047 x 1531 x 60 515 us a solve and 517, 1d2r 10,240,000 x 100 560 and 563.)
+__device__ __forceinline__ unsigned f64_ties_down(unsigned lo, int sh)
+{
+    unsigned last;
+    asm("shl.b32 %0, %1, %2;" : "=r"(last) : "r"(2u), "r"(sh));  // 0 from 31 on
+    return (lo & last) == 0u && lo != 0u ? lo - 1u : lo;
+}
 template <bool EVEN = false>
 __device__ __forceinline__ unsigned long long f64_biased_fixed(unsigned lo, unsigned hi, int eb1)
 {
     const int e = (int)((hi >> 20) & 0x7FFu);
     const int ee = max(e, 1);  // subnormals: no implicit bit, exponent 1
+    const int sh = min(eb1 - ee, 63);
+    if (EVEN) lo = f64_ties_down(lo, sh);
     const unsigned long long mant =
         ((unsigned long long)((hi & 0xFFFFFu) | (e ? 0x100000u : 0u)) << 32) | lo;
-    const int sh = min(eb1 - ee, 63);
-    const unsigned long long t = mant >> sh;
-    const unsigned up = EVEN ? ((unsigned)t >> 1 | (unsigned)min(sh, 1)) & 1u : 1u;
-    const unsigned long long x = (t + up) >> 1;
+    const unsigned long long x = ((mant >> sh) + 1) >> 1;
     const unsigned long long neg = (unsigned long long)(long long)((int)hi >> 31);  // 0 or all ones
     return ((kF64Bias - neg) + (x ^ neg)) << 1;  // kF64Bias + x, or kF64Bias - x = (kF64Bias + 1) + ~x
 }
@@ -93,8 +105,7 @@ __device__ __forceinline__ unsigned long long f64_biased_fixed(unsigned lo, unsi
 // PTX defines a shift by more than 63 (C++ does not). Half up in magnitude with
 // the sign applied first: with t = floor(m / 2^sh), the arithmetic shift of ~m
 // is -t - 1 whether or not bits were lost, and (-t - 1 + 1) >> 1 = -((t + 1) >> 1).
-// To even: a tie (sh = 0, bit 0 set) goes down if bit 1 is clear, as m without
-// bit 0 does. (Four of 15 integer operations less per point than with the sign
+// (Four of 15 integer operations less per point than with the sign
 // at the end; GB300, us a launch:
 // star3d1r 512^3 933 and 897, box2d1r 8192^2 in threes 358 and 353.)
 constexpr int kFastExp = 128;
@@ -102,7 +113,7 @@ template <bool EVEN = false>
 __device__ __forceinline__ unsigned long long f64_biased_fixed_fast(unsigned lo, unsigned hi, int eb1)
 {
     const int sh = eb1 - (int)((hi >> 20) & 0x7FFu);
-    if (EVEN && ((lo & 2u) | (unsigned)sh) == 0u) lo &= ~1u;
+    if (EVEN) lo = f64_ties_down(lo, sh);
     const unsigned neg = (unsigned)((int)hi >> 31);
     const unsigned long long m = ((unsigned long long)(((hi & 0xFFFFFu) | 0x100000u) ^ neg) << 32) | (lo ^ neg);
     unsigned long long t;
