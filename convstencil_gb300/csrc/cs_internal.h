@@ -82,10 +82,12 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 // on tcgen05, integer recombination to FP64. Layout conditions as above.
 // radius not 0: any pitch and first column (whole rows of the halo in the
 // buffer), points past a halo of `radius` read as zero; the grid goes on for
-// `above` and `below` rows before and after the ones swept.
+// `above` and `below` rows before and after the ones swept. fine: no larger an
+// error than FP64 FMA sums (always so with a radius).
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
                                  const double *in_base, double *out_base, const TcWait &wait,
-                                 cudaStream_t stream, int radius = 0, long long above = 0, long long below = 0);
+                                 cudaStream_t stream, int radius = 0, long long above = 0, long long below = 0,
+                                 bool fine = false);
 // `steps` (1..3) steps of a 2D radius-1 grid (FP64 or split) in one launch: wT
 // is the 7x7 kernel of that many steps, w3x3 the weights of one. tma false
 // (FP64): as a radius above.
@@ -133,9 +135,10 @@ cudaError_t launch_split_sweep_tc3d(const GridView &g, const Weights &w, long lo
 // the FP64 bits with integer operations, exact level sums, one rounding to
 // FP64 per output (an output whose parts had different plane exponents is
 // summed in FP64). Same layout conditions.
+// (fine: see launch_fp64_sweep_tc.)
 cudaError_t launch_fp64_sweep_tc3d(const GridView &g, const Weights &w, long long origin, long long elements,
                                    const double *in_base, double *out_base, const TcWait &wait,
-                                   cudaStream_t stream);
+                                   cudaStream_t stream, bool fine = false);
 // FP64 sweep of a 3D radius-3 kernel (343 weights, any pattern) on tcgen05
 // (cs_kernels_tc3d_r3.cu), any layout. rows_whole: whole rows and planes of the
 // buffer hold the halo, as the windows' tensor map wants.

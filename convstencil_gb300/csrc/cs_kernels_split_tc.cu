@@ -24,6 +24,11 @@
 //     dropped levels >= 6 weigh below 2^-48 of (tile max x largest weight)
 //     in the worst case (about 2^-53 for data without adversarial digits).
 //
+//   * FP64 with seven levels (FmtF64Fine): the forms that AUTO takes in the
+//     place of FP64 FMA sweeps (several steps per launch, odd layouts, 1D, small
+//     served grids), whose errors must not be larger than those sweeps'. Level
+//     6 is kept too, inputs round to even and the weights keep their sum, so a
+//     launch errs by its inputs' and its outputs' rounding.
 //   * split with six digits (FmtSplit6): the launches of several steps, below,
 //     of split plans, whose errors would otherwise grow with the steps' weights.
 //
@@ -111,9 +116,10 @@ using namespace tc;
 // kCols: columns drained at a time. Four leave the FP64 kernels' registers
 // free of spills (three-step 8192^2 launch, GB300: 370 us with eight, 359 with
 // four; with twelve or sixteen slicer warps, 80 or 72 registers, 403 and 420).
+// kLevels: levels kept, from 0; digits d of x and e of w meet in level d + e.
 struct FmtSplit {
     static constexpr bool kF64 = false;
-    static constexpr int kDigits = split::kDigits;  // 5
+    static constexpr int kDigits = split::kDigits, kLevels = split::kDigits;  // 5
     static constexpr int kEpiWarps = 4, kSliceWarps = 8, kCols = 8;
     using Out = float2;
     using Digits = split::SliceWeights;
@@ -125,7 +131,7 @@ struct FmtSplit {
 // format holds, so a launch's error is the rounding of its results to pairs.
 struct FmtSplit6 {
     static constexpr bool kF64 = false;
-    static constexpr int kDigits = 6;
+    static constexpr int kDigits = 6, kLevels = 6;
     static constexpr int kEpiWarps = 4, kSliceWarps = 8, kCols = 8;
     using Out = float2;
     using Digits = F64Weights;
@@ -133,10 +139,22 @@ struct FmtSplit6 {
 
 struct FmtF64 {
     static constexpr bool kF64 = true;
-    static constexpr int kDigits = 6;
+    static constexpr int kDigits = 6, kLevels = 6;
     static constexpr int kEpiWarps = 8, kSliceWarps = 8, kCols = 4;
     using Out = double;
     using Digits = F64Weights;
+};
+
+// Level 6 (27 digit pairs per tap) costs an MMA and 24 % more columns of B, no
+// shared memory (rows of B that are there). Without it what the dropped pairs
+// weigh, 2^-53 of the tile's largest value on average, is a launch's largest
+// error. (Error of the norm with six levels, with seven and of FP64 FMA sweeps,
+// uniform data: star2d1r 1024^2 x 100 5.7e-16, 1.06e-16, 1.12e-16; odd box2d3r x 20
+// 2.3e-16, 6.5e-17, 1.7e-16; 1d2r 1,000,000 x 100 4.1e-16, 1.2e-16, 1.5e-16. GB300, us
+// a solve: star2d1r 476 and 476, box2d1r 2047 x 1531 x 60 516 and 524, 1d2r
+// 10,240,000 x 100 563 and 563: set by the slicers, not the MMAs.)
+struct FmtF64Fine : FmtF64 {
+    static constexpr int kLevels = 7;
 };
 
 // Warp roles.
@@ -190,8 +208,8 @@ static_assert(FmtSplit::kEpiWarps == 4 && FmtF64::kEpiWarps == 8 && R == 4,
 template <class F>
 struct Smem {
     static constexpr int D = F::kDigits;
-    static constexpr int NCOL = NLV * D;       // level L at NLV * L
-    static_assert(NCOL <= kAccStride, "an accumulator must fit between the two TMEM bases");
+    static constexpr int NCOL = NLV * D;       // rows of B: digit e at NLV * e
+    static_assert(NLV * F::kLevels <= kAccStride, "an accumulator must fit between the two TMEM bases");
     uint4 stage[F::kF64 ? kStageF64 : NPAIR];  // windows: pairs of 8-byte points
     __half planes[2][D][PL];                   // digit planes, two tiles
     __half bmat[NOFF][NCOL * 16];              // B_i, K-major 8x16-byte core matrices
@@ -207,7 +225,7 @@ struct Smem {
     int redi[2][kMaxSliceWarps];                  // FP64: per-warp max biased exponent
 };
 
-static_assert(sizeof(Smem<FmtF64>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 128 <= 232448 &&
+static_assert(sizeof(Smem<FmtF64Fine>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 128 <= 232448 &&
                   sizeof(Smem<FmtSplit6>) + 128 <= 232448,
               "shared memory of one CTA must stay within 227 KB");
 
@@ -222,36 +240,57 @@ static_assert(sizeof(Smem<FmtF64>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 1
 // one: it initialises the accumulator. (6 %
 // of the columns; GB300, 8192^2: split 284.0 -> 281.8 us a sweep, FP64 three steps
 // 358.0 -> 357.1.)
+//
+// With more levels than digits, digit 1 is the first to reach the last level:
+// its first MMA stops short of it and one of its own initialises it.
 __host__ __device__ constexpr int nth_offset(int j) { return j == 0 ? 3 : j <= 3 ? j - 1 : j; }
-template <int D, int J, int DG>
+// Levels that digit DG feeds, from level DG on: the B rows of as many digits of w.
+template <class F>
+__host__ __device__ constexpr int levels_of(int dg)
+{
+    return F::kLevels - dg < F::kDigits ? F::kLevels - dg : F::kDigits;
+}
+template <class F, int J, int DG>
 __device__ __forceinline__ void tile_mma(unsigned d_base, unsigned long long a0, unsigned long long b0)
 {
+    constexpr int D = F::kDigits, L = F::kLevels, W = levels_of<F>(DG);
     constexpr int NCOL = NLV * D, I = nth_offset(J), LO = I >= 8 ? 16 : 0, HI = I <= 1 ? 16 : 0;
     constexpr unsigned long long a_off = ((unsigned long long)DG * PL * 2 + I * kRowBytes) >> 4;
     constexpr unsigned long long b_off = ((unsigned long long)I * NCOL * 16 * 2 + LO / 8 * 256) >> 4;
     static_assert(((unsigned long long)DG * PL * 2 + I * kRowBytes) % 16 == 0 && (NCOL * 16 * 2) % 16 == 0,
                   "descriptor offsets must be 16-byte multiples");
-    mma_f16(d_base + (unsigned)(NLV * DG + LO), a0 + a_off, b0 + b_off, instr_desc(NLV * (D - DG) - LO - HI),
-            (J | DG) != 0 ? 1u : 0u);
+    static_assert(L <= D + 1);
+    if constexpr (L > D && J == 0 && DG == 1) {
+        mma_f16(d_base + (unsigned)NLV, a0 + a_off, b0 + b_off, instr_desc(NLV * (W - 1)), 1u);
+        mma_f16(d_base + (unsigned)(NLV * D), a0 + a_off, b0 + b_off + (NLV * (W - 1) * 16 * 2 >> 4), instr_desc(NLV), 0u);
+    } else {
+        mma_f16(d_base + (unsigned)(NLV * DG + LO), a0 + a_off, b0 + b_off, instr_desc(NLV * W - LO - HI),
+                (J | DG) != 0 ? 1u : 0u);
+    }
     if constexpr (DG + 1 < D)
-        tile_mma<D, J, DG + 1>(d_base, a0, b0);
+        tile_mma<F, J, DG + 1>(d_base, a0, b0);
     else if constexpr (J + 1 < NOFF)
-        tile_mma<D, J + 1, 0>(d_base, a0, b0);
+        tile_mma<F, J + 1, 0>(d_base, a0, b0);
 }
 
 // The MMAs of one 1D tile: K step KK, input digit DG.
-template <int D, int KK, int DG>
+template <class F, int KK, int DG>
 __device__ __forceinline__ void tile_mma_1d(unsigned d_base, unsigned long long a0, unsigned long long b0)
 {
+    constexpr int D = F::kDigits, L = F::kLevels, W = levels_of<F>(DG);
     constexpr unsigned long long a_off =
         ((unsigned long long)DG * PL * 2 + (KK & 1) * 2 * kPhase1d + (KK >> 1) * 16) >> 4;
     constexpr unsigned long long b_off = ((unsigned long long)KK * NLV * D * 16 * 2) >> 4;
-    mma_f16(d_base + (unsigned)(NLV * DG), a0 + a_off, b0 + b_off, instr_desc(NLV * (D - DG)),
-            (KK | DG) != 0 ? 1u : 0u);
+    if constexpr (L > D && KK == 0 && DG == 1) {
+        mma_f16(d_base + (unsigned)NLV, a0 + a_off, b0 + b_off, instr_desc(NLV * (W - 1)), 1u);
+        mma_f16(d_base + (unsigned)(NLV * D), a0 + a_off, b0 + b_off + (NLV * (W - 1) * 16 * 2 >> 4), instr_desc(NLV), 0u);
+    } else {
+        mma_f16(d_base + (unsigned)(NLV * DG), a0 + a_off, b0 + b_off, instr_desc(NLV * W), (KK | DG) != 0 ? 1u : 0u);
+    }
     if constexpr (DG + 1 < D)
-        tile_mma_1d<D, KK, DG + 1>(d_base, a0, b0);
+        tile_mma_1d<F, KK, DG + 1>(d_base, a0, b0);
     else if constexpr (KK + 1 < kSteps1d)
-        tile_mma_1d<D, KK + 1, 0>(d_base, a0, b0);
+        tile_mma_1d<F, KK + 1, 0>(d_base, a0, b0);
 }
 
 // One grid of a batch (batch mode): its tensor map, output, sizes, tile
@@ -355,8 +394,8 @@ __device__ __forceinline__ int grid_of(const TcGrid<F> *grids, int ngrids, int t
 
 // What one launch computes.
 constexpr int kModeGrid = 0;    // one sweep of a 2D grid
-constexpr int kMode1d = 1;      // several steps of a 1D grid (FP64)
-constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid (FP64)
+constexpr int kMode1d = 1;      // several steps of a 1D grid
+constexpr int kModeSteps = 2;   // several steps of a 2D radius-1 grid
 
 // kModeSteps: T steps of a 3x3 stencil are one sweep of its T-fold
 // self-convolution (7x7 at T = 3) wherever the window of every intermediate
@@ -751,9 +790,9 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 const unsigned d_base = tmem + (unsigned)(kAccStride * buf);
                 const unsigned long long a0 = buf ? a_desc_buf1 : a_desc_buf0;
                 if constexpr (ONED)
-                    tile_mma_1d<D, 0, 0>(d_base, a0, b_desc0);
+                    tile_mma_1d<F, 0, 0>(d_base, a0, b_desc0);
                 else
-                    tile_mma<D, 0, 0>(d_base, a0, b_desc0);
+                    tile_mma<F, 0, 0>(d_base, a0, b_desc0);
                 mma_commit(bar2(S.planes_empty, buf));  // planes may be overwritten
                 mma_commit(bar2(S.acc_full, buf));      // accumulator ready
             }
@@ -882,7 +921,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                 return ONED ? (idx >> 2 & 3) * (kPhase1d / 4) + (idx >> 4) * 4 + (idx & 3) : idx;
             };
             if constexpr (F::kF64) {
-                constexpr bool EVEN = STEPS || ONED || ODD;
+                constexpr bool EVEN = F::kLevels > 6;
                 if (ex >= kFastExp) {
 #pragma unroll
                     for (int q = 0; q < PER; ++q) {
@@ -967,9 +1006,9 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             for (int pass = 0; pass < kPasses; ++pass) {
                 const int rho = kRowsPerWarp * h + pass * C / 8;
                 const int c0 = pass * C % 8;  // first of the C columns of this pass
-                float acc[D][C];
+                float acc[F::kLevels][C];
 #pragma unroll
-                for (int L = 0; L < D; ++L)
+                for (int L = 0; L < F::kLevels; ++L)
                     tmem_ldc(tmem + lane_bits + (unsigned)(kAccStride * buf + NLV * L + 8 * rho + c0), acc[L]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (pass == kPasses - 1) {  // accumulator drained: hand it back to the MMA warp
@@ -985,8 +1024,14 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
                     long long t[C];
 #pragma unroll
                     for (int j = 0; j < C; ++j) {
-                        const float lv[6] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4][j], acc[5][j]};
-                        t[j] = f64_combine(lv);
+                        if constexpr (F::kLevels == 7) {
+                            const float lv[7] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j],
+                                                 acc[4][j], acc[5][j], acc[6][j]};
+                            t[j] = f64_combine(lv, sw.rest);
+                        } else {
+                            const float lv[6] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4][j], acc[5][j]};
+                            t[j] = f64_combine(lv);
+                        }
                     }
                     if (f64_scale_is_plain(c)) {
 #pragma unroll
@@ -1196,16 +1241,18 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
                                  const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st, int radius,
-                                 long long above, long long below)
+                                 long long above, long long below, bool fine)
 {
     const WaitCfg wc{wt.limit_ns, wt.skip_loads};
-    if (radius == 0) return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base, wc, st);
-    StepArgs<FmtF64> sa{};
+    if (radius == 0 && !fine) return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base, wc, st);
+    const F64Weights digits = f64_slice_weights(w, 49, &tap_order(Taps::kSquare7));
+    if (radius == 0) return launch_tc<FmtF64Fine>(g, digits, origin, elements, in_base, out_base, wc, st);
+    StepArgs<FmtF64Fine> sa{};
     sa.in = in_base + origin;
     sa.radius = radius;
     sa.above = (int)std::min(above, 3LL);
     sa.below = (int)std::min(below, 3LL);
-    return launch_tc<FmtF64, kModeGrid, true>(g, f64_slice_weights(w, 49, true), origin, elements, in_base, out_base, wc, st, sa);
+    return launch_tc<FmtF64Fine, kModeGrid, true>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
 }
 
 namespace {
@@ -1239,7 +1286,7 @@ cudaError_t launch_steps_2d(const GridView &g, const Weights &wT, const Weights 
         sa.w[t] = step_weight(w3x3.v[t], Out{});
         if (w3x3.v[t] != 0.0) sa.taps |= 1u << t;
     }
-    const F64Weights digits = f64_slice_weights(wT, 49, true);
+    const F64Weights digits = f64_slice_weights(wT, 49, &tap_order(Taps::kSquare7));
     const WaitCfg wc{wt.limit_ns, wt.skip_loads};
     if constexpr (F::kF64)
         if (!tma) return launch_tc<F, kModeSteps, true>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
@@ -1266,7 +1313,7 @@ cudaError_t launch_steps_1d(long long n, const double *taps, int radius, const d
     note_launch();
     return launch_programmatic(k2d_tc<F, false, kMode1d>, std::min(tiles, device_sm_count()), kThreads<F>,
                                sizeof(Smem<F>) + 128, st, unused, reinterpret_cast<Out *>(out_base) + origin, 1,
-                               (int)n, 0LL, 1, tiles, 0, 0, f64_slice_weights(wT, 49, true),
+                               (int)n, 0LL, 1, tiles, 0, 0, f64_slice_weights(wT, 49, &tap_order(Taps::kLine49)),
                                WaitCfg{wt.limit_ns, wt.skip_loads}, static_cast<const TcGrid<F> *>(nullptr), 0, sa);
 }
 
@@ -1276,7 +1323,7 @@ cudaError_t launch_steps_tc(bool fp64, const GridView &g, const Weights &wT, con
                             long long origin, long long elements, const void *in_base, void *out_base,
                             const TcWait &wt, cudaStream_t st, bool tma)
 {
-    return fp64 ? launch_steps_2d<FmtF64>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, tma)
+    return fp64 ? launch_steps_2d<FmtF64Fine>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, tma)
                 : launch_steps_2d<FmtSplit6>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, true);
 }
 
@@ -1284,7 +1331,7 @@ cudaError_t launch_steps_tc_1d(bool fp64, long long n, const double *taps, int r
                                long long origin, const void *in_base, void *out_base, const TcWait &wt,
                                cudaStream_t st)
 {
-    return fp64 ? launch_steps_1d<FmtF64>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st)
+    return fp64 ? launch_steps_1d<FmtF64Fine>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st)
                 : launch_steps_1d<FmtSplit6>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st);
 }
 

@@ -71,7 +71,8 @@ using namespace tc;
 
 // Number formats: split (FP32 (hi, lo) grids, five digits, a ring of four
 // 128-column TMEM blocks) and FP64 (FP64 grids, six digits cut with integer
-// operations as in the 2D kernel, a ring of three 160-column blocks).
+// operations as in the 2D kernel, a ring of three 160-column blocks). LV: levels
+// kept; kBlk: TMEM columns from one input plane's block to the next.
 //
 // FP64 is bound by its epilogue and the slicers' integer operations: 155
 // instructions an output, 0.6 of the schedulers' slots (GB300, star3d1r 512^3, 861
@@ -82,17 +83,26 @@ using namespace tc;
 // 1126), two planes per loop iteration (930 against 897, spills).
 struct F3Split {
     static constexpr bool kF64 = false;
-    static constexpr int D = split::kDigits;  // 5
-    static constexpr int NBLK = 4;
+    static constexpr int D = split::kDigits, LV = D;  // 5
+    static constexpr int NBLK = 4, kBlk = 128;
     using Out = float2;
     using Digits = SliceWeights;
 };
 struct F3F64 {
     static constexpr bool kF64 = true;
-    static constexpr int D = 6;
-    static constexpr int NBLK = 3;
+    static constexpr int D = 6, LV = 6;
+    static constexpr int NBLK = 3, kBlk = 160;
     using Out = double;
     using Digits = F64Weights;
+};
+// FP64 with level 6 too, inputs rounded to even and the weights' sum kept, as
+// the 2D kernel's FmtF64Fine: errors no larger than those of FP64 FMA sweeps
+// (box3d1r, uniform data, error of the norm: 64 x 60 x 66 x 30 sweeps 3.0e-15 with
+// six levels, 7.5e-17 so, FP64 FMA 1.4e-16; 128 x 130 x 125 x 100 9.9e-15, 8.0e-17,
+// 1.4e-16. star3d1r 160 x 128 x 125 x 100 1.25e-16 against 9.2e-17 of its seven FMA, so
+// the server keeps it on those).
+struct F3F64Fine : F3F64 {
+    static constexpr int LV = 7, kBlk = 168;
 };
 
 // Warp roles. Warp w issues from the SM's scheduler w % 4, and an epilogue
@@ -129,11 +139,13 @@ constexpr int NLV = 24;                      // TMEM columns per level: 3 tap pl
 // N of an MMA that feeds `levels` levels: M = 128 wants multiples of 16, so odd
 // counts take 8 columns more, of a level that does not exist; they lie behind
 // the block's last level and are not read.
+// With seven levels there is no room behind it: the 8 columns come first, from 8
+// zero rows before B_i's (kFront).
 __host__ __device__ constexpr int mma_n(int levels) { return (NLV * levels + 15) / 16 * 16; }
 template <class F>
-constexpr int kNcol = mma_n(F::D);           // rows of B_i: 128 split, 144 FP64
+constexpr int kFront = F::LV > F::D ? 8 : 0;
 template <class F>
-constexpr int kBlk = F::kF64 ? 160 : 128;    // TMEM columns from one input plane's block to the next
+constexpr int kNcol = kFront<F> + mma_n(F::D);  // rows of B_i: 128 split, 144 FP64 (152)
 constexpr int kTmemCols = 512;
 constexpr int kStages = 2 * kGroups;         // TMA window buffers (two per slicer group)
 constexpr int NPL = 7;                       // digit-plane sets (ring); also keeps one CTA per SM
@@ -146,7 +158,8 @@ constexpr unsigned kStageBytes = ST_X * ST_Y * 8;  // 10,368 (8-byte points)
 // zero weights, so they only need to be finite).
 constexpr int PAIRS = ST_X / 2, CUT0 = 1, NCUTX = 34, NCUT = ST_Y * NCUTX;  // 36, 612
 constexpr int PER = (NCUT + kGroupThreads - 1) / kGroupThreads;            // 5
-static_assert(F3Split::NBLK * kBlk<F3Split> <= kTmemCols && F3F64::NBLK * kBlk<F3F64> <= kTmemCols,
+static_assert(F3Split::NBLK * F3Split::kBlk <= kTmemCols && F3F64::NBLK * F3F64::kBlk <= kTmemCols &&
+                  F3F64Fine::NBLK * F3F64Fine::kBlk <= kTmemCols && NLV * F3F64Fine::LV <= F3F64Fine::kBlk,
               "TMEM blocks exceed the allocation");
 static_assert(kEpiWarps == 8, "two epilogue warps per TMEM lane quarter, four columns each");
 static_assert(kStageBytes % 128 == 0, "TMA destinations stay 128-byte aligned");
@@ -165,7 +178,7 @@ struct Smem {
     float red[kGroups][2][kGroupWarps];           // split: per-warp max |hi|
     int redi[kGroups][2][kGroupWarps];            // FP64: per-warp max biased exponent
 };
-static_assert(sizeof(Smem<F3F64>) + 128 <= 232448 && sizeof(Smem<F3Split>) + 128 <= 232448,
+static_assert(sizeof(Smem<F3F64Fine>) + 128 <= 232448 && sizeof(Smem<F3Split>) + 128 <= 232448,
               "shared memory of one CTA must stay within 227 KB");
 
 // The MMAs of one input plane: window row offset I, input digit D. `a`
@@ -179,8 +192,24 @@ __device__ __forceinline__ void plane_mma(unsigned d_base, unsigned long long a,
     constexpr unsigned long long b_off = ((unsigned long long)I * NCOL * 16 * 2) >> 4;
     static_assert(((unsigned long long)D * PL * 2 + I * kRowBytes) % 16 == 0 && (NCOL * 16 * 2) % 16 == 0,
                   "descriptor offsets must be 16-byte multiples");
-    mma_f16(d_base + (unsigned)(NLV * D), a + a_off, b0 + b_off, instr_desc(mma_n(F::D - D)),
-            (I | D) != 0 ? 1u : 0u);
+    if constexpr (F::LV == F::D) {
+        mma_f16(d_base + (unsigned)(NLV * D), a + a_off, b0 + b_off, instr_desc(mma_n(F::D - D)),
+                (I | D) != 0 ? 1u : 0u);
+    } else {
+        // Levels D .. D + W - 1 (fewer: level 6 of the first row offset comes
+        // from an MMA of its own, below).
+        static_assert(F::LV == 7 && F::D == 6 && kFront<F> == 8);
+        constexpr int W = (I == 0 && D == 1) ? 5 : F::LV - D < F::D ? F::LV - D : F::D, pad = NLV * W % 16;
+        constexpr unsigned long long row = (unsigned long long)(kFront<F> - pad) * 32 >> 4;  // 8 rows: 256 bytes
+        if constexpr (I == 0 && D == 0) {
+            // Digit 1 with the weights' digit 5 initialises level 6, and with it
+            // the 8 columns before it, which digit 0 initialises next.
+            mma_f16(d_base + (unsigned)(NLV * 6 - 8), a + (PL * 2 >> 4), b0 + (unsigned long long)((8 + NLV * 5 - 8) * 32 >> 4),
+                    instr_desc(32), 0u);
+        }
+        mma_f16(d_base + (unsigned)(NLV * D - pad), a + a_off, b0 + b_off + row, instr_desc(NLV * W + pad),
+                (I | D) != 0 ? 1u : 0u);
+    }
     if constexpr (D + 1 < F::D)
         plane_mma<F, I, D + 1>(d_base, a, b0);
     else if constexpr (I + 1 < NOFF)
@@ -285,12 +314,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     // so 10.2 and 8.0.)
     for (int idx = tid; idx < NOFF * NCOL * 2; idx += kThreads) {
         const int i = idx / (NCOL * 2), rem = idx - i * (NCOL * 2), kc = rem / NCOL, nn = rem - kc * NCOL;
-        const int e = nn / NLV, dz = nn % NLV >> 3, c = nn & 7;
+        const int n0 = nn - kFront<F>, e = n0 / NLV, dz = n0 % NLV >> 3, c = nn & 7;
         unsigned long long lo = 0, hi = 0;
 #pragma unroll
         for (int tj = 0; tj < 3; ++tj) {
             const int k = c + 3 + tj - 8 * kc;
-            if (e >= D || k < 0 || k >= 8) continue;
+            if (n0 < 0 || e >= D || k < 0 || k >= 8) continue;
             const unsigned long long v = __half_as_ushort(sw.d[e][(dz * 3 + i) * 3 + tj]);
             if (k < 4)
                 lo |= v << 16 * k;
@@ -344,7 +373,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     break;
                 tc_fence_after();
                 if (elect_one()) {
-                    plane_mma<F, 0, 0>(tmem + (unsigned)(kBlk<F> * blk), a_desc0 + kSetUnits * slot, b_desc0);
+                    plane_mma<F, 0, 0>(tmem + (unsigned)(F::kBlk * blk), a_desc0 + kSetUnits * slot, b_desc0);
                     mma_commit(bar(S.blk_full, blk));       // block ready for the epilogue
                     mma_commit(bar(S.planes_empty, slot));  // digit planes may be overwritten
                 }
@@ -442,14 +471,14 @@ __global__ void __launch_bounds__(kThreads, 1)
                         for (int k = 0; k < PER; ++k) {
                             const int u = st + k * kGroupThreads;
                             if (u < NCUT)
-                                f64_cut_fast<false, PL / 2>(v[k], ex, dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX);
+                                f64_cut_fast<(F::LV > 6), PL / 2>(v[k], ex, dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX);
                         }
                     } else {
 #pragma unroll
                         for (int k = 0; k < PER; ++k) {
                             const int u = st + k * kGroupThreads;
                             if (u < NCUT)
-                                f64_cut_any<false, PL / 2>(v[k], ex, dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX);
+                                f64_cut_any<(F::LV > 6), PL / 2>(v[k], ex, dst0 + (u / NCUTX) * PAIRS + CUT0 + u % NCUTX);
                         }
                     }
                 } else {
@@ -546,16 +575,24 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int ew = sw.ew;
             // Integer sums start at -3 kRawBias, so that they are right once
             // all three parts are in; `left` parts are missing before this one.
-            auto add_raw = [](long long (&sm)[4], const float (&acc)[D][4]) {
+            constexpr unsigned long long bias = kRawBias<F::LV == 7 ? 0 : 3>;
+            auto add_raw = [&](long long (&sm)[4], const float (&acc)[F::LV][4]) {
 #pragma unroll
                 for (int c = 0; c < 4; c += 2) {
+                    if constexpr (F::LV == 7) {
+                        float u[7], v[7];
+#pragma unroll
+                        for (int L = 0; L < 7; ++L) u[L] = acc[L][c], v[L] = acc[L][c + 1];
+                        f64_add_raw2(u, v, sw.rest, sm[c], sm[c + 1]);
+                        continue;
+                    }
                     const float u[6] = {acc[0][c], acc[1][c], acc[2][c], acc[3][c], acc[4][c], acc[5][c]};
                     const float v[6] = {acc[0][c + 1], acc[1][c + 1], acc[2][c + 1],
                                         acc[3][c + 1], acc[4][c + 1], acc[5][c + 1]};
                     f64_add_raw2(u, v, sm[c], sm[c + 1]);
                 }
             };
-            auto add_part = [&](long long (&sm)[4], int &se, bool &fl, bool &nf, const float (&acc)[D][4],
+            auto add_part = [&](long long (&sm)[4], int &se, bool &fl, bool &nf, const float (&acc)[F::LV][4],
                                 int ex, int left) {
                 if (nf) return;
                 if (ex == kNonFiniteTile) {
@@ -569,22 +606,22 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!fl) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
-                        sm[c] = __double_as_longlong(f64_from_fixed((long long)((unsigned long long)sm[c] + left * kRawBias), se + ew - 1080));
+                        sm[c] = __double_as_longlong(f64_from_fixed((long long)((unsigned long long)sm[c] + left * bias), se + ew - 1080));
                     fl = true;
                 }
-                const long long none = (long long)(0 - kRawBias);
+                const long long none = (long long)(0 - bias);
                 long long t[4] = {none, none, none, none};
                 add_raw(t, acc);
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
                     sm[c] = __double_as_longlong(__longlong_as_double(sm[c]) + f64_from_fixed(t[c], ex + ew - 1080));
             };
-            auto load_issue = [&](int dz, float (&acc)[D][4]) {
-                const unsigned col = (unsigned)(kBlk<F> * blk + 8 * dz + 4 * hh);
+            auto load_issue = [&](int dz, float (&acc)[F::LV][4]) {
+                const unsigned col = (unsigned)(F::kBlk * blk + 8 * dz + 4 * hh);
 #pragma unroll
-                for (int L = 0; L < D; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
+                for (int L = 0; L < F::LV; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
             };
-            auto load_part = [&](int dz, float (&acc)[D][4]) {
+            auto load_part = [&](int dz, float (&acc)[F::LV][4]) {
                 load_issue(dz, acc);
                 tmem_wait_ld();
             };
@@ -592,7 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!(ok = wait(bar(S.blk_full, blk), full))) break;
                 tc_fence_after();
                 const int ex = S.scale_exp[q % kScaleRing];
-                float acc[D][4];
+                float acc[F::LV][4];
                 // The usual plane: every sum it goes to has its exponent, and
                 // nothing rare is under way. (All of this is the same in the
                 // whole CTA: the loads want full warps.)
@@ -615,7 +652,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         a[c] = b[c];
-                        b[c] = (long long)(0 - 3 * kRawBias);
+                        b[c] = (long long)(0 - 3 * bias);
                     }
                     add_raw(b, acc);
                     double res[4];
@@ -668,7 +705,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {  // rotate: p - 1 becomes p - 2, p starts
                     a[c] = b[c];
-                    b[c] = (long long)(0 - 3 * kRawBias);
+                    b[c] = (long long)(0 - 3 * bias);
                 }
                 ea = eb2;
                 fa = fb;
@@ -748,7 +785,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
             };
             auto load_part = [&](int dz, float (&acc)[D][4]) {
-                const unsigned col = (unsigned)(kBlk<F> * blk + 8 * dz + 4 * hh);
+                const unsigned col = (unsigned)(F::kBlk * blk + 8 * dz + 4 * hh);
 #pragma unroll
                 for (int L = 0; L < D; ++L) tmem_ld4(tmem + lane_bits + col + NLV * L, acc[L]);
                 tmem_wait_ld();
@@ -929,8 +966,9 @@ cudaError_t launch_split_sweep_tc3d(const GridView &g, const Weights &w, long lo
 }
 
 cudaError_t launch_fp64_sweep_tc3d(const GridView &g, const Weights &w, long long origin, long long elements,
-                                   const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st)
+                                   const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st, bool fine)
 {
+    if (fine) return launch_tc3d<F3F64Fine>(g, f64_slice_weights(w, 27, &tap_order(Taps::kCube3)), origin, elements, in_base, out_base, wt, st);
     return launch_tc3d<F3F64>(g, f64_slice_weights(w, 27), origin, elements, in_base, out_base, wt, st);
 }
 

@@ -586,8 +586,9 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     // five digits err more than double-float, 1.7e-12 against 1e-14 in the norm
     // after tens of sweeps, so requests below 2e6 points keep that); FP64 7x7
     // 256^2 18.7 FMA, 9.5 tcgen05 (an FMA tile takes 14 us however few there
-    // are); box3d1r 32^3 5.7, 8.4, 48^3 12.3, 8.9; star3d1r 96^3 13.5, 18.4, 128^3
-    // 29.8, 29.0; star2d1r 512^2 6.4, 4.4 (three steps a launch). The fused
+    // are); box3d1r 32^3 5.7, 8.4, 48^3 12.3, 8.9; star2d1r 512^2 6.4, 4.4 (three
+    // steps a launch). star3d1r stays on FP64 FMA, whose seven taps err less
+    // (9.2e-17 of the norm, tcgen05 1.25e-16; 128^3 29.8 and 29.0). The fused
     // 7x7x7 box costs 343 FMA per point, 171 us at 64^3 against 41; its
     // octahedron 63, about as long at 64^3.
     const bool box3d = d->shape == CS_SHAPE_BOX3D1R, in3d = box3d || d->shape == CS_SHAPE_STAR3D1R;
@@ -606,13 +607,16 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     } else {
         bool tc;
         if (in3d)
-            tc = pts >= (fused ? (box3d ? 3.2e4 : 2.6e5) : (box3d ? 6e4 : 2e6));
+            tc = pts >= (fused ? (box3d ? 3.2e4 : 2.6e5) : 6e4) && (fused || box3d);
         else if (in1d)
             tc = pts >= 2.6e5;
         else  // radius 3 any size, radius 1 from 64 tiles
             tc = fused || d->shape == CS_SHAPE_BOX2D3R || d->shape == CS_SHAPE_STAR2D3R ||
                  ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64) >= 64;
-        r->sweeps_per_launch = cs::plan_fix_fp64(r->plan, tc);
+        // A client cannot ask for FP64 FMA sums: only 7x7 kernels of at least four
+        // 64 x 64 tiles per SM run on the kernel whose error is larger.
+        const long long tiles = in3d || in1d ? 0 : ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64);
+        r->sweeps_per_launch = cs::plan_fix_fp64(r->plan, tc, tiles < 4LL * s->sm_count);
     }
     // The FP64 FMA 2D kernel's tile rows: fixed here (the plan tuner would
     // time both on the worker thread); results do not depend on them.

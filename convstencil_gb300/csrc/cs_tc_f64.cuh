@@ -7,7 +7,9 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "cs_internal.h"
 #include "cs_split_common.cuh"
@@ -21,14 +23,69 @@ namespace tc {
 struct F64Weights {
     __half d[6][49];
     int ew;
+    float rest;  // see keep_sum
 };
 
-// keep_sum: six digits hold a weight to 2^-45 of the top digit's unit, and
-// what rounding leaves of one weight is carried to the next, so the sum of
-// the weights keeps its value to half a unit (an error in the sum scales a
-// smooth grid by the same factor in every sweep, where the errors of single
-// weights average out). Used by the launches of several steps.
-inline F64Weights f64_slice_weights(const Weights &w, int taps = 49, bool keep_sum = false)
+// The taps of a line of 49, of a 7x7, a 3x3x3 or a 7x7x7, farthest first.
+struct TapOrder {
+    std::vector<int> tap;
+    std::vector<double> x, y, z;  // where it lies
+};
+enum class Taps { kLine49, kSquare7, kCube3, kCube7 };
+inline const TapOrder &tap_order(Taps t)
+{
+    auto make = [](int nx, int ny, int nz) {
+        TapOrder o;
+        auto px = [=](int i) { return i % nx - nx / 2; };
+        auto py = [=](int i) { return i / nx % ny - ny / 2; };
+        auto pz = [=](int i) { return i / (nx * ny) - nz / 2; };
+        auto far = [&](int i) { return px(i) * px(i) + py(i) * py(i) + pz(i) * pz(i); };
+        for (int i = 0; i < nx * ny * nz; ++i) o.tap.push_back(i);
+        std::stable_sort(o.tap.begin(), o.tap.end(), [&](int a, int b) { return far(a) > far(b); });
+        for (int i : o.tap) o.x.push_back(px(i)), o.y.push_back(py(i)), o.z.push_back(pz(i));
+        return o;
+    };
+    static const TapOrder orders[4] = {make(49, 1, 1), make(7, 7, 1), make(3, 3, 3), make(7, 7, 7)};
+    return orders[(int)t];
+}
+
+// Rounds weights to integers (units of their last digit) so that their sum and
+// first moments keep their values. An error of the sum scales a smooth grid by
+// the same factor in every sweep, one of the moments moves it, where the errors
+// of single weights average out; so each weight, from the farthest in, goes up
+// or down as the sums of the errors so far want it. (To the nearest, each error
+// carried on to the next tap, the moment along a row of a 7x7 was off by 3.8
+// units; so all three by 0.4 to 0.5.)
+struct KeepSums {
+    double r0 = 0.0, rx = 0.0, ry = 0.0, rz = 0.0;  // errors so far
+    double round(double v, double x, double y, double z)
+    {
+        const double below = std::floor(v), d = below - v, u = d + 1.0;
+        auto miss = [&](double q) {
+            return (r0 + q) * (r0 + q) + (rx + q * x) * (rx + q * x) + (ry + q * y) * (ry + q * y) +
+                   (rz + q * z) * (rz + q * z);
+        };
+        const bool down = d == 0.0 || miss(d) <= miss(u);
+        const double q = down ? d : u;
+        r0 += q, rx += q * x, ry += q * y, rz += q * z;
+        return down ? below : below + 1.0;
+    }
+};
+
+// What is left of a sum, as a factor of the level-0 sum: r0 is in units of 2^-45,
+// the number it goes to in units of 2^-42 of level 0's.
+inline float rest_of(const KeepSums &k, double sum, double size)
+{
+    return std::fabs(sum) > size * 0x1p-6 ? (float)(-k.r0 * 0.125 / sum) : 0.0f;
+}
+
+// keep: where the taps lie whose sum and first moments keep their values
+// (KeepSums; six digits hold a weight to 2^-45 of the top digit's unit), or null.
+// What is then left of the sum goes to the recombination as `rest`, the factor
+// of the level-0 sum that makes up for it there (f64_combine; 0 where the
+// weights cancel). 100 steps of star2d1r 1024^2, uniform data: error of the norm
+// 5.7e-16 with six levels, 1.3e-16 with seven and carried errors, 1.06e-16 so.
+inline F64Weights f64_slice_weights(const Weights &w, int taps = 49, const TapOrder *keep = nullptr)
 {
     F64Weights s{};
     double mx = 0.0;
@@ -39,20 +96,22 @@ inline F64Weights f64_slice_weights(const Weights &w, int taps = 49, bool keep_s
         e += 2;              // |w| / 2^ew < 1/4
     }
     s.ew = e;
-    double carry = 0.0;
-    for (int i = 0; i < taps; ++i) {
+    KeepSums kept;
+    double sum = 0.0, size = 0.0;
+    for (int k = 0; k < taps; ++k) {
+        const int i = keep ? keep->tap[k] : k;
         double a = std::ldexp(w.v[i], split::kDigitBits - e);  // |a| < 128, exact
-        if (keep_sum && a != 0.0) {
-            const double t = a;
-            a = std::ldexp(std::rint(std::ldexp(t, 45) + carry), -45);
-            carry += std::ldexp(t - a, 45);
-        }
-        for (int k = 0; k < 6; ++k) {
+        sum += a;
+        size += std::fabs(a);
+        if (keep && a != 0.0)
+            a = std::ldexp(kept.round(std::ldexp(a, 45), keep->x[k], keep->y[k], keep->z[k]), -45);
+        for (int t = 0; t < 6; ++t) {
             const double d = std::rint(a);
-            s.d[k][i] = __float2half_rn((float)d);
+            s.d[t][i] = __float2half_rn((float)d);
             a = (a - d) * 512.0;  // exact: a - d is a multiple of a's last bit
         }
     }
+    s.rest = keep ? rest_of(kept, sum, size) : 0.0f;
     return s;
 }
 
@@ -153,6 +212,26 @@ __device__ __forceinline__ long long f64_combine(const float (&lv)[6])
     return t;
 }
 
+// The same with what the weights' sum lacks (F64Weights::rest), of six levels or
+// seven: the last ones come in as one number, rounded to T's unit (2^-42 of level
+// 0's, below 2^-52 of T itself but for sums that cancel).
+template <int LV>
+__device__ __forceinline__ long long f64_combine(const float (&lv)[LV], float rest)
+{
+    static_assert(LV == 6 || LV == 7);
+    float last = lv[0] * rest;
+    if constexpr (LV == 7) last = fmaf(lv[6], 0x1p-12f, last);
+    long long t = __float2int_rn(fmaf(lv[5], 0.125f, last));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(__float2int_rn(lv[4])), "r"(1 << 6));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(__float2int_rn(lv[3])), "r"(1 << 15));
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(__float2int_rn(lv[2])), "r"(1 << 24));
+    unsigned tl, th;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(tl), "=r"(th) : "l"(t));
+    th += (unsigned)(__float2int_rn(lv[1]) * 2 + __float2int_rn(lv[0]) * 1024);
+    asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "r"(tl), "r"(th));
+    return t;
+}
+
 // f64_combine for two outputs whose level sums are below 2^22 in magnitude
 // (one z tap of a 3D input plane: 9 taps, so level L sums at most 9 * 5 * 2^16 <
 // 2^22), added to their running 64-bit sums: an FP32 addition of 1.5 * 2^23
@@ -163,8 +242,12 @@ __device__ __forceinline__ long long f64_combine(const float (&lv)[6])
 // off once per sum. (GB300, star3d1r 512^3: 1128 us a sweep with the bias taken
 // off every level, 1112 so.)
 constexpr unsigned kRaw = 0x4B400000u;
-constexpr unsigned long long kRawBias = (kRaw >> 3) + (unsigned long long)kRaw * ((1u << 6) + (1u << 15) + (1u << 24)) +
+// LOW: level 5's bits below T's unit (none of seven levels' sum, below).
+template <int LOW = 3>
+constexpr unsigned long long kRawBias = (kRaw >> LOW) +
+                                        (unsigned long long)kRaw * ((1u << 6) + (1u << 15) + (1u << 24)) +
                                         ((unsigned long long)(kRaw * 1026u) << 32);
+template <int LOW = 3>
 __device__ __forceinline__ void f64_add_raw2(const float (&u)[6], const float (&v)[6], long long &su, long long &sv)
 {
     int a[6], b[6];
@@ -176,7 +259,7 @@ __device__ __forceinline__ void f64_add_raw2(const float (&u)[6], const float (&
         asm("mov.b64 {%0, %1}, %2;" : "=r"(a[L]), "=r"(b[L]) : "l"(x));
     }
     auto sum = [](const int (&r)[6], long long &t) {
-        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[5] >> 3), "r"(1));
+        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[5] >> LOW), "r"(1));
         asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[4]), "r"(1 << 6));
         asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[3]), "r"(1 << 15));
         asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(t) : "r"(r[2]), "r"(1 << 24));
@@ -187,6 +270,17 @@ __device__ __forceinline__ void f64_add_raw2(const float (&u)[6], const float (&
     };
     sum(a, su);
     sum(b, sv);
+}
+// The same of seven levels: level 5, level 6 and what the weights' sum lacks
+// (F64Weights::rest) come in as one number, rounded to T's unit: cut off there, as
+// above, every part loses half a unit, the same way each sweep (star3d1r 160 x 128 x
+// 125, 100 sweeps: 9.5e-16 of the norm so). A call adds kRawBias<0>.
+__device__ __forceinline__ void f64_add_raw2(const float (&u)[7], const float (&v)[7], float rest, long long &su,
+                                             long long &sv)
+{
+    const float p[6] = {u[0], u[1], u[2], u[3], u[4], fmaf(u[5], 0.125f, fmaf(u[6], 0x1p-12f, u[0] * rest))};
+    const float q[6] = {v[0], v[1], v[2], v[3], v[4], fmaf(v[5], 0.125f, fmaf(v[6], 0x1p-12f, v[0] * rest))};
+    f64_add_raw2<0>(p, q, su, sv);
 }
 
 // Results outside the normal FP64 range (subnormal or overflowing): FP64

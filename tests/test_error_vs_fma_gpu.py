@@ -85,3 +85,63 @@ def test_fused_3d(shape, kind):
     w, dense = w / dense.sum(), dense / dense.sum()
     tc, fma = errors(shape, ext, w, dense, 10, 30, kind, lambda: cs.Plan(shape, ext, w, semantics=cs.Semantics.FUSED))
     assert tc <= fma
+
+
+# Two sets of roundings of the same size differ by a few per cent.
+ABOUT = 1.05
+
+
+@pytest.mark.parametrize("odd", [False, True])
+@pytest.mark.parametrize("shape,ext,steps", [("star2d1r", (1024, 1024), 100), ("box2d1r", (1027, 1409), 60),
+                                             ("box2d3r", (1025, 1409), 20), ("star2d3r", (1025, 1409), 20)])
+def test_2d(shape, ext, steps, odd):
+    if not odd and "3r" in shape:
+        pytest.skip("one step per launch on even layouts: the kernel that ran there before")
+    info = cs.SHAPE_INFO[cs.SHAPE_BY_NAME[shape]]
+    w = O.seeded_weights(info[1], 32)
+    w /= w.sum()
+    dense = {"star2d1r": O.star2d1r_to_dense, "star2d3r": O.star2d3r_to_dense}.get(shape, lambda v: v)(w)
+    k = 3 if "1r" in shape else 7
+    ld = ext[1] + 9
+    lay = {"dims": 2, "halo": k // 2, "extent": list(ext), "pitch": [ld, 1], "origin": 3 * ld + 5,
+           "elements": (ext[0] + 6) * ld} if odd else None
+    tc, fma = errors(shape, ext, w, dense.reshape(k, k), steps, steps, "uniform",
+                     lambda: cs.Plan(shape, ext, w, **({"layout": lay} if odd else {})))
+    assert tc <= ABOUT * fma
+
+
+@pytest.mark.parametrize("shape,n,steps", [("1d1r", 1_000_000, 100), ("1d2r", 1_000_001, 100), ("1d2r", 300_007, 33)])
+def test_1d(shape, n, steps):
+    w = O.seeded_weights(3 if shape == "1d1r" else 5, 33)
+    w /= w.sum()
+    tc, fma = errors(shape, (n,), w, w, steps, steps, "uniform", lambda: cs.Plan(shape, (n,), w))
+    assert tc <= ABOUT * fma
+
+
+@pytest.mark.parametrize("shape,ext,steps,fused", [
+    ("box2d3r", (256, 250), 40, 0), ("star2d3r", (96, 130), 10, 0), ("star2d1r", (256, 250), 60, 1),
+    ("star2d1r", (520, 600), 60, 0), ("1d2r", (300_007,), 60, 0), ("box3d1r", (64, 60, 66), 100, 0),
+    ("star3d1r", (132, 128, 125), 60, 0), ("box3d1r", (40, 44, 50), 60, 1), ("star3d1r", (70, 66, 64), 60, 1)])
+def test_served(shape, ext, steps, fused):
+    """Requests: a client cannot choose the kernel."""
+    info = cs.SHAPE_INFO[cs.SHAPE_BY_NAME[shape]]
+    w = O.seeded_weights(info[1 + fused], 34)
+    r = info[4 + fused]
+    expand = {("star2d1r", 0): O.star2d1r_to_dense, ("star2d3r", 0): O.star2d3r_to_dense,
+              ("star3d1r", 0): O.star3d1r_to_dense, ("star3d1r", 1): O.star3d_params_to_dense,
+              ("box3d1r", 1): O.box3d_planes_to_dense}.get((shape, fused), lambda v: v)
+    dense = expand(w).reshape((2 * r + 1,) * len(ext))
+    w, dense = w / dense.sum(), dense / dense.sum()
+    sweeps = steps // info[3] if fused else steps
+    x = field(ext, "uniform")
+    hi, lo = two_doubles(x, dense, sweeps)
+    server = cs.Server(hbm_fraction=0.05)
+    got, _ = server.wait(server.submit(shape, x.cpu().numpy(), w, steps, semantics=cs.Semantics(fused)))
+    p = cs.Plan(shape, ext, w, semantics=cs.Semantics(fused))
+    p.set_option(cs.Option.ALGO, cs.Algo.FP64_FMA)
+    a = torch.from_numpy(p.pack(x.cpu().numpy())).cuda()
+    b = torch.zeros_like(a)
+    in_b = p.run(a, b, steps)
+    fma = p.unpack((b if in_b else a).cpu().numpy())
+    err = [float(((torch.from_numpy(g).cuda() - hi) - lo).norm()) for g in (got, fma)]
+    assert err[0] <= ABOUT * err[1]
