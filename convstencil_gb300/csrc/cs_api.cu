@@ -398,15 +398,25 @@ int steps_per_launch(const cs_plan *p, const void *in_base, const void *out_base
     return tiles >= 64 ? p->max_steps : 1;
 }
 
+// Whether an Inf or NaN reaches only the outputs that read it where tcgen05
+// launches stand for other kernels (TcForm::redo). A caller who pins FP64_TC gets
+// its tiles as they are: NaN.
+bool redo_of(const cs_plan *p) { return p->algo != CS_ALGO_FP64_TC || p->fine; }
+
 // `steps` (1 .. steps_per_launch) steps in one launch, on FP64 or split grids.
-cudaError_t launch_steps(const cs_plan *p, bool fp64, int steps, const void *in_base, void *out_base, cudaStream_t st)
+// tuning: a timing run, of the usual launch whatever the grid holds (no redo).
+cudaError_t launch_steps(const cs_plan *p, bool fp64, int steps, const void *in_base, void *out_base, cudaStream_t st,
+                         bool tuning = false)
 {
+    const bool redo = !tuning && redo_of(p);
     if (p->dims == 1)
         return cs::launch_steps_tc_1d(fp64, p->view.ext[0], p->w1_steps[steps - 1], p->radius, p->w.v, steps,
-                                      p->layout.origin, in_base, out_base, p->wait, st);
+                                      p->layout.origin, in_base, out_base, p->wait, st, redo);
+    cs::TcForm form{1, p->pattern};
+    form.odd = !fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base);
+    form.redo = redo;
     return cs::launch_steps_tc(fp64, p->view, p->w_steps[steps - 1], p->w, steps, p->layout.origin,
-                               p->layout.elements, in_base, out_base, p->wait, st,
-                               fp64_tc_window_ok(p->view, p->layout.origin, in_base, out_base));
+                               p->layout.elements, in_base, out_base, p->wait, st, form);
 }
 
 // One sweep over the slabs [row0, row0 + rows) of the slowest axis (rows of
@@ -415,7 +425,7 @@ cudaError_t launch_steps(const cs_plan *p, bool fp64, int steps, const void *in_
 // temporally blocked kernels, which treat everything outside their grid as
 // zero, are never launched here.
 cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, void *out_base, long long row0,
-                              long long rows, cudaStream_t st)
+                              long long rows, cudaStream_t st, bool tuning = false)
 {
     GridView v = p->view;
     v.ext[0] = rows;
@@ -423,21 +433,25 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
     if (p->prec == CS_PREC_FP64) {
         const double *in = (const double *)in_base + off;
         double *out = (double *)out_base + off;
+        cs::TcForm form{p->radius, p->pattern};
+        form.redo = !tuning && redo_of(p);
         if (algo == CS_ALGO_FP64_MMA) return cs::launch_fp64_mma_2d(v, p->w, in, out, st);
         if (algo == CS_ALGO_FP64_TC && fp64_tc1d_ok(p) && row0 == 0 && rows == p->view.ext[0])
-            return launch_steps(p, true, 1, in_base, out_base, st);
+            return launch_steps(p, true, 1, in_base, out_base, st, tuning);
         if (algo == CS_ALGO_FP64_TC && fp64_tc3d_ok(p) && p->rows_whole &&
             cs::split_tc3d_layout_ok(v, off, in_base, out_base))
             return cs::launch_fp64_sweep_tc3d(v, p->w, off, p->layout.elements, (const double *)in_base,
-                                              (double *)out_base, p->wait, st, p->fine);
+                                              (double *)out_base, p->wait, st, p->fine ? &form : nullptr);
         if (algo == CS_ALGO_FP64_TC && fp64_tc3d_r3_ok(p))
             return cs::launch_fp64_sweep_tc3d_r3(v, p->w, off, p->layout.elements, (const double *)in_base,
-                                                 (double *)out_base, p->rows_whole, p->wait, st);
-        if (algo == CS_ALGO_FP64_TC && fp64_tc_ok(p) && tc_bases_ok(in_base, out_base))
+                                                 (double *)out_base, p->rows_whole, form, p->wait, st);
+        if (algo == CS_ALGO_FP64_TC && fp64_tc_ok(p) && tc_bases_ok(in_base, out_base)) {
+            form.odd = !fp64_tc_window_ok(v, off, in_base, out_base);
+            form.above = row0;
+            form.below = p->view.ext[0] - row0 - rows;
             return cs::launch_fp64_sweep_tc(v, p->w7, off, p->layout.elements, (const double *)in_base,
-                                            (double *)out_base, p->wait, st,
-                                            fp64_tc_window_ok(v, off, in_base, out_base) ? 0 : p->radius, row0,
-                                            p->view.ext[0] - row0 - rows, p->fine);
+                                            (double *)out_base, p->wait, st, form.odd || p->fine ? &form : nullptr);
+        }
         return cs::launch_fp64_fma(v, p->radius, p->pattern, p->w, in, out, st, p->active_rows);
     }
     // The tensor-core split kernels store float4 (two points) at even element
@@ -468,9 +482,10 @@ cudaError_t launch_sweep_rows(const cs_plan *p, int algo, const void *in_base, v
                                   in, out, st);
 }
 
-cudaError_t launch_sweep(const cs_plan *p, int algo, const void *in_base, void *out_base, cudaStream_t st)
+cudaError_t launch_sweep(const cs_plan *p, int algo, const void *in_base, void *out_base, cudaStream_t st,
+                         bool tuning = false)
 {
-    return launch_sweep_rows(p, algo, in_base, out_base, 0, p->view.ext[0], st);
+    return launch_sweep_rows(p, algo, in_base, out_base, 0, p->view.ext[0], st, tuning);
 }
 
 int size_class(const cs_plan *p)
@@ -569,7 +584,7 @@ cs_status choose_algo(cs_plan *p, const void *a, void *b, cudaStream_t st, int *
         for (int ci = 0; ci < nc; ++ci) {
             const int c = cand[ci];
             CS_CUDA(cudaEventRecord(e0, st));
-            for (int i = 0; i < reps; ++i) CS_CUDA(launch_sweep(p, c, a, b, st));
+            for (int i = 0; i < reps; ++i) CS_CUDA(launch_sweep(p, c, a, b, st, true));
             CS_CUDA(cudaEventRecord(e1, st));
             CS_CUDA(cudaEventSynchronize(e1));
             float ms = 0.f;
@@ -689,10 +704,10 @@ cs_status choose_steps(cs_plan *p, const void *a, void *b, cudaStream_t st, long
                                                       (const float2 *)a + p->layout.origin,
                                                       (float2 *)b + p->layout.origin, st));
                 else
-                    CS_CUDA(launch_sweep(p, algo, a, b, st));
+                    CS_CUDA(launch_sweep(p, algo, a, b, st, true));
             }
             CS_CUDA(cudaEventRecord(e[1], st));
-            for (int i = 0; i < reps; ++i) CS_CUDA(launch_steps(p, fp64, t, a, b, st));
+            for (int i = 0; i < reps; ++i) CS_CUDA(launch_steps(p, fp64, t, a, b, st, true));
             CS_CUDA(cudaEventRecord(e[2], st));
             CS_CUDA(cudaEventSynchronize(e[2]));
         }

@@ -80,20 +80,22 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 // The same pipeline on FP64 grids (2D dense 7x7): six exact 9-bit digits per
 // operand cut from the FP64 bits by integer operations, exact FP32 level sums
 // on tcgen05, integer recombination to FP64. Layout conditions as above.
-// radius not 0: any pitch and first column (whole rows of the halo in the
-// buffer), points past a halo of `radius` read as zero; the grid goes on for
-// `above` and `below` rows before and after the ones swept. fine: no larger an
-// error than FP64 FMA sums (always so with a radius).
+// With a form: in the place of FP64 FMA sums, with no larger an error.
+struct TcForm {
+    int radius, pattern;         // of the plan's kernel
+    bool odd = false;            // any pitch and first column (whole rows of the halo in the buffer);
+                                 // points past a halo of `radius` read as zero
+    long long above = 0, below = 0;  // rows by which the grid goes on before and after the ones swept
+    bool redo = false;           // an Inf or NaN reaches the outputs that read it only, not its tile
+};
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
                                  const double *in_base, double *out_base, const TcWait &wait,
-                                 cudaStream_t stream, int radius = 0, long long above = 0, long long below = 0,
-                                 bool fine = false);
+                                 cudaStream_t stream, const TcForm *form = nullptr);
 // `steps` (1..3) steps of a 2D radius-1 grid (FP64 or split) in one launch: wT
-// is the 7x7 kernel of that many steps, w3x3 the weights of one. tma false
-// (FP64): as a radius above.
+// is the 7x7 kernel of that many steps, w3x3 the weights of one. (odd: FP64.)
 cudaError_t launch_steps_tc(bool fp64, const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
                             long long origin, long long elements, const void *in_base, void *out_base,
-                            const TcWait &wait, cudaStream_t stream, bool tma);
+                            const TcWait &wait, cudaStream_t stream, const TcForm &form);
 // Batches of 2D radius-3 grids on the tcgen05 kernels (split or FP64): one
 // device record per grid (tc_batch_record_bytes each, 128-byte aligned)
 // holding its tensor map over `in_base`, output, sizes, first tile and
@@ -114,11 +116,11 @@ cudaError_t encode_split_window_map(CUtensorMap *map, const float2 *base, long l
 // `steps` steps of a 1D grid (FP64 or split) of n >= 64 points in one launch
 // of the tcgen05 digit kernel, steps * radius <= kTcReach1d: taps are the 49
 // taps of that many steps (the output's own at 24), w the 2 radius + 1 weights
-// of one.
+// of one; redo: see TcForm.
 constexpr int kTcReach1d = 24;
 cudaError_t launch_steps_tc_1d(bool fp64, long long n, const double *taps, int radius, const double *w, int steps,
                                long long origin, const void *in_base, void *out_base, const TcWait &wait,
-                               cudaStream_t stream);
+                               cudaStream_t stream, bool redo);
 // 3D tensor map: `planes` planes of pitch ldz, rows of pitch ld; box
 // box_x x box_y x 1.
 cudaError_t encode_split_window_map_3d(CUtensorMap *map, const float2 *base, long long ld, long long ldz,
@@ -135,16 +137,16 @@ cudaError_t launch_split_sweep_tc3d(const GridView &g, const Weights &w, long lo
 // the FP64 bits with integer operations, exact level sums, one rounding to
 // FP64 per output (an output whose parts had different plane exponents is
 // summed in FP64). Same layout conditions.
-// (fine: see launch_fp64_sweep_tc.)
+// form: see launch_fp64_sweep_tc.
 cudaError_t launch_fp64_sweep_tc3d(const GridView &g, const Weights &w, long long origin, long long elements,
                                    const double *in_base, double *out_base, const TcWait &wait,
-                                   cudaStream_t stream, bool fine = false);
+                                   cudaStream_t stream, const TcForm *form = nullptr);
 // FP64 sweep of a 3D radius-3 kernel (343 weights, any pattern) on tcgen05
 // (cs_kernels_tc3d_r3.cu), any layout. rows_whole: whole rows and planes of the
 // buffer hold the halo, as the windows' tensor map wants.
 cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long long origin, long long elements,
-                                      const double *in_base, double *out_base, bool rows_whole, const TcWait &wait,
-                                      cudaStream_t stream);
+                                      const double *in_base, double *out_base, bool rows_whole, const TcForm &form,
+                                      const TcWait &wait, cudaStream_t stream);
 int device_sm_count();
 // Bounded device-side waits that expired since the last reset (TMA/mma.sync
 // kernel, 2D and 3D tcgen05 kernels).

@@ -157,6 +157,10 @@ struct FmtF64Fine : FmtF64 {
     static constexpr int kLevels = 7;
 };
 
+// Formats whose launches may stand for kernels without digits (Redo).
+template <class F>
+constexpr bool kRedoable = F::kDigits == 6 && (F::kLevels == 7 || !F::kF64);
+
 // Warp roles.
 constexpr int kWarpTma = 0, kWarpMma = 1, kWarpSlice0 = 2;
 template <class F>
@@ -223,6 +227,7 @@ struct Smem {
     int scale_exp[4];                          // per-tile input scale, ring of 4
     float red[2][kMaxSliceWarps];                 // split: per-warp max |hi|, by tile parity
     int redi[2][kMaxSliceWarps];                  // FP64: per-warp max biased exponent
+    std::conditional_t<kRedoable<F>, Redo, NoRedo> redo;  // tiles to compute again
 };
 
 static_assert(sizeof(Smem<FmtF64Fine>) + 128 <= 232448 && sizeof(Smem<FmtSplit>) + 128 <= 232448 &&
@@ -425,17 +430,19 @@ struct OddRows {
     unsigned late[2];    // points by which its rows are late
 };
 
-template <class F>
+template <class F, int MODE>
 struct StepArgs {
     const typename F::Out *in;  // interior point (0, 0) of the source
     int steps;                  // T
     int radius;                 // of one step
     int aligned;                // 1D: the buffers and the interior are 16-byte aligned
-    unsigned taps;              // bit t: weight t is not zero
+    unsigned taps;              // 2D steps, bit t: weight t belongs to the pattern
     int frame_cta;              // CTAs from this one on compute the frame
-    typename F::Out w[9];       // weights of one step
+    typename F::Out w[MODE == kModeGrid ? 49 : 9];  // weights of one step (kModeGrid: at the centre of a 7x7)
     OddRows rows;               // odd layouts
     int above, below;           // odd layouts: rows of the grid before and after the ones swept
+    int pattern;                // of the weights
+    int redo;                   // tiles that hold an Inf or NaN are computed again (else: NaN)
 };
 
 // The frame's arithmetic, that of single sweeps: FP64 FMA, or double-float.
@@ -517,7 +524,7 @@ __device__ __forceinline__ void frame_strip(const V *__restrict__ in, V *__restr
 
 // The frame of an m x n grid, strip by strip, shared by `nwarps` warps.
 template <class F>
-__device__ __noinline__ void frame_steps(const StepArgs<F> &s, typename F::Out *__restrict__ out, int m, int n,
+__device__ __noinline__ void frame_steps(const StepArgs<F, kModeSteps> &s, typename F::Out *__restrict__ out, int m, int n,
                                          long long ld, int warp, int nwarps)
 {
     constexpr int S = 32 - 2 * kMaxSteps;  // outputs per strip
@@ -550,7 +557,7 @@ __device__ __noinline__ void frame_steps(const StepArgs<F> &s, typename F::Out *
 // points -r .. 2 T r - r - 1 counted from that end, two per lane, in `buf`
 // (level l's in buf[l % 2]); every level's last r points fall out of use.
 template <class F>
-__device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out *__restrict__ out, long long n, bool left,
+__device__ __noinline__ void frame_end_1d(const StepArgs<F, kMode1d> &s, typename F::Out *__restrict__ out, long long n, bool left,
                                           typename F::Out (*buf)[kFrame1d])
 {
     using V = typename F::Out;
@@ -575,6 +582,85 @@ __device__ __noinline__ void frame_end_1d(const StepArgs<F> &s, typename F::Out 
     for (int i = r + lane; i < s.steps * r; i += 32) out[at(i)] = buf[s.steps & 1][i];
 }
 
+// A tile's outputs computed again (Redo), by the whole CTA: FP64 FMA or double-
+// float sums of single steps on windows in shared memory (`a`, then `b` and `a`
+// by turns). Points outside the grid and its halo are zeros that meet no output:
+// those next to the boundary are the frame's.
+template <class F, int MODE>
+__device__ __forceinline__ void redo_tile(const StepArgs<F, MODE> &s, typename F::Out *__restrict__ out, int m, int n,
+                                          long long ld, int tiles_x, int tile, typename F::Out *a, typename F::Out *b)
+{
+    using V = typename F::Out;
+    const int tid = threadIdx.x, nt = blockDim.x, r = s.radius;
+    if constexpr (MODE == kMode1d) {
+        const int reach = s.steps * r, frame = reach - r;
+        const long long at = (long long)tile * kOut1d;
+        for (int i = tid; i < kOut1d + 2 * reach; i += nt) {
+            const long long x = at + i - reach;
+            a[i] = x >= -r && x < (long long)n + r ? s.in[x] : V{};
+        }
+        __syncthreads();
+        for (int level = 1, len = kOut1d + 2 * (reach - r); level <= s.steps; ++level, len -= 2 * r) {
+            for (int i = tid; i < len; i += nt) {
+                V v{};
+                for (int t = 0; t <= 2 * r; ++t) tap_acc(v, s.w[t], a[i + t]);
+                b[i] = tap_sum(v);
+                if (level == s.steps && at + i >= frame && at + i < (long long)n - frame) out[at + i] = b[i];
+            }
+            __syncthreads();
+            V *const c = a;
+            a = b;
+            b = c;
+        }
+    } else {
+        constexpr bool STEPS = MODE == kModeSteps;
+        constexpr int W = TX + 2 * 3, K = STEPS ? 3 : 7;
+        const int y0 = tile / tiles_x * TY, x0 = tile % tiles_x * TX;
+        static_assert(TX == TY && W * W * 8 <= F::kDigits * PL * 2, "square tiles, whose windows fit a plane set");
+        const int steps = STEPS ? s.steps : 1, reach = STEPS ? steps : 3, frame = STEPS ? steps - 1 : 0;
+        const int top = STEPS ? -r : -r - s.above, bottom = STEPS ? m + r : m + r + s.below;
+        for (int i = tid; i < (TX + 2 * reach) * (TX + 2 * reach); i += nt) {
+            const int p = i / (TX + 2 * reach), q = i - p * (TX + 2 * reach);
+            const int y = y0 - reach + p, x = x0 - reach + q;
+            a[p * W + q] = y >= top && y < bottom && x >= -r && x < n + r ? s.in[(long long)y * ld + x] : V{};
+        }
+        __syncthreads();
+        for (int level = 1; level <= steps; ++level) {
+            const int side = TX + 2 * (steps - level);
+            for (int i = tid; i < side * side; i += nt) {
+                const int p = i / side, q = i - p * side;
+                V v{};
+                for (int t = 0; t < K * K; ++t) {
+                    const int dy = t / K, dx = t - dy * K;
+                    const bool tap = STEPS ? s.taps >> t & 1u
+                                           : max(abs(dy - 3), abs(dx - 3)) <= r &&
+                                                 in_pattern(s.pattern, 0, dy - 3, dx - 3, r);
+                    if (tap) tap_acc(v, s.w[t], a[(p + dy) * W + q + dx]);
+                }
+                b[p * W + q] = tap_sum(v);
+                const int y = y0 + p, x = x0 + q;
+                if (level == steps && y >= frame && y < m - frame && x >= frame && x < n - frame)
+                    out[(long long)y * ld + x] = b[p * W + q];
+            }
+            __syncthreads();
+            V *const c = a;
+            a = b;
+            b = c;
+        }
+    }
+}
+
+template <class F, int MODE>
+__device__ __noinline__ void redo_tiles(const StepArgs<F, MODE> &s, typename F::Out *__restrict__ out, int m, int n,
+                                        long long ld, int tiles_x, int tiles, Smem<F> &S)
+{
+    using V = typename F::Out;
+    for (int it = 0, tile = blockIdx.x; tile < tiles; ++it, tile += gridDim.x)
+        if (S.redo.holds(it, it))
+            redo_tile<F, MODE>(s, out, m, n, ld, tiles_x, tile, reinterpret_cast<V *>(S.planes[0][0]),
+                               reinterpret_cast<V *>(S.planes[1][0]));
+}
+
 // One grid (BATCH = false: kernel parameters describe it, tiles are dealt
 // round-robin) or a batch of grids (BATCH = true: `grids` describes them,
 // each CTA takes a contiguous run of the batch's tiles, and the MMA warp
@@ -584,7 +670,7 @@ template <class F, bool BATCH, int MODE = kModeGrid, bool ODD = false>
 __global__ void __launch_bounds__(kThreads<F>, 1)
     k2d_tc(const __grid_constant__ CUtensorMap tmap, typename F::Out *__restrict__ out, int m, int n,
            long long ld, int tiles_x, int tiles, int map_x, int map_y, typename F::Digits sw, WaitCfg wc,
-           const TcGrid<F> *__restrict__ grids, int ngrids, const __grid_constant__ StepArgs<F> sa)
+           const TcGrid<F> *__restrict__ grids, int ngrids, const __grid_constant__ StepArgs<F, MODE> sa)
 {
     constexpr bool ONED = MODE == kMode1d, STEPS = MODE == kModeSteps;
     static_assert(!BATCH || (MODE == kModeGrid && !ODD), "batches run one sweep of 7x7 grids");
@@ -666,6 +752,7 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             mbar_init(bar2(S.acc_empty, i), F::kEpiWarps);
         }
         S.abort = 0;
+        if constexpr (kRedoable<F>) S.redo.count = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (!ONED && my_tiles > 0 && !wc.skip_loads) {  // the first window load overlaps the set-up below
             pdl_wait();
@@ -879,11 +966,15 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             for (int q = 0; q < PER; ++q) {
                 if constexpr (F::kF64)
                     emax = max(emax, max(size_of(v[q].y), size_of(v[q].w)));
+                else if constexpr (kRedoable<F>)
+                    vmax = max_nan(vmax, max_nan(fabsf(__uint_as_float(v[q].x)), fabsf(__uint_as_float(v[q].z))));
                 else
                     vmax = fmaxf(vmax, fmaxf(fabsf(__uint_as_float(v[q].x)), fabsf(__uint_as_float(v[q].z))));
             }
             if constexpr (F::kF64) {
                 emax = __reduce_max_sync(0xffffffffu, emax) >> (STEPS ? 0 : 20);
+            } else if constexpr (kRedoable<F>) {  // (not negative: ordered as integers, a NaN above Inf)
+                vmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(vmax)));
             } else {
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
@@ -902,19 +993,30 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
             const bool free = landed && wait(bar2(S.planes_empty, buf), (use & 1) ^ 1);
             if (bar_any(kSliceBarrier, kSliceThreads, !free)) break;
             int ex;
+            bool finite = true;
             if constexpr (F::kF64) {
                 int eb = S.redi[buf][0];
 #pragma unroll
                 for (int i = 1; i < kSliceWarps; ++i) eb = max(eb, S.redi[buf][i]);
                 ex = max(eb, 1);
+                finite = ex != 2047;
             } else {
                 vmax = S.red[buf][0];
+                if constexpr (kRedoable<F>) {
 #pragma unroll
-                for (int i = 1; i < kSliceWarps; ++i) vmax = fmaxf(vmax, S.red[buf][i]);
+                    for (int i = 1; i < kSliceWarps; ++i) vmax = max_nan(vmax, S.red[buf][i]);
+                    finite = vmax <= 3.402823466e38f;
+                    if (!finite) vmax = 0.f;
+                } else {
+#pragma unroll
+                    for (int i = 1; i < kSliceWarps; ++i) vmax = fmaxf(vmax, S.red[buf][i]);
+                }
                 // six digits: |x| / 2^ex < 1/4, the top digit within 128
                 ex = split::tile_exponent(vmax) + (D == 6 ? 1 : 0);
             }
-            if (leader) S.scale_exp[it & 3] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
+            if (leader) S.scale_exp[it & 3] = (F::kF64 && !finite) ? kNonFiniteTile : ex;
+            if constexpr (kRedoable<F>)
+                if (leader && !finite && sa.redo) S.redo.add(it);
             unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[buf][0][0]);
             // 1D: chunk idx / 4 in phase (idx / 4) % 4
             auto word = [](int idx) {
@@ -1133,6 +1235,9 @@ __global__ void __launch_bounds__(kThreads<F>, 1)
     tc_fence_after();
     if (warp == kWarpTma)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kTmemCols));
+    if constexpr (kRedoable<F>) {
+        if (S.redo.count > 0 && !S.abort) redo_tiles<F, MODE>(sa, out, m, n, ld, tiles_x, tiles, S);
+    }
 }
 
 template <class F, bool BATCH, int MODE = kModeGrid, bool ODD = false>
@@ -1146,11 +1251,11 @@ cudaError_t set_smem_attr()
 template <class F, int MODE = kModeGrid, bool ODD = false>
 cudaError_t launch_tc(const GridView &g, const typename F::Digits &digits, long long origin, long long elements,
                       const void *in_base, void *out_base, const WaitCfg &wc, cudaStream_t st,
-                      const StepArgs<F> &sa = StepArgs<F>{})
+                      const StepArgs<F, MODE> &sa = StepArgs<F, MODE>{})
 {
     const long long ld = g.pitch[0];
     CUtensorMap map = {};
-    StepArgs<F> args = sa;
+    StepArgs<F, MODE> args = sa;
     cudaError_t e = cudaSuccess;
     // The maps copy 8-byte points whatever they hold ((hi, lo) pairs or FP64).
     const float2 *points = reinterpret_cast<const float2 *>(in_base);
@@ -1223,7 +1328,7 @@ cudaError_t launch_batch(const void *records, int ngrids, int total, const WaitC
     return launch_programmatic(k2d_tc<F, true>, grid, kThreads<F>, sizeof(Smem<F>) + 128, st, unused,
                                static_cast<typename F::Out *>(nullptr), 0, 0, 0LL, 0, total, 0, 0,
                                typename F::Digits{}, wc, reinterpret_cast<const TcGrid<F> *>(records), ngrids,
-                               StepArgs<F>{});
+                               StepArgs<F, kModeGrid>{});
 }
 
 split::SliceWeights split_digits(const Weights &w) { return split::slice_weights(w); }
@@ -1240,18 +1345,21 @@ cudaError_t launch_split_sweep_tc(const GridView &g, const Weights &w, long long
 }
 
 cudaError_t launch_fp64_sweep_tc(const GridView &g, const Weights &w, long long origin, long long elements,
-                                 const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st, int radius,
-                                 long long above, long long below, bool fine)
+                                 const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st,
+                                 const TcForm *form)
 {
     const WaitCfg wc{wt.limit_ns, wt.skip_loads};
-    if (radius == 0 && !fine) return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base, wc, st);
+    if (!form) return launch_tc<FmtF64>(g, f64_slice_weights(w), origin, elements, in_base, out_base, wc, st);
     const F64Weights digits = f64_slice_weights(w, 49, &tap_order(Taps::kSquare7));
-    if (radius == 0) return launch_tc<FmtF64Fine>(g, digits, origin, elements, in_base, out_base, wc, st);
-    StepArgs<FmtF64Fine> sa{};
+    StepArgs<FmtF64Fine, kModeGrid> sa{};
     sa.in = in_base + origin;
-    sa.radius = radius;
-    sa.above = (int)std::min(above, 3LL);
-    sa.below = (int)std::min(below, 3LL);
+    sa.radius = form->radius;
+    sa.above = (int)std::min(form->above, 3LL);
+    sa.below = (int)std::min(form->below, 3LL);
+    sa.pattern = form->pattern;
+    sa.redo = form->redo;
+    for (int i = 0; i < 49; ++i) sa.w[i] = w.v[i];
+    if (!form->odd) return launch_tc<FmtF64Fine>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
     return launch_tc<FmtF64Fine, kModeGrid, true>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
 }
 
@@ -1267,10 +1375,10 @@ inline float2 step_weight(double w, float2)
 template <class F>
 cudaError_t launch_steps_2d(const GridView &g, const Weights &wT, const Weights &w3x3, int steps, long long origin,
                             long long elements, const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st,
-                            bool tma)
+                            const TcForm &form)
 {
     using Out = typename F::Out;
-    StepArgs<F> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, 1, 0, 0u, 0, {}};
+    StepArgs<F, kModeSteps> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, 1, 0, 0u, 0, {}};
     // The frame's strips go to the CTAs that have no tile in the last round,
     // or to all CTAs where that is sooner. A strip keeps one of an SM's four
     // FP64 pipes for about 9,000 cycles; an epilogue warp is idle that long
@@ -1284,18 +1392,20 @@ cudaError_t launch_steps_2d(const GridView &g, const Weights &wT, const Weights 
     if (extra > 0 && 9000 * rounds(ctas - extra) - 6500 < 9000 * rounds(ctas)) sa.frame_cta = (int)extra;
     for (int t = 0; t < 9; ++t) {
         sa.w[t] = step_weight(w3x3.v[t], Out{});
-        if (w3x3.v[t] != 0.0) sa.taps |= 1u << t;
+        if (form.pattern == PAT_DENSE || t / 3 == 1 || t % 3 == 1) sa.taps |= 1u << t;
     }
+    sa.pattern = form.pattern;
+    sa.redo = form.redo;
     const F64Weights digits = f64_slice_weights(wT, 49, &tap_order(Taps::kSquare7));
     const WaitCfg wc{wt.limit_ns, wt.skip_loads};
     if constexpr (F::kF64)
-        if (!tma) return launch_tc<F, kModeSteps, true>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
+        if (form.odd) return launch_tc<F, kModeSteps, true>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
     return launch_tc<F, kModeSteps>(g, digits, origin, elements, in_base, out_base, wc, st, sa);
 }
 
 template <class F>
 cudaError_t launch_steps_1d(long long n, const double *taps, int radius, const double *w, int steps, long long origin,
-                            const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st)
+                            const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st, bool redo)
 {
     using Out = typename F::Out;
     if (steps < 1 || steps * radius > kReach1d || n < 64) return cudaErrorInvalidValue;
@@ -1303,10 +1413,11 @@ cudaError_t launch_steps_1d(long long n, const double *taps, int radius, const d
     if (e != cudaSuccess) return e;
     Weights wT;
     for (int i = 0; i < 49; ++i) wT.v[i] = taps[i];
-    StepArgs<F> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, radius, 0, 0u, 0, {}};
+    StepArgs<F, kMode1d> sa{reinterpret_cast<const Out *>(in_base) + origin, steps, radius, 0, 0u, 0, {}};
     sa.aligned = origin % 2 == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0 &&
                  reinterpret_cast<uintptr_t>(out_base) % 16 == 0;
     for (int t = 0; t <= 2 * radius; ++t) sa.w[t] = step_weight(w[t], Out{});
+    sa.redo = redo;
     CUtensorMap unused;
     std::memset(&unused, 0, sizeof unused);
     const int tiles = (int)((n + kOut1d - 1) / kOut1d);
@@ -1321,18 +1432,18 @@ cudaError_t launch_steps_1d(long long n, const double *taps, int radius, const d
 
 cudaError_t launch_steps_tc(bool fp64, const GridView &g, const Weights &wT, const Weights &w3x3, int steps,
                             long long origin, long long elements, const void *in_base, void *out_base,
-                            const TcWait &wt, cudaStream_t st, bool tma)
+                            const TcWait &wt, cudaStream_t st, const TcForm &form)
 {
-    return fp64 ? launch_steps_2d<FmtF64Fine>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, tma)
-                : launch_steps_2d<FmtSplit6>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, true);
+    return fp64 ? launch_steps_2d<FmtF64Fine>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, form)
+                : launch_steps_2d<FmtSplit6>(g, wT, w3x3, steps, origin, elements, in_base, out_base, wt, st, form);
 }
 
 cudaError_t launch_steps_tc_1d(bool fp64, long long n, const double *taps, int radius, const double *w, int steps,
                                long long origin, const void *in_base, void *out_base, const TcWait &wt,
-                               cudaStream_t st)
+                               cudaStream_t st, bool redo)
 {
-    return fp64 ? launch_steps_1d<FmtF64Fine>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st)
-                : launch_steps_1d<FmtSplit6>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st);
+    return fp64 ? launch_steps_1d<FmtF64Fine>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st, redo)
+                : launch_steps_1d<FmtSplit6>(n, taps, radius, w, steps, origin, in_base, out_base, wt, st, redo);
 }
 
 size_t tc_batch_record_bytes(bool fp64) { return fp64 ? sizeof(TcGrid<FmtF64>) : sizeof(TcGrid<FmtSplit>); }

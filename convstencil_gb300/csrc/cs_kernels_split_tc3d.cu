@@ -56,6 +56,7 @@
 #include "cs_tc_f64.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cs {
 
@@ -81,12 +82,21 @@ using namespace tc;
 // (1277), all three parts loaded first with 112 registers for the epilogue by
 // setmaxnreg (1287; split 826 against 738), sixteen epilogue warps (1171 against
 // 1126), two planes per loop iteration (930 against 897, spills).
+// Again: what computes an output again (Redo).
+struct NoAgain {
+};
+struct SumAgain {
+    const double *in;  // interior point (0, 0, 0) of the source
+    int pattern, redo;
+    double w[27];
+};
 struct F3Split {
     static constexpr bool kF64 = false;
     static constexpr int D = split::kDigits, LV = D;  // 5
     static constexpr int NBLK = 4, kBlk = 128;
     using Out = float2;
     using Digits = SliceWeights;
+    using Again = NoAgain;
 };
 struct F3F64 {
     static constexpr bool kF64 = true;
@@ -94,6 +104,7 @@ struct F3F64 {
     static constexpr int NBLK = 3, kBlk = 160;
     using Out = double;
     using Digits = F64Weights;
+    using Again = NoAgain;
 };
 // FP64 with level 6 too, inputs rounded to even and the weights' sum kept, as
 // the 2D kernel's FmtF64Fine: errors no larger than those of FP64 FMA sweeps
@@ -103,6 +114,7 @@ struct F3F64 {
 // the server keeps it on those).
 struct F3F64Fine : F3F64 {
     static constexpr int LV = 7, kBlk = 168;
+    using Again = SumAgain;
 };
 
 // Warp roles. Warp w issues from the SM's scheduler w % 4, and an epilogue
@@ -177,6 +189,7 @@ struct Smem {
     int scale_exp[kScaleRing];                 // input-plane scale exponents by plane sequence
     float red[kGroups][2][kGroupWarps];           // split: per-warp max |hi|
     int redi[kGroups][2][kGroupWarps];            // FP64: per-warp max biased exponent
+    std::conditional_t<F::LV == 7, Redo, NoRedo> redo;  // input planes that hold an Inf or NaN
 };
 static_assert(sizeof(Smem<F3F64Fine>) + 128 <= 232448 && sizeof(Smem<F3Split>) + 128 <= 232448,
               "shared memory of one CTA must stay within 227 KB");
@@ -246,14 +259,6 @@ __device__ __forceinline__ void tmem_ld4(unsigned taddr, float (&v)[4])
     for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// The larger, or NaN where one is.
-__device__ __forceinline__ float max_nan(float a, float b)
-{
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
 // Recombines five exact level sums (level L in units of 2^-9L) into a
 // double-float pair.
 __device__ __forceinline__ void recombine(const float (&acc)[split::kDigits], float &hi, float &lo)
@@ -269,7 +274,7 @@ template <class F>
 __global__ void __launch_bounds__(kThreads, 1)
     k3d_tc(const __grid_constant__ CUtensorMap tmap, typename F::Out *__restrict__ out, int h, int m, int n,
            long long ldy, long long ldz, int tiles_x, int tiles_y, int zc, int items, int map_x, int map_y,
-           int map_z, typename F::Digits sw, WaitCfg wc)
+           int map_z, typename F::Digits sw, WaitCfg wc, const __grid_constant__ typename F::Again again)
 {
     constexpr int D = F::D, NBLK = F::NBLK, NCOL = kNcol<F>;
     extern __shared__ unsigned char smem_raw[];
@@ -300,6 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(bar(S.blk_empty, i), kEpiWarps);
         }
         S.abort = 0;
+        if constexpr (F::LV == 7) S.redo.count = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kWarpTma) {
@@ -464,6 +470,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                     ex = split::tile_exponent(vmax);
                 }
                 if (leader) S.scale_exp[(unsigned)q % kScaleRing] = (F::kF64 && ex == 2047) ? kNonFiniteTile : ex;
+                if constexpr (F::LV == 7)
+                    if (leader && ex == 2047 && again.redo) S.redo.add(q);
                 unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[slot][0][0]);
                 if constexpr (F::kF64) {
                     if (ex >= kFastExp) {
@@ -905,6 +913,24 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     if (warp == kWarpTma)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kTmemCols));
+    if constexpr (F::LV == 7) {
+        if (S.redo.count > 0 && !S.abort) {  // output planes j with an Inf or NaN in their three input planes
+            int q = 0;
+            for (int item = first; item < items; item += step) {
+                const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
+                for (int j = 0; j < wi.zn; ++j) {
+                    if (!S.redo.holds(q + j, q + j + 2)) continue;
+                    for (int i = tid; i < TX * TY; i += kThreads) {
+                        const int y = wi.y0 + i / TX, x = wi.x0 + i % TX;
+                        const long long at = (long long)(wi.zs + j) * ldz + (long long)y * ldy + x;
+                        if (y < m && x < n)
+                            out[at] = fma_sum_3d<1>(again.in + at, ldy, ldz, again.w, again.pattern);
+                    }
+                }
+                q += wi.zn + 2;
+            }
+        }
+    }
 }
 
 }  // namespace
@@ -921,7 +947,8 @@ namespace {
 
 template <class F>
 cudaError_t launch_tc3d(const GridView &g, const typename F::Digits &digits, long long origin, long long elements,
-                        const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st)
+                        const void *in_base, void *out_base, const TcWait &wt, cudaStream_t st,
+                        const typename F::Again &again = typename F::Again{})
 {
     const long long ldy = g.pitch[1], ldz = g.pitch[0];
     CUtensorMap map;
@@ -953,7 +980,7 @@ cudaError_t launch_tc3d(const GridView &g, const typename F::Digits &digits, lon
     return launch_programmatic(k3d_tc<F>, grid, kThreads, smem, st, map,
                                reinterpret_cast<typename F::Out *>(out_base) + origin, h, m, n, ldy, ldz, tiles_x,
                                tiles_y, zc, items, (int)(origin % ldy), (int)((origin % ldz) / ldy),
-                               (int)(origin / ldz), digits, WaitCfg{wt.limit_ns, wt.skip_loads});
+                               (int)(origin / ldz), digits, WaitCfg{wt.limit_ns, wt.skip_loads}, again);
 }
 
 }  // namespace
@@ -966,9 +993,15 @@ cudaError_t launch_split_sweep_tc3d(const GridView &g, const Weights &w, long lo
 }
 
 cudaError_t launch_fp64_sweep_tc3d(const GridView &g, const Weights &w, long long origin, long long elements,
-                                   const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st, bool fine)
+                                   const double *in_base, double *out_base, const TcWait &wt, cudaStream_t st,
+                                   const TcForm *form)
 {
-    if (fine) return launch_tc3d<F3F64Fine>(g, f64_slice_weights(w, 27, &tap_order(Taps::kCube3)), origin, elements, in_base, out_base, wt, st);
+    if (form) {
+        SumAgain again{in_base + origin, form->pattern, form->redo, {}};
+        for (int i = 0; i < 27; ++i) again.w[i] = w.v[i];
+        return launch_tc3d<F3F64Fine>(g, f64_slice_weights(w, 27, &tap_order(Taps::kCube3)), origin, elements, in_base,
+                                      out_base, wt, st, again);
+    }
     return launch_tc3d<F3F64>(g, f64_slice_weights(w, 27), origin, elements, in_base, out_base, wt, st);
 }
 

@@ -73,6 +73,8 @@ struct Weights7 {
     __half d[D][TAPS];
     int ew;
     float rest;  // what the digits' sum lacks (f64_combine)
+    int pattern, redo;
+    double w[TAPS];  // the weights themselves (Redo)
 };
 
 constexpr int kGroups = 2, kGroupWarps = 4, kGroupThreads = 32 * kGroupWarps;
@@ -119,6 +121,7 @@ struct Smem {
     int abort;
     int scale_exp[kScaleRing];
     int redi[kGroups][2][kGroupWarps];
+    Redo redo;                               // input planes that hold an Inf or NaN
 };
 static_assert(sizeof(Smem) + 128 <= 232448, "shared memory of one CTA must stay within 227 KB");
 static_assert(D * 49 * kWz * 2 <= (int)sizeof(Smem::planes), "the staged weights fit the digit planes");
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_init(bar(S.blk_empty, i), kEpiWarps);
         }
         S.abort = 0;
+        S.redo.count = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kWarpTma) {
@@ -363,7 +367,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                 int ex = 1;
 #pragma unroll
                 for (int i = 0; i < kGroupWarps; ++i) ex = max(ex, S.redi[grp][set][i]);
-                if (leader) S.scale_exp[q % kScaleRing] = ex == 2047 ? kNonFiniteTile : ex;
+                if (leader) {
+                    S.scale_exp[q % kScaleRing] = ex == 2047 ? kNonFiniteTile : ex;
+                    if (ex == 2047 && sw.redo) S.redo.add(q);
+                }
                 unsigned *dst0 = reinterpret_cast<unsigned *>(&S.planes[slot][0][0]);
                 if (ex >= kFastExp) {
 #pragma unroll
@@ -501,15 +508,33 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     if (warp == kWarpTma)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kTmemCols));
+    if (S.redo.count > 0 && !S.abort) {  // output planes j with an Inf or NaN in their seven input planes
+        int q = 0;
+        for (int item = first; item < items; item += step) {
+            const Item wi = item_of(item, tiles_x, tiles_y, zc, h);
+            for (int j = 0; j < wi.zn; ++j) {
+                if (!S.redo.holds(q + j, q + j + 6)) continue;
+                for (int i = tid; i < TX * TY; i += kThreads) {
+                    const int y = wi.y0 + i / TX, x = wi.x0 + i % TX;
+                    const long long at = (long long)(wi.zs + j) * ldz + (long long)y * ldy + x;
+                    if (y < m && x < n) out[at] = fma_sum_3d<3>(in + at, ldy, ldz, sw.w, sw.pattern);
+                }
+            }
+            q += wi.zn + 6;
+        }
+    }
 }
 
 // Digits of the 343 weights: as f64_slice_weights with the sum and the moments
 // kept, and a scale that also holds sum |w| / 2^ew to 16. (The sum alone kept, each
 // error carried on to the next tap, and level 5 cut off at T's unit: 40 sweeps of
 // the octahedron, smooth data, erred by 3.2e-16 of the norm, FP64 FMA by 2.3e-16.)
-Weights7 slice_weights7(const Weights &w)
+Weights7 slice_weights7(const Weights &w, const TcForm &form)
 {
     Weights7 s{};
+    s.pattern = form.pattern;
+    s.redo = form.redo;
+    for (int i = 0; i < TAPS; ++i) s.w[i] = w.v[i];
     double mx = 0.0, sum = 0.0;
     for (int i = 0; i < TAPS; ++i) mx = std::fmax(mx, std::fabs(w.v[i]));
     int e = 0;
@@ -544,8 +569,8 @@ Weights7 slice_weights7(const Weights &w)
 }  // namespace
 
 cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long long origin, long long elements,
-                                      const double *in_base, double *out_base, bool rows_whole, const TcWait &wt,
-                                      cudaStream_t st)
+                                      const double *in_base, double *out_base, bool rows_whole, const TcForm &form,
+                                      const TcWait &wt, cudaStream_t st)
 {
     const long long ldy = g.pitch[1], ldz = g.pitch[0];
     const bool tma = rows_whole && ldy % 2 == 0 && ldz % ldy == 0 && reinterpret_cast<uintptr_t>(in_base) % 16 == 0;
@@ -583,7 +608,7 @@ cudaError_t launch_fp64_sweep_tc3d_r3(const GridView &g, const Weights &w, long 
     note_launch();
     return launch_programmatic(kernel, std::min(items, sms), kThreads, smem, st, map, in_base + origin,
                                out_base + origin, h, m, n, ldy, ldz, tiles_x, tiles_y, zc, items, map_x,
-                               (int)((origin % ldz) / ldy), (int)(origin / ldz), left, vec2 ? 1 : 0, slice_weights7(w),
+                               (int)((origin % ldz) / ldy), (int)(origin / ldz), left, vec2 ? 1 : 0, slice_weights7(w, form),
                                WaitCfg{wt.limit_ns, wt.skip_loads}, timeouts);
 }
 

@@ -615,8 +615,9 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
                  ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64) >= 64;
         // A client cannot ask for FP64 FMA sums: only 7x7 kernels of at least four
         // 64 x 64 tiles per SM run on the kernel whose error is larger.
-        const long long tiles = in3d || in1d ? 0 : ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64);
-        r->sweeps_per_launch = cs::plan_fix_fp64(r->plan, tc, tiles < 4LL * s->sm_count);
+        const bool r3_2d = !in3d && !in1d && (fused || d->shape == CS_SHAPE_BOX2D3R || d->shape == CS_SHAPE_STAR2D3R);
+        const bool many = ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64) >= 4LL * s->sm_count;
+        r->sweeps_per_launch = cs::plan_fix_fp64(r->plan, tc, !(r3_2d && many));
     }
     // The FP64 FMA 2D kernel's tile rows: fixed here (the plan tuner would
     // time both on the worker thread); results do not depend on them.

@@ -245,6 +245,65 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap *map
         : "memory");
 }
 
+// The larger, or NaN where one is.
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// Work of a CTA (tiles, or input planes, numbered in its order) whose window
+// held an Inf or a NaN. Digits cannot hold one, so the outputs are computed
+// again after the rest, with the plan's own weights one by one as the kernels
+// without digits do: a point that is not finite then reaches the outputs that
+// read it and no other. Lies in shared memory; work is added by the slicers'
+// leaders, who look at its scale. (Cost on finite grids, GB300, us a solve:
+// star2d1r 1024^2 x 100 481.6 and 486.7, box2d1r 2047 x 1531 x 60 525 and 529, 1d2r
+// 10,240,000 x 100 562.5 and 563.7, fused box3d1r none; noted by the epilogue
+// instead 485, 536, 574.)
+struct NoRedo {
+};
+struct Redo {
+    static constexpr int kMost = 64;
+    int count, item[kMost];
+    __device__ __forceinline__ void add(int i)
+    {
+        const int k = atomicAdd(&count, 1);
+        if (k < kMost) item[k] = i;
+    }
+    // Whether one of lo .. hi is in it (more than it holds: any may be).
+    __device__ __forceinline__ bool holds(int lo, int hi) const
+    {
+        if (count > kMost) return true;
+        for (int k = 0; k < count; ++k)
+            if (item[k] >= lo && item[k] <= hi) return true;
+        return false;
+    }
+};
+
+// Whether a tap at these offsets belongs to a kernel's pattern of radius r.
+__device__ __forceinline__ bool in_pattern(int pattern, int dz, int dy, int dx, int r)
+{
+    return pattern == PAT_DENSE  ? true
+           : pattern == PAT_STAR ? (dz != 0) + (dy != 0) + (dx != 0) <= 1
+                                 : abs(dz) + abs(dy) + abs(dx) <= r;
+}
+
+// FP64 FMA sum of a (2r+1)^3 kernel's pattern at one point of a grid.
+template <int R>
+__device__ __forceinline__ double fma_sum_3d(const double *__restrict__ at, long long ldy, long long ldz,
+                                             const double *w, int pattern)
+{
+    constexpr int K = 2 * R + 1;
+    double v = 0.0;
+    for (int t = 0; t < K * K * K; ++t) {
+        const int dz = t / (K * K) - R, dy = t / K % K - R, dx = t % K - R;
+        if (in_pattern(pattern, dz, dy, dx, R)) v = fma(w[t], at[dz * ldz + dy * ldy + dx], v);
+    }
+    return v;
+}
+
 // Untiled bulk copy: 16-byte aligned addresses, a multiple of 16 bytes.
 __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar)
 {
