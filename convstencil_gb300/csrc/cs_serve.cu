@@ -246,15 +246,20 @@ void advance(cs_server *s, Request *r)
     }
     // Chunks are whole fused sweeps: a multiple of the plan's steps per sweep.
     // For plans that take several sweeps per launch also whole launches, so
-    // the launches do not depend on the chunk length.
+    // the launches do not depend on the chunk length; a single sweep left over,
+    // which run_from takes first, is the first chunk's.
     const long long unit = r->sweeps_per_step * r->sweeps_per_launch;
     const long long full = std::max(1LL, s->cfg.chunk_steps / unit) * unit;
+    auto next_chunk = [&] {
+        const bool single = r->issued == 0 && r->sweeps_per_launch > 1 && r->steps % unit == r->sweeps_per_step;
+        return std::min(full + (single ? r->sweeps_per_step : 0), r->steps - r->issued);
+    };
     if (r->small) {
         // All chunks now, back to back on the request's high-priority stream:
         // the same kernels and re-anchoring points as chunk-by-chunk issue,
         // without a scheduling turn between chunks.
         while (r->issued < r->steps) {
-            const long long chunk = std::min(full, r->steps - r->issued);
+            const long long chunk = next_chunk();
             const cs_status st = issue_steps(r, chunk);
             if (st != CS_OK) {
                 fail_request(s, r, st, cs_last_error());
@@ -265,7 +270,7 @@ void advance(cs_server *s, Request *r)
         finish_request(r);
         return;
     }
-    const long long chunk = std::min(full, r->steps - r->issued);
+    const long long chunk = next_chunk();
     cs_status st = CS_OK;
     const bool graphable = s->cfg.use_graphs && chunk == full &&
                            (chunk / r->sweeps_per_step) % 2 == 0 && r->prec == CS_PREC_FP64 &&
