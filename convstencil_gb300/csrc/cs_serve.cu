@@ -467,30 +467,30 @@ void worker_main(cs_server *s)
     }
 }
 
-// Packs a dense interior (row-major) into the plan's layout, zero halo.
 // fn(lo, hi) over [0, n) in up to `most` threads, the caller's among them. A
-// thread that cannot be started leaves its part to the caller.
+// thread that cannot be started leaves its part to the caller. fn throws
+// nothing: out of a thread that would end the process.
 template <class Fn>
 void in_threads(long long n, long long most, const Fn &fn)
 {
     const long long t = std::max(1LL, std::min({n, most, 8LL, (long long)std::thread::hardware_concurrency()}));
-    std::vector<std::thread> ths;
-    long long own = n / t;  // the caller's share; a failed thread's is added
-    std::vector<std::pair<long long, long long>> left;
-    for (long long i = 1; i < t; ++i) {
-        const long long lo = n * i / t, hi = n * (i + 1) / t;
-        try {
-            ths.emplace_back([&fn, lo, hi] { fn(lo, hi); });
-        } catch (...) {
-            left.push_back({lo, hi});
+    std::thread ths[8];
+    long long started = 1;
+    try {
+        for (; started < t; ++started) {
+            const long long lo = n * started / t, hi = n * (started + 1) / t;
+            ths[started] = std::thread([&fn, lo, hi] { fn(lo, hi); });
         }
+    } catch (...) {  // from here on it is the caller's
     }
-    fn(0, own);
-    for (const auto &p : left) fn(p.first, p.second);
-    for (auto &th : ths) th.join();
+    fn(0, n / t);
+    if (started < t) fn(n * started / t, n);
+    for (auto &th : ths)
+        if (th.joinable()) th.join();
 }
 
-// The rows of a layout between a dense interior and a padded buffer. Grids
+// The rows of a layout between a dense interior (row-major) and a padded buffer,
+// whose halo pack() zeroes. Grids
 // above a few MB are copied by several threads: one moves 8 GB/s (result
 // arrays also take their page faults here), the link to the GPU 200.
 long long row_offset(const cs_layout &L, long long r)
@@ -748,8 +748,12 @@ CS_API cs_status cs_server_submit_many(cs_server *s, const cs_request_desc *reqs
                    cudaGetDevice(&own);
                    if (own != s->device) cudaSetDevice(s->device);
                    for (int i; (i = next.fetch_add(1)) < count;) {
-                       sts[i] = prepare_request(s, &reqs[i], rs[i], 1);
-                       if (sts[i] != CS_OK) errs[i] = cs_last_error();
+                       try {
+                           sts[i] = prepare_request(s, &reqs[i], rs[i], 1);
+                           if (sts[i] != CS_OK) errs[i] = cs_last_error();
+                       } catch (...) {
+                           sts[i] = CS_ERR_OUT_OF_MEMORY;
+                       }
                    }
                    if (own != s->device) cudaSetDevice(own);
                });
