@@ -38,6 +38,7 @@ struct GridView {
 // tile_rows (2D only): 16 or 32 rows per CTA tile of 64 columns, kSmallTile =
 // 16 rows of 8 columns, 0 = by grid size.
 constexpr int kSmallTile = -16;
+int fp64_tile_rows(const GridView &g);  // that choice
 cudaError_t launch_fp64_fma(const GridView &g, int radius, int pattern, const Weights &w,
                             const double *in, double *out, cudaStream_t stream, int tile_rows = 0);
 // FP64 tensor-core path (mma.sync m8n8k4.f64), 2D radius-3 dense kernels only.

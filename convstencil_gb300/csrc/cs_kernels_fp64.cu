@@ -19,13 +19,28 @@
 //    point. Still more FP64 work than the FMA form (49 per point), so the
 //    plan's tuner only picks it if it measures faster.
 //
-// Grids of at most one CTA per SM are launched with the programmatic stream
-// serialization attribute: the CTAs are scheduled while the previous sweep
-// finishes and wait for it (pdl_wait) before their first access. Larger ones
-// are not: scheduled among the previous sweep's CTAs they spread unevenly over
-// the SMs (box2d3r 192^2 on 288 small tiles, GB300: 9.5 us a sweep against
-// 6.1), except the small tiles of radius 1, whose FP64 work is short (star2d1r
-// 384^2, 1152 of them: 3.8 us against 5.3).
+// Grids of few CTAs are launched with the programmatic stream serialization
+// attribute: the CTAs are scheduled while the previous sweep finishes and wait
+// for it (pdl_wait) before their first access. Scheduled among the previous
+// sweep's CTAs they spread unevenly over the SMs, though, and two on one SM
+// share its FP64 pipes, so each kernel has its own limit (GB300, us a sweep with
+// launches one by one / in a graph, without and with the attribute):
+//   * 64-column tiles, 1D and radius-3 3D: a CTA for every fourth SM. 1d1r of
+//     32 CTAs 4.1 / 2.7 and 3.1 / 2.7, of 64 4.1 / 2.7 and 4.2 / 2.8, of 128 4.1 /
+//     2.7 and 7.1 / 3.6; box2d3r 384^2 of 144 18.5 / 17.2 and 17.4 / 36; fused box3d1r
+//     32^3 of 64 61 / 59 and 60 / 75. Not 32-row tiles of radius 3 (star2d3r 128^2
+//     12.3 / 10.9 and 11.5 / 11.6).
+//   * small 2D tiles: radius 1 three for two SMs (box2d1r 128^2, 128 CTAs, 4.1 / 2.3
+//     and 2.8 / 2.1; 192 x 200, 300, 4.1 / 2.6 and 4.1 / 3.1), the star two per SM
+//     (192^2, 288, 4.1 / 2.3 and 2.7 / 2.4; 240^2, 450, 4.1 / 2.5 and 4.4 / 3.2), or five
+//     and more (box2d1r 320^2, 800, 6.2 / 4.0 and 4.1 / 3.9); dense radius 3 seven for
+//     ten SMs (box2d3r 96 x 130, 102 CTAs, 6.2 / 3.8 and 4.4 to 5.4 / 3.9; 144 x 128,
+//     144, 6.2 / 3.7 and 6.1 to 8.5 / 4.3), other radius 3 one (star2d3r 128^2 4.1 /
+//     2.4 and 3.6 / 2.3; 128 x 160, 160, 4.1 / 2.7 and 4.4 / 2.7).
+//   * 3D radius 1: the star always (32^3 4.1 / 2.1 and 2.5 / 1.9, 64^3 8.2 / 5.3 and
+//     5.5 / 5.3), the box one for every second SM (24^3, 144 CTAs, 4.1 / 2.7 and
+//     8.0 / 2.5; 32^3, 256, 6.2 / 3.6 and 10.3 / 5.1; 60^3, 1800, 16.4 / 13.7 and 17.3 /
+//     16.9) or twelve and more (68^3 27.6 / 25.4 and 25.3 / 25.2).
 #include "cs_internal.h"
 #include "cs_tc_common.cuh"
 
@@ -238,7 +253,7 @@ __global__ void __launch_bounds__(256) k3d_fma(const double *__restrict__ in,
 // Radius 1: an output a thread and no shared memory. Its 7 or 27 loads are all
 // in flight together, where the march above waits for a plane at a time; the
 // neighbours' come from L1. On large grids both are bound by the FP64 pipes, so
-// this one takes every size, overlapped with the previous sweep's end. (GB300, us a
+// this one takes every size. (GB300, us a
 // sweep, the march and this: 7 points 32^3 5.9 and 2.5, 64^3 10.5 and 5.9, 128^3 39.1
 // and 30.0, 256^3 274 and 227; 27 points 8.7 and 5.6, 22.7 and 16.3, 123 and 111,
 // 933 and 863. Two and four planes a thread are no faster on large grids and
@@ -334,12 +349,18 @@ WK<K> pack(const Weights &w)
 
 unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
-// Overlapping the previous sweep's end (`always`, or at most one CTA per SM).
+// Overlapping the previous sweep's end where at most `most` of the SMs get a CTA,
+// or all of them `many` CTAs and more (0: not so; see the head of this file).
+struct Overlap {
+    double most;
+    int many = 0;
+};
 template <typename... Exp, typename... Act>
-cudaError_t launch(bool always, void (*kernel)(Exp...), dim3 grid, int block, size_t smem, cudaStream_t st,
+cudaError_t launch(Overlap o, void (*kernel)(Exp...), dim3 grid, int block, size_t smem, cudaStream_t st,
                    Act &&...args)
 {
-    const bool overlap = always || (long long)grid.x * grid.y * grid.z <= device_sm_count();
+    const double ctas = (double)grid.x * grid.y * grid.z, sms = device_sm_count();
+    const bool overlap = ctas <= o.most * sms || (o.many > 0 && ctas >= o.many * sms);
     return tc::launch_overlapped(overlap, kernel, grid, block, smem, st, std::forward<Act>(args)...);
 }
 
@@ -357,34 +378,34 @@ int z_chunk(const GridView &g)
 
 
 // Rows per CTA tile: 16 (4 per thread) or 32 (8 per thread) of 64 columns, or
-// kSmallTile: 16 of 8 columns; 0 picks that up to 2^18 points and 16 on grids
-// too small to give every SM several 32-row tiles. All tile shapes sum every point's taps in the
-// same order, so results do not depend on it.
+// kSmallTile: 16 of 8 columns; 0 by size (fp64_tile_rows). All tile shapes sum
+// every point's taps in the same order, so results do not depend on it.
 template <int R, int P>
 cudaError_t go2d(const GridView &g, const Weights &w, const double *in, double *out, int tile_rows,
                  cudaStream_t st)
 {
     constexpr int K = 2 * R + 1;
     const unsigned gx = ceil_div(g.ext[1], 64);
-    if (tile_rows == 0 && g.ext[0] * g.ext[1] <= 1 << 18) tile_rows = kSmallTile;
-    if (tile_rows == 0) tile_rows = (long long)gx * ceil_div(g.ext[0], 32) < 6LL * device_sm_count() ? 16 : 32;
+    if (tile_rows == 0) tile_rows = fp64_tile_rows(g);
     const int m = (int)g.ext[0], n = (int)g.ext[1];
     if (tile_rows == kSmallTile)
-        return launch(R == 1, k2d_fma_small<R, P>, dim3(ceil_div(n, 8), ceil_div(m, 16)), 128, 0, st, in, out,
-                                       m, n, g.pitch[0], pack<K * K>(w));
+        return launch(R == 1 ? Overlap{P == PAT_STAR ? 2.0 : 1.5, 5} : Overlap{P == PAT_DENSE ? 0.7 : 1.0},
+                      k2d_fma_small<R, P>,
+                      dim3(ceil_div(n, 8), ceil_div(m, 16)), 128, 0, st, in, out, m, n, g.pitch[0], pack<K * K>(w));
     if (tile_rows == 16)
-        return launch(false, k2d_fma<R, P, 4>, dim3(gx, ceil_div(m, 16)), 256, 0, st, in, out, m, n,
-                                       g.pitch[0], pack<K * K>(w));
-    return launch(false, k2d_fma<R, P, 8>, dim3(gx, ceil_div(m, 32)), 256, 0, st, in, out, m, n, g.pitch[0],
-                                   pack<K * K>(w));
+        return launch(Overlap{0.25}, k2d_fma<R, P, 4>, dim3(gx, ceil_div(m, 16)), 256, 0, st, in, out, m, n, g.pitch[0],
+                      pack<K * K>(w));
+    return launch(Overlap{R == 3 ? 0.0 : 0.25}, k2d_fma<R, P, 8>, dim3(gx, ceil_div(m, 32)), 256, 0, st, in, out, m, n, g.pitch[0],
+                  pack<K * K>(w));
 }
 
 template <int P>
 cudaError_t go3d_r1(const GridView &g, const Weights &w, const double *in, double *out, cudaStream_t st)
 {
     const unsigned gx = ceil_div(g.ext[2], 32), gy = ceil_div(g.ext[1], 4);
-    return launch(true, k3d_fma1<P>, dim3((unsigned)(g.ext[0] * gx * gy)), 128, 0, st, in, out, (int)g.ext[1],
-                  (int)g.ext[2], g.pitch[1], g.pitch[0], gx, gy, pack<27>(w));
+    return launch(P == PAT_STAR ? Overlap{1e9} : Overlap{0.5, 12}, k3d_fma1<P>,
+                  dim3((unsigned)(g.ext[0] * gx * gy)), 128, 0, st, in, out, (int)g.ext[1], (int)g.ext[2], g.pitch[1],
+                  g.pitch[0], gx, gy, pack<27>(w));
 }
 
 template <int R, int P>
@@ -396,19 +417,27 @@ cudaError_t go3d(const GridView &g, const Weights &w, const double *in, double *
     static_assert(smem <= 48 * 1024, "3D ring exceeds the default shared-memory window");
     const int zc = z_chunk(g);
     dim3 grid(ceil_div(g.ext[2], 32), ceil_div(g.ext[1], 16), ceil_div(g.ext[0], zc));
-    return launch(false, k3d_fma<R, P>, grid, 256, smem, st, in, out, (int)g.ext[0], (int)g.ext[1],
-                                   (int)g.ext[2], g.pitch[1], g.pitch[0], zc, pack<K * K * K>(w));
+    return launch(Overlap{0.25}, k3d_fma<R, P>, grid, 256, smem, st, in, out, (int)g.ext[0], (int)g.ext[1],
+                  (int)g.ext[2], g.pitch[1], g.pitch[0], zc, pack<K * K * K>(w));
 }
 
 template <int R>
 cudaError_t go1d(const GridView &g, const Weights &w, const double *in, double *out,
                  cudaStream_t st)
 {
-    return launch(false, k1d_fma<R>, dim3(ceil_div(g.ext[0], 1024)), 256, 0, st, in, out, g.ext[0],
-                                   pack<2 * R + 1>(w));
+    return launch(Overlap{0.25}, k1d_fma<R>, dim3(ceil_div(g.ext[0], 1024)), 256, 0, st, in, out, g.ext[0],
+                  pack<2 * R + 1>(w));
 }
 
 }  // namespace
+
+// The small tile up to 2^18 points, 16 rows on grids too small to give every SM
+// several 32-row tiles.
+int fp64_tile_rows(const GridView &g)
+{
+    if (g.ext[0] * g.ext[1] <= 1 << 18) return kSmallTile;
+    return (long long)ceil_div(g.ext[1], 64) * ceil_div(g.ext[0], 32) < 6LL * device_sm_count() ? 16 : 32;
+}
 
 bool fp64_fma_supported(int dims, int radius, int pattern)
 {
@@ -463,8 +492,8 @@ cudaError_t launch_fp64_mma_2d(const GridView &g, const Weights &w, const double
 {
     note_launch();
     dim3 grid(ceil_div(g.ext[1], 64), ceil_div(g.ext[0], 32));
-    return launch(false, k2d_mma, grid, 256, 0, st, in, out, (int)g.ext[0], (int)g.ext[1], g.pitch[0],
-                                   pack<49>(w));
+    return launch(Overlap{0.0}, k2d_mma, grid, 256, 0, st, in, out, (int)g.ext[0], (int)g.ext[1], g.pitch[0],
+                  pack<49>(w));
 }
 
 }  // namespace cs
