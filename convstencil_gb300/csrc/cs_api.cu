@@ -246,7 +246,7 @@ struct cs_plan {
     int last_algo = CS_ALGO_AUTO;  // kernel family the last cs_run used
     int time_block = 0;            // split FMA: steps per launch (0 = tuner)
     int last_time_block = 1;
-    int tile_rows = 0;             // FP64 FMA 2D: rows per CTA tile (0 = tuner)
+    int tile_rows = 0;             // FP64 FMA 2D: rows per CTA tile, or kSmallTile (0 = tuner)
     int active_rows = 0;           // the tile rows launches use now (0 = by grid size)
     long long reanchor = 100;
     cs::TcWait wait;               // bounded waits of the tcgen05 kernels
@@ -730,7 +730,7 @@ cs_status choose_tile_rows(cs_plan *p, int algo, const void *a, void *b, cudaStr
 {
     *out = 0;
     if (p->prec != CS_PREC_FP64 || algo != CS_ALGO_FP64_FMA || p->dims != 2) return CS_OK;
-    if (p->tile_rows > 0) {
+    if (p->tile_rows != 0) {
         *out = p->tile_rows;
         return CS_OK;
     }
@@ -1721,6 +1721,7 @@ int plan_fix_fp64(cs_plan *p, bool tc, bool fine)
     tc = tc && (fp64_tc_ok(p) || fp64_tc3d_ok(p) || fp64_tc3d_r3_ok(p) || fp64_tc1d_ok(p));
     p->algo = tc ? CS_ALGO_FP64_TC : CS_ALGO_FP64_FMA;
     p->fine = fine;
+    if (p->dims == 2) p->tile_rows = cs::fp64_tile_rows(p->view);
     return tc ? steps_per_launch(p, nullptr, nullptr) : 1;
 }
 

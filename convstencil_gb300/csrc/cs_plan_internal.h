@@ -22,8 +22,8 @@ struct PlanFacts {
 bool plan_facts(const cs_plan *p, PlanFacts *f);
 cs_status set_error(cs_status s, const char *msg);
 // Pins an FP64 plan's kernel without a timing run: the tcgen05 one (tc) where
-// the plan allows it, else FP64 FMA; fine: with no larger an error than FP64 FMA
-// sweeps. Returns the sweeps a launch takes on 16-byte aligned buffers.
+// the plan allows it, else FP64 FMA (in 2D with the tile of its size); fine: with
+// no larger an error than FP64 FMA sweeps. Returns the sweeps a launch takes on 16-byte aligned buffers.
 int plan_fix_fp64(cs_plan *p, bool tc, bool fine);
 
 // cs_run with the sweeps numbered from first_sweep (so chunked runs take

@@ -615,20 +615,14 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
             tc = pts >= (fused ? (box3d ? 3.2e4 : 2.6e5) : 6e4) && (fused || box3d);
         else if (in1d)
             tc = pts >= 2.6e5;
-        else  // radius 3 any size, radius 1 from 64 tiles
-            tc = fused || d->shape == CS_SHAPE_BOX2D3R || d->shape == CS_SHAPE_STAR2D3R ||
+        else  // fused kernels and box2d3r any size, star2d3r and radius 1 from 64 tiles
+            tc = fused || d->shape == CS_SHAPE_BOX2D3R ||
                  ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64) >= 64;
         // A client cannot ask for FP64 FMA sums: only 7x7 kernels of at least four
         // 64 x 64 tiles per SM run on the kernel whose error is larger.
         const bool r3_2d = !in3d && !in1d && (fused || d->shape == CS_SHAPE_BOX2D3R || d->shape == CS_SHAPE_STAR2D3R);
         const bool many = ((d->extent[0] + 63) / 64) * ((d->extent[1] + 63) / 64) >= 4LL * s->sm_count;
         r->sweeps_per_launch = cs::plan_fix_fp64(r->plan, tc, !(r3_2d && many));
-    }
-    // The FP64 FMA 2D kernel's tile rows: fixed here (the plan tuner would
-    // time both on the worker thread); results do not depend on them.
-    if (d->precision == CS_PREC_FP64 && (d->shape >= CS_SHAPE_STAR2D1R && d->shape <= CS_SHAPE_BOX2D3R)) {
-        const long long t32 = ((d->extent[1] + 63) / 64) * ((d->extent[0] + 31) / 32);
-        cs_plan_set_option(r->plan, CS_OPT_TILE_ROWS, t32 < 6LL * s->sm_count ? 16 : 32);
     }
     long long sweeps1 = 0;
     if (d->semantics == CS_SEM_FUSED) {
