@@ -188,9 +188,8 @@ void native_layout(int dims, int r, const long long *ext, cs_layout &L)
     L.halo = r;
     const long long x0 = round_up(r, 2);  // interior rows start 16-byte aligned
     if (dims == 1) {
-        // at least 4 points of halo before the interior and 60 after it: the
-        // 1D FP64 tcgen05 sweep reads 4 neighbours either side of a row of 64
-        // outputs, as whole 64-point rows of the array from origin - 4
+        // at least 4 points before the interior and 60 after it, as callers who
+        // pin FP64_TC are promised (fp64_tc1d_pin_ok); the kernel needs neither
         const long long h1 = std::max(x0, 4LL);
         L.extent[0] = ext[0];
         L.pitch[0] = 1;
@@ -1246,7 +1245,9 @@ int bands_that_pay(const cs_plan *p, long long sweeps)
     // 3.24 2.79 2.81 2.81 2.97 3.34, x 60 6.77 7.03 7.20 7.38 8.04 9.28; 8192^2 x 20
     // 12.1 9.46 8.83 8.48 8.60 8.90; 2048^2 x 20 0.99 1.15 1.22 1.34 1.56 1.83;
     // box3d1r 512^3 x 10 22.1 16.8 15.6 14.5 14.2 14.3; fused box3d1r 200 x 184 x 192 x
-    // 10 2.56 2.77 2.92 3.08 3.49 3.81.)
+    // 10 2.56 2.77 2.92 3.08 3.49 3.81.) All of that on pinned arrays; pageable ones
+    // are copied by the host, which waits for each copy out: box2d3r 4096^2 x 5
+    // 2.35 ms, x 20 3.8, 8192^2 x 20 13.2.
     constexpr double kLinkRate = 205e3;  // bytes per us each way, pinned host buffers
     const double cut_us = p->dims == 3 && p->radius > 1 ? 20.0 : 6.0;
     const double best = std::sqrt(2.0 * (double)p->layout.bytes / kLinkRate / (cut_us * (double)sweeps));

@@ -75,8 +75,10 @@
 //     the same time.
 //   * Bound: the shared memory that the MMAs read (354 KB of operands a tile
 //     split, 455 KB FP64, at 128 bytes a cycle 2,770 and 3,560 cycles) beside
-//     the slicers' and the TMA unit's ~120 KB. GB300, 8192^2: split 282 us a
-//     sweep, FP64 320, three steps of radius 1 353.
+//     the slicers' and the TMA unit's ~120 KB. That is about 70 % of the cycles
+//     a tile takes (5,400 split); the rest is the roles waiting for each other,
+//     with no unit above 60 %. GB300, 8192^2: split 280 us a sweep, FP64 321, three
+//     steps of radius 1 362.
 //
 // Every mbarrier wait is bounded (WaitCfg, 2 s by default). An expired wait
 // is counted in g_tc_wait_timeouts; the CTA then waits, again bounded, for

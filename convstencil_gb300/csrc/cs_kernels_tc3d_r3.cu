@@ -9,9 +9,11 @@
 // input plane) has level sums below 2^24, exact in FP32 in any order; they
 // combine into one 64-bit integer, and the seven z taps are added as integers
 // relative to the largest plane exponent among them (the weights' scale keeps
-// sum |w| <= 16, so |sum| <= 2^62) and rounded once to FP64. Error: as the 2D
-// kernel's, relative to the largest value of the output's 3D window times the
-// largest weight.
+// sum |w| <= 16, so |sum| <= 2^62) and rounded once to FP64. Error: relative to the
+// largest value of the output's 3D window times the largest weight, and no
+// larger in the norm than that of FP64 FMA sweeps (40 sweeps of 64 x 60 x 66, uniform
+// data: box 1.9e-16, FMA 5.1e-16; octahedron 1.5e-16, 2.2e-16). Planes with an Inf or
+// NaN are computed again (Redo).
 //
 // Mapping (M = 128, K = 16):
 //   * A work item is a column of output tiles, 16 rows x 64 columns on zc
@@ -41,8 +43,9 @@
 //     slicer shares the MMA thread's scheduler. (Eight draining four columns:
 //     7,000 cycles a plane, mostly waiting for their own TMEM loads, longer
 //     than the MMAs.) GB300, box 256^3: 545 us a sweep with lane == 0 and
-//     eight, 466 with elect_one, 398 with sixteen: 42 G outputs/s; the FP64
-//     FMA kernel 1.5 (box), 8.3 (octahedron).
+//     eight, 466 with elect_one, 398 with sixteen, 391 with the second half's
+//     24 columns a level: 43 G outputs/s; the FP64 FMA kernel 1.5 (box), 8.3
+//     (octahedron).
 //   * Windows arrive by TMA where the layout allows it (even pitches,
 //     16-byte aligned base, the halo in whole rows and planes); the window then starts 4 columns left of the
 //     tile, or 3 where the interior's first column is odd, so that its
@@ -393,8 +396,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if ((kEpiMask >> warp) & 1u) {
         // ------------------------------------------------ epilogue
         // Warp w reads TMEM lanes 32 (w % 4) ..; lane -> D row m = (output row
-        // er, block eb); of the two warps of a lane quarter hh = 0, 1 takes
-        // columns 8 eb + 4 hh .. + 3. s[dz] is the running sum of the output
+        // er, block eb); of the four warps of a lane quarter hh = 0 .. 3 takes
+        // columns 8 eb + 2 hh, + 1. s[dz] is the running sum of the output
         // whose z tap dz the current input plane is, in units of its largest
         // plane exponent so far, se[dz] (the same in every thread).
         const int quarter = warp & 3, hh = quarter == 1 ? (warp - 9) >> 2 : warp >> 2;

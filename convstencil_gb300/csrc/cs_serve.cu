@@ -590,12 +590,12 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
     // split box3d1r 64^3 10.5 double-float, 8.0 tcgen05, 96^3 18.7, 13.3 (but its
     // five digits err more than double-float, 1.7e-12 against 1e-14 in the norm
     // after tens of sweeps, so requests below 2e6 points keep that); FP64 7x7
-    // 256^2 18.7 FMA, 9.5 tcgen05 (an FMA tile takes 14 us however few there
-    // are); box3d1r 32^3 5.7, 8.4, 48^3 12.3, 8.9; star2d1r 512^2 6.4, 4.4 (three
-    // steps a launch). star3d1r stays on FP64 FMA, whose seven taps err less
-    // (9.2e-17 of the norm, tcgen05 1.25e-16; 128^3 29.8 and 29.0). The fused
-    // 7x7x7 box costs 343 FMA per point, 171 us at 64^3 against 41; its
-    // octahedron 63, about as long at 64^3.
+    // 256^2 10.3 FMA, 8.8 tcgen05; star2d3r (13 taps) 256^2 6.2, 8.9, 512^2 11.8, 9.6;
+    // box3d1r 32^3 6.2, 11.7, 48^3 12.3, 9.7, 128^3 109, 32; star2d1r 448^2 (FMA) 6.2,
+    // 512^2 (three steps a launch) 4.2. star3d1r stays on FP64 FMA, whose seven
+    // taps err less (9.2e-17 of the norm, tcgen05 1.25e-16). The fused 7x7x7 box
+    // costs 343 FMA per point, 218 us at 64^3 against 37; its octahedron 63, 51
+    // against 37 at 64^3.
     const bool box3d = d->shape == CS_SHAPE_BOX3D1R, in3d = box3d || d->shape == CS_SHAPE_STAR3D1R;
     const bool in1d = d->shape == CS_SHAPE_1D1R || d->shape == CS_SHAPE_1D2R;
     const bool fused = d->semantics == CS_SEM_FUSED;
@@ -651,8 +651,8 @@ cs_status prepare_request(cs_server *s, const cs_request_desc *d, std::unique_pt
         r->small = work < kSmallWork;
     }
     {
-        // Packable: small FP64 requests, 2D (not radius 3: those run tcgen05
-        // alone from four tiles per SM) or 3D, on the FP64 FMA kernels whose
+        // Packable: small FP64 requests, 2D (not radius 3: the batch kernels
+        // run those on tcgen05) or 3D, on the FP64 FMA kernels whose
         // per-point arithmetic and form the batch kernels repeat. Split
         // requests stay alone: their own kernels (temporal blocking in 2D, the
         // z-queue star and packed-pair box in 3D) beat the batch's generic

@@ -65,18 +65,26 @@ typedef enum cs_shape {
 typedef enum cs_semantics { CS_SEM_STEP = 0, CS_SEM_FUSED = 1 } cs_semantics;
 
 /* Arithmetic of the sweep.
- * CS_PREC_FP64 : FP64 grids. FP64 FMA or FP64 MMA arithmetic, or, for 2D
- *                kernels up to 7x7 and 3D radius-1 kernels, the FP64-accurate
- *                tensor-core form (CS_ALGO_FP64_TC) when the tuner measures
- *                it faster: every
+ * CS_PREC_FP64 : FP64 grids. FP64 FMA or FP64 MMA arithmetic, or the
+ *                FP64-accurate tensor-core form (CS_ALGO_FP64_TC) when the
+ *                tuner measures it faster: every
  *                product and level sum is exact, inputs keep 52 bits below
- *                their 64x70 tile's largest value and weights 53 below the
- *                largest weight (relative error per sweep ~1e-16 of the
- *                tile's scale). On 2D radius-1 plans of at least 64 tiles
+ *                their tile's largest value (a window of 64x70 points in 2D,
+ *                4,144 in 1D, one plane's 16x64 tile and its halo in 3D) and
+ *                weights 53 below the largest weight (relative error per sweep
+ *                ~1e-16 of the tile's scale, so a value 2^-k below it keeps
+ *                52 - k bits, where FP64 FMA keeps 53 of each value). On 2D
+ *                radius-1 plans of at least 64 tiles
  *                of 64x64 that form takes three steps per launch (as one
  *                7x7 kernel, the frame along the boundary step by step; a
  *                run cut into calls of other lengths agrees to rounding, not
- *                bitwise). Pin CS_ALGO_FP64_FMA for IEEE FP64 sums.
+ *                bitwise), on 1D plans 3 to 23. Launches of several steps, 1D,
+ *                odd layouts (odd pitch or first column) and 3D radius 3 round
+ *                so that their error is no larger in the norm than that of FP64
+ *                FMA sweeps on uniform data, and an Inf or NaN reaches only the
+ *                outputs that read it; 2D 7x7 and 3D radius-1 sweeps, and any
+ *                pinned CS_ALGO_FP64_TC, make the tile that holds one NaN.
+ *                Pin CS_ALGO_FP64_FMA for IEEE FP64 sums.
  * CS_PREC_SPLIT: grids stored as FP32 (hi, lo) pairs (8 bytes per point,
  *                about 48 significant bits); no FP64 arithmetic in the sweep.
  *                Dense 7x7 kernels contract exact 9-bit fixed-point slices
@@ -87,7 +95,9 @@ typedef enum cs_semantics { CS_SEM_STEP = 0, CS_SEM_FUSED = 1 } cs_semantics;
  *                faster, 3 to 23 steps per launch, with six digits per
  *                operand: inputs keep 52 bits below their tile's largest
  *                value, results are rounded to pairs once per launch. Relative
- *                error per sweep ~1e-13. Inputs must be finite. Pin
+ *                error per sweep ~1e-13. Inputs must be finite (where launches
+ *                of several steps stand for double-float sweeps, an Inf or NaN
+ *                gives NaN where it is read and nowhere else). Pin
  *                CS_ALGO_SPLIT_FMA for double-float sums. */
 typedef enum cs_precision { CS_PREC_FP64 = 0, CS_PREC_SPLIT = 1 } cs_precision;
 
@@ -131,8 +141,10 @@ typedef enum cs_option {
                                      steps fused per launch by temporal blocking
                                      (0 = tuner picks 1..4, or a tensor-core launch of several
                                      steps, default; 1 = off) */
-    CS_OPT_TILE_ROWS = 6,         /* FP64 FMA 2D kernel: rows per CTA tile, 16 or 32 (0 = tuner,
-                                     default: the first run times both; results do not depend on it) */
+    CS_OPT_TILE_ROWS = 6,         /* FP64 FMA 2D kernel: rows per CTA tile of 64 columns, 16 or 32
+                                     (0 = tuner, default: the first run times both and, up to 2^20
+                                     points, tiles of 16 rows and 8 columns; results do not depend
+                                     on it) */
     CS_OPT_WAIT_LIMIT_US = 4,     /* bound of each device-side wait of the tcgen05 kernels, in
                                      microseconds (default 2,000,000; 1 .. 60,000,000) */
     CS_OPT_WAIT_TEST_SKIP_LOADS = 5 /* test hook (0/1): the tcgen05 kernels issue no TMA loads,
@@ -226,7 +238,8 @@ CS_API cs_status cs_split_to_fp64(const cs_plan *plan, const void *src, double *
  * re-anchor sweep is involved, the copies of 2D and 3D grids overlap the
  * sweeps: the grid moves in bands, the sweeps of a band run as soon as it is
  * there, and rows return after their last sweep (results bitwise those of
- * whole-grid sweeps). The two device grids are allocated by the plan's first call and kept for its later calls until
+ * whole-grid sweeps of one step per launch, and the same from call to call).
+ * The two device grids are allocated by the plan's first call and kept for its later calls until
  * cs_plan_destroy (a call that finds them in use by another thread allocates
  * and frees its own). Returns CS_ERR_TIMEOUT (result incomplete) if a
  * bounded device-side wait expired during the call. */
